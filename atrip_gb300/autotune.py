@@ -5,7 +5,8 @@ candidate launch parameters of the chosen form on sample windows of the
 tuple list (device time from CUDA events, ``atrip_result.device_ms``) and
 keeps the fastest:
 
-* FP64 form: the register tile (32 or 64 rows of (p,q) pairs per CTA pass),
+* FP64 form: the engine's own choice (the tensor-core kernel for all but tiny
+  systems) against the kernel of FP64 instructions with the register tile (32 or 64 rows of (p,q) pairs per CTA pass),
   the kernel's register budget (compiler's choice, or capped at 128 for two
   resident CTAs per SM) and the tuples a CTA claims per queue access;
 * split forms: the slice format first -- the cheapest of 2 FP16 slices
@@ -138,13 +139,14 @@ def _time(ctx, wins, form, slices, tuning, reps=3):
 def tune_fp64(ctx: capi.Context, flops: float = 2e12, m: int = 8) -> dict:
     n = capi.n_tuples(ctx.Nv)
     wins = windows(n, m, window_size(ctx.No, ctx.Nv, m, flops))
-    cands = [{"fp64_tile_rows": 64, "fp64_min_blocks": 0},
+    cands = [{},  # the engine's choice: the tensor-core kernel where it applies
+             {"fp64_tile_rows": 64, "fp64_min_blocks": 0},
              {"fp64_tile_rows": 64, "fp64_min_blocks": 2},
              {"fp64_tile_rows": 32, "fp64_min_blocks": 0}]
     run_windows(ctx, wins[:1], "fp64")  # warm-up
     timed = [(_time(ctx, wins, "fp64", 0, c), c) for c in cands]
     best_ms, best = min(timed, key=lambda x: x[0])
-    for claim in (2, 4):
+    for claim in (2, 4) if best else ():
         c = dict(best, tuples_per_claim=claim)
         t = _time(ctx, wins, "fp64", 0, c)
         if t < 0.98 * best_ms:

@@ -132,6 +132,18 @@ double **direct_slot(atrip_gpu_context *c, int t) {
   }
 }
 
+// Tensors the digit slices are cut from.
+bool contraction_operand(int t) {
+  return t == ATRIP_TABIJ || t == ATRIP_VIJKA || t == ATRIP_VABCI || t == ATRIP_JIJKA ||
+         t == ATRIP_JABCI;
+}
+
+// The FP64 slices are a copy the engine can do without: give them back.
+void free_tc(atrip_gpu_context *c) {
+  tc_free(c->tc);
+  tc_buffers_free(c->tcb);
+}
+
 void free_tensor(atrip_gpu_context *c, int t) {
   if (double **d = direct_slot(c, t)) {
     cudaFree(*d);
@@ -145,6 +157,7 @@ void free_tensor(atrip_gpu_context *c, int t) {
   }
   c->have[t] = false;
   split_invalidate(c->split);
+  if (contraction_operand(t)) tc_free(c->tc);
 }
 
 // Host uploads above this many elements are staged in chunks (default 2^28
@@ -172,6 +185,7 @@ int upload_impl(atrip_gpu_context *c, int32_t tensor, const double *src, int64_t
   if (!src && n > 0) return fail(ATRIP_ERR_ARGUMENT, "null source pointer");
   ATRIP_CUDA_TRY(cudaSetDevice(c->device));
   if (c->have[tensor]) free_tensor(c, tensor);
+  if (contraction_operand(tensor)) free_tc(c);  // a new operand, and its memory
   const cudaMemcpyKind kind = src_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   const bool cplx = c->field == ATRIP_FIELD_COMPLEX;
   const size_t elem = sizeof(double) * (cplx ? 2 : 1);
@@ -431,8 +445,49 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
     if (rc != ATRIP_OK) return rc;
     order = c->d_order;
   }
+  // the FP64 form runs on the tensor cores unless the system is tiny, its
+  // data or the free memory rule that out, or a launch parameter of the DFMA
+  // kernel is set
+  const bool dfma_tuned = c->tune.fp64_tile_rows != 0 || c->tune.fp64_min_blocks != 0 ||
+                          c->tune.fp64_ctas_per_sm != 0 || c->tune.tuples_per_claim != 0;
+  bool tc = form == ATRIP_FORM_FP64 && n > 0 && !dfma_tuned &&
+            tc_sizes_ok(c->No, c->Nv, c->n_tuples, cplx);
+  double sums[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   ATRIP_CUDA_TRY(cudaEventRecord(c->ev0, st));
-  if (n > 0) {
+  if (tc) {
+    const int rc = tc_prepare(c->tc, c->dt, c->No, c->Nv, use_j, st, &launches, &tc);
+    if (rc != ATRIP_OK) return rc;
+  }
+  if (tc) {
+    const TcSystem ts = {&c->tc, &c->dt, c->No, c->Nv, c->n_triples, c->d_tuples, c->d_triples,
+                         t_begin, t_end, use_j, c->d_e, c->d_ect};
+    int rc = tc_launch_prepare(&ts, 1, opts->ijkabc ? -1.0 : 1.0, c->sm_count, c->tcb);
+    if (rc == ATRIP_ERR_OUT_OF_MEMORY) {  // no room for its W buffers
+      cudaGetLastError();
+      clear_error();
+      free_tc(c);
+      c->tc.tried = true;
+      tc = false;
+    } else if (rc != ATRIP_OK) {
+      return rc;
+    }
+  }
+  if (tc) {
+    int rc = tc_launch_enqueue(c->tcb, order, st, &launches);
+    if (rc != ATRIP_OK) return rc;
+    ATRIP_CUDA_TRY(launch_energy_sum(c->d_e + t_begin, c->d_ect + t_begin, n, c->d_partials,
+                                     c->d_sum, st));
+    launches += 2;
+    ATRIP_CUDA_TRY(cudaEventRecord(c->ev1, st));
+    ATRIP_CUDA_TRY(cudaMemcpyAsync(sums, c->d_sum, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
+    ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+    TcState *state = &c->tc;
+    bool rerun = false;
+    rc = tc_launch_check(c->tcb, &state, &rerun);
+    if (rc != ATRIP_OK) return rc;
+    tc = !rerun;
+  }
+  if (n > 0 && !tc) {
     ATRIP_CUDA_TRY(cudaMemsetAsync(c->d_queue, 0, sizeof(unsigned long long) * 4, st));
     if (form == ATRIP_FORM_FP64) {
       const int rows_tile = c->tune.fp64_tile_rows == 32 ? 32 : 64;
@@ -497,17 +552,27 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
                          c->n_triples, t_begin, t_end, order, opts->ijkabc ? -1.0 : 1.0, use_j,
                          slices,
                          c->d_queue, c->d_e, c->d_ect, st, &launches);
+      if (rc == ATRIP_ERR_OUT_OF_MEMORY && c->tc.impl) {  // the FP64 slices make room
+        cudaGetLastError();
+        clear_error();
+        free_tc(c);
+        rc = split_run(c->split, c->dt, c->No, c->Nv, ctas, c->d_tuples, c->d_triples,
+                       c->n_triples, t_begin, t_end, order, opts->ijkabc ? -1.0 : 1.0, use_j,
+                       slices, c->d_queue, c->d_e, c->d_ect, st, &launches);
+      }
       if (rc != ATRIP_OK) return rc;
     }
     ATRIP_CUDA_TRY(launch_energy_sum(c->d_e + t_begin, c->d_ect + t_begin, n, c->d_partials,
                                      c->d_sum, st));
     launches += 2;
   }
-  ATRIP_CUDA_TRY(cudaEventRecord(c->ev1, st));
-  double sums[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  if (n > 0)
-    ATRIP_CUDA_TRY(cudaMemcpyAsync(sums, c->d_sum, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
-  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+  if (!tc) {
+    ATRIP_CUDA_TRY(cudaEventRecord(c->ev1, st));
+    if (n > 0)
+      ATRIP_CUDA_TRY(
+          cudaMemcpyAsync(sums, c->d_sum, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
+    ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+  }
   ATRIP_CUDA_TRY(cudaGetLastError());
   float ms = 0.f;
   ATRIP_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
@@ -607,6 +672,7 @@ int atrip_gpu_destroy(atrip_gpu_context *c) {
   for (int t = 0; t < ATRIP_N_TENSORS; ++t)
     if (c->have[t]) free_tensor(c, t);
   split_free(c->split);
+  free_tc(c);
   cudaFree(c->d_tuples);
   cudaFree(c->d_triples);
   cudaFree(c->d_e);

@@ -9,6 +9,7 @@
 
 #include "atrip_gb300.h"
 #include "engine.cuh"
+#include "fp64_tc.cuh"
 #include "split.cuh"
 
 struct atrip_gpu_context {
@@ -30,6 +31,8 @@ struct atrip_gpu_context {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   atrip_gb300::SplitState split;
+  atrip_gb300::TcState tc;  // FP64 form on the tensor cores
+  atrip_gb300::TcBuffers tcb;
   atrip_tuning tune = {};
   // processing order of the last range (tuple_block > 1), see build_order
   std::vector<uint32_t> h_tuples;  // packed list, host copy

@@ -1,0 +1,1272 @@
+// FP64 form of the triples kernel on the tensor cores.
+//
+// FP64 arithmetic on this part runs at ~1.25 TFLOP/s whichever instruction
+// does it, BF16 MMAs at ~1900.  So the contractions are done as the Ozaki
+// scheme does them (Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59,
+// 2012): an FP64 operand is cut into integer digit slices, the slices are
+// multiplied exactly by the matrix units, and the products are added up in
+// wide integers and FP64.  With e the exponent above the tensor's largest
+// element,
+//     x = 2^(e-7) sum_{s<8} q_s 2^(-8s),   q_s integer, |q_s| <= 128,
+// holds x to 2^(e-64).  Every q_s is exact in BF16, q q' is below 2^14, and
+// a sum of products is exact in the FP32 accumulator while it stays below
+// 2^24.  Products are grouped by level L = s + s'; levels 0..7 are kept (36
+// of the 64 slice products).  What is dropped lies 2^-58 below a typical
+// element of W, where the DFMA kernel's own rounding is at 2^-51.
+//
+// When that holds is examined, not assumed (tc_prepare and the kernel's
+// overflow flag): operands must be finite; the largest element of every
+// slab a tuple reads must lie within 2^kRangeBits of its tensor's largest
+// (product of both operands' ratios); the partial sums of levels 0..2 are
+// bounded below 2^24 by the rows' digit norms (Cauchy-Schwarz); sums of the
+// higher levels, random in sign for any data whose low-order bits are not
+// correlated, are checked to end below 2^22, a quarter of the exact range.
+// Whatever fails this is run by the DFMA kernel instead.
+//
+// Contraction structure: the six fused particle+hole terms of
+// src/atrip/Equations.cxx:455-728 pair up by their column index into three
+// K-concatenated GEMMs (the partner's rows read from a transposed copy)
+//   G0  rows (i,j), column k:  T_a V_bc - Vh_b T_ac + T_b V_ac - Vh_a T_bc
+//   G1  rows (i,k), column j:  T_a V_cb - Vh_c T_ab + T_c V_ab - Vh_a T_bc
+//   G2  rows (j,k), column i:  T_b V_ca - Vh_c T_ab + T_c V_ba - Vh_b T_ac
+// An item is 128 rows of one group.  A operand: one slice of those rows per
+// ring slot; B operand: the 8 slices of the columns stacked in shared memory
+// (slice s at rows s P, P = columns rounded up to 8), loaded once per K
+// chunk.  Slice sa of A times slices 0..7-sa of B is one MMA (two above
+// N = 256) whose result columns are the level accumulators sa..7, which lie
+// side by side in TMEM: no product is padded but for P.
+//
+// Kernel roles (512 threads, one persistent CTA per SM):
+//   warp 0            TMA producer, owner of the tuple queue
+//   warp 1            TMEM owner and single-thread tcgen05.mma issuer
+//   warps 4..7        epilogue: level accumulators to exact integers, stored
+//                     as the group's W cells
+//   warps 2, 3, 8..15 energy: W in FP64, Zijk, get_energy_{distinct,same}
+//                     (src/atrip/Equations.cxx:101-238), one tuple behind
+//
+// What bounds it: shared memory.  An MMA of N columns reads 4 KB of A and
+// 32 N bytes of B at ~118 B per cycle, so the narrow ones (the last slices,
+// few columns) cost 35 + 0.27 N cycles instead of N / 2, and the TMA's writes
+// of the next tiles take their part of the same bandwidth.  Whole runs
+// measured against the DFMA kernel: No=24/Nv=240, 8000 tuples, 316 -> 15.3 ms
+// (1.11 -> 23 TFLOP/s FP64-equivalent); No=37/Nv=151 with (cT), 900 tuples,
+// 229.6 -> 12.0 ms; No=8/Nv=40, the whole list, 6.2 -> 2.2 ms.  Error of the
+// tuple energies against quad precision, 2-norm: 1.0e-16 and 2.2e-16 for
+// (cT), DFMA kernel 1.0e-16 and 4.5e-16 (No = 8..33).
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cudaTypedefs.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <string>
+
+#include "engine.cuh"
+#include "fp64_tc.cuh"
+#include "sm100.cuh"
+
+namespace atrip_gb300 {
+namespace {
+
+using namespace sm100;
+
+constexpr int kThreads = 512;
+constexpr int kS = 8;                       // digit slices and levels
+constexpr int kKChunk = 64;                 // BF16 elements per 128-byte row
+constexpr int kATile = 128 * 128;           // one slice of 128 rows
+constexpr int kMaxSlots = 12;               // A ring
+constexpr int kBSlots = 2;
+constexpr int kTupleSlots = 4;
+constexpr int kEnergyWarps = 10;
+constexpr int kEnergyThreads = kEnergyWarps * 32;
+constexpr int kSmemLimit = 232448;
+constexpr int kTailBytes = 512 + 3 * 64 * 8 + 16 * 8;
+constexpr double kRangeBits = 8.0;
+
+enum : int { kErrFull = 1, kErrEmpty = 2, kErrAccFull = 3, kErrAccEmpty = 4 };
+
+struct TcMaps {
+  CUtensorMap TaN, TaT, VhN, VhT, Vp, TpN, TpT, JhN, JhT, Jp;
+};
+
+struct TcDesc {
+  TcMaps maps;
+  const double *epsi, *epsa, *tai, *Vhh;
+  const uint32_t *tuples, *triples;
+  double *e, *ect;
+  double unit, unit_j;  // weight of a W cell's high part
+  double tai_sign;
+  int64_t t_begin;
+  int No, Nv, P, rows, n_triples, use_j;
+};
+
+struct TcArgs {
+  const TcDesc *sys;
+  const int64_t *prefix;
+  int nsys;
+  int64_t total;
+  const uint32_t *order;  // processing order of a single system's range
+  unsigned long long *queue;
+  int *flags;
+  longlong2 *planes;  // [CTA][parity][pass][group][cell]
+  double *wd;         // [CTA][pass][cell]
+  int lay_cells, lay_pass, nslots, bslot;
+};
+
+__device__ __forceinline__ void bar_sync(int id, int n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+__device__ __forceinline__ bool bar_and(int id, int n, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)v), "r"(id), "r"(n)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void tensormap_acquire(const void *map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(
+                   reinterpret_cast<uint64_t>(map))
+               : "memory");
+}
+
+// Wait for a phase whatever the status says, with a limit of its own.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
+  for (int it = 0; it < (1 << 20) && !mbar_try_wait(bar, parity); ++it) {
+  }
+}
+
+// |n| < 2^51: 1.5 2^52 + n holds n in its low mantissa bits.
+__device__ __forceinline__ double i64_to_f64(long long n) {
+  return __longlong_as_double(0x4338000000000000ll + n) - 6755399441055744.0;
+}
+
+// Operand sources of group g, part pt (0 natural particle, 1 natural hole,
+// 2 transposed particle, 3 transposed hole) of tuple (a,b,c).
+struct TcPart {
+  const CUtensorMap *amap, *bmap;
+  int ax, bz, by;
+  bool particle;
+};
+__device__ __forceinline__ TcPart part_of(const TcMaps &m, int g, int pt, int a, int b, int c,
+                                          int pass) {
+  int x, w, y, z, u, v, flip;
+  const bool tr = pt >= 2;
+  if (g == 0) {
+    if (!tr) { x = a; w = b; y = b; z = c; u = a; v = c; flip = 0; }
+    else     { x = b; w = a; y = a; z = c; u = b; v = c; flip = 0; }
+  } else if (g == 1) {
+    if (!tr) { x = a; w = c; y = c; z = b; u = a; v = b; flip = 0; }
+    else     { x = c; w = a; y = a; z = b; u = b; v = c; flip = 1; }
+  } else {
+    if (!tr) { x = b; w = c; y = c; z = a; u = a; v = b; flip = 1; }
+    else     { x = c; w = b; y = b; z = a; u = a; v = c; flip = 1; }
+  }
+  TcPart p;
+  p.particle = (pt & 1) == 0;
+  if (p.particle) {
+    p.amap = tr ? &m.TaT : &m.TaN;
+    p.ax = x;
+    p.bmap = pass ? &m.Jp : &m.Vp;
+    p.bz = z;
+    p.by = y;
+  } else {
+    p.amap = pass ? (tr ? &m.JhT : &m.JhN) : (tr ? &m.VhT : &m.VhN);
+    p.ax = w;
+    p.bmap = flip ? &m.TpT : &m.TpN;
+    p.bz = v;
+    p.by = u;
+  }
+  return p;
+}
+
+struct TcSlot {
+  int64_t t;  // list position, -1 = no more work
+  int a, b, c, s;
+};
+
+struct TcSinglesCtx {
+  const double *Vbc, *Vac, *Vab;
+  const double *ta, *tb, *tc;
+};
+
+__device__ __forceinline__ double zval(const double *W, const TcSinglesCtx &s, int No, int i, int j,
+                                       int k) {
+  double z = W[i + No * j + No * No * k];
+  z += s.ta[i] * s.Vbc[j + k * No];
+  z += s.tb[j] * s.Vac[i + k * No];
+  z += s.tc[k] * s.Vab[i + j * No];
+  return z;
+}
+
+// This thread's part of a tuple's energy, T from Tb and Z from Wz + singles:
+// the expressions of the DFMA kernel's energy loop, with its division.
+__device__ __forceinline__ double energy_partial(const TcDesc &d, const double *Tb,
+                                                 const double *Wz, const TcSinglesCtx &s,
+                                                 bool distinct, double epsabc, int er) {
+  const int No = d.No;
+  double sum = 0.0;
+  for (int n = er; n < d.n_triples; n += kEnergyThreads) {
+    const uint32_t pk = d.triples[n];
+    const int i = pk & 0xff, j = (pk >> 8) & 0xff, k = (pk >> 16) & 0xff;
+    const double fac = (j == k ? 0.5 : 1.0) * (i == j ? 0.5 : 1.0);
+    const double denominator = epsabc - ((d.epsi[i] + d.epsi[j]) + d.epsi[k]);
+    double value;
+    if (distinct) {
+      const double U = zval(Wz, s, No, i, j, k), V = zval(Wz, s, No, i, k, j),
+                   W = zval(Wz, s, No, j, i, k), X = zval(Wz, s, No, j, k, i),
+                   Y = zval(Wz, s, No, k, i, j), Z = zval(Wz, s, No, k, j, i);
+      const double A = Tb[i + No * j + No * No * k], B = Tb[i + No * k + No * No * j],
+                   C = Tb[j + No * i + No * No * k], D = Tb[j + No * k + No * No * i],
+                   E = Tb[k + No * i + No * No * j], F = Tb[k + No * j + No * No * i];
+      const double UXY = U + (X + Y), VWZ = V + (W + Z), ADE = A + (D + E), BCF = B + (C + F);
+      const double first = A * U + (B * V + (C * W + (D * X + (E * Y + F * Z))));
+      value = 3.0 * first + ((UXY - 2.0 * VWZ) * ADE + (VWZ - 2.0 * UXY) * BCF);
+    } else {
+      const double U = zval(Wz, s, No, i, j, k), V = zval(Wz, s, No, j, k, i),
+                   W = zval(Wz, s, No, k, i, j);
+      const double A = Tb[i + No * j + No * No * k], B = Tb[j + No * k + No * No * i],
+                   C = Tb[k + No * i + No * No * j];
+      value = 3.0 * ((A * U + B * V) + C * W) - (A + (B + C)) * (U + (V + W));
+    }
+    sum += (2.0 * value / denominator) * fac;
+  }
+  return sum;
+}
+
+__global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcArgs g) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *smem = reinterpret_cast<unsigned char *>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char *ring = smem;
+  unsigned char *bring = ring + g.nslots * kATile;
+  unsigned char *tail = bring + kBSlots * g.bslot;
+  uint64_t *afull = reinterpret_cast<uint64_t *>(tail);
+  uint64_t *aempty = afull + kMaxSlots;
+  uint64_t *bfull = aempty + kMaxSlots;
+  uint64_t *bempty = bfull + kBSlots;
+  uint64_t *accf = bempty + kBSlots;
+  uint64_t *acce = accf + 2;
+  uint64_t *tfull = acce + 2;
+  uint64_t *tempty = tfull + kTupleSlots;
+  uint64_t *wfull = tempty + kTupleSlots;
+  uint64_t *wfree = wfull + 2;
+  uint64_t *drain = wfree + 2;
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(drain + 1);
+  TcSlot *tslot = reinterpret_cast<TcSlot *>(tail + 384);
+  double *ta = reinterpret_cast<double *>(tail + 512);
+  double *tb = ta + 64, *tc = tb + 64, *red = tc + 64;
+  static_assert((2 * kMaxSlots + 2 * kBSlots + 4 + 2 * kTupleSlots + 5) * 8 + 8 <= 384, "tail");
+  static_assert(kTupleSlots * sizeof(TcSlot) <= 128, "tuple slots");
+
+  int *status = g.flags;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < g.nslots; ++s) {
+      mbar_init(&afull[s], 1);
+      mbar_init(&aempty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&bfull[b], 1);
+      mbar_init(&bempty[b], 1);
+      mbar_init(&accf[b], 1);
+      mbar_init(&acce[b], 128);
+      mbar_init(&wfull[b], 1);
+      mbar_init(&wfree[b], 1);
+    }
+    for (int s = 0; s < kTupleSlots; ++s) {
+      mbar_init(&tfull[s], 1);
+      mbar_init(&tempty[s], 3);
+    }
+    mbar_init(drain, 1);
+    fence_mbar_init();
+  }
+  // rows that no load writes (past a system's box, past the last stack row)
+  // feed accumulator rows and columns nobody reads: any finite value will do
+  for (int i = threadIdx.x; i < (g.nslots * kATile + kBSlots * g.bslot) / 16; i += kThreads)
+    reinterpret_cast<uint4 *>(ring)[i] = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (warp == 1) {
+    tmem_alloc(tmem_holder, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_holder;
+  const size_t cells = (size_t)g.lay_cells;
+  longlong2 *planes = g.planes + (size_t)blockIdx.x * 2 * g.lay_pass * 3 * cells;
+
+  if (warp == 0) {
+    // ------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      int st = 0, bs = 0;
+      uint32_t use = 0, buse = 0;
+      int cur = -1;
+      int64_t cur_lo = 0, cur_hi = 0;
+      bool alive = true;
+      for (uint32_t k = 0;; ++k) {
+        const int ts = k % kTupleSlots;
+        const uint32_t tuse = k / kTupleSlots;
+        if (tuse > 0 && !mbar_wait(&tempty[ts], (tuse - 1) & 1, status, kErrEmpty)) alive = false;
+        const int64_t q = alive ? (int64_t)atomicAdd(g.queue, 1ull) : g.total;
+        const bool stop = !alive || q >= g.total || *reinterpret_cast<volatile int *>(status) != 0;
+        TcSlot s;
+        s.a = s.b = s.c = s.s = 0;
+        s.t = -1;
+        if (!stop) {
+          if (q >= cur_hi) {  // queue positions only grow: walk on to the tuple's system
+            int lo = cur < 0 ? 0 : cur;
+            while (lo + 1 < g.nsys && g.prefix[lo + 1] <= q) ++lo;
+            cur = lo;
+            cur_lo = g.prefix[lo];
+            cur_hi = g.prefix[lo + 1];
+            const CUtensorMap *m = &g.sys[lo].maps.TaN;
+            const int nm = g.sys[lo].use_j ? 10 : 7;
+            for (int i = 0; i < nm; ++i) tensormap_acquire(m + i);
+          }
+          const TcDesc &d = g.sys[cur];
+          s.s = cur;
+          s.t = d.t_begin + (g.order ? (int64_t)g.order[q] : q - cur_lo);
+          const uint32_t pk = d.tuples[s.t];
+          s.a = pk & 0x3ff;
+          s.b = (pk >> 10) & 0x3ff;
+          s.c = (pk >> 20) & 0x3ff;
+        }
+        tslot[ts] = s;
+        mbar_arrive(&tfull[ts]);
+        if (stop) break;
+        const TcDesc &d = g.sys[cur];
+        const int No2 = d.No * d.No, rows = d.rows, ntiles = (No2 + rows - 1) / rows;
+        const int kp = d.Nv, kh = d.No, npass = d.use_j ? 2 : 1;
+        const uint32_t a_bytes = rows * 128, b_bytes = kS * d.P * 128;
+        for (int gi = 0; gi < 3 * npass && alive; ++gi)
+          for (int mt = 0; mt < ntiles && alive; ++mt)
+            for (int pt = 0; pt < 4 && alive; ++pt) {
+              const TcPart p = part_of(d.maps, gi % 3, pt, s.a, s.b, s.c, gi / 3);
+              const int nch = ((p.particle ? kp : kh) + kKChunk - 1) / kKChunk;
+              for (int ch = 0; ch < nch && alive; ++ch) {
+                if (buse > 0 && !mbar_wait(&bempty[bs], (buse - 1) & 1, status, kErrEmpty)) {
+                  alive = false;
+                  break;
+                }
+                mbar_arrive_expect_tx(&bfull[bs], b_bytes);
+                tma_load_5d(bring + bs * g.bslot, p.bmap, &bfull[bs], ch * kKChunk, 0, p.bz, p.by,
+                            0);
+                if (++bs == kBSlots) {
+                  bs = 0;
+                  ++buse;
+                }
+                for (int sa = 0; sa < kS; ++sa) {
+                  if (use > 0 && !mbar_wait(&aempty[st], (use - 1) & 1, status, kErrEmpty)) {
+                    alive = false;
+                    break;
+                  }
+                  mbar_arrive_expect_tx(&afull[st], a_bytes);
+                  tma_load_4d(ring + st * kATile, p.amap, &afull[st], ch * kKChunk, mt * rows,
+                              p.ax, sa);
+                  if (++st == g.nslots) {
+                    st = 0;
+                    ++use;
+                  }
+                }
+              }
+            }
+      }
+      if (!alive) {  // wait for the copies still in flight
+        for (int i = 0; i < g.nslots; ++i) {
+          const uint32_t n = use + (i < st ? 1 : 0);
+          if (n > 0) mbar_drain(&afull[i], (n - 1) & 1);
+        }
+        for (int i = 0; i < kBSlots; ++i) {
+          const uint32_t n = buse + (i < bs ? 1 : 0);
+          if (n > 0) mbar_drain(&bfull[i], (n - 1) & 1);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // -------------------------------------------------------- MMA issuer
+    const bool leader = elect_one();
+    int st = 0, bs = 0;
+    uint32_t ph = 0, bph = 0, item = 0;
+    int prev = -1;
+    bool alive = true;
+    const uint64_t desc0 = sdesc_sw128(0);
+    const uint32_t ring_a = uniform(smem_u32(ring)), ring_b = uniform(smem_u32(bring));
+    const uint32_t tm = uniform(tmem);
+    for (uint32_t k = 0; alive; ++k) {
+      const int ts = k % kTupleSlots;
+      if (!mbar_wait(&tfull[ts], (k / kTupleSlots) & 1, status, kErrFull)) break;
+      const int stop = uniform(tslot[ts].t < 0 ? 1 : 0);
+      const int sys = uniform(tslot[ts].s);
+      __syncwarp();
+      if (leader) mbar_arrive(&tempty[ts]);
+      if (stop) break;
+      const TcDesc &d = g.sys[sys];
+      const bool fresh = sys != prev;  // its accumulators may lie elsewhere
+      prev = sys;
+      const int P = uniform(d.P), kp = uniform(d.Nv), kh = uniform(d.No);
+      const int rows = uniform(d.rows), ntiles = (kh * kh + rows - 1) / rows;
+      const int nitems = 3 * (uniform(d.use_j) ? 2 : 1) * ntiles;
+      const int bufcols = kS * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
+      for (int it = 0; it < nitems && alive; ++it, ++item) {
+        const int buf = nbuf == 2 ? (int)(item & 1) : 0;
+        // buffer `item & 1`'s barrier is used for every item, whichever
+        // columns it holds: use u of it is item 2u + (item & 1)
+        const int bb = item & 1;
+        const uint32_t u = item >> 1;
+        if (u > 0 && !mbar_wait(&acce[bb], (u - 1) & 1, status, kErrAccEmpty)) {
+          alive = false;
+          break;
+        }
+        if ((nbuf == 1 || (it == 0 && fresh)) && item > 0) {
+          // one accumulator, or another layout than the item before had:
+          // that item must be drained too
+          const int pb = (item - 1) & 1;
+          const uint32_t pu = (item - 1) >> 1;
+          if (!mbar_wait(&acce[pb], pu & 1, status, kErrAccEmpty)) {
+            alive = false;
+            break;
+          }
+        }
+        tc_fence_after();
+        const uint32_t dbase = tm + buf * bufcols;
+        uint32_t acc = 0;
+        for (int pt = 0; pt < 4 && alive; ++pt) {
+          const int K = (pt & 1) == 0 ? kp : kh;
+          for (int k0 = 0; k0 < K && alive; k0 += kKChunk) {
+            const int nkk = (min(kKChunk, K - k0) + 15) / 16;
+            if (!mbar_wait(&bfull[bs], bph, status, kErrFull)) {
+              alive = false;
+              break;
+            }
+            const uint64_t bdesc = desc0 + ((ring_b + (uint32_t)(bs * g.bslot)) >> 4);
+            uint32_t dcol = dbase;
+            int n = kS * P;
+#pragma unroll 1
+            for (int sa = 0; sa < kS; ++sa, n -= P, dcol += P) {
+              if (!mbar_wait(&afull[st], ph, status, kErrFull)) {
+                alive = false;
+                break;
+              }
+              tc_fence_after();
+              const uint64_t adesc = desc0 + ((ring_a + (uint32_t)(st * kATile)) >> 4);
+              const int n16 = (n + 15) & ~15;
+              // above N = 256 two MMAs of about half the columns each
+              const int n1 = n16 <= 256 ? n16 : ((n16 >> 1) + 15) & ~15, n2 = n16 - n1;
+              const uint32_t id1 = idesc_bf16_f32(128, 0) | ((uint32_t)(n1 >> 3) << 17);
+              if (leader) {
+#pragma unroll
+                for (int kk = 0; kk < kKChunk / 16; ++kk)
+                  if (kk < nkk)
+                    mma_bf16(dcol, adesc + 2 * kk, bdesc + 2 * kk, id1, kk == 0 ? acc : 1u);
+                if (n2 > 0) {
+                  const uint32_t id2 = idesc_bf16_f32(128, 0) | ((uint32_t)(n2 >> 3) << 17);
+                  const uint64_t bdesc2 = bdesc + (uint32_t)(n1 * 8);
+#pragma unroll
+                  for (int kk = 0; kk < kKChunk / 16; ++kk)
+                    if (kk < nkk)
+                      mma_bf16(dcol + n1, adesc + 2 * kk, bdesc2 + 2 * kk, id2,
+                               kk == 0 ? acc : 1u);
+                }
+                mma_commit(&aempty[st]);
+              }
+              __syncwarp();
+              acc = 1;
+              if (++st == g.nslots) {
+                st = 0;
+                ph ^= 1u;
+              }
+            }
+            if (leader) mma_commit(&bempty[bs]);
+            __syncwarp();
+            if (++bs == kBSlots) {
+              bs = 0;
+              bph ^= 1u;
+            }
+          }
+        }
+        if (leader && alive) mma_commit(&accf[bb]);
+        __syncwarp();
+      }
+    }
+    // no MMA outlives this role (after a failed wait some may be in flight)
+    if (leader) {
+      mma_commit(drain);
+      mbar_drain(drain, 0);
+    }
+    __syncwarp();
+  } else if (warp >= 4 && warp < 8) {
+    // ------------------------------------------------ epilogue (4 warps)
+    const int quarter = warp - 4;
+    const int l = quarter * 32 + lane;
+    uint32_t item = 0;
+    bool alive = true;
+    for (uint32_t k = 0; alive; ++k) {
+      const int ts = k % kTupleSlots;
+      bool ok = mbar_wait(&tfull[ts], (k / kTupleSlots) & 1, status, kErrFull);
+      const int64_t t = tslot[ts].t;
+      const int sys = tslot[ts].s;
+      const TcDesc &d = g.sys[sys];
+      uint32_t over = 0;
+      ok = bar_and(1, 128, ok);
+      if (threadIdx.x == 128) mbar_arrive(&tempty[ts]);
+      if (!ok || t < 0) break;
+      const int No = d.No, No2 = No * No, P = d.P, rows = d.rows;
+      const int ntiles = (No2 + rows - 1) / rows, npass = d.use_j ? 2 : 1;
+      const int bufcols = kS * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
+      const int wb = k & 1;
+      const uint32_t wuse = k >> 1;
+      ok = wuse == 0 || mbar_wait(&wfree[wb], (wuse - 1) & 1, status, kErrEmpty);
+      for (int it = 0; it < 3 * npass * ntiles; ++it, ++item) {
+        const int gi = it / ntiles, mt = it - gi * ntiles, grp = gi % 3, pass = gi / 3;
+        longlong2 *plane = planes + (size_t)((wb * g.lay_pass + pass) * 3 + grp) * cells;
+        const int bb = item & 1, buf = nbuf == 2 ? bb : 0;
+        bool okw = ok && alive && mbar_wait(&accf[bb], (item >> 1) & 1, status, kErrAccFull);
+        okw = bar_and(1, 128, okw);
+        if (!okw) {
+          alive = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + buf * bufcols;
+        const int m = mt * rows + l;
+        const bool valid = l < rows && m < No2;
+        for (int c0 = 0; c0 < No; c0 += 8) {
+          float v[kS][8];
+          __syncwarp();
+#pragma unroll
+          for (int L = 0; L < kS; ++L) tmem_ld8(tbase + L * P + c0, v[L]);
+          tmem_wait_ld();
+          if (c0 + 8 >= No) {  // everything is read: the accumulator is free
+            tc_fence_before();
+            mbar_arrive(&acce[bb]);
+          }
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            const int r = c0 + x;
+            if (r < No && valid) {
+              // |level sum| < 2^22 for L >= 1 (flagged otherwise): adding
+              // 1.5 2^23 leaves the integer in the low mantissa bits
+              constexpr float kMagic = 12582912.f;
+              constexpr uint32_t kBits = 0x4B400000u;
+              long long hi = (long long)__float2int_rn(v[0][x]) << 24, lo = 0;
+#pragma unroll
+              for (int L = 1; L < kS; ++L) {
+                const uint32_t b = __float_as_uint(v[L][x] + kMagic);
+                over |= b ^ 0x4B000000u;  // exponent bits differ outside that range
+                const long long n = (long long)((int)b - (int)kBits);
+                if (L < 4) hi += n << (24 - 8 * L); else lo += n << (56 - 8 * L);
+              }
+              plane[(size_t)r * No2 + m] = make_longlong2(hi, lo);
+            }
+          }
+        }
+      }
+      if (!alive) break;
+      __threadfence_block();
+      bar_sync(1, 128);
+      if (threadIdx.x == 128) mbar_arrive(&wfull[wb]);
+      if (over & 0xFF800000u) atomicOr(&g.flags[1 + sys], 1);
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------ energy (10 warps)
+    const int er = ((warp < 4 ? warp - 2 : warp - 6) << 5) | lane;
+    double *wd = g.wd + (size_t)blockIdx.x * g.lay_pass * cells;
+    for (uint32_t k = 0;; ++k) {
+      const int ts = k % kTupleSlots;
+      bool ok = mbar_wait(&tfull[ts], (k / kTupleSlots) & 1, status, kErrFull);
+      const TcSlot s = tslot[ts];
+      ok = bar_and(2, kEnergyThreads, ok);
+      if (er == 0) mbar_arrive(&tempty[ts]);
+      if (!ok || s.t < 0) break;
+      const TcDesc &d = g.sys[s.s];
+      const int No = d.No, No2 = No * No, No3 = No2 * No;
+      const int64_t Nv = d.Nv;
+      const int a = s.a, b = s.b, c = s.c;
+      // W, Z and the singles in units of a cell's high part (a power of two)
+      const double inv = d.tai_sign / d.unit;
+      if (er < No) {
+        ta[er] = d.tai[a + er * Nv] * inv;
+        tb[er] = d.tai[b + er * Nv] * inv;
+        tc[er] = d.tai[c + er * Nv] * inv;
+      }
+      const int wb = k & 1;
+      ok = mbar_wait(&wfull[wb], (k >> 1) & 1, status, kErrAccFull);
+      const uint32_t magic = 0xffffffffu / (uint32_t)No + 1u;  // idx / No = umulhi, idx < 2^18
+      const int npass = d.use_j ? 2 : 1;
+      for (int pass = 0; pass < npass; ++pass) {
+        const longlong2 *p0 = planes + (size_t)((wb * g.lay_pass + pass) * 3) * cells;
+        const longlong2 *p1 = p0 + cells, *p2 = p1 + cells;
+        double *W = wd + pass * cells;
+        constexpr int kU = 4;
+        for (int i0 = er; i0 < No3; i0 += kU * kEnergyThreads) {
+          longlong2 v[kU][3];
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            const int idx = i0 + u * kEnergyThreads;
+            if (idx < No3) {
+              const int jk = No == 1 ? idx : (int)__umulhi((uint32_t)idx, magic), i = idx - jk * No;
+              const int kx = No == 1 ? jk : (int)__umulhi((uint32_t)jk, magic), j = jk - kx * No;
+              v[u][0] = p0[idx];
+              v[u][1] = p1[j * No2 + i + No * kx];
+              v[u][2] = p2[i * No2 + j + No * kx];
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            const int idx = i0 + u * kEnergyThreads;
+            if (idx < No3) {
+              // both sums are exact; one rounding where they are joined
+              const long long hi = v[u][0].x + v[u][1].x + v[u][2].x;
+              const long long lo = v[u][0].y + v[u][1].y + v[u][2].y;
+              W[idx] = fma(i64_to_f64(lo), 0x1p-32, i64_to_f64(hi));
+            }
+          }
+        }
+      }
+      __threadfence_block();
+      bar_sync(2, kEnergyThreads);
+      if (er == 0) mbar_arrive(&wfree[wb]);
+      int cls = 0;  // src/atrip/Atrip.cxx:640-642
+      if (a == b) cls++;
+      if (b == c) cls--;
+      const double epsabc = d.epsa[a] + d.epsa[b] + d.epsa[c];
+      TcSinglesCtx sc;
+      sc.Vbc = d.Vhh + ((int64_t)b * Nv + c) * No2;
+      sc.Vac = d.Vhh + ((int64_t)a * Nv + c) * No2;
+      sc.Vab = d.Vhh + ((int64_t)a * Nv + b) * No2;
+      sc.ta = ta;
+      sc.tb = tb;
+      sc.tc = tc;
+      double en[2];
+      for (int pass = 0; pass < npass; ++pass) {
+        double sum = ok ? energy_partial(d, wd + pass * cells, wd, sc, cls == 0, epsabc, er) : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) red[er >> 5] = sum;
+        bar_sync(2, kEnergyThreads);
+        double e = 0.0;
+        for (int w = 0; w < kEnergyWarps; ++w) e += red[w];
+        bar_sync(2, kEnergyThreads);  // red, ta.. and wd are reused
+        en[pass] = e * d.unit * (pass ? d.unit_j : d.unit);
+      }
+      if (er == 0) {
+        d.e[s.t] = en[0];
+        d.ect[s.t] = npass == 2 ? en[1] : en[0];
+      }
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem, 512);
+}
+
+// ------------------------------------------------------------------ prep
+
+// stats[0] = max |x| over the tensor, stats[1] = min over its nonzero slabs
+// (n elements each) of the slab's max, as FP64 bit patterns (ordered like
+// the magnitudes; infinities and NaN sort above every finite value).
+__global__ void slab_max_kernel(const double *__restrict__ x, int64_t slabs, int64_t n,
+                                unsigned long long *__restrict__ stats) {
+  __shared__ unsigned long long sh[8];
+  for (int64_t s = blockIdx.x; s < slabs; s += gridDim.x) {
+    const double *p = x + s * n;
+    unsigned long long m = 0;
+    for (int64_t i = threadIdx.x; i < n; i += 256) {
+      const unsigned long long b =
+          (unsigned long long)__double_as_longlong(p[i]) & 0x7fffffffffffffffull;
+      m = b > m ? b : m;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
+      m = v > m ? v : m;
+    }
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) m = sh[w] > m ? sh[w] : m;
+      if (m > *(volatile unsigned long long *)&stats[0]) atomicMax(&stats[0], m);
+      if (m != 0 && m < *(volatile unsigned long long *)&stats[1]) atomicMin(&stats[1], m);
+    }
+    __syncthreads();
+  }
+}
+
+// dst[s][R][k] (pitch Kp) = digit_s(sign src(R, k)), row R = (o n1 + r1) n2
+// + r2.  norms[s], s < 3: the largest row sum of q_s^2.
+struct CutJob {
+  const double *src;
+  __nv_bfloat16 *dst;
+  int64_t nrows, n1, n2, so, s1, s2, sk;
+  int K, Kp, e, neg;
+  unsigned int *norms;
+};
+
+// round(x 2^(63-e)) for |x| <= 127/128 2^e, with integer instructions.
+__device__ __forceinline__ long long fixed63(double x, int e) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int ex = (int)((b >> 52) & 0x7ff);
+  if (ex == 0) return 0;  // zero or subnormal: below 2^(e-64) for any e accepted
+  const long long m = (long long)((b & 0xfffffffffffffull) | 0x10000000000000ull);
+  const int sh = ex - 1075 + 63 - e;  // <= 10
+  long long v;
+  if (sh >= 0) v = m << sh;
+  else if (sh < -54) v = 0;
+  else v = (m + (1ll << (-sh - 1))) >> -sh;
+  return (long long)b < 0 ? -v : v;
+}
+
+__global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
+  const int64_t plane = j.nrows * j.Kp;
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * 8;
+  unsigned int best[3] = {0, 0, 0};
+  for (int64_t R = blockIdx.x * 8 + (threadIdx.x >> 5); R < j.nrows; R += nw) {
+    const int64_t r2 = R % j.n2, t = R / j.n2, r1 = t % j.n1, o = t / j.n1;
+    const double *src = j.src + o * j.so + r1 * j.s1 + r2 * j.s2;
+    __nv_bfloat16 *dst = j.dst + R * j.Kp;
+    unsigned int nrm[3] = {0, 0, 0};
+    for (int k = 2 * lane; k < j.Kp; k += 64) {
+      unsigned long long y[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        long long X = k + h < j.K ? fixed63(src[(k + h) * j.sk], j.e) : 0;
+        if (j.neg) X = -X;
+        // bytes of X plus 128 in each of the seven lower ones: digit + 128
+        y[h] = (unsigned long long)X + 0x0080808080808080ull;
+      }
+#pragma unroll
+      for (int s = 0; s < kS; ++s) {
+        float q[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (s == 0)
+            q[h] = (float)(int)((long long)y[h] >> 56);
+          else
+            q[h] = __uint_as_float(0x4B000000u | (uint32_t)((y[h] >> (56 - 8 * s)) & 0xff)) -
+                   8388736.f;
+          if (s < 3) nrm[s] += (unsigned int)(int)(q[h] * q[h]);
+        }
+        *reinterpret_cast<__nv_bfloat162 *>(dst + s * plane + k) =
+            __floats2bfloat162_rn(q[0], q[1]);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      unsigned int v = nrm[s];
+#pragma unroll
+      for (int o2 = 16; o2 > 0; o2 >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o2);
+      best[s] = v > best[s] ? v : best[s];
+    }
+  }
+  if (lane < 3) {
+    const unsigned int v = lane == 0 ? best[0] : lane == 1 ? best[1] : best[2];
+    if (v > *(volatile unsigned int *)&j.norms[lane]) atomicMax(&j.norms[lane], v);
+  }
+}
+
+// ------------------------------------------------------------------ host
+
+struct TcImpl {
+  int No = 0, Nv = 0, P = 0, rows = 0, Kp = 0, Kh = 0;
+  int eT = 0, eV = 0, eJ = 0;
+  double max_t = 0, min_t = 0;  // T: largest element, smallest nonzero slab maximum
+  double nT[3], nU[3];          // digit norms of the T rows (over E; over L)
+  double unit = 1.0, unit_j = 1.0;
+  char *arena = nullptr, *arena_j = nullptr;
+  TcMaps maps;
+};
+
+PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
+                                         &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+  }();
+  return fn;
+}
+
+// BF16 tensor map of `rank` dimensions, dims[0] = K extent (fastest, pitch
+// elements apart per row), 128-byte swizzle.
+int make_map(CUtensorMap *m, void *base, int rank, const uint64_t *dims, uint64_t pitch,
+             const uint32_t *box) {
+  auto fn = encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled not available from the driver");
+    return ATRIP_ERR_CUDA;
+  }
+  uint64_t strides[4], s = pitch * 2;
+  for (int i = 1; i < rank; ++i) {
+    strides[i - 1] = s;
+    s *= dims[i];
+  }
+  const uint32_t one[5] = {1, 1, 1, 1, 1};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, base, dims, strides, box, one,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed with CUresult " + std::to_string((int)r));
+    return ATRIP_ERR_CUDA;
+  }
+  return ATRIP_OK;
+}
+
+int map_a(CUtensorMap *m, void *base, const TcImpl &p, int K, int pitch) {
+  const uint64_t d[4] = {(uint64_t)K, (uint64_t)p.No * p.No, (uint64_t)p.Nv, kS};
+  const uint32_t box[4] = {kKChunk, (uint32_t)p.rows, 1, 1};
+  return make_map(m, base, 4, d, pitch, box);
+}
+int map_b(CUtensorMap *m, void *base, const TcImpl &p, int K, int pitch) {
+  const uint64_t d[5] = {(uint64_t)K, (uint64_t)p.No, (uint64_t)p.Nv, (uint64_t)p.Nv, kS};
+  const uint32_t box[5] = {kKChunk, (uint32_t)p.P, 1, 1, kS};
+  return make_map(m, base, 5, d, pitch, box);
+}
+
+// Smallest e with x <= 127/128 2^e (the top digit then stays below 128).
+int exponent_of(double x) {
+  int e = std::ilogb(x) + 1;
+  if (x > std::ldexp(127.0 / 128.0, e)) ++e;
+  return e;
+}
+
+double as_double(unsigned long long b) {
+  double d;
+  std::memcpy(&d, &b, sizeof(d));
+  return d;
+}
+
+struct DeviceStats {
+  unsigned long long m[4][2];  // slab statistics of up to four tensor views
+  unsigned int n[8][4];        // digit norms of up to eight cut jobs
+};
+
+cudaError_t slab_max(const double *x, int64_t slabs, int64_t n, unsigned long long *out,
+                     cudaStream_t st) {
+  const int grid = (int)std::min<int64_t>(slabs, 152 * 16);
+  slab_max_kernel<<<grid, 256, 0, st>>>(x, slabs, n, out);
+  return cudaGetLastError();
+}
+
+cudaError_t cut(CutJob j, cudaStream_t st) {
+  const int grid = (int)std::min<int64_t>((j.nrows + 7) / 8, 152 * 8);
+  cut_kernel<<<grid, 256, 0, st>>>(j);
+  return cudaGetLastError();
+}
+
+size_t up(size_t x) { return (x + 1023) / 1024 * 1024; }
+
+// The slices may take at most half of the memory that is free: the rest is
+// the host program's.  false (no error) when they do not fit.
+bool alloc_arena(char **p, size_t bytes) {
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || bytes > fr / 2 ||
+      cudaMalloc(p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    return false;
+  }
+  return true;
+}
+
+bool exponent_ok(int e) { return e >= -200 && e <= 200; }
+
+// Bound of |partial sums| of levels 1 and 2 (level 0 is far smaller a
+// count): twice (natural and transposed part) the Cauchy-Schwarz products.
+bool sums_exact(const double *nT, const double *nV, const double *nH, const double *nU) {
+  for (int L = 0; L < 3; ++L) {
+    double b = 0;
+    for (int s = 0; s <= L; ++s)
+      b += 2.0 * (std::sqrt(nT[s] * nV[L - s]) + std::sqrt(nH[s] * nU[L - s]));
+    if (!(b < 16777216.0)) return false;
+  }
+  return true;
+}
+
+void set_norms(double *out, const unsigned int *x) {
+  for (int s = 0; s < 3; ++s) out[s] = (double)x[s];
+}
+void max_norms(double *out, const unsigned int *x) {
+  for (int s = 0; s < 3; ++s) out[s] = std::max(out[s], (double)x[s]);
+}
+
+// Cut V_pphp / V_hhhp (or the J pair): slices at hN, hT (rows natural and
+// transposed) and vp, scale 2^e shared by both.
+int cut_pair(const TcImpl &p, const double *vht, const double *vpt, int e, __nv_bfloat16 *hN,
+             __nv_bfloat16 *hT, __nv_bfloat16 *vp, DeviceStats *ds, cudaStream_t st,
+             int64_t *launches) {
+  const int64_t No = p.No, Nv = p.Nv, No2 = No * No;
+  CutJob j;
+  j.e = e;
+  j.neg = 0;
+  j.src = vht; j.dst = hN; j.nrows = Nv * No2; j.n1 = No; j.n2 = No;
+  j.so = No2 * No; j.s1 = No2; j.s2 = No; j.sk = 1; j.K = p.No; j.Kp = p.Kh;
+  j.norms = ds->n[4];
+  ATRIP_CUDA_TRY(cut(j, st));
+  j.dst = hT; j.s1 = No; j.s2 = No2;
+  ATRIP_CUDA_TRY(cut(j, st));
+  j.src = vpt; j.dst = vp; j.nrows = Nv * Nv * No; j.n1 = Nv; j.n2 = No;
+  j.so = Nv * No * Nv; j.s1 = No * Nv; j.s2 = Nv; j.sk = 1; j.K = p.Nv; j.Kp = p.Kp;
+  j.norms = ds->n[5];
+  ATRIP_CUDA_TRY(cut(j, st));
+  *launches += 3;
+  return ATRIP_OK;
+}
+
+void free_impl(TcImpl *p) {
+  if (!p) return;
+  cudaFree(p->arena);
+  cudaFree(p->arena_j);
+  delete p;
+}
+
+struct ScopedDevice {  // device allocation freed on scope exit
+  void *p = nullptr;
+  ~ScopedDevice() { cudaFree(p); }
+};
+
+int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStream_t st,
+                 int64_t *launches) {
+  auto *p = new TcImpl();
+  s.impl = p;
+  p->No = No_;
+  p->Nv = Nv_;
+  p->P = (No_ + 7) / 8 * 8;
+  p->rows = std::min(128, (No_ * No_ + 7) / 8 * 8);
+  p->Kp = (Nv_ + 7) / 8 * 8;
+  p->Kh = (No_ + 7) / 8 * 8;
+  const int64_t No = No_, Nv = Nv_, No2 = No * No;
+  const size_t nTa = up((size_t)2 * kS * Nv * No2 * p->Kp), nVh = up((size_t)2 * kS * Nv * No2 * p->Kh),
+               nVp = up((size_t)2 * kS * Nv * Nv * No * p->Kp),
+               nTp = up((size_t)2 * kS * Nv * Nv * No * p->Kh);
+  if (!alloc_arena(&p->arena, 2 * nTa + 2 * nVh + nVp + 2 * nTp)) return ATRIP_OK;
+  ScopedDevice tmp;
+  ATRIP_CUDA_TRY(cudaMalloc(&tmp.p, sizeof(DeviceStats)));
+  auto *ds = static_cast<DeviceStats *>(tmp.p);
+  DeviceStats h;
+  std::memset(&h, 0, sizeof(h));
+  for (auto &m : h.m) m[1] = ~0ull;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(ds, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+  ATRIP_CUDA_TRY(slab_max(dt.Ta, Nv, No2 * Nv, ds->m[0], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Tp, Nv * Nv, No2, ds->m[1], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Vpt, Nv * Nv, No * Nv, ds->m[2], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Vht, Nv, No2 * No, ds->m[3], st));
+  *launches += 4;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
+  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+  const unsigned long long mT = h.m[0][0], mV = std::max(h.m[2][0], h.m[3][0]);
+  constexpr unsigned long long kInf = 0x7ff0000000000000ull;
+  if (mT == 0 || mV == 0 || mT >= kInf || mV >= kInf) return ATRIP_OK;
+  p->max_t = as_double(mT);
+  p->min_t = as_double(std::min(h.m[0][1], h.m[1][1]));
+  const double max_v = as_double(mV), min_v = as_double(std::min(h.m[2][1], h.m[3][1]));
+  p->eT = exponent_of(p->max_t);
+  p->eV = exponent_of(max_v);
+  if (!exponent_ok(p->eT) || !exponent_ok(p->eV)) return ATRIP_OK;
+  if (std::log2(p->max_t / p->min_t) + std::log2(max_v / min_v) > kRangeBits) return ATRIP_OK;
+  p->unit = std::ldexp(1.0, p->eT + p->eV - 14 - 24);
+
+  char *q = p->arena;
+  auto take = [&](size_t n) {
+    char *r = q;
+    q += n;
+    return reinterpret_cast<__nv_bfloat16 *>(r);
+  };
+  __nv_bfloat16 *TaN = take(nTa), *TaT = take(nTa), *VhN = take(nVh), *VhT = take(nVh),
+                *Vp = take(nVp), *TpN = take(nTp), *TpT = take(nTp);
+  CutJob j;
+  j.e = p->eT;
+  j.neg = 0;
+  // rows (p,q) of T_x over E, p fastest and q fastest
+  j.src = dt.Ta; j.dst = TaN; j.nrows = Nv * No2; j.n1 = No; j.n2 = No;
+  j.so = No2 * Nv; j.s1 = No * Nv; j.s2 = Nv; j.sk = 1; j.K = Nv_; j.Kp = p->Kp;
+  j.norms = ds->n[0];
+  ATRIP_CUDA_TRY(cut(j, st));
+  j.dst = TaT; j.s1 = Nv; j.s2 = No * Nv;
+  ATRIP_CUDA_TRY(cut(j, st));
+  // columns r of -T[u,v,L,r] and -T[u,v,r,L] over L
+  j.neg = 1;
+  j.src = dt.Tp; j.dst = TpN; j.nrows = Nv * Nv * No; j.n1 = Nv; j.n2 = No;
+  j.so = Nv * No2; j.s1 = No2; j.s2 = No; j.sk = 1; j.K = No_; j.Kp = p->Kh;
+  j.norms = ds->n[1];
+  ATRIP_CUDA_TRY(cut(j, st));
+  j.dst = TpT; j.s2 = 1; j.sk = No;
+  j.norms = ds->n[2];
+  ATRIP_CUDA_TRY(cut(j, st));
+  *launches += 4;
+  int rc = cut_pair(*p, dt.Vht, dt.Vpt, p->eV, VhN, VhT, Vp, ds, st, launches);
+  if (rc != ATRIP_OK) return rc;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
+  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+  set_norms(p->nT, h.n[0]);
+  set_norms(p->nU, h.n[1]);
+  max_norms(p->nU, h.n[2]);
+  double nH[3], nV[3];
+  set_norms(nH, h.n[4]);
+  set_norms(nV, h.n[5]);
+  if (!sums_exact(p->nT, nV, nH, p->nU)) return ATRIP_OK;
+
+  if ((rc = map_a(&p->maps.TaN, TaN, *p, Nv_, p->Kp)) || (rc = map_a(&p->maps.TaT, TaT, *p, Nv_, p->Kp)) ||
+      (rc = map_a(&p->maps.VhN, VhN, *p, No_, p->Kh)) || (rc = map_a(&p->maps.VhT, VhT, *p, No_, p->Kh)) ||
+      (rc = map_b(&p->maps.Vp, Vp, *p, Nv_, p->Kp)) || (rc = map_b(&p->maps.TpN, TpN, *p, No_, p->Kh)) ||
+      (rc = map_b(&p->maps.TpT, TpT, *p, No_, p->Kh)))
+    return rc;
+  p->maps.JhN = p->maps.VhN;
+  p->maps.JhT = p->maps.VhT;
+  p->maps.Jp = p->maps.Vp;
+  s.usable = true;
+  return ATRIP_OK;
+}
+
+int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *launches) {
+  auto *p = static_cast<TcImpl *>(s.impl);
+  const int64_t No = p->No, Nv = p->Nv, No2 = No * No;
+  const size_t nVh = up((size_t)2 * kS * Nv * No2 * p->Kh), nVp = up((size_t)2 * kS * Nv * Nv * No * p->Kp);
+  if (!alloc_arena(&p->arena_j, 2 * nVh + nVp)) return ATRIP_OK;
+  ScopedDevice tmp;
+  ATRIP_CUDA_TRY(cudaMalloc(&tmp.p, sizeof(DeviceStats)));
+  auto *ds = static_cast<DeviceStats *>(tmp.p);
+  DeviceStats h;
+  std::memset(&h, 0, sizeof(h));
+  for (auto &m : h.m) m[1] = ~0ull;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(ds, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+  ATRIP_CUDA_TRY(slab_max(dt.Jpt, Nv * Nv, No * Nv, ds->m[2], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Jht, Nv, No2 * No, ds->m[3], st));
+  *launches += 2;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
+  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+  const unsigned long long mV = std::max(h.m[2][0], h.m[3][0]);
+  if (mV == 0 || mV >= 0x7ff0000000000000ull) return ATRIP_OK;
+  const double max_v = as_double(mV), min_v = as_double(std::min(h.m[2][1], h.m[3][1]));
+  p->eJ = exponent_of(max_v);
+  if (!exponent_ok(p->eJ) ||
+      std::log2(p->max_t / p->min_t) + std::log2(max_v / min_v) > kRangeBits)
+    return ATRIP_OK;
+  p->unit_j = std::ldexp(1.0, p->eT + p->eJ - 14 - 24);
+  auto *hN = reinterpret_cast<__nv_bfloat16 *>(p->arena_j);
+  auto *hT = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + nVh);
+  auto *vp = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + 2 * nVh);
+  int rc = cut_pair(*p, dt.Jht, dt.Jpt, p->eJ, hN, hT, vp, ds, st, launches);
+  if (rc != ATRIP_OK) return rc;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
+  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+  double nH[3], nV[3];
+  set_norms(nH, h.n[4]);
+  set_norms(nV, h.n[5]);
+  if (!sums_exact(p->nT, nV, nH, p->nU)) return ATRIP_OK;
+  if ((rc = map_a(&p->maps.JhN, hN, *p, p->No, p->Kh)) || (rc = map_a(&p->maps.JhT, hT, *p, p->No, p->Kh)) ||
+      (rc = map_b(&p->maps.Jp, vp, *p, p->Nv, p->Kp)))
+    return rc;
+  s.usable_j = true;
+  return ATRIP_OK;
+}
+
+// Free what an unusable preparation left behind (the verdict stays).
+void drop_impl(TcState &s) {
+  free_impl(static_cast<TcImpl *>(s.impl));
+  s.impl = nullptr;
+  s.usable = s.usable_j = false;
+}
+
+}  // namespace
+
+void tc_free(TcState &s) {
+  if (s.impl) {
+    drop_impl(s);
+    s.generation++;
+  }
+  s.tried = s.tried_j = s.usable = s.usable_j = false;
+}
+
+// The line: the work of the system's whole list, so that every range of one
+// system takes the same kernel.  Cutting the slices costs ~2 ms in
+// allocations, launches and tensor maps the first time, about what the DFMA
+// kernel needs for 1e9 FLOPs at these sizes (No=4/Nv=12, 4.5e6: 0.1 ms).
+bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx) {
+  return !cplx && No >= 2 && (double)n_tuples * 12.0 * No * No * No * (No + Nv) >= 1e9;
+}
+
+int tc_prepare(TcState &s, const DeviceTensors &dt, int No, int Nv, bool use_j, cudaStream_t st,
+               int64_t *launches, bool *usable) {
+  *usable = false;
+  if (!s.tried) {
+    const int rc = prepare_main(s, dt, No, Nv, st, launches);
+    if (rc != ATRIP_OK || !s.usable) drop_impl(s);
+    s.generation++;
+    if (rc != ATRIP_OK) return rc;
+    s.tried = true;
+  }
+  if (!s.usable) return ATRIP_OK;
+  if (use_j && !s.tried_j) {
+    const int rc = prepare_j(s, dt, st, launches);
+    if (rc != ATRIP_OK || !s.usable_j) {
+      auto *p = static_cast<TcImpl *>(s.impl);
+      cudaFree(p->arena_j);
+      p->arena_j = nullptr;
+    }
+    s.generation++;
+    if (rc != ATRIP_OK) return rc;
+    s.tried_j = true;
+  }
+  *usable = !use_j || s.usable_j;
+  return ATRIP_OK;
+}
+
+void tc_buffers_free(TcBuffers &b) {
+  cudaFreeHost(b.h_desc);
+  cudaFree(b.d_desc);
+  cudaFreeHost(b.h_prefix);
+  cudaFree(b.d_prefix);
+  cudaFree(b.planes);
+  cudaFreeHost(b.h_flags);
+  cudaFree(b.d_flags);
+  cudaFree(b.d_queue);
+  b = TcBuffers();
+}
+
+int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count, TcBuffers &b) {
+  if (b.cap < n) {
+    cudaFreeHost(b.h_desc);
+    cudaFree(b.d_desc);
+    cudaFreeHost(b.h_prefix);
+    cudaFree(b.d_prefix);
+    cudaFreeHost(b.h_flags);
+    cudaFree(b.d_flags);
+    b.h_desc = b.d_desc = nullptr;
+    b.h_prefix = b.d_prefix = nullptr;
+    b.h_flags = b.d_flags = nullptr;
+    b.cap = 0;
+    ATRIP_CUDA_TRY(cudaMallocHost(&b.h_desc, sizeof(TcDesc) * n));
+    ATRIP_CUDA_TRY(cudaMalloc(&b.d_desc, sizeof(TcDesc) * n));
+    ATRIP_CUDA_TRY(cudaMallocHost(&b.h_prefix, sizeof(int64_t) * (n + 1)));
+    ATRIP_CUDA_TRY(cudaMalloc(&b.d_prefix, sizeof(int64_t) * (n + 1)));
+    ATRIP_CUDA_TRY(cudaMallocHost(&b.h_flags, sizeof(int) * (n + 1)));
+    ATRIP_CUDA_TRY(cudaMalloc(&b.d_flags, sizeof(int) * (n + 1)));
+    b.cap = n;
+  }
+  if (!b.d_queue) ATRIP_CUDA_TRY(cudaMalloc(&b.d_queue, sizeof(unsigned long long)));
+  auto *h = static_cast<TcDesc *>(b.h_desc);
+  int P = 0;
+  b.lay_no = 0;
+  b.lay_pass = 1;
+  b.h_prefix[0] = 0;
+  for (int k = 0; k < n; ++k) {
+    const TcSystem &m = sys[k];
+    auto *p = static_cast<TcImpl *>(m.state->impl);
+    if (!p || !m.state->usable || (m.use_j && !m.state->usable_j)) {
+      set_error("tensor-core FP64 form: operands not prepared");
+      return ATRIP_ERR_STATE;
+    }
+    TcDesc d;
+    std::memset(&d, 0, sizeof(d));
+    d.maps = p->maps;
+    d.epsi = m.dt->epsi;
+    d.epsa = m.dt->epsa;
+    d.tai = m.dt->tai;
+    d.Vhh = m.dt->Vhh;
+    d.tuples = m.tuples;
+    d.triples = m.triples;
+    d.e = m.e;
+    d.ect = m.ect;
+    d.unit = p->unit;
+    d.unit_j = p->unit_j;
+    d.tai_sign = tai_sign;
+    d.t_begin = m.t_begin;
+    d.No = m.No;
+    d.Nv = m.Nv;
+    d.P = p->P;
+    d.rows = p->rows;
+    d.n_triples = m.n_triples;
+    d.use_j = m.use_j ? 1 : 0;
+    h[k] = d;
+    P = std::max(P, p->P);
+    b.lay_no = std::max(b.lay_no, m.No);
+    if (m.use_j) b.lay_pass = 2;
+    b.h_prefix[k + 1] = b.h_prefix[k] + std::max<int64_t>(0, m.t_end - m.t_begin);
+  }
+  b.n = n;
+  b.total = b.h_prefix[n];
+  b.grid = (int)std::min<int64_t>(b.total, sm_count);
+  b.lay_cells = b.lay_no * b.lay_no * b.lay_no;
+  // stack of 8 slices of P rows; an MMA's N, a multiple of 16, may read 8 rows more
+  b.bslot = kS * P * 128 + 1024;
+  b.nslots = std::min(kMaxSlots, (kSmemLimit - 1024 - kTailBytes - kBSlots * b.bslot) / kATile);
+  b.smem = 1024 + (size_t)b.nslots * kATile + kBSlots * b.bslot + kTailBytes;
+  const size_t per_cta = ((size_t)2 * 3 * 16 + 8) * b.lay_pass * b.lay_cells;
+  const size_t need = per_cta * std::max(b.grid, 1);
+  if (need > b.planes_bytes) {
+    cudaFree(b.planes);
+    b.planes = nullptr;
+    b.planes_bytes = 0;
+    ATRIP_CUDA_TRY(cudaMalloc(&b.planes, need));
+    b.planes_bytes = need;
+  }
+  return ATRIP_OK;
+}
+
+int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st,
+                      int64_t *launches) {
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(b.d_desc, b.h_desc, sizeof(TcDesc) * b.n, cudaMemcpyHostToDevice,
+                                 st));
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(b.d_prefix, b.h_prefix, sizeof(int64_t) * (b.n + 1),
+                                 cudaMemcpyHostToDevice, st));
+  ATRIP_CUDA_TRY(cudaMemsetAsync(b.d_queue, 0, sizeof(unsigned long long), st));
+  ATRIP_CUDA_TRY(cudaMemsetAsync(b.d_flags, 0, sizeof(int) * (b.n + 1), st));
+  if (b.total == 0) return ATRIP_OK;
+  TcArgs a;
+  a.sys = static_cast<const TcDesc *>(b.d_desc);
+  a.prefix = b.d_prefix;
+  a.nsys = b.n;
+  a.total = b.total;
+  a.order = order;
+  a.queue = b.d_queue;
+  a.flags = b.d_flags;
+  a.planes = static_cast<longlong2 *>(b.planes);
+  a.wd = reinterpret_cast<double *>(static_cast<char *>(b.planes) +
+                                    (size_t)b.grid * 2 * 3 * 16 * b.lay_pass * b.lay_cells);
+  a.lay_cells = b.lay_cells;
+  a.lay_pass = b.lay_pass;
+  a.nslots = b.nslots;
+  a.bslot = b.bslot;
+  ATRIP_CUDA_TRY(cudaFuncSetAttribute(triples_fp64_tc_kernel,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem));
+  triples_fp64_tc_kernel<<<b.grid, kThreads, b.smem, st>>>(a);
+  ATRIP_CUDA_TRY(cudaGetLastError());
+  *launches += 1;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(b.h_flags, b.d_flags, sizeof(int) * (b.n + 1),
+                                 cudaMemcpyDeviceToHost, st));
+  return ATRIP_OK;
+}
+
+int tc_launch_check(const TcBuffers &b, TcState *const *states, bool *rerun) {
+  *rerun = false;
+  if (b.total == 0) return ATRIP_OK;
+  if (b.h_flags[0] != 0) {
+    set_error("tensor-core FP64 kernel: a bounded wait gave up (code " +
+              std::to_string(b.h_flags[0]) + ")");
+    return ATRIP_ERR_TIMEOUT;
+  }
+  for (int k = 0; k < b.n; ++k)
+    if (b.h_flags[1 + k] != 0) {
+      *rerun = true;
+      drop_impl(*states[k]);
+      states[k]->generation++;
+    }
+  return ATRIP_OK;
+}
+
+}  // namespace atrip_gb300

@@ -65,7 +65,10 @@ enum atrip_tensor {
 
 /* Arithmetic form of the contractions. */
 enum atrip_form {
-  ATRIP_FORM_FP64 = 0,       /* FP64 throughout                               */
+  ATRIP_FORM_FP64 = 0,       /* FP64 results: exact digit-slice products on   */
+                             /* the tensor cores where sizes and data allow   */
+                             /* (error no larger than FP64 dot products'),    */
+                             /* else FP64 instructions throughout             */
   ATRIP_FORM_SPLIT_BF16 = 1, /* operands cut into BF16 slices, tensor cores,  */
                              /* FP32 accumulation, FP64 recombination         */
   ATRIP_FORM_AUTO = 2,       /* split-BF16 for real inputs (3 slices unless  */
@@ -153,7 +156,9 @@ int atrip_gpu_release(atrip_gpu_context *ctx, int32_t tensor);
 int atrip_gpu_run(atrip_gpu_context *ctx, const atrip_run_options *opts, atrip_result *out);
 
 /* Launch parameters chosen by the autotuner (atrip_gb300/autotune.py);
- * a zero field keeps the built-in choice.  No counterpart in the reference,
+ * a zero field keeps the built-in choice.  The fp64_* fields and
+ * tuples_per_claim describe the kernel of FP64 instructions: one that is set
+ * selects that kernel for the FP64 form.  No counterpart in the reference,
  * whose only tuning knob for this loop is the tuple distribution.          */
 typedef struct {
   int32_t fp64_ctas_per_sm; /* FP64 form: resident CTAs per SM (0 = occupancy max) */

@@ -1,0 +1,61 @@
+"""FP64 form on the tensor cores (8-bit digit slices, exact sums) against the
+DFMA kernel, which an explicit fp64_tile_rows selects, and the CPU oracle.
+
+Both kernels round W like an FP64 dot product of K = 2 (Nv + No) terms: per
+tuple they agree within K 2^-52 of the largest tuple energy.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from atrip_gb300 import capi, synth
+
+pytestmark = pytest.mark.gpu
+NAMES = ("epsi", "epsa", "Tai", "Tabij", "Vabij", "Vijka", "Vabci")
+DFMA_LAUNCHES = 3  # the kernel and the two stages of the energy sum
+
+
+def _ctx(d, j=False):
+    ctx = capi.Context(d["No"], d["Nv"], 0)
+    for n in NAMES + (("Jijka", "Jabci") if j else ()):
+        ctx.upload(n, d[n])
+    return ctx
+
+
+def _both(ctx, **kw):
+    """(tensor-core result, its energies, DFMA energies) over one range."""
+    r = ctx.run(form="fp64", **kw)
+    t0, n = kw.get("first_iteration", 0), r.tuples_done
+    e, ect = ctx.tuple_energies(t0, n)
+    ctx.set_tuning(fp64_tile_rows=64)
+    rd = ctx.run(form="fp64", **kw)
+    assert rd.kernel_launches == DFMA_LAUNCHES
+    d, dct = ctx.tuple_energies(t0, n)
+    ctx.set_tuning()
+    return r, (e, ect), (d, dct)
+
+
+def _close(x, y, K):
+    assert np.max(np.abs(x - y)) <= K * 2.0 ** -52 * np.max(np.abs(y))
+
+
+# P = No rounded up to 8; N = 8 P of the widest MMA splits above 256; TMEM
+# holds two accumulators up to No = 32; 128-row tiles end in No^2's remainder
+@pytest.mark.parametrize("No,Nv,j", [
+    (4, 80, False), (5, 66, True), (8, 40, True), (9, 47, False), (11, 64, False), (12, 65, True),
+    (16, 33, False), (17, 33, True), (24, 30, False), (25, 21, False), (32, 18, True),
+    (33, 20, False), (40, 24, True), (47, 16, False), (56, 14, False), (64, 12, False)])
+def test_matches_dfma_and_oracle(No, Nv, j):
+    d = synth.make_inputs(No, Nv, 11, with_j=j)
+    n = min(synth.n_tuples(Nv), 700)
+    with _ctx(d, j) as ctx:
+        r, (e, ect), (f, fct) = _both(ctx, max_iterations=n - 1, use_j=j)
+        assert r.kernel_launches > DFMA_LAUNCHES  # the slices were cut
+        again = ctx.run(form="fp64", max_iterations=n - 1, use_j=j)
+        assert again.energy == r.energy and again.kernel_launches == DFMA_LAUNCHES
+        K = 2 * (Nv + No)
+        _close(e, f, K)
+        _close(ect, fct, K)
+        pr = oracle.Problem(d)
+        o = oracle.tuple_energies(pr, 0, 12)[0]
+        assert np.max(np.abs(e[:12] - o)) <= K * 2.0 ** -52 * np.max(np.abs(f))
