@@ -3,8 +3,9 @@
 // FP64: one persistent launch of the batch kernel over the concatenated
 // tuple lists of all systems (a single device work-queue cursor; the table of
 // per-system descriptors is ordered by per-tuple cost, largest first, so the
-// queue drains the expensive tuples before the cheap ones), then one kernel
-// that reduces every system's energies.  Split form: one persistent launch
+// queue drains the expensive tuples before the cheap ones), and one of the
+// tensor-core kernel over the systems that it serves, then one kernel that
+// reduces every system's energies.  Split form: one persistent launch
 // per system (each has its own pre-split operands and tensor maps) and the
 // same reduction.  Either sequence is captured once into a CUDA graph and
 // replayed; the descriptor table is a graph node that copies from pinned host
@@ -52,6 +53,7 @@ struct atrip_gpu_batch {
   int max_per_sm = 1;      // CTAs per SM the workspace is sized for
   SplitMultiBuffers multi;  // split form: every system in one launch
   bool multi_used = false;  // the captured graph holds that one launch
+  TcBuffers tcb;            // FP64 form: the systems on the tensor-core kernel
 };
 
 namespace {
@@ -226,8 +228,51 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
   const double tai_sign = opts->ijkabc ? -1.0 : 1.0;
   std::vector<int64_t> prefix;
   fill_table(b, opts->first_iteration, opts->max_iterations, tai_sign, opts->use_j != 0, prefix);
-  std::copy(prefix.begin(), prefix.end(), b->h_prefix);
   int64_t prep_launches = 0;
+
+  // FP64 form: the systems the tensor-core kernel serves leave the DFMA
+  // kernel's queue (their stretch of prefix is empty), unless a launch
+  // parameter of the DFMA kernel is set
+  std::vector<TcSystem> tc;
+  std::vector<TcState *> tc_states;
+  const bool dfma_tuned = b->tune.fp64_min_blocks != 0 || b->tune.fp64_ctas_per_sm != 0 ||
+                          b->tune.tuples_per_claim != 0;
+  if (form == ATRIP_FORM_FP64 && !dfma_tuned) {
+    for (int k = 0; k < n; ++k) {
+      atrip_gpu_context *c = b->sys[b->order[k]];
+      const TriplesArgs &a = b->h_table[k];
+      bool ok = a.t_end > a.t_begin && c->tune.fp64_tile_rows == 0 &&
+                tc_sizes_ok(c->No, c->Nv, c->n_tuples, false);
+      if (!ok) continue;
+      const int rc = tc_prepare(c->tc, c->dt, c->No, c->Nv, a.use_j != 0, st, &prep_launches, &ok);
+      if (rc != ATRIP_OK) return rc;
+      if (!ok) continue;
+      tc.push_back({&c->tc, &c->dt, c->No, c->Nv, a.n_triples, a.tuples, a.triples, a.t_begin,
+                    a.t_end, a.use_j != 0, a.e, a.ect});
+      tc_states.push_back(&c->tc);
+    }
+    if (!tc.empty()) {
+      const int rc = tc_launch_prepare(tc.data(), (int)tc.size(), tai_sign, b->sm_count, b->tcb);
+      if (rc == ATRIP_ERR_OUT_OF_MEMORY) {  // no room for its W buffers
+        cudaGetLastError();
+        clear_error();
+        tc.clear();
+      } else if (rc != ATRIP_OK) {
+        return rc;
+      }
+      ATRIP_CUDA_TRY(cudaStreamSynchronize(st));  // slices cut on st, replayed on another stream
+    }
+  }
+  size_t next_tc = 0;
+  for (int k = 0; k < n; ++k) {
+    int64_t count = b->h_table[k].t_end - b->h_table[k].t_begin;
+    if (next_tc < tc.size() && tc[next_tc].e == b->h_table[k].e) {
+      ++next_tc;
+      count = 0;
+    }
+    prefix[k + 1] = prefix[k] + count;
+  }
+  std::copy(prefix.begin(), prefix.end(), b->h_prefix);
 
   // What the captured graph depends on besides the table (copied at replay).
   std::vector<uintptr_t> key = {(uintptr_t)form, (uintptr_t)(form == ATRIP_FORM_FP64 ? 0 : slices),
@@ -297,6 +342,14 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
     // the split operands were cut on st; the capture stream must see them
     ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
   }
+  if (!tc.empty()) {
+    const uintptr_t more[] = {(uintptr_t)tc.size(), (uintptr_t)b->tcb.total, (uintptr_t)b->tcb.grid,
+                              (uintptr_t)b->tcb.planes, (uintptr_t)b->tcb.d_desc,
+                              (uintptr_t)b->tcb.smem, (uintptr_t)b->tcb.lay_cells,
+                              (uintptr_t)b->tcb.lay_pass, (uintptr_t)b->tcb.bslot,
+                              (uintptr_t)b->tcb.nslots};
+    key.insert(key.end(), std::begin(more), std::end(more));
+  }
   if (!b->exec || key != b->key) {
     destroy_graph(b);
     BatchArgs ba;
@@ -323,6 +376,10 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
           ATRIP_CUDA_TRY(launch_triples_fp64_batch(ba, b->max_no, b->tune.fp64_min_blocks, grid,
                                                    b->stream));
           launches += 1;
+        }
+        if (!tc.empty()) {
+          const int rc2 = tc_launch_enqueue(b->tcb, nullptr, b->stream, &launches);
+          if (rc2 != ATRIP_OK) return rc2;
         }
       } else if (b->multi_used) {
         ATRIP_CUDA_TRY(cudaMemsetAsync(b->multi.d_status, 0, sizeof(int), b->stream));
@@ -370,6 +427,13 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
   ATRIP_CUDA_TRY(cudaGetLastError());
   float ms = 0.f;
   ATRIP_CUDA_TRY(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
+  if (!tc.empty()) {
+    bool rerun = false;
+    const int rc = tc_launch_check(b->tcb, tc_states.data(), &rerun);
+    if (rc != ATRIP_OK) return rc;
+    // systems whose sums left the exact range are barred now: run again
+    if (rerun) return atrip_gpu_batch_run(b, opts, results);
+  }
   for (int s = 0; s < n; ++s) {
     const int rc = split_status_check(b->h_status[s]);
     if (rc != ATRIP_OK)
@@ -417,6 +481,7 @@ int atrip_gpu_batch_destroy(atrip_gpu_batch *b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   destroy_graph(b);
   split_multi_free(b->multi);
+  tc_buffers_free(b->tcb);
   cudaFreeHost(b->h_table);
   cudaFreeHost(b->h_prefix);
   cudaFreeHost(b->h_sums);
