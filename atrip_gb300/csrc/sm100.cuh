@@ -63,6 +63,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *s
   }
 }
 
+// The same for a whole converged warp: every lane gets the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, int *status,
+                                               int code, long long limit = kWaitCycles) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code, limit));
+}
+
 // True in one lane of a converged warp.  A role that issues tcgen05 or TMA
 // instructions keeps its whole warp in the loop and lets this lane issue:
 // their operands live in uniform registers, and in code that the compiler
@@ -82,20 +89,24 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 
 // ---------------------------------------------------------------------- TMA
-__device__ __forceinline__ void tma_load_5d(void *dst, const void *map, uint64_t *bar, int c0,
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const void *map, uint64_t *bar, int c0,
                                             int c1, int c2, int c3, int c4) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(smem_u32(dst)),
+      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
       "r"(c4)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_4d(void *dst, const void *map, uint64_t *bar, int c0,
+__device__ __forceinline__ void tma_load_5d(void *dst, const void *map, uint64_t *bar, int c0,
+                                            int c1, int c2, int c3, int c4) {
+  tma_load_5d(smem_u32(dst), map, bar, c0, c1, c2, c3, c4);
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void *map, uint64_t *bar, int c0,
                                             int c1, int c2, int c3) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(dst)),
+      " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
