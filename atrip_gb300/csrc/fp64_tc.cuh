@@ -53,7 +53,8 @@ struct TcBuffers {
   unsigned long long *d_queue = nullptr;
   int cap = 0;
   // launch layout of the last tc_launch_prepare
-  int n = 0, lay_no = 0, lay_cells = 0, lay_pass = 1, nslots = 0, bslot = 0, grid = 0;
+  int n = 0, lay_no = 0, lay_cells = 0, lay_pass = 1, nslots = 0, nbslots = 0, aslot = 0,
+      bslot = 0, grid = 0;
   size_t smem = 0;
   int64_t total = 0;
 };

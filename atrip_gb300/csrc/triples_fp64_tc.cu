@@ -75,14 +75,13 @@ using namespace sm100;
 constexpr int kThreads = 512;
 constexpr int kS = 8;                       // digit slices and levels
 constexpr int kKChunk = 64;                 // BF16 elements per 128-byte row
-constexpr int kATile = 128 * 128;           // one slice of 128 rows
-constexpr int kMaxSlots = 12;               // A ring
-constexpr int kBSlots = 2;
+constexpr int kMaxSlots = 10;               // A ring
+constexpr int kMaxBSlots = 8;               // B ring
 constexpr int kTupleSlots = 4;
 constexpr int kEnergyWarps = 10;
 constexpr int kEnergyThreads = kEnergyWarps * 32;
 constexpr int kSmemLimit = 232448;
-constexpr int kTailBytes = 512 + 3 * 64 * 8 + 16 * 8;
+constexpr int kTailBytes = 576 + 3 * 64 * 8 + 16 * 8;
 constexpr double kRangeBits = 8.0;
 
 enum : int { kErrFull = 1, kErrEmpty = 2, kErrAccFull = 3, kErrAccEmpty = 4 };
@@ -99,7 +98,7 @@ struct TcDesc {
   double unit, unit_j;  // weight of a W cell's high part
   double tai_sign;
   int64_t t_begin;
-  int No, Nv, P, rows, n_triples, use_j;
+  int No, Nv, P, rows, spp, n_triples, use_j;
 };
 
 struct TcArgs {
@@ -112,7 +111,7 @@ struct TcArgs {
   int *flags;
   longlong2 *planes;  // [CTA][parity][pass][group][cell]
   double *wd;         // [CTA][pass][cell]
-  int lay_cells, lay_pass, nslots, bslot;
+  int lay_cells, lay_pass, nslots, nbslots, aslot, bslot;
 };
 
 __device__ __forceinline__ void bar_sync(int id, int n) {
@@ -240,18 +239,123 @@ __device__ __forceinline__ double energy_partial(const TcDesc &d, const double *
   return sum;
 }
 
+// The MMA issuer's state, carried from tuple to tuple.
+struct MmaRole {
+  int st, bs;              // A and B ring slots of the next operands
+  uint32_t ph, bph, item;  // their phases; items so far
+  int nslots, nbslots, aslot, bslot;
+  uint32_t ring_a, ring_b, tm;
+  uint64_t *afull, *aempty, *bfull, *bempty, *accf, *acce;
+  bool leader;
+  int kp, kh, rows, spp, nitems;  // the tuple's system
+};
+
+// One slice of A times the slices of B that still give a kept level: result
+// columns sa P .. 8 P - 1, above N = 256 by two MMAs of about half of them.
+// NKK K steps (the run-time nkk of them where NKK is 0).
+template <int P, int SA, int NKK>
+__device__ __forceinline__ void mma_slice(uint32_t d, uint64_t ad, uint64_t bd, int nkk,
+                                          uint32_t acc) {
+  constexpr int n = ((kS - SA) * P + 15) & ~15;
+  constexpr int n1 = n <= 256 ? n : ((n >> 1) + 15) & ~15, n2 = n - n1;
+  constexpr int kMax = NKK ? NKK : kKChunk / 16;
+#pragma unroll
+  for (int kk = 0; kk < kMax; ++kk)
+    if (NKK || kk < nkk)
+      mma_bf16(d + SA * P, ad + 2 * kk, bd + 2 * kk, idesc_bf16_f32(128, n1),
+               kk == 0 && SA == 0 ? acc : 1u);
+  if constexpr (n2 > 0) {
+#pragma unroll
+    for (int kk = 0; kk < kMax; ++kk)
+      if (NKK || kk < nkk)
+        mma_bf16(d + SA * P + n1, ad + 2 * kk, bd + n1 * 8 + 2 * kk, idesc_bf16_f32(128, n2),
+                 kk == 0 && SA == 0 ? acc : 1u);
+  }
+}
+
+// A K chunk: the 8 slices of A from the ring, spp to a slot.
+template <int P, int SA, int NKK>
+__device__ __forceinline__ bool mma_chunk(MmaRole &m, uint32_t d, uint64_t &ad, uint64_t bd,
+                                          int nkk, uint32_t acc, int *status) {
+  if constexpr (SA < kS) {
+    if ((SA & (m.spp - 1)) == 0) {
+      if (!mbar_wait_warp(&m.afull[m.st], m.ph, status, kErrFull)) return false;
+      tc_fence_after();
+      ad = sdesc_sw128(0) + ((m.ring_a + (uint32_t)(m.st * m.aslot)) >> 4);
+    }
+    if (m.leader) mma_slice<P, SA, NKK>(d, ad, bd, nkk, acc);
+    ad += (uint32_t)(m.rows * 8);
+    if ((SA & (m.spp - 1)) == m.spp - 1) {
+      if (m.leader) mma_commit(&m.aempty[m.st]);
+      if (++m.st == m.nslots) {
+        m.st = 0;
+        m.ph ^= 1u;
+      }
+    }
+    __syncwarp();
+    return mma_chunk<P, SA + 1, NKK>(m, d, ad, bd, nkk, acc, status);
+  }
+  return true;
+}
+
+// All items of a tuple.  The column count P is a template parameter so that
+// every MMA's column offset and instruction descriptor are constants: a warp
+// needs ~5 cycles for each instruction between two MMAs of 50 to 130.
+template <int P>
+__device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
+  constexpr int bufcols = kS * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
+  for (int it = 0; it < m.nitems; ++it, ++m.item) {
+    // barrier `item & 1` serves every second item, whichever columns the
+    // item has: its use u is item 2u + (item & 1)
+    const int bb = m.item & 1, buf = nbuf == 2 ? bb : 0;
+    const uint32_t u = m.item >> 1;
+    if (u > 0 && !mbar_wait_warp(&m.acce[bb], (u - 1) & 1, status, kErrAccEmpty)) return false;
+    if ((nbuf == 1 || (it == 0 && fresh)) && m.item > 0) {
+      // one accumulator, or another layout than the item before had: that
+      // item must be drained too
+      const uint32_t p = m.item - 1;
+      if (!mbar_wait_warp(&m.acce[p & 1], (p >> 1) & 1, status, kErrAccEmpty)) return false;
+    }
+    tc_fence_after();
+    const uint32_t d = m.tm + buf * bufcols;
+    uint32_t acc = 0;
+    for (int pt = 0; pt < 4; ++pt) {
+      const int K = (pt & 1) == 0 ? m.kp : m.kh;
+      for (int k0 = 0; k0 < K; k0 += kKChunk) {
+        if (!mbar_wait_warp(&m.bfull[m.bs], m.bph, status, kErrFull)) return false;
+        const uint64_t bd = sdesc_sw128(0) + ((m.ring_b + (uint32_t)(m.bs * m.bslot)) >> 4);
+        uint64_t ad = 0;
+        const int nkk = (min(kKChunk, K - k0) + 15) / 16;
+        const bool ok = nkk == 4 ? mma_chunk<P, 0, 4>(m, d, ad, bd, 4, acc, status)
+                                 : mma_chunk<P, 0, 0>(m, d, ad, bd, nkk, acc, status);
+        if (!ok) return false;
+        acc = 1;
+        if (m.leader) mma_commit(&m.bempty[m.bs]);
+        __syncwarp();
+        if (++m.bs == m.nbslots) {
+          m.bs = 0;
+          m.bph ^= 1u;
+        }
+      }
+    }
+    if (m.leader) mma_commit(&m.accf[bb]);
+    __syncwarp();
+  }
+  return true;
+}
+
 __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcArgs g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char *ring = smem;
-  unsigned char *bring = ring + g.nslots * kATile;
-  unsigned char *tail = bring + kBSlots * g.bslot;
+  unsigned char *bring = ring + g.nslots * g.aslot;
+  unsigned char *tail = bring + g.nbslots * g.bslot;
   uint64_t *afull = reinterpret_cast<uint64_t *>(tail);
   uint64_t *aempty = afull + kMaxSlots;
   uint64_t *bfull = aempty + kMaxSlots;
-  uint64_t *bempty = bfull + kBSlots;
-  uint64_t *accf = bempty + kBSlots;
+  uint64_t *bempty = bfull + kMaxBSlots;
+  uint64_t *accf = bempty + kMaxBSlots;
   uint64_t *acce = accf + 2;
   uint64_t *tfull = acce + 2;
   uint64_t *tempty = tfull + kTupleSlots;
@@ -259,10 +363,10 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
   uint64_t *wfree = wfull + 2;
   uint64_t *drain = wfree + 2;
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(drain + 1);
-  TcSlot *tslot = reinterpret_cast<TcSlot *>(tail + 384);
-  double *ta = reinterpret_cast<double *>(tail + 512);
+  TcSlot *tslot = reinterpret_cast<TcSlot *>(tail + 448);
+  double *ta = reinterpret_cast<double *>(tail + 576);
   double *tb = ta + 64, *tc = tb + 64, *red = tc + 64;
-  static_assert((2 * kMaxSlots + 2 * kBSlots + 4 + 2 * kTupleSlots + 5) * 8 + 8 <= 384, "tail");
+  static_assert((2 * kMaxSlots + 2 * kMaxBSlots + 4 + 2 * kTupleSlots + 5) * 8 + 8 <= 448, "tail");
   static_assert(kTupleSlots * sizeof(TcSlot) <= 128, "tuple slots");
 
   int *status = g.flags;
@@ -272,9 +376,11 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       mbar_init(&afull[s], 1);
       mbar_init(&aempty[s], 1);
     }
+    for (int s = 0; s < g.nbslots; ++s) {
+      mbar_init(&bfull[s], 1);
+      mbar_init(&bempty[s], 1);
+    }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&bfull[b], 1);
-      mbar_init(&bempty[b], 1);
       mbar_init(&accf[b], 1);
       mbar_init(&acce[b], 128);
       mbar_init(&wfull[b], 1);
@@ -289,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
   }
   // rows that no load writes (past a system's box, past the last stack row)
   // feed accumulator rows and columns nobody reads: any finite value will do
-  for (int i = threadIdx.x; i < (g.nslots * kATile + kBSlots * g.bslot) / 16; i += kThreads)
+  for (int i = threadIdx.x; i < (g.nslots * g.aslot + g.nbslots * g.bslot) / 16; i += kThreads)
     reinterpret_cast<uint4 *>(ring)[i] = make_uint4(0, 0, 0, 0);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (warp == 1) {
@@ -305,105 +411,132 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int st = 0, bs = 0;
-      uint32_t use = 0, buse = 0;
-      int cur = -1;
-      int64_t cur_lo = 0, cur_hi = 0;
-      bool alive = true;
-      for (uint32_t k = 0;; ++k) {
-        const int ts = k % kTupleSlots;
-        const uint32_t tuse = k / kTupleSlots;
-        if (tuse > 0 && !mbar_wait(&tempty[ts], (tuse - 1) & 1, status, kErrEmpty)) alive = false;
-        const int64_t q = alive ? (int64_t)atomicAdd(g.queue, 1ull) : g.total;
-        const bool stop = !alive || q >= g.total || *reinterpret_cast<volatile int *>(status) != 0;
-        TcSlot s;
-        s.a = s.b = s.c = s.s = 0;
-        s.t = -1;
-        if (!stop) {
-          if (q >= cur_hi) {  // queue positions only grow: walk on to the tuple's system
-            int lo = cur < 0 ? 0 : cur;
-            while (lo + 1 < g.nsys && g.prefix[lo + 1] <= q) ++lo;
-            cur = lo;
-            cur_lo = g.prefix[lo];
-            cur_hi = g.prefix[lo + 1];
-            const CUtensorMap *m = &g.sys[lo].maps.TaN;
-            const int nm = g.sys[lo].use_j ? 10 : 7;
-            for (int i = 0; i < nm; ++i) tensormap_acquire(m + i);
-          }
-          const TcDesc &d = g.sys[cur];
-          s.s = cur;
-          s.t = d.t_begin + (g.order ? (int64_t)g.order[q] : q - cur_lo);
-          const uint32_t pk = d.tuples[s.t];
-          s.a = pk & 0x3ff;
-          s.b = (pk >> 10) & 0x3ff;
-          s.c = (pk >> 20) & 0x3ff;
+    const bool leader = elect_one();
+    int st = 0, bs = 0;
+    uint32_t use = 0, buse = 0;
+    int cur = -1;
+    int64_t cur_lo = 0, cur_hi = 0;
+    bool alive = true;
+    const uint32_t ring_a = uniform(smem_u32(ring)), ring_b = uniform(smem_u32(bring));
+    for (uint32_t k = 0;; ++k) {
+      const int ts = k % kTupleSlots;
+      const uint32_t tuse = k / kTupleSlots;
+      if (tuse > 0 && !mbar_wait_warp(&tempty[ts], (tuse - 1) & 1, status, kErrEmpty))
+        alive = false;
+      int64_t q = g.total;
+      if (alive && leader && *reinterpret_cast<volatile int *>(status) == 0)
+        q = (int64_t)atomicAdd(g.queue, 1ull);
+      q = __shfl_sync(0xffffffffu, q, __ffs(__ballot_sync(0xffffffffu, leader)) - 1);
+      const bool stop = q >= g.total;
+      TcSlot s;
+      s.a = s.b = s.c = s.s = 0;
+      s.t = -1;
+      if (!stop) {
+        if (q >= cur_hi) {  // queue positions only grow: walk on to the tuple's system
+          int lo = cur < 0 ? 0 : cur;
+          while (lo + 1 < g.nsys && g.prefix[lo + 1] <= q) ++lo;
+          cur = uniform(lo);
+          cur_lo = g.prefix[cur];
+          cur_hi = g.prefix[cur + 1];
+          const CUtensorMap *m = &g.sys[cur].maps.TaN;
+          const int nm = g.sys[cur].use_j ? 10 : 7;
+          for (int i = 0; i < nm; ++i) tensormap_acquire(m + i);
         }
+        const TcDesc &d = g.sys[cur];
+        s.s = cur;
+        s.t = d.t_begin + (g.order ? (int64_t)g.order[q] : q - cur_lo);
+        const int pk = uniform((int)d.tuples[s.t]);
+        s.a = pk & 0x3ff;
+        s.b = (pk >> 10) & 0x3ff;
+        s.c = (pk >> 20) & 0x3ff;
+      }
+      if (leader) {
         tslot[ts] = s;
         mbar_arrive(&tfull[ts]);
-        if (stop) break;
-        const TcDesc &d = g.sys[cur];
-        const int No2 = d.No * d.No, rows = d.rows, ntiles = (No2 + rows - 1) / rows;
-        const int kp = d.Nv, kh = d.No, npass = d.use_j ? 2 : 1;
-        const uint32_t a_bytes = rows * 128, b_bytes = kS * d.P * 128;
-        for (int gi = 0; gi < 3 * npass && alive; ++gi)
-          for (int mt = 0; mt < ntiles && alive; ++mt)
-            for (int pt = 0; pt < 4 && alive; ++pt) {
-              const TcPart p = part_of(d.maps, gi % 3, pt, s.a, s.b, s.c, gi / 3);
-              const int nch = ((p.particle ? kp : kh) + kKChunk - 1) / kKChunk;
-              for (int ch = 0; ch < nch && alive; ++ch) {
-                if (buse > 0 && !mbar_wait(&bempty[bs], (buse - 1) & 1, status, kErrEmpty)) {
+      }
+      __syncwarp();
+      if (stop) break;
+      const TcDesc &d = g.sys[cur];
+      const int kp = uniform(d.Nv), kh = uniform(d.No), rows = uniform(d.rows);
+      const int ntiles = (kh * kh + rows - 1) / rows, npass = uniform(d.use_j) ? 2 : 1;
+      const int spp = uniform(d.spp);
+      const uint32_t a_bytes = spp * rows * 128, b_bytes = kS * uniform(d.P) * 128;
+      for (int gi = 0; gi < 3 * npass && alive; ++gi)
+        for (int mt = 0; mt < ntiles && alive; ++mt)
+          for (int pt = 0; pt < 4 && alive; ++pt) {
+            const TcPart p = part_of(d.maps, gi % 3, pt, s.a, s.b, s.c, gi / 3);
+            const int K = p.particle ? kp : kh;
+            for (int k0 = 0; k0 < K && alive; k0 += kKChunk) {
+              if (buse > 0 && !mbar_wait_warp(&bempty[bs], (buse - 1) & 1, status, kErrEmpty)) {
+                alive = false;
+                break;
+              }
+              if (leader) {
+                mbar_arrive_expect_tx(&bfull[bs], b_bytes);
+                tma_load_5d(ring_b + (uint32_t)(bs * g.bslot), p.bmap, &bfull[bs], k0, 0, p.bz,
+                            p.by, 0);
+              }
+              __syncwarp();
+              if (++bs == g.nbslots) {
+                bs = 0;
+                ++buse;
+              }
+#pragma unroll 1
+              for (int sa = 0; sa < kS; sa += spp) {
+                if (use > 0 && !mbar_wait_warp(&aempty[st], (use - 1) & 1, status, kErrEmpty)) {
                   alive = false;
                   break;
                 }
-                mbar_arrive_expect_tx(&bfull[bs], b_bytes);
-                tma_load_5d(bring + bs * g.bslot, p.bmap, &bfull[bs], ch * kKChunk, 0, p.bz, p.by,
-                            0);
-                if (++bs == kBSlots) {
-                  bs = 0;
-                  ++buse;
-                }
-                for (int sa = 0; sa < kS; ++sa) {
-                  if (use > 0 && !mbar_wait(&aempty[st], (use - 1) & 1, status, kErrEmpty)) {
-                    alive = false;
-                    break;
-                  }
+                if (leader) {
                   mbar_arrive_expect_tx(&afull[st], a_bytes);
-                  tma_load_4d(ring + st * kATile, p.amap, &afull[st], ch * kKChunk, mt * rows,
+                  tma_load_4d(ring_a + (uint32_t)(st * g.aslot), p.amap, &afull[st], k0, mt * rows,
                               p.ax, sa);
-                  if (++st == g.nslots) {
-                    st = 0;
-                    ++use;
-                  }
+                }
+                __syncwarp();
+                if (++st == g.nslots) {
+                  st = 0;
+                  ++use;
                 }
               }
             }
+          }
+    }
+    if (!alive && leader) {  // wait for the copies still in flight
+      for (int i = 0; i < g.nslots; ++i) {
+        const uint32_t n = use + (i < st ? 1 : 0);
+        if (n > 0) mbar_drain(&afull[i], (n - 1) & 1);
       }
-      if (!alive) {  // wait for the copies still in flight
-        for (int i = 0; i < g.nslots; ++i) {
-          const uint32_t n = use + (i < st ? 1 : 0);
-          if (n > 0) mbar_drain(&afull[i], (n - 1) & 1);
-        }
-        for (int i = 0; i < kBSlots; ++i) {
-          const uint32_t n = buse + (i < bs ? 1 : 0);
-          if (n > 0) mbar_drain(&bfull[i], (n - 1) & 1);
-        }
+      for (int i = 0; i < g.nbslots; ++i) {
+        const uint32_t n = buse + (i < bs ? 1 : 0);
+        if (n > 0) mbar_drain(&bfull[i], (n - 1) & 1);
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------- MMA issuer
     const bool leader = elect_one();
-    int st = 0, bs = 0;
-    uint32_t ph = 0, bph = 0, item = 0;
+    MmaRole m;
+    m.st = m.bs = 0;
+    m.ph = m.bph = m.item = 0;
+    m.nslots = g.nslots;
+    m.nbslots = g.nbslots;
+    m.aslot = g.aslot;
+    m.bslot = g.bslot;
+    m.ring_a = uniform(smem_u32(ring));
+    m.ring_b = uniform(smem_u32(bring));
+    m.tm = uniform(tmem);
+    m.afull = afull;
+    m.aempty = aempty;
+    m.bfull = bfull;
+    m.bempty = bempty;
+    m.accf = accf;
+    m.acce = acce;
+    m.leader = leader;
     int prev = -1;
     bool alive = true;
-    const uint64_t desc0 = sdesc_sw128(0);
-    const uint32_t ring_a = uniform(smem_u32(ring)), ring_b = uniform(smem_u32(bring));
-    const uint32_t tm = uniform(tmem);
     for (uint32_t k = 0; alive; ++k) {
       const int ts = k % kTupleSlots;
-      if (!mbar_wait(&tfull[ts], (k / kTupleSlots) & 1, status, kErrFull)) break;
+      if (!mbar_wait_warp(&tfull[ts], (k / kTupleSlots) & 1, status, kErrFull)) break;
       const int stop = uniform(tslot[ts].t < 0 ? 1 : 0);
       const int sys = uniform(tslot[ts].s);
       __syncwarp();
@@ -412,89 +545,20 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       const TcDesc &d = g.sys[sys];
       const bool fresh = sys != prev;  // its accumulators may lie elsewhere
       prev = sys;
-      const int P = uniform(d.P), kp = uniform(d.Nv), kh = uniform(d.No);
-      const int rows = uniform(d.rows), ntiles = (kh * kh + rows - 1) / rows;
-      const int nitems = 3 * (uniform(d.use_j) ? 2 : 1) * ntiles;
-      const int bufcols = kS * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
-      for (int it = 0; it < nitems && alive; ++it, ++item) {
-        const int buf = nbuf == 2 ? (int)(item & 1) : 0;
-        // buffer `item & 1`'s barrier is used for every item, whichever
-        // columns it holds: use u of it is item 2u + (item & 1)
-        const int bb = item & 1;
-        const uint32_t u = item >> 1;
-        if (u > 0 && !mbar_wait(&acce[bb], (u - 1) & 1, status, kErrAccEmpty)) {
-          alive = false;
-          break;
-        }
-        if ((nbuf == 1 || (it == 0 && fresh)) && item > 0) {
-          // one accumulator, or another layout than the item before had:
-          // that item must be drained too
-          const int pb = (item - 1) & 1;
-          const uint32_t pu = (item - 1) >> 1;
-          if (!mbar_wait(&acce[pb], pu & 1, status, kErrAccEmpty)) {
-            alive = false;
-            break;
-          }
-        }
-        tc_fence_after();
-        const uint32_t dbase = tm + buf * bufcols;
-        uint32_t acc = 0;
-        for (int pt = 0; pt < 4 && alive; ++pt) {
-          const int K = (pt & 1) == 0 ? kp : kh;
-          for (int k0 = 0; k0 < K && alive; k0 += kKChunk) {
-            const int nkk = (min(kKChunk, K - k0) + 15) / 16;
-            if (!mbar_wait(&bfull[bs], bph, status, kErrFull)) {
-              alive = false;
-              break;
-            }
-            const uint64_t bdesc = desc0 + ((ring_b + (uint32_t)(bs * g.bslot)) >> 4);
-            uint32_t dcol = dbase;
-            int n = kS * P;
-#pragma unroll 1
-            for (int sa = 0; sa < kS; ++sa, n -= P, dcol += P) {
-              if (!mbar_wait(&afull[st], ph, status, kErrFull)) {
-                alive = false;
-                break;
-              }
-              tc_fence_after();
-              const uint64_t adesc = desc0 + ((ring_a + (uint32_t)(st * kATile)) >> 4);
-              const int n16 = (n + 15) & ~15;
-              // above N = 256 two MMAs of about half the columns each
-              const int n1 = n16 <= 256 ? n16 : ((n16 >> 1) + 15) & ~15, n2 = n16 - n1;
-              const uint32_t id1 = idesc_bf16_f32(128, 0) | ((uint32_t)(n1 >> 3) << 17);
-              if (leader) {
-#pragma unroll
-                for (int kk = 0; kk < kKChunk / 16; ++kk)
-                  if (kk < nkk)
-                    mma_bf16(dcol, adesc + 2 * kk, bdesc + 2 * kk, id1, kk == 0 ? acc : 1u);
-                if (n2 > 0) {
-                  const uint32_t id2 = idesc_bf16_f32(128, 0) | ((uint32_t)(n2 >> 3) << 17);
-                  const uint64_t bdesc2 = bdesc + (uint32_t)(n1 * 8);
-#pragma unroll
-                  for (int kk = 0; kk < kKChunk / 16; ++kk)
-                    if (kk < nkk)
-                      mma_bf16(dcol + n1, adesc + 2 * kk, bdesc2 + 2 * kk, id2,
-                               kk == 0 ? acc : 1u);
-                }
-                mma_commit(&aempty[st]);
-              }
-              __syncwarp();
-              acc = 1;
-              if (++st == g.nslots) {
-                st = 0;
-                ph ^= 1u;
-              }
-            }
-            if (leader) mma_commit(&bempty[bs]);
-            __syncwarp();
-            if (++bs == kBSlots) {
-              bs = 0;
-              bph ^= 1u;
-            }
-          }
-        }
-        if (leader && alive) mma_commit(&accf[bb]);
-        __syncwarp();
+      m.kp = uniform(d.Nv);
+      m.kh = uniform(d.No);
+      m.rows = uniform(d.rows);
+      m.spp = uniform(d.spp);
+      m.nitems = 3 * (uniform(d.use_j) ? 2 : 1) * ((m.kh * m.kh + m.rows - 1) / m.rows);
+      switch (uniform(d.P)) {
+        case 8: alive = mma_tuple<8>(m, fresh, status); break;
+        case 16: alive = mma_tuple<16>(m, fresh, status); break;
+        case 24: alive = mma_tuple<24>(m, fresh, status); break;
+        case 32: alive = mma_tuple<32>(m, fresh, status); break;
+        case 40: alive = mma_tuple<40>(m, fresh, status); break;
+        case 48: alive = mma_tuple<48>(m, fresh, status); break;
+        case 56: alive = mma_tuple<56>(m, fresh, status); break;
+        default: alive = mma_tuple<64>(m, fresh, status); break;
       }
     }
     // no MMA outlives this role (after a failed wait some may be in flight)
@@ -779,7 +843,7 @@ __global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
 // ------------------------------------------------------------------ host
 
 struct TcImpl {
-  int No = 0, Nv = 0, P = 0, rows = 0, Kp = 0, Kh = 0;
+  int No = 0, Nv = 0, P = 0, rows = 0, spp = 0, Kp = 0, Kh = 0;
   int eT = 0, eV = 0, eJ = 0;
   double max_t = 0, min_t = 0;  // T: largest element, smallest nonzero slab maximum
   double nT[3], nU[3];          // digit norms of the T rows (over E; over L)
@@ -801,16 +865,17 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// BF16 tensor map of `rank` dimensions, dims[0] = K extent (fastest, pitch
-// elements apart per row), 128-byte swizzle.
-int make_map(CUtensorMap *m, void *base, int rank, const uint64_t *dims, uint64_t pitch,
-             const uint32_t *box) {
+// BF16 tensor map of `rank` dimensions, K fastest, 128-byte swizzle.  The K
+// extent is the padded one, whole chunks: a box that leaves the tensor in its
+// innermost dimension takes ~7 cycles a row (18 B per cycle), one inside it
+// 1.1 (119 B per cycle); rows past the other extents cost nothing extra.
+int make_map(CUtensorMap *m, void *base, int rank, const uint64_t *dims, const uint32_t *box) {
   auto fn = encode_fn();
   if (!fn) {
     set_error("cuTensorMapEncodeTiled not available from the driver");
     return ATRIP_ERR_CUDA;
   }
-  uint64_t strides[4], s = pitch * 2;
+  uint64_t strides[4], s = dims[0] * 2;
   for (int i = 1; i < rank; ++i) {
     strides[i - 1] = s;
     s *= dims[i];
@@ -826,15 +891,15 @@ int make_map(CUtensorMap *m, void *base, int rank, const uint64_t *dims, uint64_
   return ATRIP_OK;
 }
 
-int map_a(CUtensorMap *m, void *base, const TcImpl &p, int K, int pitch) {
+int map_a(CUtensorMap *m, void *base, const TcImpl &p, int K) {
   const uint64_t d[4] = {(uint64_t)K, (uint64_t)p.No * p.No, (uint64_t)p.Nv, kS};
-  const uint32_t box[4] = {kKChunk, (uint32_t)p.rows, 1, 1};
-  return make_map(m, base, 4, d, pitch, box);
+  const uint32_t box[4] = {kKChunk, (uint32_t)p.rows, 1, (uint32_t)p.spp};
+  return make_map(m, base, 4, d, box);
 }
-int map_b(CUtensorMap *m, void *base, const TcImpl &p, int K, int pitch) {
+int map_b(CUtensorMap *m, void *base, const TcImpl &p, int K) {
   const uint64_t d[5] = {(uint64_t)K, (uint64_t)p.No, (uint64_t)p.Nv, (uint64_t)p.Nv, kS};
   const uint32_t box[5] = {kKChunk, (uint32_t)p.P, 1, 1, kS};
-  return make_map(m, base, 5, d, pitch, box);
+  return make_map(m, base, 5, d, box);
 }
 
 // Smallest e with x <= 127/128 2^e (the top digit then stays below 128).
@@ -946,9 +1011,15 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStre
   p->No = No_;
   p->Nv = Nv_;
   p->P = (No_ + 7) / 8 * 8;
-  p->rows = std::min(128, (No_ * No_ + 7) / 8 * 8);
-  p->Kp = (Nv_ + 7) / 8 * 8;
-  p->Kh = (No_ + 7) / 8 * 8;
+  // rows of an item: the No^2 rows in equal shares of at most 128
+  const int nt = (No_ * No_ + 127) / 128;
+  p->rows = ((No_ * No_ + nt - 1) / nt + 7) / 8 * 8;
+  // slices per copy: as many as 32 KB hold (a ring slot).  A warp needs
+  // ~400 cycles for a wait, a copy and its bookkeeping whatever the size, so
+  // 16 KB copies fed the ring 33 B per cycle; 32 KB ones twice that
+  p->spp = p->rows > 64 ? 2 : p->rows > 32 ? 4 : 8;
+  p->Kp = (Nv_ + kKChunk - 1) / kKChunk * kKChunk;
+  p->Kh = kKChunk;
   const int64_t No = No_, Nv = Nv_, No2 = No * No;
   const size_t nTa = up((size_t)2 * kS * Nv * No2 * p->Kp), nVh = up((size_t)2 * kS * Nv * No2 * p->Kh),
                nVp = up((size_t)2 * kS * Nv * Nv * No * p->Kp),
@@ -1020,10 +1091,10 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStre
   set_norms(nV, h.n[5]);
   if (!sums_exact(p->nT, nV, nH, p->nU)) return ATRIP_OK;
 
-  if ((rc = map_a(&p->maps.TaN, TaN, *p, Nv_, p->Kp)) || (rc = map_a(&p->maps.TaT, TaT, *p, Nv_, p->Kp)) ||
-      (rc = map_a(&p->maps.VhN, VhN, *p, No_, p->Kh)) || (rc = map_a(&p->maps.VhT, VhT, *p, No_, p->Kh)) ||
-      (rc = map_b(&p->maps.Vp, Vp, *p, Nv_, p->Kp)) || (rc = map_b(&p->maps.TpN, TpN, *p, No_, p->Kh)) ||
-      (rc = map_b(&p->maps.TpT, TpT, *p, No_, p->Kh)))
+  if ((rc = map_a(&p->maps.TaN, TaN, *p, p->Kp)) || (rc = map_a(&p->maps.TaT, TaT, *p, p->Kp)) ||
+      (rc = map_a(&p->maps.VhN, VhN, *p, p->Kh)) || (rc = map_a(&p->maps.VhT, VhT, *p, p->Kh)) ||
+      (rc = map_b(&p->maps.Vp, Vp, *p, p->Kp)) || (rc = map_b(&p->maps.TpN, TpN, *p, p->Kh)) ||
+      (rc = map_b(&p->maps.TpT, TpT, *p, p->Kh)))
     return rc;
   p->maps.JhN = p->maps.VhN;
   p->maps.JhT = p->maps.VhT;
@@ -1068,8 +1139,8 @@ int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *lau
   set_norms(nH, h.n[4]);
   set_norms(nV, h.n[5]);
   if (!sums_exact(p->nT, nV, nH, p->nU)) return ATRIP_OK;
-  if ((rc = map_a(&p->maps.JhN, hN, *p, p->No, p->Kh)) || (rc = map_a(&p->maps.JhT, hT, *p, p->No, p->Kh)) ||
-      (rc = map_b(&p->maps.Jp, vp, *p, p->Nv, p->Kp)))
+  if ((rc = map_a(&p->maps.JhN, hN, *p, p->Kh)) || (rc = map_a(&p->maps.JhT, hT, *p, p->Kh)) ||
+      (rc = map_b(&p->maps.Jp, vp, *p, p->Kp)))
     return rc;
   s.usable_j = true;
   return ATRIP_OK;
@@ -1160,9 +1231,10 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   }
   if (!b.d_queue) ATRIP_CUDA_TRY(cudaMalloc(&b.d_queue, sizeof(unsigned long long)));
   auto *h = static_cast<TcDesc *>(b.h_desc);
-  int P = 0;
+  int P = 0, spp = kS;
   b.lay_no = 0;
   b.lay_pass = 1;
+  b.aslot = 0;
   b.h_prefix[0] = 0;
   for (int k = 0; k < n; ++k) {
     const TcSystem &m = sys[k];
@@ -1190,10 +1262,13 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     d.Nv = m.Nv;
     d.P = p->P;
     d.rows = p->rows;
+    d.spp = p->spp;
     d.n_triples = m.n_triples;
     d.use_j = m.use_j ? 1 : 0;
     h[k] = d;
     P = std::max(P, p->P);
+    b.aslot = std::max(b.aslot, p->spp * p->rows * 128);
+    spp = std::min(spp, p->spp);
     b.lay_no = std::max(b.lay_no, m.No);
     if (m.use_j) b.lay_pass = 2;
     b.h_prefix[k + 1] = b.h_prefix[k] + std::max<int64_t>(0, m.t_end - m.t_begin);
@@ -1204,8 +1279,12 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   b.lay_cells = b.lay_no * b.lay_no * b.lay_no;
   // stack of 8 slices of P rows; an MMA's N, a multiple of 16, may read 8 rows more
   b.bslot = kS * P * 128 + 1024;
-  b.nslots = std::min(kMaxSlots, (kSmemLimit - 1024 - kTailBytes - kBSlots * b.bslot) / kATile);
-  b.smem = 1024 + (size_t)b.nslots * kATile + kBSlots * b.bslot + kTailBytes;
+  // rings: a K chunk takes one B slot and (at the largest system) 8 / spp A
+  // slots; as many chunks in flight as fit, two B slots at least
+  const int room = kSmemLimit - 1024 - kTailBytes, chunk = kS / spp * b.aslot + b.bslot;
+  b.nbslots = std::min(kMaxBSlots, std::max(2, room / chunk + 1));
+  b.nslots = std::min(kMaxSlots, (room - b.nbslots * b.bslot) / b.aslot);
+  b.smem = 1024 + (size_t)b.nslots * b.aslot + (size_t)b.nbslots * b.bslot + kTailBytes;
   const size_t per_cta = ((size_t)2 * 3 * 16 + 8) * b.lay_pass * b.lay_cells;
   const size_t need = per_cta * std::max(b.grid, 1);
   if (need > b.planes_bytes) {
@@ -1241,6 +1320,8 @@ int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st
   a.lay_cells = b.lay_cells;
   a.lay_pass = b.lay_pass;
   a.nslots = b.nslots;
+  a.nbslots = b.nbslots;
+  a.aslot = b.aslot;
   a.bslot = b.bslot;
   ATRIP_CUDA_TRY(cudaFuncSetAttribute(triples_fp64_tc_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem));
