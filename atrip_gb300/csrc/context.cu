@@ -458,6 +458,14 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
     const int rc = tc_prepare(c->tc, c->dt, c->No, c->Nv, use_j, st, &launches, &tc);
     if (rc != ATRIP_OK) return rc;
   }
+  if (tc && c->tune.tuple_block == 0) {
+    const int block = tc_tuple_block(c->No, c->Nv, c->sm_count);
+    if (block > 0) {
+      const int rc = build_order(c, t_begin, t_end, block, st);
+      if (rc != ATRIP_OK) return rc;
+      order = c->d_order;
+    }
+  }
   if (tc) {
     const TcSystem ts = {&c->tc, &c->dt, c->No, c->Nv, c->n_triples, c->d_tuples, c->d_triples,
                          t_begin, t_end, use_j, c->d_e, c->d_ect};

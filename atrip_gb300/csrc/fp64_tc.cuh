@@ -25,6 +25,9 @@ void tc_free(TcState &s);
 // Whether this form serves a system of these sizes at all.
 bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx);
 
+// The processing order of its tuples (see build_order), 0 = list order.
+int tc_tuple_block(int No, int Nv, int sm_count);
+
 // Examine the operands, cut the slices and build the tensor maps, once per
 // upload.  ATRIP_OK with *usable = false where the data or the free memory
 // rule the form out (the caller then runs the DFMA kernel).

@@ -44,6 +44,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// Whether the phase is complete now; never suspends.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Wait for the phase with the given parity to complete.  Returns false (and
 // sets *status to code if it was 0) when the wait exceeds `limit` SM cycles
 // (default kWaitCycles) or another thread already reported a failure.
@@ -85,8 +97,11 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(p));
   return p != 0;
 }
-// A value every lane holds, as one the compiler knows to be warp-uniform.
-__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+// A value every lane holds (not negative), in a uniform register: a warp
+// reduction's result lives there, a shuffle's does not.
+__device__ __forceinline__ int uniform(int v) {
+  return (int)__reduce_max_sync(0xffffffffu, (unsigned)v);
+}
 
 // ---------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const void *map, uint64_t *bar, int c0,

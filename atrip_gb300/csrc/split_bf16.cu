@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                                g.wait_cycles);
             }))
           break;
-        const int stop = uniform(tslot[ts].t < 0 ? 1 : 0);
+        const bool stop = __any_sync(0xffffffffu, tslot[ts].t < 0);
         const int sys = MULTI ? uniform(tslot[ts].s) : 0;
         __syncwarp();
         if (leader) mbar_arrive(&tempty[ts]);

@@ -76,7 +76,6 @@ constexpr int kThreads = 512;
 constexpr int kS = 8;                       // digit slices and levels
 constexpr int kKChunk = 64;                 // BF16 elements per 128-byte row
 constexpr int kMaxSlots = 10;               // A ring
-constexpr int kMaxBSlots = 8;               // B ring
 constexpr int kTupleSlots = 4;
 constexpr int kEnergyWarps = 10;
 constexpr int kEnergyThreads = kEnergyWarps * 32;
@@ -106,6 +105,7 @@ struct TcArgs {
   const int64_t *prefix;
   int nsys;
   int64_t total;
+  int claim;              // tuples taken from the queue at once, <= 32
   const uint32_t *order;  // processing order of a single system's range
   unsigned long long *queue;
   int *flags;
@@ -242,12 +242,12 @@ __device__ __forceinline__ double energy_partial(const TcDesc &d, const double *
 // The MMA issuer's state, carried from tuple to tuple.
 struct MmaRole {
   int st, bs;              // A and B ring slots of the next operands
-  uint32_t ph, bph, item;  // their phases; items so far
+  uint32_t ph, item;       // the A slot's phase; items so far
   int nslots, nbslots, aslot, bslot;
   uint32_t ring_a, ring_b, tm;
-  uint64_t *afull, *aempty, *bfull, *bempty, *accf, *acce;
+  uint64_t *afull, *aempty, *accf, *acce;
   bool leader;
-  int kp, kh, rows, spp, nitems;  // the tuple's system
+  int P, kp, kh, rows, spp, nitems;  // the tuple's system
 };
 
 // One slice of A times the slices of B that still give a kept level: result
@@ -322,7 +322,6 @@ __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
     for (int pt = 0; pt < 4; ++pt) {
       const int K = (pt & 1) == 0 ? m.kp : m.kh;
       for (int k0 = 0; k0 < K; k0 += kKChunk) {
-        if (!mbar_wait_warp(&m.bfull[m.bs], m.bph, status, kErrFull)) return false;
         const uint64_t bd = sdesc_sw128(0) + ((m.ring_b + (uint32_t)(m.bs * m.bslot)) >> 4);
         uint64_t ad = 0;
         const int nkk = (min(kKChunk, K - k0) + 15) / 16;
@@ -330,12 +329,7 @@ __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
                                  : mma_chunk<P, 0, 0>(m, d, ad, bd, nkk, acc, status);
         if (!ok) return false;
         acc = 1;
-        if (m.leader) mma_commit(&m.bempty[m.bs]);
-        __syncwarp();
-        if (++m.bs == m.nbslots) {
-          m.bs = 0;
-          m.bph ^= 1u;
-        }
+        if (++m.bs == m.nbslots) m.bs = 0;
       }
     }
     if (m.leader) mma_commit(&m.accf[bb]);
@@ -353,9 +347,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
   unsigned char *tail = bring + g.nbslots * g.bslot;
   uint64_t *afull = reinterpret_cast<uint64_t *>(tail);
   uint64_t *aempty = afull + kMaxSlots;
-  uint64_t *bfull = aempty + kMaxSlots;
-  uint64_t *bempty = bfull + kMaxBSlots;
-  uint64_t *accf = bempty + kMaxBSlots;
+  uint64_t *accf = aempty + kMaxSlots;
   uint64_t *acce = accf + 2;
   uint64_t *tfull = acce + 2;
   uint64_t *tempty = tfull + kTupleSlots;
@@ -366,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
   TcSlot *tslot = reinterpret_cast<TcSlot *>(tail + 448);
   double *ta = reinterpret_cast<double *>(tail + 576);
   double *tb = ta + 64, *tc = tb + 64, *red = tc + 64;
-  static_assert((2 * kMaxSlots + 2 * kMaxBSlots + 4 + 2 * kTupleSlots + 5) * 8 + 8 <= 448, "tail");
+  static_assert((2 * kMaxSlots + 4 + 2 * kTupleSlots + 5) * 8 + 8 <= 448, "tail");
   static_assert(kTupleSlots * sizeof(TcSlot) <= 128, "tuple slots");
 
   int *status = g.flags;
@@ -375,10 +367,6 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
     for (int s = 0; s < g.nslots; ++s) {
       mbar_init(&afull[s], 1);
       mbar_init(&aempty[s], 1);
-    }
-    for (int s = 0; s < g.nbslots; ++s) {
-      mbar_init(&bfull[s], 1);
-      mbar_init(&bempty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&accf[b], 1);
@@ -413,39 +401,67 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
     // ------------------------------------------------------ TMA producer
     const bool leader = elect_one();
     int st = 0, bs = 0;
-    uint32_t use = 0, buse = 0;
+    uint32_t use = 0;
     int cur = -1;
-    int64_t cur_lo = 0, cur_hi = 0;
+    int64_t cur_hi = 0;
     bool alive = true;
     const uint32_t ring_a = uniform(smem_u32(ring)), ring_b = uniform(smem_u32(bring));
+    const TcDesc *d = g.sys;
+    int kp = 0, kh = 0, rows = 0, ntiles = 0, npass = 0, spp = 0;
+    uint32_t a_bytes = 0, b_bytes = 0;
+    // queue positions are claimed g.claim at a time; a claim's tuples are
+    // looked up together, one to a lane
+    int64_t q0 = 0, pos = 0;
+    int have = 0, next = 0;
+    uint32_t packed = 0;
     for (uint32_t k = 0;; ++k) {
       const int ts = k % kTupleSlots;
       const uint32_t tuse = k / kTupleSlots;
       if (tuse > 0 && !mbar_wait_warp(&tempty[ts], (tuse - 1) & 1, status, kErrEmpty))
         alive = false;
-      int64_t q = g.total;
-      if (alive && leader && *reinterpret_cast<volatile int *>(status) == 0)
-        q = (int64_t)atomicAdd(g.queue, 1ull);
-      q = __shfl_sync(0xffffffffu, q, __ffs(__ballot_sync(0xffffffffu, leader)) - 1);
-      const bool stop = q >= g.total;
+      if (next == have) {
+        q0 = g.total;
+        if (alive && leader && *reinterpret_cast<volatile int *>(status) == 0)
+          q0 = (int64_t)atomicAdd(g.queue, (unsigned long long)g.claim);
+        q0 = __shfl_sync(0xffffffffu, q0, __ffs(__ballot_sync(0xffffffffu, leader)) - 1);
+        have = q0 >= g.total ? 0 : (int)min((int64_t)g.claim, g.total - q0);
+        next = 0;
+        if (lane < have) {
+          const int64_t q = q0 + lane;
+          int lo = max(cur, 0);  // queue positions only grow: walk on from the last system
+          while (lo + 1 < g.nsys && g.prefix[lo + 1] <= q) ++lo;
+          pos = g.sys[lo].t_begin + (g.order ? (int64_t)g.order[q] : q - g.prefix[lo]);
+          packed = g.sys[lo].tuples[pos];
+        }
+        __syncwarp();
+      }
+      const bool stop = next == have || !alive;
       TcSlot s;
       s.a = s.b = s.c = s.s = 0;
       s.t = -1;
       if (!stop) {
-        if (q >= cur_hi) {  // queue positions only grow: walk on to the tuple's system
-          int lo = cur < 0 ? 0 : cur;
+        const int64_t q = q0 + next;
+        if (q >= cur_hi) {
+          int lo = max(cur, 0);
           while (lo + 1 < g.nsys && g.prefix[lo + 1] <= q) ++lo;
           cur = uniform(lo);
-          cur_lo = g.prefix[cur];
           cur_hi = g.prefix[cur + 1];
-          const CUtensorMap *m = &g.sys[cur].maps.TaN;
-          const int nm = g.sys[cur].use_j ? 10 : 7;
-          for (int i = 0; i < nm; ++i) tensormap_acquire(m + i);
+          d = g.sys + cur;
+          const int nm = d->use_j ? 10 : 7;
+          for (int i = 0; i < nm; ++i) tensormap_acquire(&d->maps.TaN + i);
+          kp = uniform(d->Nv);
+          kh = uniform(d->No);
+          rows = uniform(d->rows);
+          ntiles = (kh * kh + rows - 1) / rows;
+          npass = uniform(d->use_j) ? 2 : 1;
+          spp = uniform(d->spp);
+          a_bytes = spp * rows * 128;
+          b_bytes = kS * uniform(d->P) * 128;
         }
-        const TcDesc &d = g.sys[cur];
         s.s = cur;
-        s.t = d.t_begin + (g.order ? (int64_t)g.order[q] : q - cur_lo);
-        const int pk = uniform((int)d.tuples[s.t]);
+        s.t = __shfl_sync(0xffffffffu, pos, next);
+        const int pk = __shfl_sync(0xffffffffu, (int)packed, next);
+        ++next;
         s.a = pk & 0x3ff;
         s.b = (pk >> 10) & 0x3ff;
         s.c = (pk >> 20) & 0x3ff;
@@ -456,31 +472,12 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       }
       __syncwarp();
       if (stop) break;
-      const TcDesc &d = g.sys[cur];
-      const int kp = uniform(d.Nv), kh = uniform(d.No), rows = uniform(d.rows);
-      const int ntiles = (kh * kh + rows - 1) / rows, npass = uniform(d.use_j) ? 2 : 1;
-      const int spp = uniform(d.spp);
-      const uint32_t a_bytes = spp * rows * 128, b_bytes = kS * uniform(d.P) * 128;
       for (int gi = 0; gi < 3 * npass && alive; ++gi)
         for (int mt = 0; mt < ntiles && alive; ++mt)
           for (int pt = 0; pt < 4 && alive; ++pt) {
-            const TcPart p = part_of(d.maps, gi % 3, pt, s.a, s.b, s.c, gi / 3);
+            const TcPart p = part_of(d->maps, gi % 3, pt, s.a, s.b, s.c, gi / 3);
             const int K = p.particle ? kp : kh;
             for (int k0 = 0; k0 < K && alive; k0 += kKChunk) {
-              if (buse > 0 && !mbar_wait_warp(&bempty[bs], (buse - 1) & 1, status, kErrEmpty)) {
-                alive = false;
-                break;
-              }
-              if (leader) {
-                mbar_arrive_expect_tx(&bfull[bs], b_bytes);
-                tma_load_5d(ring_b + (uint32_t)(bs * g.bslot), p.bmap, &bfull[bs], k0, 0, p.bz,
-                            p.by, 0);
-              }
-              __syncwarp();
-              if (++bs == g.nbslots) {
-                bs = 0;
-                ++buse;
-              }
 #pragma unroll 1
               for (int sa = 0; sa < kS; sa += spp) {
                 if (use > 0 && !mbar_wait_warp(&aempty[st], (use - 1) & 1, status, kErrEmpty)) {
@@ -488,7 +485,12 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
                   break;
                 }
                 if (leader) {
-                  mbar_arrive_expect_tx(&afull[st], a_bytes);
+                  mbar_arrive_expect_tx(&afull[st], sa == 0 ? a_bytes + b_bytes : a_bytes);
+                  // the chunk's B stack comes with its first A slot; its ring
+                  // is one chunk deeper than A's, so that slot is free too
+                  if (sa == 0)
+                    tma_load_5d(ring_b + (uint32_t)(bs * g.bslot), p.bmap, &afull[st], k0, 0, p.bz,
+                                p.by, 0);
                   tma_load_4d(ring_a + (uint32_t)(st * g.aslot), p.amap, &afull[st], k0, mt * rows,
                               p.ax, sa);
                 }
@@ -498,6 +500,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
                   ++use;
                 }
               }
+              if (++bs == g.nbslots) bs = 0;
             }
           }
     }
@@ -506,10 +509,6 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
         const uint32_t n = use + (i < st ? 1 : 0);
         if (n > 0) mbar_drain(&afull[i], (n - 1) & 1);
       }
-      for (int i = 0; i < g.nbslots; ++i) {
-        const uint32_t n = buse + (i < bs ? 1 : 0);
-        if (n > 0) mbar_drain(&bfull[i], (n - 1) & 1);
-      }
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -517,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
     const bool leader = elect_one();
     MmaRole m;
     m.st = m.bs = 0;
-    m.ph = m.bph = m.item = 0;
+    m.ph = m.item = 0;
     m.nslots = g.nslots;
     m.nbslots = g.nbslots;
     m.aslot = g.aslot;
@@ -527,8 +526,6 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
     m.tm = uniform(tmem);
     m.afull = afull;
     m.aempty = aempty;
-    m.bfull = bfull;
-    m.bempty = bempty;
     m.accf = accf;
     m.acce = acce;
     m.leader = leader;
@@ -537,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
     for (uint32_t k = 0; alive; ++k) {
       const int ts = k % kTupleSlots;
       if (!mbar_wait_warp(&tfull[ts], (k / kTupleSlots) & 1, status, kErrFull)) break;
-      const int stop = uniform(tslot[ts].t < 0 ? 1 : 0);
+      const bool stop = __any_sync(0xffffffffu, tslot[ts].t < 0);
       const int sys = uniform(tslot[ts].s);
       __syncwarp();
       if (leader) mbar_arrive(&tempty[ts]);
@@ -545,12 +542,15 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       const TcDesc &d = g.sys[sys];
       const bool fresh = sys != prev;  // its accumulators may lie elsewhere
       prev = sys;
-      m.kp = uniform(d.Nv);
-      m.kh = uniform(d.No);
-      m.rows = uniform(d.rows);
-      m.spp = uniform(d.spp);
-      m.nitems = 3 * (uniform(d.use_j) ? 2 : 1) * ((m.kh * m.kh + m.rows - 1) / m.rows);
-      switch (uniform(d.P)) {
+      if (fresh) {
+        m.P = uniform(d.P);
+        m.kp = uniform(d.Nv);
+        m.kh = uniform(d.No);
+        m.rows = uniform(d.rows);
+        m.spp = uniform(d.spp);
+        m.nitems = 3 * (uniform(d.use_j) ? 2 : 1) * ((m.kh * m.kh + m.rows - 1) / m.rows);
+      }
+      switch (m.P) {
         case 8: alive = mma_tuple<8>(m, fresh, status); break;
         case 16: alive = mma_tuple<16>(m, fresh, status); break;
         case 24: alive = mma_tuple<24>(m, fresh, status); break;
@@ -618,17 +618,23 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
             const int r = c0 + x;
             if (r < No && valid) {
               // |level sum| < 2^22 for L >= 1 (flagged otherwise): adding
-              // 1.5 2^23 leaves the integer in the low mantissa bits
-              constexpr float kMagic = 12582912.f;
+              // 1.5 2^23 leaves the integer n in the low mantissa bits b =
+              // n + kBits.  Pairs of levels join in 32 bits (256 n + n' <
+              // 2^31; the kBits cancel modulo 2^32), pairs of pairs in 64.
               constexpr uint32_t kBits = 0x4B400000u;
-              long long hi = (long long)__float2int_rn(v[0][x]) << 24, lo = 0;
+              uint32_t b[kS];
 #pragma unroll
               for (int L = 1; L < kS; ++L) {
-                const uint32_t b = __float_as_uint(v[L][x] + kMagic);
-                over |= b ^ 0x4B000000u;  // exponent bits differ outside that range
-                const long long n = (long long)((int)b - (int)kBits);
-                if (L < 4) hi += n << (24 - 8 * L); else lo += n << (56 - 8 * L);
+                b[L] = __float_as_uint(v[L][x] + 12582912.f);
+                over |= b[L] ^ 0x4B000000u;  // exponent bits differ outside that range
               }
+              const int n1 = (int)(b[1] - kBits);
+              const int n23 = (int)(b[2] * 256u + b[3] - kBits * 257u);
+              const int n45 = (int)(b[4] * 256u + b[5] - kBits * 257u);
+              const int n67 = (int)(b[6] * 256u + b[7] - kBits * 257u);
+              const long long hi = (long long)__float2int_rn(v[0][x]) * (1 << 24) +
+                                   ((long long)n1 * 65536 + n23);
+              const long long lo = (long long)n45 * 65536 + n67;
               plane[(size_t)r * No2 + m] = make_longlong2(hi, lo);
             }
           }
@@ -1014,10 +1020,9 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStre
   // rows of an item: the No^2 rows in equal shares of at most 128
   const int nt = (No_ * No_ + 127) / 128;
   p->rows = ((No_ * No_ + nt - 1) / nt + 7) / 8 * 8;
-  // slices per copy: as many as 32 KB hold (a ring slot).  A warp needs
-  // ~400 cycles for a wait, a copy and its bookkeeping whatever the size, so
-  // 16 KB copies fed the ring 33 B per cycle; 32 KB ones twice that
-  p->spp = p->rows > 64 ? 2 : p->rows > 32 ? 4 : 8;
+  // slices per copy (a ring slot): up to 32 KB.  A role's warp needs ~200 cycles for a wait and a signal whatever the
+  // size, so a slot should hold several MMAs' work
+  p->spp = p->rows > 64 ? 2 : 4;
   p->Kp = (Nv_ + kKChunk - 1) / kKChunk * kKChunk;
   p->Kh = kKChunk;
   const int64_t No = No_, Nv = Nv_, No2 = No * No;
@@ -1171,6 +1176,16 @@ bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx) {
   return !cplx && No >= 2 && (double)n_tuples * 12.0 * No * No * No * (No + Nv) >= 1e9;
 }
 
+// Side of the (a,b,c) blocks tuples are processed in, 0 = list order.  In list
+// order the ~150 tuples in flight read as many T_c slabs; where those exceed
+// the L2 (129 MB, each die caching what it reads) blocks of side 6 keep them
+// resident: No=24/Nv=240 13.3 -> 11.3 ms, No=40/Nv=240 10.4 -> 9.2 ms (sides
+// 3, 4, 8: 11.5, 13.1, 11.4 and 9.2, 9.1, 9.2); below it they gain nothing.
+int tc_tuple_block(int No, int Nv, int sm_count) {
+  const double slab = 16.0 * No * No * ((Nv + kKChunk - 1) / kKChunk * kKChunk);
+  return slab * std::min(sm_count, Nv) > 64e6 ? 6 : 0;
+}
+
 int tc_prepare(TcState &s, const DeviceTensors &dt, int No, int Nv, bool use_j, cudaStream_t st,
                int64_t *launches, bool *usable) {
   *usable = false;
@@ -1231,7 +1246,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   }
   if (!b.d_queue) ATRIP_CUDA_TRY(cudaMalloc(&b.d_queue, sizeof(unsigned long long)));
   auto *h = static_cast<TcDesc *>(b.h_desc);
-  int P = 0, spp = kS;
+  int P = 0, spp = 1;
   b.lay_no = 0;
   b.lay_pass = 1;
   b.aslot = 0;
@@ -1268,7 +1283,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     h[k] = d;
     P = std::max(P, p->P);
     b.aslot = std::max(b.aslot, p->spp * p->rows * 128);
-    spp = std::min(spp, p->spp);
+    spp = std::max(spp, p->spp);
     b.lay_no = std::max(b.lay_no, m.No);
     if (m.use_j) b.lay_pass = 2;
     b.h_prefix[k + 1] = b.h_prefix[k] + std::max<int64_t>(0, m.t_end - m.t_begin);
@@ -1279,11 +1294,17 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   b.lay_cells = b.lay_no * b.lay_no * b.lay_no;
   // stack of 8 slices of P rows; an MMA's N, a multiple of 16, may read 8 rows more
   b.bslot = kS * P * 128 + 1024;
-  // rings: a K chunk takes one B slot and (at the largest system) 8 / spp A
-  // slots; as many chunks in flight as fit, two B slots at least
-  const int room = kSmemLimit - 1024 - kTailBytes, chunk = kS / spp * b.aslot + b.bslot;
-  b.nbslots = std::min(kMaxBSlots, std::max(2, room / chunk + 1));
-  b.nslots = std::min(kMaxSlots, (room - b.nbslots * b.bslot) / b.aslot);
+  // rings: a K chunk takes 8 / spp A slots and one B slot, of which there is
+  // one more than chunks (of the largest slots) can be in flight
+  const int room = kSmemLimit - 1024 - kTailBytes;
+  auto b_for = [&](int nslots) { return (nslots * spp + kS - 1) / kS + 1; };
+  b.nslots = kMaxSlots;
+  while (b.nslots > 1 && b.nslots * b.aslot + b_for(b.nslots) * b.bslot > room) --b.nslots;
+  b.nbslots = b_for(b.nslots);
+  if (b.nslots * b.aslot + b.nbslots * b.bslot > room || b.nslots < 2) {
+    set_error("tensor-core FP64 form: shared memory too small");
+    return ATRIP_ERR_UNSUPPORTED;
+  }
   b.smem = 1024 + (size_t)b.nslots * b.aslot + (size_t)b.nbslots * b.bslot + kTailBytes;
   const size_t per_cta = ((size_t)2 * 3 * 16 + 8) * b.lay_pass * b.lay_cells;
   const size_t need = per_cta * std::max(b.grid, 1);
@@ -1311,6 +1332,8 @@ int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st
   a.prefix = b.d_prefix;
   a.nsys = b.n;
   a.total = b.total;
+  // several tuples a claim where every CTA has many (the tail stays even)
+  a.claim = (int)std::max<int64_t>(1, std::min<int64_t>(8, b.total / (b.grid * 16ll)));
   a.order = order;
   a.queue = b.d_queue;
   a.flags = b.d_flags;
