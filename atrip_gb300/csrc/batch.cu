@@ -244,7 +244,7 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
       bool ok = a.t_end > a.t_begin && c->tune.fp64_tile_rows == 0 &&
                 tc_sizes_ok(c->No, c->Nv, c->n_tuples, false);
       if (!ok) continue;
-      const int rc = tc_prepare(c->tc, c->dt, c->No, c->Nv, a.use_j != 0, st, &prep_launches, &ok);
+      const int rc = tc_prepare(c->tc, c->dt, c->No, c->Nv, false, a.use_j != 0, st, &prep_launches, &ok);
       if (rc != ATRIP_OK) return rc;
       if (!ok) continue;
       tc.push_back({&c->tc, &c->dt, c->No, c->Nv, a.n_triples, a.tuples, a.triples, a.t_begin,

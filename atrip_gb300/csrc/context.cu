@@ -455,7 +455,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
   double sums[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   ATRIP_CUDA_TRY(cudaEventRecord(c->ev0, st));
   if (tc) {
-    const int rc = tc_prepare(c->tc, c->dt, c->No, c->Nv, use_j, st, &launches, &tc);
+    const int rc = tc_prepare(c->tc, c->dt, c->No, c->Nv, cplx, use_j, st, &launches, &tc);
     if (rc != ATRIP_OK) return rc;
   }
   if (tc && c->tune.tuple_block == 0) {

@@ -31,8 +31,8 @@ int tc_tuple_block(int No, int Nv, int sm_count);
 // Examine the operands, cut the slices and build the tensor maps, once per
 // upload.  ATRIP_OK with *usable = false where the data or the free memory
 // rule the form out (the caller then runs the DFMA kernel).
-int tc_prepare(TcState &s, const DeviceTensors &dt, int No, int Nv, bool use_j, cudaStream_t st,
-               int64_t *launches, bool *usable);
+int tc_prepare(TcState &s, const DeviceTensors &dt, int No, int Nv, bool cplx, bool use_j,
+               cudaStream_t st, int64_t *launches, bool *usable);
 
 // One system of a launch.
 struct TcSystem {
@@ -56,7 +56,7 @@ struct TcBuffers {
   unsigned long long *d_queue = nullptr;
   int cap = 0;
   // launch layout of the last tc_launch_prepare
-  int n = 0, lay_no = 0, lay_cells = 0, lay_pass = 1, nslots = 0, nbslots = 0, aslot = 0,
+  int n = 0, nc = 1, lay_no = 0, lay_cells = 0, lay_pass = 1, nslots = 0, nbslots = 0, aslot = 0,
       bslot = 0, grid = 0;
   size_t smem = 0;
   int64_t total = 0;

@@ -63,6 +63,7 @@
 #include <cstring>
 #include <string>
 
+#include "complex.cuh"
 #include "engine.cuh"
 #include "fp64_tc.cuh"
 #include "sm100.cuh"
@@ -80,14 +81,21 @@ constexpr int kTupleSlots = 4;
 constexpr int kEnergyWarps = 10;
 constexpr int kEnergyThreads = kEnergyWarps * 32;
 constexpr int kSmemLimit = 232448;
-constexpr int kTailBytes = 576 + 3 * 64 * 8 + 16 * 8;
+constexpr int kT1 = 64;  // doubles per t1 row: No <= 64, or No <= 32 complex
+constexpr int kTailBytes = 576 + 3 * kT1 * 8 + 16 * 8;
 constexpr double kRangeBits = 8.0;
+constexpr int kBlocksZ = 3;                 // column blocks stored for a complex operand
 
 enum : int { kErrFull = 1, kErrEmpty = 2, kErrAccFull = 3, kErrAccEmpty = 4 };
 
+// A operands by row order (natural, transposed) and component ([1]: imaginary
+// parts of a complex system); B operands.
 struct TcMaps {
-  CUtensorMap TaN, TaT, VhN, VhT, Vp, TpN, TpT, JhN, JhT, Jp;
+  CUtensorMap Ta[2][2], Vh[2][2], Vp, TpN, TpT;
+  CUtensorMap Jh[2][2], Jp;  // (cT) intermediates in place of V_hhhp, V_pphp
 };
+constexpr int kMapsMain = 11, kMaps = 16;
+static_assert(sizeof(TcMaps) == kMaps * sizeof(CUtensorMap), "maps are contiguous");
 
 struct TcDesc {
   TcMaps maps;
@@ -146,17 +154,29 @@ __device__ __forceinline__ double i64_to_f64(long long n) {
   return __longlong_as_double(0x4338000000000000ll + n) - 6755399441055744.0;
 }
 
-// Operand sources of group g, part pt (0 natural particle, 1 natural hole,
-// 2 transposed particle, 3 transposed hole) of tuple (a,b,c).
+// Operand sources of group g, part pt of tuple (a,b,c): natural, then
+// transposed rows; in each the particle, then the hole contraction; for a
+// complex system in each of those A's real, then its imaginary parts.
+// A complex product is four real ones: columns [re | im] of
+//   A_re [V_re | V_im] + A_im [-V_im | V_re]              (particle)
+//   A_re [-T_re | -T_im] + A_im [-T_im | T_re]            (hole, conj(V_hhhp))
+// whose column blocks are neighbours in planes (-im, re, im) of V and
+// (-re, -im, re) of T: blk is the first one.
+template <bool CPLX>
+struct TcParts {
+  static constexpr int kCount = CPLX ? 8 : 4;
+  __device__ static __forceinline__ bool hole(int pt) { return (CPLX ? pt >> 1 : pt) & 1; }
+};
 struct TcPart {
   const CUtensorMap *amap, *bmap;
-  int ax, bz, by;
-  bool particle;
+  int ax, by, bz, blk;
 };
+template <bool CPLX>
 __device__ __forceinline__ TcPart part_of(const TcMaps &m, int g, int pt, int a, int b, int c,
                                           int pass) {
   int x, w, y, z, u, v, flip;
-  const bool tr = pt >= 2;
+  const bool tr = pt >= TcParts<CPLX>::kCount / 2;
+  const int im = CPLX ? pt & 1 : 0;
   if (g == 0) {
     if (!tr) { x = a; w = b; y = b; z = c; u = a; v = c; flip = 0; }
     else     { x = b; w = a; y = a; z = c; u = b; v = c; flip = 0; }
@@ -168,19 +188,20 @@ __device__ __forceinline__ TcPart part_of(const TcMaps &m, int g, int pt, int a,
     else     { x = c; w = b; y = b; z = a; u = a; v = c; flip = 1; }
   }
   TcPart p;
-  p.particle = (pt & 1) == 0;
-  if (p.particle) {
-    p.amap = tr ? &m.TaT : &m.TaN;
+  if (!TcParts<CPLX>::hole(pt)) {
+    p.amap = &m.Ta[im][tr];
     p.ax = x;
     p.bmap = pass ? &m.Jp : &m.Vp;
     p.bz = z;
     p.by = y;
+    p.blk = im ? 0 : 1;
   } else {
-    p.amap = pass ? (tr ? &m.JhT : &m.JhN) : (tr ? &m.VhT : &m.VhN);
+    p.amap = pass ? &m.Jh[im][tr] : &m.Vh[im][tr];
     p.ax = w;
     p.bmap = flip ? &m.TpT : &m.TpN;
     p.bz = v;
     p.by = u;
+    p.blk = im ? 1 : 0;
   }
   return p;
 }
@@ -235,6 +256,66 @@ __device__ __forceinline__ double energy_partial(const TcDesc &d, const double *
       value = 3.0 * ((A * U + B * V) + C * W) - (A + (B + C)) * (U + (V + W));
     }
     sum += (2.0 * value / denominator) * fac;
+  }
+  return sum;
+}
+
+// The same for a complex system: the expressions of the complex DFMA kernel.
+// W as planes of real and imaginary parts, cells apart.
+struct TcSinglesZ {
+  const double2 *Vbc, *Vac, *Vab, *ta, *tb, *tc;
+};
+__device__ __forceinline__ double2 zval_z(const double *W, size_t cells, const TcSinglesZ &s, int No,
+                                          int i, int j, int k) {
+  const int x = i + No * j + No * No * k;
+  double2 z = make_double2(W[x], W[cells + x]);
+  z = cadd(z, cmul(s.ta[i], s.Vbc[j + k * No]));
+  z = cadd(z, cmul(s.tb[j], s.Vac[i + k * No]));
+  z = cadd(z, cmul(s.tc[k], s.Vab[i + j * No]));
+  return z;
+}
+__device__ __forceinline__ double energy_partial_z(const TcDesc &d, const double *Tb,
+                                                   const double *Wz, size_t cells,
+                                                   const TcSinglesZ &s, bool distinct,
+                                                   double epsabc, int er) {
+  const int No = d.No;
+  const double2 *epsi = reinterpret_cast<const double2 *>(d.epsi);
+  double sum = 0.0;
+  for (int n = er; n < d.n_triples; n += kEnergyThreads) {
+    const uint32_t pk = d.triples[n];
+    const int i = pk & 0xff, j = (pk >> 8) & 0xff, k = (pk >> 16) & 0xff;
+    const double fac = (j == k ? 0.5 : 1.0) * (i == j ? 0.5 : 1.0);
+    const double2 eijk = cadd(cadd(epsi[i], epsi[j]), epsi[k]);
+    const double2 den = make_double2(epsabc - eijk.x, -eijk.y);
+    auto T = [&](int p, int q, int r) {
+      const int x = p + No * q + No * No * r;
+      return make_double2(Tb[x], -Tb[cells + x]);  // conj(T)
+    };
+    auto Z = [&](int p, int q, int r) { return zval_z(Wz, cells, s, No, p, q, r); };
+    double2 value;
+    if (distinct) {
+      // one permutation after the other: sums over the even (ijk, jki, kij)
+      // and the odd ones, and the products
+      double2 first = make_double2(0.0, 0.0), zs[2], ts[2];
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        const int p = i, q = o ? k : j, r = o ? j : k;
+        const double2 z0 = Z(p, q, r), z1 = Z(q, r, p), z2 = Z(r, p, q);
+        const double2 t0 = T(p, q, r), t1 = T(q, r, p), t2 = T(r, p, q);
+        first = cadd(first, cadd(cmul(t0, z0), cadd(cmul(t1, z1), cmul(t2, z2))));
+        zs[o] = cadd(z0, cadd(z1, z2));
+        ts[o] = cadd(t0, cadd(t1, t2));
+      }
+      const double2 second = cmul(csub(zs[0], cscale(2.0, zs[1])), ts[0]);
+      const double2 third = cmul(csub(zs[1], cscale(2.0, zs[0])), ts[1]);
+      value = cadd(cscale(3.0, first), cadd(second, third));
+    } else {
+      const double2 U = Z(i, j, k), V = Z(j, k, i), W = Z(k, i, j);
+      const double2 A = T(i, j, k), B = T(j, k, i), C = T(k, i, j);
+      value = csub(cscale(3.0, cadd(cadd(cmul(A, U), cmul(B, V)), cmul(C, W))),
+                   cmul(cadd(A, cadd(B, C)), cadd(U, cadd(V, W))));
+    }
+    sum += cdiv_re(cscale(2.0, value), den) * fac;
   }
   return sum;
 }
@@ -301,7 +382,7 @@ __device__ __forceinline__ bool mma_chunk(MmaRole &m, uint32_t d, uint64_t &ad, 
 // All items of a tuple.  The column count P is a template parameter so that
 // every MMA's column offset and instruction descriptor are constants: a warp
 // needs ~5 cycles for each instruction between two MMAs of 50 to 130.
-template <int P>
+template <int P, bool CPLX>
 __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
   constexpr int bufcols = kS * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
   for (int it = 0; it < m.nitems; ++it, ++m.item) {
@@ -319,8 +400,8 @@ __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
     tc_fence_after();
     const uint32_t d = m.tm + buf * bufcols;
     uint32_t acc = 0;
-    for (int pt = 0; pt < 4; ++pt) {
-      const int K = (pt & 1) == 0 ? m.kp : m.kh;
+    for (int pt = 0; pt < TcParts<CPLX>::kCount; ++pt) {
+      const int K = TcParts<CPLX>::hole(pt) ? m.kh : m.kp;
       for (int k0 = 0; k0 < K; k0 += kKChunk) {
         const uint64_t bd = sdesc_sw128(0) + ((m.ring_b + (uint32_t)(m.bs * m.bslot)) >> 4);
         uint64_t ad = 0;
@@ -338,6 +419,7 @@ __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
   return true;
 }
 
+template <bool CPLX>
 __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcArgs g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
@@ -357,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(drain + 1);
   TcSlot *tslot = reinterpret_cast<TcSlot *>(tail + 448);
   double *ta = reinterpret_cast<double *>(tail + 576);
-  double *tb = ta + 64, *tc = tb + 64, *red = tc + 64;
+  double *tb = ta + kT1, *tc = tb + kT1, *red = tc + kT1;  // complex: (re, im) pairs
   static_assert((2 * kMaxSlots + 4 + 2 * kTupleSlots + 5) * 8 + 8 <= 448, "tail");
   static_assert(kTupleSlots * sizeof(TcSlot) <= 128, "tuple slots");
 
@@ -395,7 +477,8 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
   tc_fence_after();
   const uint32_t tmem = *tmem_holder;
   const size_t cells = (size_t)g.lay_cells;
-  longlong2 *planes = g.planes + (size_t)blockIdx.x * 2 * g.lay_pass * 3 * cells;
+  constexpr int kComp = CPLX ? 2 : 1;
+  longlong2 *planes = g.planes + (size_t)blockIdx.x * 2 * g.lay_pass * 3 * kComp * cells;
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
@@ -447,8 +530,8 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
           cur = uniform(lo);
           cur_hi = g.prefix[cur + 1];
           d = g.sys + cur;
-          const int nm = d->use_j ? 10 : 7;
-          for (int i = 0; i < nm; ++i) tensormap_acquire(&d->maps.TaN + i);
+          const int nm = d->use_j ? kMaps : kMapsMain;
+          for (int i = 0; i < nm; ++i) tensormap_acquire(&d->maps.Ta[0][0] + i);
           kp = uniform(d->Nv);
           kh = uniform(d->No);
           rows = uniform(d->rows);
@@ -474,9 +557,10 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       if (stop) break;
       for (int gi = 0; gi < 3 * npass && alive; ++gi)
         for (int mt = 0; mt < ntiles && alive; ++mt)
-          for (int pt = 0; pt < 4 && alive; ++pt) {
-            const TcPart p = part_of(d->maps, gi % 3, pt, s.a, s.b, s.c, gi / 3);
-            const int K = p.particle ? kp : kh;
+          for (int pt = 0; pt < TcParts<CPLX>::kCount && alive; ++pt) {
+            const TcPart p = part_of<CPLX>(d->maps, gi % 3, pt, s.a, s.b, s.c, gi / 3);
+            const int K = TcParts<CPLX>::hole(pt) ? kh : kp;
+            const int c2 = CPLX ? p.blk : p.bz, c3 = CPLX ? p.by * kp + p.bz : p.by;
             for (int k0 = 0; k0 < K && alive; k0 += kKChunk) {
 #pragma unroll 1
               for (int sa = 0; sa < kS; sa += spp) {
@@ -489,8 +573,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
                   // the chunk's B stack comes with its first A slot; its ring
                   // is one chunk deeper than A's, so that slot is free too
                   if (sa == 0)
-                    tma_load_5d(ring_b + (uint32_t)(bs * g.bslot), p.bmap, &afull[st], k0, 0, p.bz,
-                                p.by, 0);
+                    tma_load_5d(ring_b + (uint32_t)(bs * g.bslot), p.bmap, &afull[st], k0, 0, c2, c3, 0);
                   tma_load_4d(ring_a + (uint32_t)(st * g.aslot), p.amap, &afull[st], k0, mt * rows,
                               p.ax, sa);
                 }
@@ -550,15 +633,24 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
         m.spp = uniform(d.spp);
         m.nitems = 3 * (uniform(d.use_j) ? 2 : 1) * ((m.kh * m.kh + m.rows - 1) / m.rows);
       }
-      switch (m.P) {
-        case 8: alive = mma_tuple<8>(m, fresh, status); break;
-        case 16: alive = mma_tuple<16>(m, fresh, status); break;
-        case 24: alive = mma_tuple<24>(m, fresh, status); break;
-        case 32: alive = mma_tuple<32>(m, fresh, status); break;
-        case 40: alive = mma_tuple<40>(m, fresh, status); break;
-        case 48: alive = mma_tuple<48>(m, fresh, status); break;
-        case 56: alive = mma_tuple<56>(m, fresh, status); break;
-        default: alive = mma_tuple<64>(m, fresh, status); break;
+      if constexpr (CPLX) {  // P = 2 round_up(No, 8)
+        switch (m.P) {
+          case 16: alive = mma_tuple<16, true>(m, fresh, status); break;
+          case 32: alive = mma_tuple<32, true>(m, fresh, status); break;
+          case 48: alive = mma_tuple<48, true>(m, fresh, status); break;
+          default: alive = mma_tuple<64, true>(m, fresh, status); break;
+        }
+      } else {
+        switch (m.P) {
+          case 8: alive = mma_tuple<8, false>(m, fresh, status); break;
+          case 16: alive = mma_tuple<16, false>(m, fresh, status); break;
+          case 24: alive = mma_tuple<24, false>(m, fresh, status); break;
+          case 32: alive = mma_tuple<32, false>(m, fresh, status); break;
+          case 40: alive = mma_tuple<40, false>(m, fresh, status); break;
+          case 48: alive = mma_tuple<48, false>(m, fresh, status); break;
+          case 56: alive = mma_tuple<56, false>(m, fresh, status); break;
+          default: alive = mma_tuple<64, false>(m, fresh, status); break;
+        }
       }
     }
     // no MMA outlives this role (after a failed wait some may be in flight)
@@ -591,7 +683,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       ok = wuse == 0 || mbar_wait(&wfree[wb], (wuse - 1) & 1, status, kErrEmpty);
       for (int it = 0; it < 3 * npass * ntiles; ++it, ++item) {
         const int gi = it / ntiles, mt = it - gi * ntiles, grp = gi % 3, pass = gi / 3;
-        longlong2 *plane = planes + (size_t)((wb * g.lay_pass + pass) * 3 + grp) * cells;
+        longlong2 *plane0 = planes + (size_t)((wb * g.lay_pass + pass) * 3 + grp) * kComp * cells;
         const int bb = item & 1, buf = nbuf == 2 ? bb : 0;
         bool okw = ok && alive && mbar_wait(&accf[bb], (item >> 1) & 1, status, kErrAccFull);
         okw = bar_and(1, 128, okw);
@@ -603,13 +695,18 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
         const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + buf * bufcols;
         const int m = mt * rows + l;
         const bool valid = l < rows && m < No2;
-        for (int c0 = 0; c0 < No; c0 += 8) {
+        const int P1 = P / kComp;
+        for (int cc = 0; cc < kComp * No;) {
+          // column block (component) and its next 8 columns
+          const int comp = kComp == 2 && cc >= No ? 1 : 0, c0 = cc - comp * No;
+          cc += min(8, No - c0);
+          longlong2 *plane = plane0 + comp * cells;
           float v[kS][8];
           __syncwarp();
 #pragma unroll
-          for (int L = 0; L < kS; ++L) tmem_ld8(tbase + L * P + c0, v[L]);
+          for (int L = 0; L < kS; ++L) tmem_ld8(tbase + L * P + comp * P1 + c0, v[L]);
           tmem_wait_ld();
-          if (c0 + 8 >= No) {  // everything is read: the accumulator is free
+          if (cc == kComp * No) {  // everything is read: the accumulator is free
             tc_fence_before();
             mbar_arrive(&acce[bb]);
           }
@@ -650,7 +747,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
   } else {
     // ------------------------------------------------ energy (10 warps)
     const int er = ((warp < 4 ? warp - 2 : warp - 6) << 5) | lane;
-    double *wd = g.wd + (size_t)blockIdx.x * g.lay_pass * cells;
+    double *wd = g.wd + (size_t)blockIdx.x * g.lay_pass * kComp * cells;
     for (uint32_t k = 0;; ++k) {
       const int ts = k % kTupleSlots;
       bool ok = mbar_wait(&tfull[ts], (k / kTupleSlots) & 1, status, kErrFull);
@@ -665,18 +762,23 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       // W, Z and the singles in units of a cell's high part (a power of two)
       const double inv = d.tai_sign / d.unit;
       if (er < No) {
-        ta[er] = d.tai[a + er * Nv] * inv;
-        tb[er] = d.tai[b + er * Nv] * inv;
-        tc[er] = d.tai[c + er * Nv] * inv;
+#pragma unroll
+        for (int h = 0; h < kComp; ++h) {
+          ta[kComp * er + h] = d.tai[kComp * (a + er * Nv) + h] * inv;
+          tb[kComp * er + h] = d.tai[kComp * (b + er * Nv) + h] * inv;
+          tc[kComp * er + h] = d.tai[kComp * (c + er * Nv) + h] * inv;
+        }
       }
       const int wb = k & 1;
       ok = mbar_wait(&wfull[wb], (k >> 1) & 1, status, kErrAccFull);
       const uint32_t magic = 0xffffffffu / (uint32_t)No + 1u;  // idx / No = umulhi, idx < 2^18
       const int npass = d.use_j ? 2 : 1;
-      for (int pass = 0; pass < npass; ++pass) {
-        const longlong2 *p0 = planes + (size_t)((wb * g.lay_pass + pass) * 3) * cells;
-        const longlong2 *p1 = p0 + cells, *p2 = p1 + cells;
-        double *W = wd + pass * cells;
+      for (int pc = 0; pc < npass * kComp; ++pc) {
+        const int pass = pc / kComp, comp = pc % kComp;
+        const longlong2 *p0 =
+            planes + (size_t)((wb * g.lay_pass + pass) * 3 * kComp + comp) * cells;
+        const longlong2 *p1 = p0 + kComp * cells, *p2 = p1 + kComp * cells;
+        double *W = wd + pc * cells;
         constexpr int kU = 4;
         for (int i0 = er; i0 < No3; i0 += kU * kEnergyThreads) {
           longlong2 v[kU][3];
@@ -709,17 +811,24 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       int cls = 0;  // src/atrip/Atrip.cxx:640-642
       if (a == b) cls++;
       if (b == c) cls--;
-      const double epsabc = d.epsa[a] + d.epsa[b] + d.epsa[c];
-      TcSinglesCtx sc;
-      sc.Vbc = d.Vhh + ((int64_t)b * Nv + c) * No2;
-      sc.Vac = d.Vhh + ((int64_t)a * Nv + c) * No2;
-      sc.Vab = d.Vhh + ((int64_t)a * Nv + b) * No2;
-      sc.ta = ta;
-      sc.tb = tb;
-      sc.tc = tc;
+      const double epsabc = d.epsa[kComp * a] + d.epsa[kComp * b] + d.epsa[kComp * c];
+      const double *Vbc = d.Vhh + ((int64_t)b * Nv + c) * No2 * kComp;
+      const double *Vac = d.Vhh + ((int64_t)a * Nv + c) * No2 * kComp;
+      const double *Vab = d.Vhh + ((int64_t)a * Nv + b) * No2 * kComp;
       double en[2];
       for (int pass = 0; pass < npass; ++pass) {
-        double sum = ok ? energy_partial(d, wd + pass * cells, wd, sc, cls == 0, epsabc, er) : 0.0;
+        double sum = 0.0;
+        if constexpr (CPLX) {
+          const TcSinglesZ sc = {
+              reinterpret_cast<const double2 *>(Vbc), reinterpret_cast<const double2 *>(Vac),
+              reinterpret_cast<const double2 *>(Vab), reinterpret_cast<const double2 *>(ta),
+              reinterpret_cast<const double2 *>(tb), reinterpret_cast<const double2 *>(tc)};
+          if (ok)
+            sum = energy_partial_z(d, wd + pass * 2 * cells, wd, cells, sc, cls == 0, epsabc, er);
+        } else {
+          const TcSinglesCtx sc = {Vbc, Vac, Vab, ta, tb, tc};
+          if (ok) sum = energy_partial(d, wd + pass * cells, wd, sc, cls == 0, epsabc, er);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (lane == 0) red[er >> 5] = sum;
@@ -781,6 +890,7 @@ struct CutJob {
   int64_t nrows, n1, n2, so, s1, s2, sk;
   int K, Kp, e, neg;
   unsigned int *norms;
+  int nblk = 1, blk = 0;  // dst holds nblk blocks of n2 rows for each of src's: this is block blk
 };
 
 // round(x 2^(63-e)) for |x| <= 127/128 2^e, with integer instructions.
@@ -798,14 +908,14 @@ __device__ __forceinline__ long long fixed63(double x, int e) {
 }
 
 __global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
-  const int64_t plane = j.nrows * j.Kp;
+  const int64_t plane = j.nrows * j.nblk * j.Kp;
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * 8;
   unsigned int best[3] = {0, 0, 0};
   for (int64_t R = blockIdx.x * 8 + (threadIdx.x >> 5); R < j.nrows; R += nw) {
     const int64_t r2 = R % j.n2, t = R / j.n2, r1 = t % j.n1, o = t / j.n1;
     const double *src = j.src + o * j.so + r1 * j.s1 + r2 * j.s2;
-    __nv_bfloat16 *dst = j.dst + R * j.Kp;
+    __nv_bfloat16 *dst = j.dst + ((t * j.nblk + j.blk) * j.n2 + r2) * j.Kp;
     unsigned int nrm[3] = {0, 0, 0};
     for (int k = 2 * lane; k < j.Kp; k += 64) {
       unsigned long long y[2];
@@ -849,6 +959,7 @@ __global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
 // ------------------------------------------------------------------ host
 
 struct TcImpl {
+  int nc = 1;  // doubles per element: 2 for a complex system
   int No = 0, Nv = 0, P = 0, rows = 0, spp = 0, Kp = 0, Kh = 0;
   int eT = 0, eV = 0, eJ = 0;
   double max_t = 0, min_t = 0;  // T: largest element, smallest nonzero slab maximum
@@ -903,6 +1014,11 @@ int map_a(CUtensorMap *m, void *base, const TcImpl &p, int K) {
   return make_map(m, base, 4, d, box);
 }
 int map_b(CUtensorMap *m, void *base, const TcImpl &p, int K) {
+  if (p.nc == 2) {  // (K, r, block, (y,z), slice): two neighbouring column blocks of three
+    const uint64_t d[5] = {(uint64_t)K, (uint64_t)p.No, kBlocksZ, (uint64_t)p.Nv * p.Nv, kS};
+    const uint32_t box[5] = {kKChunk, (uint32_t)p.P / 2, 2, 1, kS};
+    return make_map(m, base, 5, d, box);
+  }
   const uint64_t d[5] = {(uint64_t)K, (uint64_t)p.No, (uint64_t)p.Nv, (uint64_t)p.Nv, kS};
   const uint32_t box[5] = {kKChunk, (uint32_t)p.P, 1, 1, kS};
   return make_map(m, base, 5, d, box);
@@ -956,13 +1072,14 @@ bool alloc_arena(char **p, size_t bytes) {
 
 bool exponent_ok(int e) { return e >= -200 && e <= 200; }
 
-// Bound of |partial sums| of levels 1 and 2 (level 0 is far smaller a
-// count): twice (natural and transposed part) the Cauchy-Schwarz products.
-bool sums_exact(const double *nT, const double *nV, const double *nH, const double *nU) {
+// Bound of |partial sums| of levels 0, 1 and 2: twice (natural and transposed
+// part; four times for a complex system, whose rows meet real and imaginary
+// columns) the Cauchy-Schwarz products.
+bool sums_exact(int nc, const double *nT, const double *nV, const double *nH, const double *nU) {
   for (int L = 0; L < 3; ++L) {
     double b = 0;
     for (int s = 0; s <= L; ++s)
-      b += 2.0 * (std::sqrt(nT[s] * nV[L - s]) + std::sqrt(nH[s] * nU[L - s]));
+      b += 2.0 * nc * (std::sqrt(nT[s] * nV[L - s]) + std::sqrt(nH[s] * nU[L - s]));
     if (!(b < 16777216.0)) return false;
   }
   return true;
@@ -975,27 +1092,61 @@ void max_norms(double *out, const unsigned int *x) {
   for (int s = 0; s < 3; ++s) out[s] = std::max(out[s], (double)x[s]);
 }
 
-// Cut V_pphp / V_hhhp (or the J pair): slices at hN, hT (rows natural and
-// transposed) and vp, scale 2^e shared by both.
-int cut_pair(const TcImpl &p, const double *vht, const double *vpt, int e, __nv_bfloat16 *hN,
-             __nv_bfloat16 *hT, __nv_bfloat16 *vp, DeviceStats *ds, cudaStream_t st,
+// A column operand: its one block, or the three of a complex system, of
+// components comp[] and signs.
+int cut_blocks(const TcImpl &p, CutJob j, const int *comp, const int *neg, cudaStream_t st,
+               int64_t *launches) {
+  const double *src = j.src;
+  j.nblk = p.nc == 2 ? kBlocksZ : 1;
+  for (int b = 0; b < j.nblk; ++b) {
+    j.blk = b;
+    j.src = src + comp[b];
+    j.neg = neg[b];
+    ATRIP_CUDA_TRY(cut(j, st));
+    *launches += 1;
+  }
+  return ATRIP_OK;
+}
+
+// A row operand, natural and transposed rows (r1 and r2 exchanged), one
+// component after the other at dst[].
+int cut_rows(const TcImpl &p, CutJob j, __nv_bfloat16 *const *dst, cudaStream_t st,
              int64_t *launches) {
-  const int64_t No = p.No, Nv = p.Nv, No2 = No * No;
+  const double *src = j.src;
+  for (int c = 0; c < p.nc; ++c)
+    for (int tr = 0; tr < 2; ++tr) {
+      j.src = src + c;
+      j.dst = dst[2 * c + tr];
+      ATRIP_CUDA_TRY(cut(j, st));
+      std::swap(j.s1, j.s2);
+      *launches += 1;
+    }
+  return ATRIP_OK;
+}
+
+constexpr int kCompV[kBlocksZ] = {1, 0, 1}, kNegV[kBlocksZ] = {1, 0, 0};
+constexpr int kCompT[kBlocksZ] = {0, 1, 0}, kNegT[kBlocksZ] = {1, 1, 0};
+constexpr int kReal[1] = {0}, kPos[1] = {0}, kNeg[1] = {1};
+
+// Cut V_pphp / V_hhhp (or the J pair), scale 2^e shared by both.
+int cut_pair(const TcImpl &p, const double *vht, const double *vpt, int e,
+             __nv_bfloat16 *const *vh, __nv_bfloat16 *vp, DeviceStats *ds, cudaStream_t st,
+             int64_t *launches) {
+  const int64_t No = p.No, Nv = p.Nv, No2 = No * No, nc = p.nc;
   CutJob j;
   j.e = e;
   j.neg = 0;
-  j.src = vht; j.dst = hN; j.nrows = Nv * No2; j.n1 = No; j.n2 = No;
-  j.so = No2 * No; j.s1 = No2; j.s2 = No; j.sk = 1; j.K = p.No; j.Kp = p.Kh;
+  j.src = vht; j.nrows = Nv * No2; j.n1 = No; j.n2 = No;
+  j.so = No2 * No * nc; j.s1 = No2 * nc; j.s2 = No * nc; j.sk = nc; j.K = p.No; j.Kp = p.Kh;
   j.norms = ds->n[4];
-  ATRIP_CUDA_TRY(cut(j, st));
-  j.dst = hT; j.s1 = No; j.s2 = No2;
-  ATRIP_CUDA_TRY(cut(j, st));
+  const int rc = cut_rows(p, j, vh, st, launches);
+  if (rc != ATRIP_OK) return rc;
   j.src = vpt; j.dst = vp; j.nrows = Nv * Nv * No; j.n1 = Nv; j.n2 = No;
-  j.so = Nv * No * Nv; j.s1 = No * Nv; j.s2 = Nv; j.sk = 1; j.K = p.Nv; j.Kp = p.Kp;
+  j.so = Nv * No * Nv * nc; j.s1 = No * Nv * nc; j.s2 = Nv * nc; j.sk = nc;
+  j.K = p.Nv; j.Kp = p.Kp;
   j.norms = ds->n[5];
-  ATRIP_CUDA_TRY(cut(j, st));
-  *launches += 3;
-  return ATRIP_OK;
+  return nc == 2 ? cut_blocks(p, j, kCompV, kNegV, st, launches)
+                 : cut_blocks(p, j, kReal, kPos, st, launches);
 }
 
 void free_impl(TcImpl *p) {
@@ -1010,26 +1161,28 @@ struct ScopedDevice {  // device allocation freed on scope exit
   ~ScopedDevice() { cudaFree(p); }
 };
 
-int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStream_t st,
-                 int64_t *launches) {
+int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cplx,
+                 cudaStream_t st, int64_t *launches) {
   auto *p = new TcImpl();
   s.impl = p;
+  p->nc = cplx ? 2 : 1;
   p->No = No_;
   p->Nv = Nv_;
-  p->P = (No_ + 7) / 8 * 8;
+  p->P = p->nc * ((No_ + 7) / 8 * 8);
   // rows of an item: the No^2 rows in equal shares of at most 128
   const int nt = (No_ * No_ + 127) / 128;
   p->rows = ((No_ * No_ + nt - 1) / nt + 7) / 8 * 8;
-  // slices per copy (a ring slot): up to 32 KB.  A role's warp needs ~200 cycles for a wait and a signal whatever the
-  // size, so a slot should hold several MMAs' work
+  // slices per copy (a ring slot): up to 32 KB.  A role's warp needs ~200
+  // cycles for a wait and a signal whatever the size, so a slot should hold
+  // several MMAs' work
   p->spp = p->rows > 64 ? 2 : 4;
   p->Kp = (Nv_ + kKChunk - 1) / kKChunk * kKChunk;
   p->Kh = kKChunk;
-  const int64_t No = No_, Nv = Nv_, No2 = No * No;
+  const int64_t No = No_, Nv = Nv_, No2 = No * No, nc = p->nc, nblk = cplx ? kBlocksZ : 1;
   const size_t nTa = up((size_t)2 * kS * Nv * No2 * p->Kp), nVh = up((size_t)2 * kS * Nv * No2 * p->Kh),
-               nVp = up((size_t)2 * kS * Nv * Nv * No * p->Kp),
-               nTp = up((size_t)2 * kS * Nv * Nv * No * p->Kh);
-  if (!alloc_arena(&p->arena, 2 * nTa + 2 * nVh + nVp + 2 * nTp)) return ATRIP_OK;
+               nVp = up((size_t)2 * kS * Nv * Nv * No * nblk * p->Kp),
+               nTp = up((size_t)2 * kS * Nv * Nv * No * nblk * p->Kh);
+  if (!alloc_arena(&p->arena, 2 * nc * (nTa + nVh) + nVp + 2 * nTp)) return ATRIP_OK;
   ScopedDevice tmp;
   ATRIP_CUDA_TRY(cudaMalloc(&tmp.p, sizeof(DeviceStats)));
   auto *ds = static_cast<DeviceStats *>(tmp.p);
@@ -1037,10 +1190,10 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStre
   std::memset(&h, 0, sizeof(h));
   for (auto &m : h.m) m[1] = ~0ull;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(ds, &h, sizeof(h), cudaMemcpyHostToDevice, st));
-  ATRIP_CUDA_TRY(slab_max(dt.Ta, Nv, No2 * Nv, ds->m[0], st));
-  ATRIP_CUDA_TRY(slab_max(dt.Tp, Nv * Nv, No2, ds->m[1], st));
-  ATRIP_CUDA_TRY(slab_max(dt.Vpt, Nv * Nv, No * Nv, ds->m[2], st));
-  ATRIP_CUDA_TRY(slab_max(dt.Vht, Nv, No2 * No, ds->m[3], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Ta, Nv, No2 * Nv * nc, ds->m[0], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Tp, Nv * Nv, No2 * nc, ds->m[1], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Vpt, Nv * Nv, No * Nv * nc, ds->m[2], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Vht, Nv, No2 * No * nc, ds->m[3], st));
   *launches += 4;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1062,29 +1215,29 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStre
     q += n;
     return reinterpret_cast<__nv_bfloat16 *>(r);
   };
-  __nv_bfloat16 *TaN = take(nTa), *TaT = take(nTa), *VhN = take(nVh), *VhT = take(nVh),
-                *Vp = take(nVp), *TpN = take(nTp), *TpT = take(nTp);
+  __nv_bfloat16 *Ta[4], *Vh[4];
+  for (int i = 0; i < 2 * nc; ++i) Ta[i] = take(nTa);
+  for (int i = 0; i < 2 * nc; ++i) Vh[i] = take(nVh);
+  __nv_bfloat16 *Vp = take(nVp), *TpN = take(nTp), *TpT = take(nTp);
   CutJob j;
   j.e = p->eT;
   j.neg = 0;
   // rows (p,q) of T_x over E, p fastest and q fastest
-  j.src = dt.Ta; j.dst = TaN; j.nrows = Nv * No2; j.n1 = No; j.n2 = No;
-  j.so = No2 * Nv; j.s1 = No * Nv; j.s2 = Nv; j.sk = 1; j.K = Nv_; j.Kp = p->Kp;
+  j.src = dt.Ta; j.nrows = Nv * No2; j.n1 = No; j.n2 = No;
+  j.so = No2 * Nv * nc; j.s1 = No * Nv * nc; j.s2 = Nv * nc; j.sk = nc; j.K = Nv_; j.Kp = p->Kp;
   j.norms = ds->n[0];
-  ATRIP_CUDA_TRY(cut(j, st));
-  j.dst = TaT; j.s1 = Nv; j.s2 = No * Nv;
-  ATRIP_CUDA_TRY(cut(j, st));
+  int rc = cut_rows(*p, j, Ta, st, launches);
+  if (rc != ATRIP_OK) return rc;
   // columns r of -T[u,v,L,r] and -T[u,v,r,L] over L
-  j.neg = 1;
+  const int *comp = cplx ? kCompT : kReal, *neg = cplx ? kNegT : kNeg;
   j.src = dt.Tp; j.dst = TpN; j.nrows = Nv * Nv * No; j.n1 = Nv; j.n2 = No;
-  j.so = Nv * No2; j.s1 = No2; j.s2 = No; j.sk = 1; j.K = No_; j.Kp = p->Kh;
+  j.so = Nv * No2 * nc; j.s1 = No2 * nc; j.s2 = No * nc; j.sk = nc; j.K = No_; j.Kp = p->Kh;
   j.norms = ds->n[1];
-  ATRIP_CUDA_TRY(cut(j, st));
-  j.dst = TpT; j.s2 = 1; j.sk = No;
+  if ((rc = cut_blocks(*p, j, comp, neg, st, launches)) != ATRIP_OK) return rc;
+  j.dst = TpT; j.s2 = nc; j.sk = No * nc;
   j.norms = ds->n[2];
-  ATRIP_CUDA_TRY(cut(j, st));
-  *launches += 4;
-  int rc = cut_pair(*p, dt.Vht, dt.Vpt, p->eV, VhN, VhT, Vp, ds, st, launches);
+  if ((rc = cut_blocks(*p, j, comp, neg, st, launches)) != ATRIP_OK) return rc;
+  rc = cut_pair(*p, dt.Vht, dt.Vpt, p->eV, Vh, Vp, ds, st, launches);
   if (rc != ATRIP_OK) return rc;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1094,15 +1247,18 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStre
   double nH[3], nV[3];
   set_norms(nH, h.n[4]);
   set_norms(nV, h.n[5]);
-  if (!sums_exact(p->nT, nV, nH, p->nU)) return ATRIP_OK;
+  if (!sums_exact(p->nc, p->nT, nV, nH, p->nU)) return ATRIP_OK;
 
-  if ((rc = map_a(&p->maps.TaN, TaN, *p, p->Kp)) || (rc = map_a(&p->maps.TaT, TaT, *p, p->Kp)) ||
-      (rc = map_a(&p->maps.VhN, VhN, *p, p->Kh)) || (rc = map_a(&p->maps.VhT, VhT, *p, p->Kh)) ||
-      (rc = map_b(&p->maps.Vp, Vp, *p, p->Kp)) || (rc = map_b(&p->maps.TpN, TpN, *p, p->Kh)) ||
+  for (int i = 0; i < 4; ++i) {  // [component][row order]; a real system's twice
+    const int k = i % (2 * nc);
+    if ((rc = map_a(&p->maps.Ta[i / 2][i % 2], Ta[k], *p, p->Kp)) ||
+        (rc = map_a(&p->maps.Vh[i / 2][i % 2], Vh[k], *p, p->Kh)))
+      return rc;
+  }
+  if ((rc = map_b(&p->maps.Vp, Vp, *p, p->Kp)) || (rc = map_b(&p->maps.TpN, TpN, *p, p->Kh)) ||
       (rc = map_b(&p->maps.TpT, TpT, *p, p->Kh)))
     return rc;
-  p->maps.JhN = p->maps.VhN;
-  p->maps.JhT = p->maps.VhT;
+  std::memcpy(p->maps.Jh, p->maps.Vh, sizeof(p->maps.Jh));
   p->maps.Jp = p->maps.Vp;
   s.usable = true;
   return ATRIP_OK;
@@ -1110,9 +1266,11 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, cudaStre
 
 int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *launches) {
   auto *p = static_cast<TcImpl *>(s.impl);
-  const int64_t No = p->No, Nv = p->Nv, No2 = No * No;
-  const size_t nVh = up((size_t)2 * kS * Nv * No2 * p->Kh), nVp = up((size_t)2 * kS * Nv * Nv * No * p->Kp);
-  if (!alloc_arena(&p->arena_j, 2 * nVh + nVp)) return ATRIP_OK;
+  const int64_t No = p->No, Nv = p->Nv, No2 = No * No, nc = p->nc;
+  const int64_t nblk = nc == 2 ? kBlocksZ : 1;
+  const size_t nVh = up((size_t)2 * kS * Nv * No2 * p->Kh),
+               nVp = up((size_t)2 * kS * Nv * Nv * No * nblk * p->Kp);
+  if (!alloc_arena(&p->arena_j, 2 * nc * nVh + nVp)) return ATRIP_OK;
   ScopedDevice tmp;
   ATRIP_CUDA_TRY(cudaMalloc(&tmp.p, sizeof(DeviceStats)));
   auto *ds = static_cast<DeviceStats *>(tmp.p);
@@ -1120,8 +1278,8 @@ int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *lau
   std::memset(&h, 0, sizeof(h));
   for (auto &m : h.m) m[1] = ~0ull;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(ds, &h, sizeof(h), cudaMemcpyHostToDevice, st));
-  ATRIP_CUDA_TRY(slab_max(dt.Jpt, Nv * Nv, No * Nv, ds->m[2], st));
-  ATRIP_CUDA_TRY(slab_max(dt.Jht, Nv, No2 * No, ds->m[3], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Jpt, Nv * Nv, No * Nv * nc, ds->m[2], st));
+  ATRIP_CUDA_TRY(slab_max(dt.Jht, Nv, No2 * No * nc, ds->m[3], st));
   *launches += 2;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1133,20 +1291,20 @@ int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *lau
       std::log2(p->max_t / p->min_t) + std::log2(max_v / min_v) > kRangeBits)
     return ATRIP_OK;
   p->unit_j = std::ldexp(1.0, p->eT + p->eJ - 14 - 24);
-  auto *hN = reinterpret_cast<__nv_bfloat16 *>(p->arena_j);
-  auto *hT = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + nVh);
-  auto *vp = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + 2 * nVh);
-  int rc = cut_pair(*p, dt.Jht, dt.Jpt, p->eJ, hN, hT, vp, ds, st, launches);
+  __nv_bfloat16 *vh[4];
+  for (int i = 0; i < 2 * nc; ++i) vh[i] = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + i * nVh);
+  auto *vp = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + 2 * nc * nVh);
+  int rc = cut_pair(*p, dt.Jht, dt.Jpt, p->eJ, vh, vp, ds, st, launches);
   if (rc != ATRIP_OK) return rc;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
   double nH[3], nV[3];
   set_norms(nH, h.n[4]);
   set_norms(nV, h.n[5]);
-  if (!sums_exact(p->nT, nV, nH, p->nU)) return ATRIP_OK;
-  if ((rc = map_a(&p->maps.JhN, hN, *p, p->Kh)) || (rc = map_a(&p->maps.JhT, hT, *p, p->Kh)) ||
-      (rc = map_b(&p->maps.Jp, vp, *p, p->Kp)))
-    return rc;
+  if (!sums_exact(p->nc, p->nT, nV, nH, p->nU)) return ATRIP_OK;
+  for (int i = 0; i < 4; ++i)
+    if ((rc = map_a(&p->maps.Jh[i / 2][i % 2], vh[i % (2 * nc)], *p, p->Kh))) return rc;
+  if ((rc = map_b(&p->maps.Jp, vp, *p, p->Kp))) return rc;
   s.usable_j = true;
   return ATRIP_OK;
 }
@@ -1173,7 +1331,9 @@ void tc_free(TcState &s) {
 // allocations, launches and tensor maps the first time, about what the DFMA
 // kernel needs for 1e9 FLOPs at these sizes (No=4/Nv=12, 4.5e6: 0.1 ms).
 bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx) {
-  return !cplx && No >= 2 && (double)n_tuples * 12.0 * No * No * No * (No + Nv) >= 1e9;
+  // complex: the columns of both components of 8 levels fill TMEM at No = 32
+  const double flops = (cplx ? 4.0 : 1.0) * (double)n_tuples * 12.0 * No * No * No * (No + Nv);
+  return No >= 2 && (!cplx || No <= 32) && flops >= 1e9;
 }
 
 // Side of the (a,b,c) blocks tuples are processed in, 0 = list order.  In list
@@ -1186,11 +1346,11 @@ int tc_tuple_block(int No, int Nv, int sm_count) {
   return slab * std::min(sm_count, Nv) > 64e6 ? 6 : 0;
 }
 
-int tc_prepare(TcState &s, const DeviceTensors &dt, int No, int Nv, bool use_j, cudaStream_t st,
-               int64_t *launches, bool *usable) {
+int tc_prepare(TcState &s, const DeviceTensors &dt, int No, int Nv, bool cplx, bool use_j,
+               cudaStream_t st, int64_t *launches, bool *usable) {
   *usable = false;
   if (!s.tried) {
-    const int rc = prepare_main(s, dt, No, Nv, st, launches);
+    const int rc = prepare_main(s, dt, No, Nv, cplx, st, launches);
     if (rc != ATRIP_OK || !s.usable) drop_impl(s);
     s.generation++;
     if (rc != ATRIP_OK) return rc;
@@ -1250,6 +1410,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   b.lay_no = 0;
   b.lay_pass = 1;
   b.aslot = 0;
+  b.nc = 1;
   b.h_prefix[0] = 0;
   for (int k = 0; k < n; ++k) {
     const TcSystem &m = sys[k];
@@ -1282,6 +1443,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     d.use_j = m.use_j ? 1 : 0;
     h[k] = d;
     P = std::max(P, p->P);
+    b.nc = p->nc;  // the same for all: a batch holds real systems
     b.aslot = std::max(b.aslot, p->spp * p->rows * 128);
     spp = std::max(spp, p->spp);
     b.lay_no = std::max(b.lay_no, m.No);
@@ -1306,7 +1468,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     return ATRIP_ERR_UNSUPPORTED;
   }
   b.smem = 1024 + (size_t)b.nslots * b.aslot + (size_t)b.nbslots * b.bslot + kTailBytes;
-  const size_t per_cta = ((size_t)2 * 3 * 16 + 8) * b.lay_pass * b.lay_cells;
+  const size_t per_cta = ((size_t)2 * 3 * 16 + 8) * b.nc * b.lay_pass * b.lay_cells;
   const size_t need = per_cta * std::max(b.grid, 1);
   if (need > b.planes_bytes) {
     cudaFree(b.planes);
@@ -1339,16 +1501,17 @@ int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st
   a.flags = b.d_flags;
   a.planes = static_cast<longlong2 *>(b.planes);
   a.wd = reinterpret_cast<double *>(static_cast<char *>(b.planes) +
-                                    (size_t)b.grid * 2 * 3 * 16 * b.lay_pass * b.lay_cells);
+                                    (size_t)b.grid * 2 * 3 * 16 * b.nc * b.lay_pass * b.lay_cells);
   a.lay_cells = b.lay_cells;
   a.lay_pass = b.lay_pass;
   a.nslots = b.nslots;
   a.nbslots = b.nbslots;
   a.aslot = b.aslot;
   a.bslot = b.bslot;
-  ATRIP_CUDA_TRY(cudaFuncSetAttribute(triples_fp64_tc_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem));
-  triples_fp64_tc_kernel<<<b.grid, kThreads, b.smem, st>>>(a);
+  auto kern = b.nc == 2 ? triples_fp64_tc_kernel<true> : triples_fp64_tc_kernel<false>;
+  ATRIP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)b.smem));
+  kern<<<b.grid, kThreads, b.smem, st>>>(a);
   ATRIP_CUDA_TRY(cudaGetLastError());
   *launches += 1;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(b.h_flags, b.d_flags, sizeof(int) * (b.n + 1),

@@ -15,8 +15,8 @@ NAMES = ("epsi", "epsa", "Tai", "Tabij", "Vabij", "Vijka", "Vabci")
 DFMA_LAUNCHES = 3  # the kernel and the two stages of the energy sum
 
 
-def _ctx(d, j=False):
-    ctx = capi.Context(d["No"], d["Nv"], 0)
+def _ctx(d, j=False, field="real"):
+    ctx = capi.Context(d["No"], d["Nv"], 0, field=field)
     for n in NAMES + (("Jijka", "Jabci") if j else ()):
         ctx.upload(n, d[n])
     return ctx
@@ -59,3 +59,40 @@ def test_matches_dfma_and_oracle(No, Nv, j):
         pr = oracle.Problem(d)
         o = oracle.tuple_energies(pr, 0, 12)[0]
         assert np.max(np.abs(e[:12] - o)) <= K * 2.0 ** -52 * np.max(np.abs(f))
+
+
+# complex: two column blocks of No rounded up to 8, products of K = 4 (Nv + No)
+# real terms each; complex orbital energies
+@pytest.mark.parametrize("No,Nv,j", [(5, 48, True), (8, 33, False), (9, 30, True), (13, 26, False),
+                                     (17, 21, True), (24, 16, False), (32, 12, True)])
+def test_complex_matches_dfma_and_oracle(No, Nv, j):
+    d = synth.make_inputs(No, Nv, 12, with_j=j, field="complex", eps_imag=0.05)
+    n = min(synth.n_tuples(Nv), 500)
+    with _ctx(d, j, "complex") as ctx:
+        r, (e, ect), (f, fct) = _both(ctx, max_iterations=n - 1, use_j=j, ijkabc=True)
+        assert r.kernel_launches > DFMA_LAUNCHES
+        K = 4 * (Nv + No)
+        _close(e, f, K)
+        _close(ect, fct, K)
+        o = oracle.tuple_energies(oracle.Problem(d), 0, 8, ijkabc=True)[0]
+        assert np.max(np.abs(e[:8] - o)) <= K * 2.0 ** -52 * np.max(np.abs(f))
+
+
+# data the exact sums cannot hold runs on the DFMA kernel, with its result
+@pytest.mark.parametrize("spoil", ["inf", "range", "constant"])
+def test_data_rules(spoil):
+    d = synth.make_inputs(8, 40, 13)
+    if spoil == "inf":
+        d["Vabci"][3, 4, 5, 6] = np.inf
+    elif spoil == "range":
+        d["Vabci"][:, 7] *= 2.0 ** -20
+    else:  # every level sum coherent
+        d["Tabij"][:] = 1.0 / 3.0
+        d["Vabci"][:] = 1.0 / 3.0
+    with _ctx(d) as ctx:
+        r = ctx.run(form="fp64", max_iterations=199)
+        e, _ = ctx.tuple_energies(0, 200)
+        ctx.set_tuning(fp64_tile_rows=64)
+        ctx.run(form="fp64", max_iterations=199)
+        f, _ = ctx.tuple_energies(0, 200)
+    np.testing.assert_array_equal(e, f)
