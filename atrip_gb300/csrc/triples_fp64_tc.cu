@@ -64,6 +64,7 @@
 #include <string>
 
 #include "complex.cuh"
+#include "digits.cuh"
 #include "engine.cuh"
 #include "fp64_tc.cuh"
 #include "sm100.cuh"
@@ -893,20 +894,6 @@ struct CutJob {
   int nblk = 1, blk = 0;  // dst holds nblk blocks of n2 rows for each of src's: this is block blk
 };
 
-// round(x 2^(63-e)) for |x| <= 127/128 2^e, with integer instructions.
-__device__ __forceinline__ long long fixed63(double x, int e) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int ex = (int)((b >> 52) & 0x7ff);
-  if (ex == 0) return 0;  // zero or subnormal: below 2^(e-64) for any e accepted
-  const long long m = (long long)((b & 0xfffffffffffffull) | 0x10000000000000ull);
-  const int sh = ex - 1075 + 63 - e;  // <= 10
-  long long v;
-  if (sh >= 0) v = m << sh;
-  else if (sh < -54) v = 0;
-  else v = (m + (1ll << (-sh - 1))) >> -sh;
-  return (long long)b < 0 ? -v : v;
-}
-
 __global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
   const int64_t plane = j.nrows * j.nblk * j.Kp;
   const int lane = threadIdx.x & 31;
@@ -923,19 +910,14 @@ __global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
       for (int h = 0; h < 2; ++h) {
         long long X = k + h < j.K ? fixed63(src[(k + h) * j.sk], j.e) : 0;
         if (j.neg) X = -X;
-        // bytes of X plus 128 in each of the seven lower ones: digit + 128
-        y[h] = (unsigned long long)X + 0x0080808080808080ull;
+        y[h] = biased(X);
       }
 #pragma unroll
       for (int s = 0; s < kS; ++s) {
         float q[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          if (s == 0)
-            q[h] = (float)(int)((long long)y[h] >> 56);
-          else
-            q[h] = __uint_as_float(0x4B000000u | (uint32_t)((y[h] >> (56 - 8 * s)) & 0xff)) -
-                   8388736.f;
+          q[h] = digit(y[h], s);
           if (s < 3) nrm[s] += (unsigned int)(int)(q[h] * q[h]);
         }
         *reinterpret_cast<__nv_bfloat162 *>(dst + s * plane + k) =

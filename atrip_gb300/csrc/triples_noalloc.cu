@@ -22,12 +22,24 @@
 // is the same as the FP64 form of atrip_gpu_run (six fused particle+hole
 // contractions written into W at their index permutations, Z = W + singles,
 // the get_energy_{distinct,same} terms of src/atrip/Equations.cxx:101-238).
+//
+// Two kernels do it.  The tensor-core one forms W as triples_fp64_tc.cu does,
+// from exact products of 8-bit digit slices, but has no memory for slices: it
+// cuts each K chunk of the caller's tensors into shared memory as it goes.
+// The other runs on FP64 instructions.  A call cannot ask the device and wait,
+// so where the first applies by its sizes both are queued: a few small kernels
+// examine the operands (largest elements of the tensors and of their slabs),
+// the tensor-core kernel runs if they allow exact sums, and the other one
+// returns at once if that succeeded.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "atrip_gb300.h"
+#include "digits.cuh"
 #include "engine.cuh"
+#include "sm100.cuh"
 
 namespace atrip_gb300 {
 namespace noalloc {
@@ -42,6 +54,18 @@ constexpr int kMT = 64;
 constexpr int kKC = 32;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
+
+// The first bytes of the scratch, cleared by every call.
+struct Header {
+  unsigned long long cursor;     // FP64-instruction kernel
+  unsigned long long tc_cursor;  // tensor-core kernel
+  int tc_ok;                     // the operands allow exact sums
+  int tc_overflow;               // a level sum left its exact range
+  int tc_status;                 // a bounded wait gave up
+  int e_t, e_v, e_j;             // exponents of the digit grids
+  unsigned long long vh_max[2], vh_min_not[2];  // V_hhhp, J_hhhp slabs: max, ~min (0: none)
+};
+static_assert(sizeof(Header) <= kHeaderBytes, "header");
 
 struct Args {
   int No, Nv;
@@ -227,9 +251,12 @@ __device__ double block_sum(double v, Smem &sm, int slot) {
 template <int NC>
 __global__ void __launch_bounds__(kThreads) triples_noalloc_kernel(Args g) {
   __shared__ Smem sm;
-  unsigned long long *cursor = reinterpret_cast<unsigned long long *>(g.scratch);
+  Header *h = reinterpret_cast<Header *>(g.scratch);
+  if (h->tc_ok && !h->tc_overflow && !h->tc_status) return;  // the tensor-core kernel did it
+  unsigned long long *cursor = &h->cursor;
   const int64_t No3 = (int64_t)g.No * g.No * g.No;
-  double *Wv = reinterpret_cast<double *>(g.scratch + kWorkspaceOffset) + blockIdx.x * 2 * No3;
+  double *Wv = reinterpret_cast<double *>(g.scratch + kWorkspaceOffset) +
+               blockIdx.x * (g.use_j ? 2 : 1) * No3;
   double *Wj = Wv + No3;
   const int64_t n = g.t_end - g.t_begin;
   for (;;) {
@@ -268,6 +295,490 @@ __global__ void __launch_bounds__(kThreads) triples_noalloc_kernel(Args g) {
     __syncthreads();
   }
 }
+
+// ------------------------------------------------- tensor-core kernel
+
+namespace tc {
+using namespace sm100;
+constexpr int kThreads = 512;
+constexpr int kS = 8;           // digit slices and levels
+constexpr int kChunk = 64;      // K elements per 128-byte row
+constexpr int kATile = 128 * 128;
+// K contributions an accumulator may hold: levels 0..2 stay below 2^24
+// whatever the digits are, 3 K 2^14 <= 2^24.  Longer sums are drained into W
+// in pieces.
+constexpr int kMaxK = 341;
+constexpr double kRangeBits = 8.0;
+
+__device__ __forceinline__ unsigned long long magnitude(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+
+// out[s] = largest magnitude of slab s of x[s + nslab c], c < count.
+__global__ void column_max(const double *__restrict__ x, int64_t nslab, int64_t count,
+                           unsigned long long *__restrict__ out) {
+  const int64_t s = blockIdx.x * 256ll + threadIdx.x;
+  if (s >= nslab) return;
+  unsigned long long m = 0;
+#pragma unroll 8
+  for (int64_t c = blockIdx.y; c < count; c += gridDim.y) {
+    const unsigned long long b = magnitude(x[s + nslab * c]);
+    m = b > m ? b : m;
+  }
+  atomicMax(&out[s], m);
+}
+
+// Largest magnitudes of contiguous slabs of n elements into the header.
+__global__ void slab_max(const double *__restrict__ x, int64_t slabs, int64_t n, Header *h,
+                         int which) {
+  __shared__ unsigned long long sh[8];
+  for (int64_t s = blockIdx.x; s < slabs; s += gridDim.x) {
+    unsigned long long m = 0;
+    for (int64_t i = threadIdx.x; i < n; i += 256) {
+      const unsigned long long b = magnitude(x[s * n + i]);
+      m = b > m ? b : m;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
+      m = v > m ? v : m;
+    }
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) m = sh[w] > m ? sh[w] : m;
+      atomicMax(&h->vh_max[which], m);
+      if (m != 0) atomicMax(&h->vh_min_not[which], ~m);
+    }
+    __syncthreads();
+  }
+}
+
+// Smallest e with x <= 127/128 2^e; false if the exponent is out of hand.
+__device__ bool grid_exponent(unsigned long long bits, int *e) {
+  if (bits == 0 || bits >= 0x7ff0000000000000ull) return false;
+  const double x = __longlong_as_double((long long)bits);
+  int k = ilogb(x) + 1;
+  if (x > ldexp(127.0 / 128.0, k)) ++k;
+  *e = k;
+  return k >= -200 && k <= 200;
+}
+
+// One block: the verdict from the slab maxima (T_uv, V_yz and J_yz pair
+// slabs at slabs[0 .. 3 nvnv)); the rules of triples_fp64_tc.cu.
+__global__ void decide(const unsigned long long *__restrict__ slabs, int64_t nvnv, int use_j,
+                       Header *h) {
+  __shared__ unsigned long long mx[3], mn_not[3];
+  if (threadIdx.x < 3) mx[threadIdx.x] = mn_not[threadIdx.x] = 0;
+  __syncthreads();
+  for (int t = 0; t < (use_j ? 3 : 2); ++t) {
+    unsigned long long a = 0, b = 0;
+    for (int64_t i = threadIdx.x; i < nvnv; i += blockDim.x) {
+      const unsigned long long m = slabs[t * nvnv + i];
+      a = m > a ? m : a;
+      if (m != 0 && ~m > b) b = ~m;
+    }
+    atomicMax(&mx[t], a);
+    atomicMax(&mn_not[t], b);
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  bool ok = true;
+  double range[3] = {0.0, 0.0, 0.0};
+  int e[3] = {0, 0, 0};
+  for (int t = 0; t < (use_j ? 3 : 2); ++t) {
+    unsigned long long m = mx[t], n = mn_not[t];
+    if (t > 0) {  // V_pphp and V_hhhp share a grid
+      m = max(m, h->vh_max[t - 1]);
+      n = max(n, h->vh_min_not[t - 1]);
+    }
+    ok = ok && grid_exponent(m, &e[t]);
+    if (ok)
+      range[t] = log2(__longlong_as_double((long long)m) / __longlong_as_double((long long)~n));
+  }
+  ok = ok && range[0] + range[1] <= kRangeBits && range[0] + range[2] <= kRangeBits;
+  h->e_t = e[0];
+  h->e_v = e[1];
+  h->e_j = e[2];
+  h->tc_ok = ok ? 1 : 0;
+}
+
+struct Tail {
+  uint64_t bar;
+  uint32_t tmem;
+  long long slot;
+  int abc[3];
+  double ta[64], tb[64], tc[64];
+  double red[kThreads / 32];
+};
+
+__device__ __forceinline__ double i64_to_f64(long long n) {  // |n| < 2^51
+  return __longlong_as_double(0x4338000000000000ll + n) - 6755399441055744.0;
+}
+
+// Four rows of digits at a time: the loads of all of them go out first.
+template <class Load>
+__device__ __forceinline__ void cut_rows(unsigned char *tile, int pitch, int row0, int nrows,
+                                         int e, int k0, int K, Load load) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int m0 = warp; m0 < nrows; m0 += 64) {
+    double x[4][2];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = m0 + 16 * u, k = k0 + 2 * lane + h;
+        x[u][h] = m < nrows && k < K ? load(m, k) : 0.0;
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int m = m0 + 16 * u;
+      if (m >= nrows) break;
+      const unsigned long long y0 = biased(fixed63(x[u][0], e)), y1 = biased(fixed63(x[u][1], e));
+#pragma unroll
+      for (int s = 0; s < kS; ++s) {
+        // 128-byte rows, their 16-byte groups permuted by the row (SW128)
+        const int row = row0 + m;
+        *reinterpret_cast<__nv_bfloat162 *>(tile + s * pitch + row * 128 +
+                                            ((lane * 4) ^ ((row & 7) << 4))) =
+            __floats2bfloat162_rn(digit(y0, s), digit(y1, s));
+      }
+    }
+  }
+}
+
+// W (+)= the three groups of one pass (V: pass 0, J: pass 1).
+struct Pass {
+  const double *Vh, *Vp;
+  int e;
+  double unit;
+  double *W;
+};
+
+__device__ bool build_w(const Args &g, Header *h, Tail &t, unsigned char *At, unsigned char *Bt,
+                        const Pass &ps, int a, int b, int c, uint32_t &phase, uint32_t &over) {
+  const int No = g.No, No2 = No * No, P = (No + 7) / 8 * 8;
+  const int64_t Nv = g.Nv, NvNv = Nv * Nv;
+  const int nt = (No2 + 127) / 128, rows = ((No2 + nt - 1) / nt + 7) / 8 * 8;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  for (int grp = 0; grp < 3; ++grp)
+    for (int mt = 0; mt < nt; ++mt) {
+      int held = 0;         // K in the accumulator
+      bool first = grp == 0;  // the first piece of the first group stores W
+      for (int pt = 0; pt < 4; ++pt) {
+        const bool tr = pt >= 2, hole = pt & 1;
+        int x, w, y, z, u, v, flip;
+        if (grp == 0) {
+          if (!tr) { x = a; w = b; y = b; z = c; u = a; v = c; flip = 0; }
+          else     { x = b; w = a; y = a; z = c; u = b; v = c; flip = 0; }
+        } else if (grp == 1) {
+          if (!tr) { x = a; w = c; y = c; z = b; u = a; v = b; flip = 0; }
+          else     { x = c; w = a; y = a; z = b; u = b; v = c; flip = 1; }
+        } else {
+          if (!tr) { x = b; w = c; y = c; z = a; u = a; v = b; flip = 1; }
+          else     { x = c; w = b; y = b; z = a; u = a; v = c; flip = 1; }
+        }
+        const int K = hole ? No : g.Nv;
+        for (int k0 = 0; k0 < K; k0 += kChunk) {
+          const int kc = min(kChunk, K - k0);
+          // A: rows (p,q) of this tile, p fastest (natural) or q (transposed)
+          const int m0 = mt * rows;
+          const int64_t sf = tr ? No : 1, ss = tr ? 1 : No;  // p + No q of (f, slow)
+          const double *T = g.T, *Vh = ps.Vh, *Vp = ps.Vp;
+          if (!hole)
+            cut_rows(At, kATile, 0, min(rows, No2 - m0), h->e_t, k0, K, [&](int m, int k) {
+              const int sl = (m0 + m) / No, f = (m0 + m) - sl * No;
+              return T[x + k * Nv + (f * sf + sl * ss) * NvNv];  // T[x,E,p,q]
+            });
+          else
+            cut_rows(At, kATile, 0, min(rows, No2 - m0), ps.e, k0, K, [&](int m, int k) {
+              const int sl = (m0 + m) / No, f = (m0 + m) - sl * No;
+              return Vh[f * sf + sl * ss + (int64_t)k * No2 + (int64_t)w * No2 * No];
+            });
+          // B: columns r
+          if (!hole)
+            cut_rows(Bt, P * 128, 0, No, ps.e, k0, K, [&](int r, int k) {
+              return Vp[y + z * Nv + k * NvNv + r * NvNv * Nv];  // Vp[y,z,E,r]
+            });
+          else
+            cut_rows(Bt, P * 128, 0, No, h->e_t, k0, K, [&](int r, int k) {
+              return -T[u + v * Nv + (flip ? r + (int64_t)No * k : k + (int64_t)No * r) * NvNv];
+            });
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          tc_fence_before();
+          __syncthreads();
+          if (warp == 0) {
+            tc_fence_after();
+            const bool leader = elect_one();
+            const uint64_t ad = sdesc_sw128(smem_u32(At)), bd = sdesc_sw128(smem_u32(Bt));
+            const int nkk = (kc + 15) / 16;
+            uint32_t acc = held > 0 ? 1 : 0;
+            for (int sa = 0; sa < kS; ++sa) {
+              const int n = ((kS - sa) * P + 15) & ~15;
+              const int n1 = n <= 256 ? n : ((n >> 1) + 15) & ~15;
+              const uint32_t id = idesc_bf16_f32(128, 0) | ((uint32_t)(n1 >> 3) << 17);
+              const uint32_t id2 = idesc_bf16_f32(128, 0) | ((uint32_t)((n - n1) >> 3) << 17);
+              const uint32_t d = t.tmem + sa * P;
+              if (leader)
+                for (int kk = 0; kk < nkk; ++kk) {
+                  const uint64_t as = ad + (uint32_t)(sa * (kATile >> 4)) + 2 * kk;
+                  mma_bf16(d, as, bd + 2 * kk, id, acc);
+                  if (n1 < n) mma_bf16(d + n1, as, bd + (uint32_t)(n1 * 8) + 2 * kk, id2, acc);
+                  acc = 1;
+                }
+              __syncwarp();
+              acc = 1;
+            }
+            if (leader) mma_commit(&t.bar);
+            __syncwarp();
+          }
+          held += kc;
+          const bool ok = mbar_wait(&t.bar, phase & 1, &h->tc_status, 1);
+          ++phase;
+          if (__syncthreads_or(!ok)) return false;
+          // the next chunk, if the accumulator can take it
+          const int next = k0 + kChunk < K ? min(kChunk, K - k0 - kChunk)
+                           : pt < 3        ? min(kChunk, ((pt + 1) & 1) ? No : g.Nv)
+                                           : kMaxK;
+          if (held + next <= kMaxK) continue;
+          // drain: level sums to exact integers, one rounding, into W
+          tc_fence_after();
+          const int l = (warp & 3) * 32 + lane, m = m0 + l;
+          const bool valid = l < rows && m < No2;
+          const int sl = m / No, f = m - sl * No;
+          const int base = grp == 0 ? m : grp == 1 ? f + No2 * sl : No * f + No2 * sl;
+          const int step = grp == 0 ? No2 : grp == 1 ? No : 1;
+          const uint32_t tb = t.tmem + ((uint32_t)((warp & 3) * 32) << 16);
+          for (int c0 = (warp >> 2) * 8; c0 < No; c0 += 32) {
+            float vv[kS][8];
+            __syncwarp();
+#pragma unroll
+            for (int L = 0; L < kS; ++L) tmem_ld8(tb + L * P + c0, vv[L]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const int r = c0 + q;
+              if (r >= No || !valid) continue;
+              constexpr uint32_t kBits = 0x4B400000u;  // 1.5 2^23: see triples_fp64_tc.cu
+              uint32_t bb[kS];
+#pragma unroll
+              for (int L = 1; L < kS; ++L) {
+                bb[L] = __float_as_uint(vv[L][q] + 12582912.f);
+                over |= bb[L] ^ 0x4B000000u;
+              }
+              const int n1 = (int)(bb[1] - kBits);
+              const int n23 = (int)(bb[2] * 256u + bb[3] - kBits * 257u);
+              const int n45 = (int)(bb[4] * 256u + bb[5] - kBits * 257u);
+              const int n67 = (int)(bb[6] * 256u + bb[7] - kBits * 257u);
+              const long long hi = (long long)__float2int_rn(vv[0][q]) * (1 << 24) +
+                                   ((long long)n1 * 65536 + n23);
+              const long long lo = (long long)n45 * 65536 + n67;
+              const double val = fma(i64_to_f64(lo), 0x1p-32, i64_to_f64(hi)) * ps.unit;
+              double *dst = ps.W + base + r * step;
+              *dst = first ? val : *dst + val;
+            }
+          }
+          tc_fence_before();
+          __syncthreads();  // the accumulator and W are used again
+          held = 0;
+          first = false;
+        }
+      }
+    }
+  return true;
+}
+
+// n-th (i >= j >= k) triple, n = C(i+2,3) + C(j+1,2) + k.
+__device__ __forceinline__ void triple_of(int n, int &i, int &j, int &k) {
+  i = (int)cbrtf(6.f * n);
+  while (i * (i + 1) * (i + 2) / 6 > n) --i;
+  while ((i + 1) * (i + 2) * (i + 3) / 6 <= n) ++i;
+  n -= i * (i + 1) * (i + 2) / 6;
+  j = (int)((sqrtf(8.f * n + 1.f) - 1.f) * 0.5f);
+  while (j * (j + 1) / 2 > n) --j;
+  while ((j + 1) * (j + 2) / 2 <= n) ++j;
+  k = n - j * (j + 1) / 2;
+}
+
+// This thread's part of a tuple's energy (src/atrip/Equations.cxx:101-238);
+// V: the three singles blocks V[b,c,..], V[a,c,..], V[a,b,..], No x No each.
+__device__ double energy_partial(const Args &g, const Tail &t, const double *V, const double *Tb,
+                                 const double *Wz, bool distinct, double epsabc) {
+  const int No = g.No, No2 = No * No, ntri = No * (No + 1) * (No + 2) / 6;
+  auto Z = [&](int i, int j, int k) {
+    double z = Wz[i + No * j + No2 * k];
+    z += t.ta[i] * V[j + k * No];
+    z += t.tb[j] * V[No2 + i + k * No];
+    z += t.tc[k] * V[2 * No2 + i + j * No];
+    return z;
+  };
+  auto T = [&](int i, int j, int k) { return Tb[i + No * j + No2 * k]; };
+  double sum = 0.0;
+  for (int n = threadIdx.x; n < ntri; n += kThreads) {
+    int i, j, k;
+    triple_of(n, i, j, k);
+    const double facjk = j == k ? 0.5 : 1.0, facij = i == j ? 0.5 : 1.0;
+    const double denominator = epsabc - ((g.epsi[i] + g.epsi[j]) + g.epsi[k]);
+    double value;
+    if (distinct) {
+      const double U = Z(i, j, k), V2 = Z(i, k, j), W = Z(j, i, k), X = Z(j, k, i),
+                   Y = Z(k, i, j), Zz = Z(k, j, i);
+      const double A = T(i, j, k), B = T(i, k, j), C = T(j, i, k), D = T(j, k, i),
+                   E = T(k, i, j), F = T(k, j, i);
+      const double UXY = U + (X + Y), VWZ = V2 + (W + Zz), ADE = A + (D + E), BCF = B + (C + F);
+      const double first = A * U + (B * V2 + (C * W + (D * X + (E * Y + F * Zz))));
+      value = 3.0 * first + ((UXY - 2.0 * VWZ) * ADE + (VWZ - 2.0 * UXY) * BCF);
+    } else {
+      const double U = Z(i, j, k), V2 = Z(j, k, i), W = Z(k, i, j);
+      const double A = T(i, j, k), B = T(j, k, i), C = T(k, i, j);
+      value = 3.0 * ((A * U + B * V2) + C * W) - (A + (B + C)) * (U + (V2 + W));
+    }
+    sum += (2.0 * value / denominator) * (facjk * facij);
+  }
+  return sum;
+}
+
+// One CTA of 512 threads per SM (as many as the scratch holds W for): cut a
+// chunk, multiply, in turn; W accumulates in the scratch in FP64.  Bound by
+// the cut, which each tuple repeats: single doubles read from a column-major
+// tensor (a 32-byte sector each) and ~60 instructions an element.
+// No=24/Nv=120, 2500 tuples: 19.1 ms, 70.7 on FP64 instructions.
+__global__ void __launch_bounds__(kThreads, 1) kernel(Args g) {
+  extern __shared__ __align__(1024) unsigned char raw[];
+  unsigned char *At = reinterpret_cast<unsigned char *>(
+      (reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+  const int No = g.No, No2 = No * No, P = (No + 7) / 8 * 8;
+  unsigned char *Bt = At + kS * kATile;
+  Tail &t = *reinterpret_cast<Tail *>(Bt + kS * P * 128 + 1024);
+  Header *h = reinterpret_cast<Header *>(g.scratch);
+  if (!h->tc_ok) return;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    mbar_init(&t.bar, 1);
+    fence_mbar_init();
+  }
+  for (int i = threadIdx.x; i < (kS * kATile + kS * P * 128 + 1024) / 16; i += kThreads)
+    reinterpret_cast<uint4 *>(At)[i] = make_uint4(0, 0, 0, 0);
+  if (warp == 0) {
+    tmem_alloc(&t.tmem, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const int64_t No3 = (int64_t)No2 * No, Nv = g.Nv;
+  double *Wv = reinterpret_cast<double *>(g.scratch + kWorkspaceOffset) +
+               blockIdx.x * (g.use_j ? 2 : 1) * No3;
+  double *Wj = Wv + No3;
+  const int64_t n = g.t_end - g.t_begin;
+  const Pass pv = {g.Vh, g.Vp, h->e_v, ldexp(1.0, h->e_t + h->e_v - 14 - 24), Wv};
+  const Pass pj = {g.Jh, g.Jp, h->e_j, ldexp(1.0, h->e_t + h->e_j - 14 - 24), Wj};
+  uint32_t phase = 0, over = 0;
+  bool alive = true;
+  while (alive) {
+    if (threadIdx.x == 0) {
+      const unsigned long long q = atomicAdd(&h->tc_cursor, 1ull);
+      t.slot = q < (unsigned long long)n ? (long long)q : -1;
+      if (t.slot >= 0) decode_tuple(g.t_begin + t.slot, g.Nv, t.abc[0], t.abc[1], t.abc[2]);
+    }
+    __syncthreads();
+    const long long slot = t.slot;
+    if (slot < 0) break;
+    const int a = t.abc[0], b = t.abc[1], c = t.abc[2];
+    if (threadIdx.x < No) {
+      const int i = threadIdx.x;
+      t.ta[i] = g.tai_sign * g.tai[a + i * Nv];
+      t.tb[i] = g.tai_sign * g.tai[b + i * Nv];
+      t.tc[i] = g.tai_sign * g.tai[c + i * Nv];
+    }
+    alive = build_w(g, h, t, At, Bt, pv, a, b, c, phase, over) &&
+            (!g.use_j || build_w(g, h, t, At, Bt, pj, a, b, c, phase, over));
+    if (!alive) break;
+    // the singles' blocks in place of the A tile
+    double *V = reinterpret_cast<double *>(At);
+    const int64_t pair[3] = {b + c * Nv, a + c * Nv, a + b * Nv};
+    for (int i = threadIdx.x; i < 3 * No2; i += kThreads)
+      V[i] = g.Vpp[pair[i / No2] + (i % No2) * Nv * Nv];
+    __syncthreads();
+    int cls = 0;  // src/atrip/Atrip.cxx:640-642
+    if (a == b) cls++;
+    if (b == c) cls--;
+    const double epsabc = g.epsa[a] + g.epsa[b] + g.epsa[c];
+    double e[2] = {0.0, 0.0};
+    for (int pass = 0; pass < (g.use_j ? 2 : 1); ++pass) {
+      double sum = energy_partial(g, t, V, pass ? Wj : Wv, Wv, cls == 0, epsabc);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) t.red[warp] = sum;
+      __syncthreads();
+      if (threadIdx.x == 0)
+        for (int w = 0; w < kThreads / 32; ++w) e[pass] += t.red[w];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      g.e[slot] = e[0];
+      g.ect[slot] = g.use_j ? e[1] : e[0];
+    }
+  }
+  if (over & 0xFF800000u) atomicOr(&h->tc_overflow, 1);
+  // no MMA outlives the block (after a failed wait some may be in flight)
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 0) tmem_dealloc(t.tmem, 512);
+}
+
+size_t smem_bytes(int no) {
+  return 1024 + kS * kATile + (size_t)kS * ((no + 7) / 8 * 8) * 128 + 1024 + sizeof(Tail);
+}
+
+// By sizes: slab maxima fit the scratch, and the range's work on FP64
+// instructions (~0.8 TFLOP/s here) takes several times what examining the
+// whole tensors does (~5 TB/s and a few launches).
+bool sizes_ok(const Args &a) {
+  const double Nv = a.Nv, No = a.No, n = (double)(a.t_end - a.t_begin);
+  const double nj = a.use_j ? 2.0 : 1.0;
+  const double dfma = n * nj * 12.0 * No * No * No * (No + Nv) / 0.8e12;
+  const double scan = 8.0 * (Nv * Nv * No * No + nj * Nv * No * (Nv * Nv + No * No)) / 5e12 + 4e-5;
+  return No >= 4 && dfma > 4.0 * scan &&
+         3.0 * 8.0 * Nv * Nv <= (double)(kScratchBytes - kWorkspaceOffset);
+}
+
+// Queue the examination and the kernel.
+int enqueue(const Args &a, int device, cudaStream_t st) {
+  const int64_t Nv = a.Nv, No = a.No, nvnv = Nv * Nv;
+  auto *slabs = reinterpret_cast<unsigned long long *>(a.scratch + kWorkspaceOffset);
+  Header *h = reinterpret_cast<Header *>(a.scratch);
+  ATRIP_CUDA_TRY(cudaMemsetAsync(slabs, 0, 8 * 3 * nvnv, st));
+  const dim3 blocks((unsigned)((nvnv + 255) / 256), 1);
+  auto grid = [&](int64_t count) {
+    const int64_t y = std::max<int64_t>(1, 152 * 16 / blocks.x);
+    return dim3(blocks.x, (unsigned)std::min<int64_t>(count, y));
+  };
+  column_max<<<grid(No * No), 256, 0, st>>>(a.T, nvnv, No * No, slabs);
+  column_max<<<grid(Nv * No), 256, 0, st>>>(a.Vp, nvnv, Nv * No, slabs + nvnv);
+  slab_max<<<(int)Nv, 256, 0, st>>>(a.Vh, Nv, No * No * No, h, 0);
+  if (a.use_j) {
+    column_max<<<grid(Nv * No), 256, 0, st>>>(a.Jp, nvnv, Nv * No, slabs + 2 * nvnv);
+    slab_max<<<(int)Nv, 256, 0, st>>>(a.Jh, Nv, No * No * No, h, 1);
+  }
+  decide<<<1, 1024, 0, st>>>(slabs, nvnv, a.use_j, h);
+  ATRIP_CUDA_TRY(cudaGetLastError());
+  int sms = 0;
+  ATRIP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  const size_t per_cta = sizeof(double) * (a.use_j ? 2 : 1) * (size_t)No * No * No;
+  const int64_t fit = (int64_t)((kScratchBytes - kWorkspaceOffset) / per_cta);
+  const int64_t n = a.t_end - a.t_begin;
+  const int ctas = (int)std::min<int64_t>(std::min<int64_t>(sms, fit), n);
+  const size_t smem = smem_bytes((int)No);
+  ATRIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+  kernel<<<ctas, kThreads, smem, st>>>(a);
+  ATRIP_CUDA_TRY(cudaGetLastError());
+  return ATRIP_OK;
+}
+
+}  // namespace tc
 
 __device__ __forceinline__ void neumaier(double &s, double &c, double x) {
   const double t = s + x;
@@ -331,7 +842,7 @@ int launch(const Args &a, int device, cudaStream_t st) {
   ATRIP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, triples_noalloc_kernel<NC>,
                                                                kThreads, 0));
   ATRIP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  const size_t per_cta = sizeof(double) * 2 * (size_t)a.No * a.No * a.No;
+  const size_t per_cta = sizeof(double) * (a.use_j ? 2 : 1) * (size_t)a.No * a.No * a.No;
   const int64_t fit = (int64_t)((kScratchBytes - kWorkspaceOffset) / per_cta);
   int64_t grid = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
   if (grid > fit) grid = fit;
@@ -428,7 +939,8 @@ extern "C" int atrip_gpu_run_fp64_noalloc(int32_t no, int32_t nv, const atrip_de
   ATRIP_CUDA_TRY(cudaMemsetAsync(scratch, 0, noalloc::kHeaderBytes, st));
   const int64_t n = t_end - t_begin;
   if (n > 0) {
-    int rc = ATRIP_OK;
+    int rc = noalloc::tc::sizes_ok(a) ? noalloc::tc::enqueue(a, device, st) : ATRIP_OK;
+    if (rc != ATRIP_OK) return rc;
     switch ((no + 7) / 8) {
       case 1: rc = noalloc::launch<1>(a, device, st); break;
       case 2: rc = noalloc::launch<2>(a, device, st); break;

@@ -96,3 +96,41 @@ def test_data_rules(spoil):
         ctx.run(form="fp64", max_iterations=199)
         f, _ = ctx.tuple_energies(0, 200)
     np.testing.assert_array_equal(e, f)
+
+
+# the no-allocation entry point's tensor-core kernel: tiles of 128 rows and
+# their remainders, sums drained once and in pieces (2 (Nv + No) > 341), (cT);
+# and data that sends it to its FP64-instruction kernel
+@pytest.mark.parametrize("No,Nv,j,spoil", [(8, 40, True, False), (13, 33, False, False),
+                                           (24, 26, True, False), (41, 18, False, False),
+                                           (64, 12, False, False), (6, 170, False, False),
+                                           (12, 40, False, True)])
+def test_noalloc_tensor_cores(No, Nv, j, spoil):
+    torch = pytest.importorskip("torch")
+    import ctypes
+    d = synth.make_inputs(No, Nv, 14, with_j=j)
+    if spoil:
+        d["Vabci"][:, 7] *= 2.0 ** -20
+    names = NAMES + (("Jijka", "Jabci") if j else ())
+    dev = {k: torch.from_numpy(np.ascontiguousarray(d[k].ravel(order="F"))).cuda() for k in names}
+    n = min(synth.n_tuples(Nv), 3000 if No < 10 else 900 if No < 30 else 350)
+    t0 = synth.n_tuples(Nv) - n
+    out = torch.full((2 * n + 2,), float("nan"), dtype=torch.float64, device="cuda")
+    ptrs = capi.DeviceInputs(*[dev[k].data_ptr() if k in dev else None for k in
+                               NAMES + ("Jijka", "Jabci")])
+    lib = capi.load()
+    torch.cuda.synchronize()
+    for _ in range(2):
+        capi.check(lib.atrip_gpu_run_fp64_noalloc(
+            No, Nv, ctypes.byref(ptrs), t0, t0 + n - 1, 0, 1, out.data_ptr() + 16,
+            out.data_ptr() + 16 + 8 * n, out.data_ptr(), None))
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    with _ctx(d, j) as ctx:
+        ctx.set_tuning(fp64_tile_rows=64)
+        r = ctx.run(form="fp64", first_iteration=t0, max_iterations=t0 + n - 1)
+        e, ect = ctx.tuple_energies(t0, n)
+    K = 2 * (Nv + No)
+    _close(got[2:2 + n], e, K)
+    _close(got[2 + n:], ect, K)
+    assert abs(got[0] - r.energy) <= K * 2.0 ** -52 * np.sum(np.abs(e))
