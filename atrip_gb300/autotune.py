@@ -199,11 +199,12 @@ def tune_split(ctx: capi.Context, slices: int, flops: float = 2e13, m: int = 8,
     wins = windows(n, m, window_size(ctx.No, ctx.Nv, m, flops))
     run_windows(ctx, wins[:1], form, slices)  # warm-up (cuts the slices)
     f16 = form == "split_f16"  # always the transposed kernel
-    cands = [{"split_stages": st} for st in (0, 3, 4)]
+    # {}: the engine's choice; a launch parameter selects the split kernels
+    cands = [{}] + [dict(split_variant=1, split_stages=st) for st in (0, 3, 4)]
     if ctx.No <= 24 and not f16:  # W copy in shared memory, or a deeper ring with W in L2
-        cands += [{"split_stages": st, "split_w_global": 1} for st in (0, 5)]
+        cands += [{"split_variant": 1, "split_stages": st, "split_w_global": 1} for st in (0, 5)]
     if f16:
-        cands = [{"split_variant": 2, "split_stages": st} for st in (0, 3)]
+        cands = [{}] + [{"split_variant": 2, "split_stages": st} for st in (0, 3)]
         cands += [{"split_variant": 2, "split_w_global": 1}]
         if ctx.No % 8 == 0:
             cands += [{"split_variant": 3}]
@@ -215,12 +216,12 @@ def tune_split(ctx: capi.Context, slices: int, flops: float = 2e13, m: int = 8,
             cands += [{"split_variant": 3}]
     timed = [(_time(ctx, wins, form, slices, c), c) for c in cands]
     best_ms, tuning = min(timed, key=lambda x: x[0])
-    # L2 prefetch of the next part's slab tiles
-    c = dict(tuning, split_prefetch=1)
-    t = _time(ctx, wins, form, slices, c)
-    timed.append((t, c))
-    if t < 0.98 * best_ms:
-        best_ms, tuning = t, c
+    if tuning:  # split kernels: L2 prefetch of the next part's slab tiles
+        c = dict(tuning, split_prefetch=1)
+        t = _time(ctx, wins, form, slices, c)
+        timed.append((t, c))
+        if t < 0.98 * best_ms:
+            best_ms, tuning = t, c
     # then the processing order: tuples grouped by (a, b, c) blocks of side L
     # keep the slabs of the tuples in flight in L2
     for L in (4, 6, 8, 12, 16, 24):

@@ -54,6 +54,8 @@ struct atrip_gpu_batch {
   SplitMultiBuffers multi;  // split form: every system in one launch
   bool multi_used = false;  // the captured graph holds that one launch
   TcBuffers tcb;            // FP64 form: the systems on the tensor-core kernel
+  TcBuffers tcs;            // split form: every system in one launch of that kernel
+  bool tcs_used = false;
 };
 
 namespace {
@@ -248,7 +250,7 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
       if (rc != ATRIP_OK) return rc;
       if (!ok) continue;
       tc.push_back({&c->tc, &c->dt, c->No, c->Nv, a.n_triples, a.tuples, a.triples, a.t_begin,
-                    a.t_end, a.use_j != 0, a.e, a.ect});
+                    a.t_end, a.use_j != 0, a.e, a.ect, nullptr});
       tc_states.push_back(&c->tc);
     }
     if (!tc.empty()) {
@@ -292,14 +294,45 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
         c->split.variant = c->tune.split_variant;
         c->split.prefetch = c->tune.split_prefetch != 0;
         c->split.f16 = form == ATRIP_FORM_SPLIT_F16;
-        int rc = split_prepare(c->split, c->dt, c->No, c->Nv, one_launch ? 1 : split_ctas(c),
+        int rc = split_prepare(c->split, c->dt, c->No, c->Nv,
+                               b->tcs_used ? 0 : one_launch ? 1 : split_ctas(c),
                                a.use_j != 0, slices, a.triples, a.n_triples, st, &prep_launches);
         if (rc != ATRIP_OK) return rc;
       }
       return ATRIP_OK;
     };
     b->multi_used = false;
-    if (b->tune.split_variant != 1) {
+    // one launch of the kernel of fp64_tc.cuh unless a launch parameter of the
+    // split kernels is set, for the batch or one of its systems
+    b->tcs_used = b->tune.split_variant == 0;
+    for (int s = 0; s < n && b->tcs_used; ++s) {
+      const atrip_gpu_context *c = b->sys[s];
+      const atrip_tuning &t = c->tune;
+      b->tcs_used = split_tc_eligible(slices, form == ATRIP_FORM_SPLIT_F16, c->No, c->Nv) &&
+                    t.split_variant == 0 && t.split_stages == 0 && t.split_ctas == 0 &&
+                    t.split_w_global == 0 && t.split_prefetch == 0;
+    }
+    if (b->tcs_used) {
+      int rc = prepare_all(true);
+      if (rc != ATRIP_OK) return rc;
+      std::vector<TcSystem> ts(n);
+      for (int k = 0; k < n; ++k) {
+        atrip_gpu_context *c = b->sys[b->order[k]];
+        const TriplesArgs &a = b->h_table[k];
+        ts[k] = {&c->split.tc, &c->dt, c->No, c->Nv, a.n_triples, a.tuples, a.triples, a.t_begin,
+                 a.t_end, a.use_j != 0, a.e, a.ect, nullptr};
+        if ((rc = split_tc_attach(c->split, a.use_j != 0, &ts[k].tri_ef)) != ATRIP_OK) return rc;
+      }
+      rc = tc_launch_prepare(ts.data(), n, tai_sign, b->sm_count, b->tcs);
+      if (rc != ATRIP_OK) return rc;
+      const uintptr_t more[] = {1, (uintptr_t)b->tcs.total, (uintptr_t)b->tcs.grid,
+                                (uintptr_t)b->tcs.planes, (uintptr_t)b->tcs.d_desc,
+                                (uintptr_t)b->tcs.smem, (uintptr_t)b->tcs.lay_cells,
+                                (uintptr_t)b->tcs.lay_pass, (uintptr_t)b->tcs.bslot,
+                                (uintptr_t)b->tcs.aslot, (uintptr_t)b->tcs.nslots,
+                                (uintptr_t)b->tcs.nbslots};
+      key.insert(key.end(), std::begin(more), std::end(more));
+    } else if (b->tune.split_variant != 1) {
       int rc = prepare_all(true);
       if (rc != ATRIP_OK) return rc;
       std::vector<SplitMultiSystem> ms(n);
@@ -315,7 +348,7 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
       else if (rc != ATRIP_ERR_UNSUPPORTED) return rc;
       clear_error();
     }
-    if (!b->multi_used) {
+    if (!b->multi_used && !b->tcs_used) {
       const int rc = prepare_all(false);  // one launch per system (batch split_variant 1)
       if (rc != ATRIP_OK) return rc;
     }
@@ -381,6 +414,9 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
           const int rc2 = tc_launch_enqueue(b->tcb, nullptr, b->stream, &launches);
           if (rc2 != ATRIP_OK) return rc2;
         }
+      } else if (b->tcs_used) {
+        const int rc2 = tc_launch_enqueue(b->tcs, nullptr, b->stream, &launches);
+        if (rc2 != ATRIP_OK) return rc2;
       } else if (b->multi_used) {
         ATRIP_CUDA_TRY(cudaMemsetAsync(b->multi.d_status, 0, sizeof(int), b->stream));
         int rc2 = split_multi_enqueue(b->multi, tai_sign, b->sm_count, b->stream, &launches);
@@ -434,6 +470,13 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
     // systems whose sums left the exact range are barred now: run again
     if (rerun) return atrip_gpu_batch_run(b, opts, results);
   }
+  if (form != ATRIP_FORM_FP64 && b->tcs_used) {
+    std::vector<TcState *> states(n);
+    for (int k = 0; k < n; ++k) states[k] = &b->sys[b->order[k]]->split.tc;
+    bool rerun = false;
+    const int rc = tc_launch_check(b->tcs, states.data(), &rerun);
+    if (rc != ATRIP_OK) return rc;
+  }
   for (int s = 0; s < n; ++s) {
     const int rc = split_status_check(b->h_status[s]);
     if (rc != ATRIP_OK)
@@ -482,6 +525,7 @@ int atrip_gpu_batch_destroy(atrip_gpu_batch *b) {
   destroy_graph(b);
   split_multi_free(b->multi);
   tc_buffers_free(b->tcb);
+  tc_buffers_free(b->tcs);
   cudaFreeHost(b->h_table);
   cudaFreeHost(b->h_prefix);
   cudaFreeHost(b->h_sums);

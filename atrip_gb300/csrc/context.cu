@@ -468,7 +468,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
   }
   if (tc) {
     const TcSystem ts = {&c->tc, &c->dt, c->No, c->Nv, c->n_triples, c->d_tuples, c->d_triples,
-                         t_begin, t_end, use_j, c->d_e, c->d_ect};
+                         t_begin, t_end, use_j, c->d_e, c->d_ect, nullptr};
     int rc = tc_launch_prepare(&ts, 1, opts->ijkabc ? -1.0 : 1.0, c->sm_count, c->tcb);
     if (rc == ATRIP_ERR_OUT_OF_MEMORY) {  // no room for its W buffers
       cudaGetLastError();
@@ -495,6 +495,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
     if (rc != ATRIP_OK) return rc;
     tc = !rerun;
   }
+  bool split_on_tc = false;
   if (n > 0 && !tc) {
     ATRIP_CUDA_TRY(cudaMemsetAsync(c->d_queue, 0, sizeof(unsigned long long) * 4, st));
     if (form == ATRIP_FORM_FP64) {
@@ -556,19 +557,40 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
       c->split.f16 = form == ATRIP_FORM_SPLIT_F16;
       const int ctas = c->tune.split_ctas > 0 ? std::min(c->sm_count, (int)c->tune.split_ctas)
                                               : c->sm_count;
-      int rc = split_run(c->split, c->dt, c->No, c->Nv, ctas, c->d_tuples, c->d_triples,
-                         c->n_triples, t_begin, t_end, order, opts->ijkabc ? -1.0 : 1.0, use_j,
-                         slices,
-                         c->d_queue, c->d_e, c->d_ect, st, &launches);
+      // the kernel of fp64_tc.cuh unless a launch parameter of the split
+      // kernels is set
+      const atrip_tuning &tn = c->tune;
+      bool on_tc = split_tc_eligible(slices, c->split.f16, c->No, c->Nv) &&
+                   tn.split_variant == 0 && tn.split_stages == 0 && tn.split_ctas == 0 &&
+                   tn.split_w_global == 0 && tn.split_prefetch == 0 &&
+                   tn.split_wait_kcycles == 0 && tn.split_test_unpublished == 0 &&
+                   tn.split_profile == 0;
+      const double tai_sign = opts->ijkabc ? -1.0 : 1.0;
+      auto run_split = [&]() -> int {
+        if (on_tc) {
+          int rc = split_prepare(c->split, c->dt, c->No, c->Nv, 0, use_j, slices, c->d_triples,
+                                 c->n_triples, st, &launches);
+          if (rc != ATRIP_OK) return rc;
+          TcSystem ts = {&c->split.tc, &c->dt, c->No, c->Nv, c->n_triples, c->d_tuples,
+                         c->d_triples, t_begin, t_end, use_j, c->d_e, c->d_ect, nullptr};
+          if ((rc = split_tc_attach(c->split, use_j, &ts.tri_ef)) != ATRIP_OK) return rc;
+          if ((rc = tc_launch_prepare(&ts, 1, tai_sign, c->sm_count, c->tcs)) != ATRIP_OK)
+            return rc;
+          return tc_launch_enqueue(c->tcs, order, st, &launches);
+        }
+        return split_run(c->split, c->dt, c->No, c->Nv, ctas, c->d_tuples, c->d_triples,
+                         c->n_triples, t_begin, t_end, order, tai_sign, use_j, slices, c->d_queue,
+                         c->d_e, c->d_ect, st, &launches);
+      };
+      int rc = run_split();
       if (rc == ATRIP_ERR_OUT_OF_MEMORY && c->tc.impl) {  // the FP64 slices make room
         cudaGetLastError();
         clear_error();
         free_tc(c);
-        rc = split_run(c->split, c->dt, c->No, c->Nv, ctas, c->d_tuples, c->d_triples,
-                       c->n_triples, t_begin, t_end, order, opts->ijkabc ? -1.0 : 1.0, use_j,
-                       slices, c->d_queue, c->d_e, c->d_ect, st, &launches);
+        rc = run_split();
       }
       if (rc != ATRIP_OK) return rc;
+      split_on_tc = on_tc;
     }
     ATRIP_CUDA_TRY(launch_energy_sum(c->d_e + t_begin, c->d_ect + t_begin, n, c->d_partials,
                                      c->d_sum, st));
@@ -580,6 +602,12 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
       ATRIP_CUDA_TRY(
           cudaMemcpyAsync(sums, c->d_sum, sizeof(double) * 6, cudaMemcpyDeviceToHost, st));
     ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+    if (split_on_tc) {
+      TcState *state = &c->split.tc;
+      bool rerun = false;
+      const int rc = tc_launch_check(c->tcs, &state, &rerun);
+      if (rc != ATRIP_OK) return rc;
+    }
   }
   ATRIP_CUDA_TRY(cudaGetLastError());
   float ms = 0.f;
@@ -681,6 +709,7 @@ int atrip_gpu_destroy(atrip_gpu_context *c) {
     if (c->have[t]) free_tensor(c, t);
   split_free(c->split);
   free_tc(c);
+  tc_buffers_free(c->tcs);
   cudaFree(c->d_tuples);
   cudaFree(c->d_triples);
   cudaFree(c->d_e);

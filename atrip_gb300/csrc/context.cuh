@@ -33,6 +33,7 @@ struct atrip_gpu_context {
   atrip_gb300::SplitState split;
   atrip_gb300::TcState tc;  // FP64 form on the tensor cores
   atrip_gb300::TcBuffers tcb;
+  atrip_gb300::TcBuffers tcs;  // split forms on the same kernel
   atrip_tuning tune = {};
   // processing order of the last range (tuple_block > 1), see build_order
   std::vector<uint32_t> h_tuples;  // packed list, host copy

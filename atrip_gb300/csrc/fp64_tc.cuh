@@ -34,6 +34,14 @@ int tc_tuple_block(int No, int Nv, int sm_count);
 int tc_prepare(TcState &s, const DeviceTensors &dt, int No, int Nv, bool cplx, bool use_j,
                cudaStream_t st, int64_t *launches, bool *usable);
 
+// The split-precision forms' slices on the same kernel: S slices of the
+// operands ops[] = {T rows natural, transposed, V_hhhp natural, transposed,
+// V_pphp, T_uv, T_uv^T} (pitch Kp, holes 64), unit the weight of level 0; the
+// (cT) pair {J_hhhp natural, transposed, J_pphp}.  s owns none of them.
+int tc_split_attach(TcState &s, int S, bool f16, int No, int Nv, int Kp, double unit,
+                    void *const *ops);
+int tc_split_attach_j(TcState &s, double unit_j, void *const *ops);
+
 // One system of a launch.
 struct TcSystem {
   TcState *state;
@@ -43,6 +51,7 @@ struct TcSystem {
   int64_t t_begin, t_end;
   bool use_j;
   double *e, *ect;
+  const double2 *tri_ef;  // split forms: denominator part and weight of each triple
 };
 
 // Buffers of a launch, owned by a context or a batch.
@@ -56,7 +65,9 @@ struct TcBuffers {
   unsigned long long *d_queue = nullptr;
   int cap = 0;
   // launch layout of the last tc_launch_prepare
-  int n = 0, nc = 1, lay_no = 0, lay_cells = 0, lay_pass = 1, nslots = 0, nbslots = 0, aslot = 0,
+  int n = 0, S = 8, nc = 1;
+  bool split = false, f16 = false;
+  int lay_no = 0, lay_cells = 0, lay_pass = 1, nslots = 0, nbslots = 0, aslot = 0,
       bslot = 0, grid = 0;
   size_t smem = 0;
   int64_t total = 0;

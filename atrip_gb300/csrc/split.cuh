@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "engine.cuh"
+#include "fp64_tc.cuh"
 
 namespace atrip_gb300 {
 
@@ -22,6 +23,7 @@ struct SplitState {
   long long wait_cycles = 0;  // bounded-wait limit in SM cycles (0 = built-in ~2 s)
   bool unpublished = false;   // test: the producer publishes no tuple
   bool profile = false;       // launch the kernel built with role counters
+  TcState tc;                 // the slices' maps for the tensor-core kernel of fp64_tc.cuh
 };
 
 void split_invalidate(SplitState &s);
@@ -34,6 +36,14 @@ void split_free(SplitState &s);
 int split_prepare(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm_count,
                   bool use_j, int slices, const uint32_t *triples, int n_triples,
                   cudaStream_t st, int64_t *launches);
+// Whether the kernel of fp64_tc.cuh takes these slices: levels exact as the
+// kernels here keep them, BF16 with K = 2 (Nv + No) <= 1024, FP16 within
+// their own limits.  It is the one run unless a launch parameter of the
+// kernels here is set.
+bool split_tc_eligible(int slices, bool f16, int No, int Nv);
+// The prepared slices' maps for it, and the triple table it reads.
+int split_tc_attach(SplitState &s, bool use_j, const double2 **tri_ef);
+
 // Queue one launch over tuples [t_begin, t_end) on st (no host sync; may be
 // captured into a CUDA graph).  The caller zeroes *queue first.
 int split_enqueue(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm_count,

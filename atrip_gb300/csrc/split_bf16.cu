@@ -51,6 +51,7 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "recip.cuh"
 #include "sm100.cuh"
 #include "split.cuh"
 
@@ -145,46 +146,6 @@ __global__ void triple_table_kernel(const uint32_t *__restrict__ triples, int n,
     const double fac = (j == k ? 0.5 : 1.0) * (i == j ? 0.5 : 1.0);
     out[t] = make_double2((epsi[i] + epsi[j]) + epsi[k], 2.0 * fac);
   }
-}
-
-__device__ __noinline__ double recip_div(double d) { return 1.0 / d; }
-
-// Exact conversions to FP64 done with integer instructions.  The energy
-// warps are bound by this GPU's narrow FP64 pipe; integer operations run
-// beside it.
-// |n| < 2^51: 1.5 2^52 + n has ulp 1, so its bit pattern is that of
-// 1.5 2^52 plus n in the low mantissa bits; subtracting 1.5 2^52 is exact.
-__device__ __forceinline__ double i64_to_f64_exact(long long n) {
-  return __longlong_as_double(0x4338000000000000ll + n) - 6755399441055744.0;
-}
-// Normal FP32 values: same sign and mantissa, exponent rebiased (127 ->
-// 1023); zero, subnormal, infinity and NaN take the conversion instruction.
-__device__ __forceinline__ double f32_to_f64_exact(float f) {
-  const uint32_t u = __float_as_uint(f);
-  const uint32_t e = (u >> 23) & 0xffu;
-  if (e == 0u || e == 0xffu) return (double)f;
-  const unsigned long long bits = ((unsigned long long)(u & 0x80000000u) << 32) |
-                                  ((unsigned long long)(e + 896u) << 52) |
-                                  ((unsigned long long)(u & 0x7fffffu) << 29);
-  return __longlong_as_double((long long)bits);
-}
-
-// 1/d for the energy denominators: d truncated to FP32 (integer
-// operations), its FP32 reciprocal (rounded to nearest), widened exactly,
-// refined by one Newton-Raphson step x1 = x0 + x0 (1 - d x0) in FP64.
-// With |x0 d - 1| <= ~1.5 2^-23 the relative error of x1 is about its
-// square (< 2^-44) plus one rounding; outside the FP32 exponent range it
-// falls back to the division (out of line: the orbital-energy gaps never
-// get there).
-__device__ __forceinline__ double recip_nr(double d) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-  const int e = (int)((b >> 52) & 0x7ffu) - 1023;
-  if (e < -125 || e > 126) return recip_div(d);
-  const uint32_t fb = ((uint32_t)(b >> 32) & 0x80000000u) | ((uint32_t)(e + 127) << 23) |
-                      ((uint32_t)(b >> 29) & 0x7fffffu);
-  const double x0 = f32_to_f64_exact(__frcp_rn(__uint_as_float(fb)));
-  const double err = fma(-d, x0, 1.0);
-  return fma(x0, err, x0);
 }
 
 // dst[s][R][k] (pitch Kp) = sign * digit_s(src(R, k) * scale) for k < K,
@@ -1919,6 +1880,7 @@ int split_profile_read(const SplitState &s, unsigned long long *out, int n) {
 void split_invalidate(SplitState &s) { s.valid = false; }
 
 void split_free(SplitState &s) {
+  tc_free(s.tc);
   free_impl(static_cast<SplitImpl *>(s.impl));
   s.impl = nullptr;
   s.valid = false;
@@ -2064,6 +2026,32 @@ int split_enqueue(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
   if (rc != ATRIP_OK) return rc;
   *launches += 1;
   return ATRIP_OK;
+}
+
+bool split_tc_eligible(int slices, bool f16, int No, int Nv) {
+  if (No < 2) return false;  // one triple a tuple, whose energy is 0 but for rounding
+  if (f16) return slices == 2 && No <= 64 && 2 * (Nv + No) < 2048;
+  return slices >= 2 && slices <= 4 && 2 * (Nv + No) <= 1024;
+}
+
+int split_tc_attach(SplitState &s, bool use_j, const double2 **tri_ef) {
+  auto *p = static_cast<SplitImpl *>(s.impl);
+  if (!s.valid || !p || (use_j && !p->has_j)) {
+    set_error("split form: operands not prepared");
+    return ATRIP_ERR_STATE;
+  }
+  int rc = ATRIP_OK;
+  if (!s.tc.usable) {
+    void *const ops[7] = {p->TaS, p->TaST, p->VhS, p->VhST, p->VpS, p->TpS, p->TpTS};
+    rc = tc_split_attach(s.tc, p->S, p->bits == 11, p->No, p->Nv, p->Ep, p->unit, ops);
+  }
+  if (rc == ATRIP_OK && use_j && !s.tc.usable_j) {
+    void *const ops[3] = {p->JhS, p->JhST, p->JpS};
+    rc = tc_split_attach_j(s.tc, p->unit_j, ops);
+  }
+  if (rc != ATRIP_OK) tc_free(s.tc);
+  *tri_ef = p->tri_ef;
+  return rc;
 }
 
 const int *split_status_ptr(const SplitState &s) {

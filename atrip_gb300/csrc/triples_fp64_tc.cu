@@ -62,11 +62,13 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "complex.cuh"
 #include "digits.cuh"
 #include "engine.cuh"
 #include "fp64_tc.cuh"
+#include "recip.cuh"
 #include "sm100.cuh"
 
 namespace atrip_gb300 {
@@ -75,7 +77,7 @@ namespace {
 using namespace sm100;
 
 constexpr int kThreads = 512;
-constexpr int kS = 8;                       // digit slices and levels
+constexpr int kS = 8;                       // digit slices and levels of the FP64 form
 constexpr int kKChunk = 64;                 // BF16 elements per 128-byte row
 constexpr int kMaxSlots = 10;               // A ring
 constexpr int kTupleSlots = 4;
@@ -102,6 +104,7 @@ struct TcDesc {
   TcMaps maps;
   const double *epsi, *epsa, *tai, *Vhh;
   const uint32_t *tuples, *triples;
+  const double2 *tri_ef;
   double *e, *ect;
   double unit, unit_j;  // weight of a W cell's high part
   double tai_sign;
@@ -118,7 +121,7 @@ struct TcArgs {
   const uint32_t *order;  // processing order of a single system's range
   unsigned long long *queue;
   int *flags;
-  longlong2 *planes;  // [CTA][parity][pass][group][cell]
+  void *planes;       // [CTA][parity][pass][group][cell]
   double *wd;         // [CTA][pass][cell]
   int lay_cells, lay_pass, nslots, nbslots, aslot, bslot;
 };
@@ -207,6 +210,22 @@ __device__ __forceinline__ TcPart part_of(const TcMaps &m, int g, int pt, int a,
   return p;
 }
 
+// What a kernel instantiation multiplies: S digit slices and levels; CPLX a
+// complex system; SPLIT the split-precision forms' slices, BF16 of radix 2^8
+// or (F16) FP16 of radix 2^11, and their energy arithmetic.
+template <int S_, bool CPLX_, bool SPLIT_, bool F16_>
+struct Fmt {
+  static constexpr int S = S_;
+  static constexpr bool CPLX = CPLX_;
+  static constexpr bool SPLIT = SPLIT_;  // an A ring slot holds all slices of a chunk
+  __device__ static constexpr int radix() { return F16_ ? 2048 : 256; }
+  __device__ static constexpr uint32_t idesc(int n) {
+    return F16_ ? idesc_f16_f32(128, n) : idesc_bf16_f32(128, n);
+  }
+};
+using FmtFp64 = Fmt<kS, false, false, false>;
+using FmtZ = Fmt<kS, true, false, false>;
+
 struct TcSlot {
   int64_t t;  // list position, -1 = no more work
   int a, b, c, s;
@@ -228,6 +247,9 @@ __device__ __forceinline__ double zval(const double *W, const TcSinglesCtx &s, i
 
 // This thread's part of a tuple's energy, T from Tb and Z from Wz + singles:
 // the expressions of the DFMA kernel's energy loop, with its division.
+// SPLIT: the split forms' arithmetic, the occupied part of the denominator
+// and the weight from a table and a refined reciprocal for the division.
+template <bool SPLIT>
 __device__ __forceinline__ double energy_partial(const TcDesc &d, const double *Tb,
                                                  const double *Wz, const TcSinglesCtx &s,
                                                  bool distinct, double epsabc, int er) {
@@ -236,8 +258,10 @@ __device__ __forceinline__ double energy_partial(const TcDesc &d, const double *
   for (int n = er; n < d.n_triples; n += kEnergyThreads) {
     const uint32_t pk = d.triples[n];
     const int i = pk & 0xff, j = (pk >> 8) & 0xff, k = (pk >> 16) & 0xff;
-    const double fac = (j == k ? 0.5 : 1.0) * (i == j ? 0.5 : 1.0);
-    const double denominator = epsabc - ((d.epsi[i] + d.epsi[j]) + d.epsi[k]);
+    const double2 ef = SPLIT ? d.tri_ef[n] : make_double2(0.0, 0.0);
+    const double fac = SPLIT ? ef.y : (j == k ? 0.5 : 1.0) * (i == j ? 0.5 : 1.0);
+    const double denominator =
+        epsabc - (SPLIT ? ef.x : (d.epsi[i] + d.epsi[j]) + d.epsi[k]);
     double value;
     if (distinct) {
       const double U = zval(Wz, s, No, i, j, k), V = zval(Wz, s, No, i, k, j),
@@ -256,7 +280,10 @@ __device__ __forceinline__ double energy_partial(const TcDesc &d, const double *
                    C = Tb[k + No * i + No * No * j];
       value = 3.0 * ((A * U + B * V) + C * W) - (A + (B + C)) * (U + (V + W));
     }
-    sum += (2.0 * value / denominator) * fac;
+    if constexpr (SPLIT)
+      sum = fma(value, recip_nr(denominator) * fac, sum);
+    else
+      sum += (2.0 * value / denominator) * fac;
   }
   return sum;
 }
@@ -335,39 +362,38 @@ struct MmaRole {
 // One slice of A times the slices of B that still give a kept level: result
 // columns sa P .. 8 P - 1, above N = 256 by two MMAs of about half of them.
 // NKK K steps (the run-time nkk of them where NKK is 0).
-template <int P, int SA, int NKK>
+template <class F, int P, int SA, int NKK>
 __device__ __forceinline__ void mma_slice(uint32_t d, uint64_t ad, uint64_t bd, int nkk,
                                           uint32_t acc) {
-  constexpr int n = ((kS - SA) * P + 15) & ~15;
+  constexpr int n = ((F::S - SA) * P + 15) & ~15;
   constexpr int n1 = n <= 256 ? n : ((n >> 1) + 15) & ~15, n2 = n - n1;
   constexpr int kMax = NKK ? NKK : kKChunk / 16;
 #pragma unroll
   for (int kk = 0; kk < kMax; ++kk)
     if (NKK || kk < nkk)
-      mma_bf16(d + SA * P, ad + 2 * kk, bd + 2 * kk, idesc_bf16_f32(128, n1),
-               kk == 0 && SA == 0 ? acc : 1u);
+      mma_bf16(d + SA * P, ad + 2 * kk, bd + 2 * kk, F::idesc(n1), kk == 0 && SA == 0 ? acc : 1u);
   if constexpr (n2 > 0) {
 #pragma unroll
     for (int kk = 0; kk < kMax; ++kk)
       if (NKK || kk < nkk)
-        mma_bf16(d + SA * P + n1, ad + 2 * kk, bd + n1 * 8 + 2 * kk, idesc_bf16_f32(128, n2),
+        mma_bf16(d + SA * P + n1, ad + 2 * kk, bd + n1 * 8 + 2 * kk, F::idesc(n2),
                  kk == 0 && SA == 0 ? acc : 1u);
   }
 }
 
-// A K chunk: the 8 slices of A from the ring, spp to a slot.
-template <int P, int SA, int NKK>
+// A K chunk: the slices of A from the ring, spp to a slot.
+template <class F, int P, int SA, int NKK>
 __device__ __forceinline__ bool mma_chunk(MmaRole &m, uint32_t d, uint64_t &ad, uint64_t bd,
                                           int nkk, uint32_t acc, int *status) {
-  if constexpr (SA < kS) {
-    if ((SA & (m.spp - 1)) == 0) {
+  if constexpr (SA < F::S) {
+    if (F::SPLIT ? SA == 0 : (SA & (m.spp - 1)) == 0) {
       if (!mbar_wait_warp(&m.afull[m.st], m.ph, status, kErrFull)) return false;
       tc_fence_after();
       ad = sdesc_sw128(0) + ((m.ring_a + (uint32_t)(m.st * m.aslot)) >> 4);
     }
-    if (m.leader) mma_slice<P, SA, NKK>(d, ad, bd, nkk, acc);
+    if (m.leader) mma_slice<F, P, SA, NKK>(d, ad, bd, nkk, acc);
     ad += (uint32_t)(m.rows * 8);
-    if ((SA & (m.spp - 1)) == m.spp - 1) {
+    if (F::SPLIT ? SA == F::S - 1 : (SA & (m.spp - 1)) == m.spp - 1) {
       if (m.leader) mma_commit(&m.aempty[m.st]);
       if (++m.st == m.nslots) {
         m.st = 0;
@@ -375,7 +401,7 @@ __device__ __forceinline__ bool mma_chunk(MmaRole &m, uint32_t d, uint64_t &ad, 
       }
     }
     __syncwarp();
-    return mma_chunk<P, SA + 1, NKK>(m, d, ad, bd, nkk, acc, status);
+    return mma_chunk<F, P, SA + 1, NKK>(m, d, ad, bd, nkk, acc, status);
   }
   return true;
 }
@@ -383,9 +409,9 @@ __device__ __forceinline__ bool mma_chunk(MmaRole &m, uint32_t d, uint64_t &ad, 
 // All items of a tuple.  The column count P is a template parameter so that
 // every MMA's column offset and instruction descriptor are constants: a warp
 // needs ~5 cycles for each instruction between two MMAs of 50 to 130.
-template <int P, bool CPLX>
+template <class F, int P>
 __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
-  constexpr int bufcols = kS * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
+  constexpr int bufcols = F::S * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
   for (int it = 0; it < m.nitems; ++it, ++m.item) {
     // barrier `item & 1` serves every second item, whichever columns the
     // item has: its use u is item 2u + (item & 1)
@@ -401,14 +427,14 @@ __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
     tc_fence_after();
     const uint32_t d = m.tm + buf * bufcols;
     uint32_t acc = 0;
-    for (int pt = 0; pt < TcParts<CPLX>::kCount; ++pt) {
-      const int K = TcParts<CPLX>::hole(pt) ? m.kh : m.kp;
+    for (int pt = 0; pt < TcParts<F::CPLX>::kCount; ++pt) {
+      const int K = TcParts<F::CPLX>::hole(pt) ? m.kh : m.kp;
       for (int k0 = 0; k0 < K; k0 += kKChunk) {
         const uint64_t bd = sdesc_sw128(0) + ((m.ring_b + (uint32_t)(m.bs * m.bslot)) >> 4);
         uint64_t ad = 0;
         const int nkk = (min(kKChunk, K - k0) + 15) / 16;
-        const bool ok = nkk == 4 ? mma_chunk<P, 0, 4>(m, d, ad, bd, 4, acc, status)
-                                 : mma_chunk<P, 0, 0>(m, d, ad, bd, nkk, acc, status);
+        const bool ok = nkk == 4 ? mma_chunk<F, P, 0, 4>(m, d, ad, bd, 4, acc, status)
+                                 : mma_chunk<F, P, 0, 0>(m, d, ad, bd, nkk, acc, status);
         if (!ok) return false;
         acc = 1;
         if (++m.bs == m.nbslots) m.bs = 0;
@@ -420,8 +446,10 @@ __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
   return true;
 }
 
-template <bool CPLX>
-__global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcArgs g) {
+template <class F>
+__global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g) {
+  constexpr bool CPLX = F::CPLX;
+  constexpr int S = F::S;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -479,7 +507,11 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
   const uint32_t tmem = *tmem_holder;
   const size_t cells = (size_t)g.lay_cells;
   constexpr int kComp = CPLX ? 2 : 1;
-  longlong2 *planes = g.planes + (size_t)blockIdx.x * 2 * g.lay_pass * 3 * kComp * cells;
+  // a W cell: the level sums joined exactly -- (high, low) halves of levels
+  // 0..3 and 4..7, or all levels of a split form in one integer
+  using Cell = typename std::conditional<F::SPLIT, long long, longlong2>::type;
+  Cell *planes =
+      static_cast<Cell *>(g.planes) + (size_t)blockIdx.x * 2 * g.lay_pass * 3 * kComp * cells;
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
@@ -540,7 +572,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
           npass = uniform(d->use_j) ? 2 : 1;
           spp = uniform(d->spp);
           a_bytes = spp * rows * 128;
-          b_bytes = kS * uniform(d->P) * 128;
+          b_bytes = S * uniform(d->P) * 128;
         }
         s.s = cur;
         s.t = __shfl_sync(0xffffffffu, pos, next);
@@ -564,7 +596,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
             const int c2 = CPLX ? p.blk : p.bz, c3 = CPLX ? p.by * kp + p.bz : p.by;
             for (int k0 = 0; k0 < K && alive; k0 += kKChunk) {
 #pragma unroll 1
-              for (int sa = 0; sa < kS; sa += spp) {
+              for (int sa = 0; sa < S; sa += spp) {
                 if (use > 0 && !mbar_wait_warp(&aempty[st], (use - 1) & 1, status, kErrEmpty)) {
                   alive = false;
                   break;
@@ -636,21 +668,21 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       }
       if constexpr (CPLX) {  // P = 2 round_up(No, 8)
         switch (m.P) {
-          case 16: alive = mma_tuple<16, true>(m, fresh, status); break;
-          case 32: alive = mma_tuple<32, true>(m, fresh, status); break;
-          case 48: alive = mma_tuple<48, true>(m, fresh, status); break;
-          default: alive = mma_tuple<64, true>(m, fresh, status); break;
+          case 16: alive = mma_tuple<F, 16>(m, fresh, status); break;
+          case 32: alive = mma_tuple<F, 32>(m, fresh, status); break;
+          case 48: alive = mma_tuple<F, 48>(m, fresh, status); break;
+          default: alive = mma_tuple<F, 64>(m, fresh, status); break;
         }
       } else {
         switch (m.P) {
-          case 8: alive = mma_tuple<8, false>(m, fresh, status); break;
-          case 16: alive = mma_tuple<16, false>(m, fresh, status); break;
-          case 24: alive = mma_tuple<24, false>(m, fresh, status); break;
-          case 32: alive = mma_tuple<32, false>(m, fresh, status); break;
-          case 40: alive = mma_tuple<40, false>(m, fresh, status); break;
-          case 48: alive = mma_tuple<48, false>(m, fresh, status); break;
-          case 56: alive = mma_tuple<56, false>(m, fresh, status); break;
-          default: alive = mma_tuple<64, false>(m, fresh, status); break;
+          case 8: alive = mma_tuple<F, 8>(m, fresh, status); break;
+          case 16: alive = mma_tuple<F, 16>(m, fresh, status); break;
+          case 24: alive = mma_tuple<F, 24>(m, fresh, status); break;
+          case 32: alive = mma_tuple<F, 32>(m, fresh, status); break;
+          case 40: alive = mma_tuple<F, 40>(m, fresh, status); break;
+          case 48: alive = mma_tuple<F, 48>(m, fresh, status); break;
+          case 56: alive = mma_tuple<F, 56>(m, fresh, status); break;
+          default: alive = mma_tuple<F, 64>(m, fresh, status); break;
         }
       }
     }
@@ -678,13 +710,13 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       if (!ok || t < 0) break;
       const int No = d.No, No2 = No * No, P = d.P, rows = d.rows;
       const int ntiles = (No2 + rows - 1) / rows, npass = d.use_j ? 2 : 1;
-      const int bufcols = kS * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
+      const int bufcols = S * P + (P & 8), nbuf = 2 * bufcols <= 512 ? 2 : 1;
       const int wb = k & 1;
       const uint32_t wuse = k >> 1;
       ok = wuse == 0 || mbar_wait(&wfree[wb], (wuse - 1) & 1, status, kErrEmpty);
       for (int it = 0; it < 3 * npass * ntiles; ++it, ++item) {
         const int gi = it / ntiles, mt = it - gi * ntiles, grp = gi % 3, pass = gi / 3;
-        longlong2 *plane0 = planes + (size_t)((wb * g.lay_pass + pass) * 3 + grp) * kComp * cells;
+        Cell *plane0 = planes + (size_t)((wb * g.lay_pass + pass) * 3 + grp) * kComp * cells;
         const int bb = item & 1, buf = nbuf == 2 ? bb : 0;
         bool okw = ok && alive && mbar_wait(&accf[bb], (item >> 1) & 1, status, kErrAccFull);
         okw = bar_and(1, 128, okw);
@@ -701,11 +733,11 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
           // column block (component) and its next 8 columns
           const int comp = kComp == 2 && cc >= No ? 1 : 0, c0 = cc - comp * No;
           cc += min(8, No - c0);
-          longlong2 *plane = plane0 + comp * cells;
-          float v[kS][8];
+          Cell *plane = plane0 + comp * cells;
+          float v[S][8];
           __syncwarp();
 #pragma unroll
-          for (int L = 0; L < kS; ++L) tmem_ld8(tbase + L * P + comp * P1 + c0, v[L]);
+          for (int L = 0; L < S; ++L) tmem_ld8(tbase + L * P + comp * P1 + c0, v[L]);
           tmem_wait_ld();
           if (cc == kComp * No) {  // everything is read: the accumulator is free
             tc_fence_before();
@@ -714,15 +746,23 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
 #pragma unroll
           for (int x = 0; x < 8; ++x) {
             const int r = c0 + x;
-            if (r < No && valid) {
+            if constexpr (F::SPLIT) {
+              if (r < No && valid) {
+                long long n = __float2int_rn(v[0][x]);
+#pragma unroll
+                for (int L = 1; L < S; ++L)
+                  n = n * F::radix() + __float2int_rn(v[L][x]);
+                plane[(size_t)r * No2 + m] = n;
+              }
+            } else if (r < No && valid) {
               // |level sum| < 2^22 for L >= 1 (flagged otherwise): adding
               // 1.5 2^23 leaves the integer n in the low mantissa bits b =
               // n + kBits.  Pairs of levels join in 32 bits (256 n + n' <
               // 2^31; the kBits cancel modulo 2^32), pairs of pairs in 64.
               constexpr uint32_t kBits = 0x4B400000u;
-              uint32_t b[kS];
+              uint32_t b[S];
 #pragma unroll
-              for (int L = 1; L < kS; ++L) {
+              for (int L = 1; L < S; ++L) {
                 b[L] = __float_as_uint(v[L][x] + 12582912.f);
                 over |= b[L] ^ 0x4B000000u;  // exponent bits differ outside that range
               }
@@ -776,13 +816,13 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
       const int npass = d.use_j ? 2 : 1;
       for (int pc = 0; pc < npass * kComp; ++pc) {
         const int pass = pc / kComp, comp = pc % kComp;
-        const longlong2 *p0 =
+        const Cell *p0 =
             planes + (size_t)((wb * g.lay_pass + pass) * 3 * kComp + comp) * cells;
-        const longlong2 *p1 = p0 + kComp * cells, *p2 = p1 + kComp * cells;
+        const Cell *p1 = p0 + kComp * cells, *p2 = p1 + kComp * cells;
         double *W = wd + pc * cells;
         constexpr int kU = 4;
         for (int i0 = er; i0 < No3; i0 += kU * kEnergyThreads) {
-          longlong2 v[kU][3];
+          Cell v[kU][3];
 #pragma unroll
           for (int u = 0; u < kU; ++u) {
             const int idx = i0 + u * kEnergyThreads;
@@ -798,10 +838,14 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
           for (int u = 0; u < kU; ++u) {
             const int idx = i0 + u * kEnergyThreads;
             if (idx < No3) {
-              // both sums are exact; one rounding where they are joined
-              const long long hi = v[u][0].x + v[u][1].x + v[u][2].x;
-              const long long lo = v[u][0].y + v[u][1].y + v[u][2].y;
-              W[idx] = fma(i64_to_f64(lo), 0x1p-32, i64_to_f64(hi));
+              if constexpr (F::SPLIT) {  // below 2^50: exact
+                W[idx] = i64_to_f64(v[u][0] + v[u][1] + v[u][2]);
+              } else {
+                // both sums are exact; one rounding where they are joined
+                const long long hi = v[u][0].x + v[u][1].x + v[u][2].x;
+                const long long lo = v[u][0].y + v[u][1].y + v[u][2].y;
+                W[idx] = fma(i64_to_f64(lo), 0x1p-32, i64_to_f64(hi));
+              }
             }
           }
         }
@@ -828,7 +872,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_fp64_tc_kernel(const TcAr
             sum = energy_partial_z(d, wd + pass * 2 * cells, wd, cells, sc, cls == 0, epsabc, er);
         } else {
           const TcSinglesCtx sc = {Vbc, Vac, Vab, ta, tb, tc};
-          if (ok) sum = energy_partial(d, wd + pass * cells, wd, sc, cls == 0, epsabc, er);
+          if (ok) sum = energy_partial<F::SPLIT>(d, wd + pass * cells, wd, sc, cls == 0, epsabc, er);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -941,6 +985,8 @@ __global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
 // ------------------------------------------------------------------ host
 
 struct TcImpl {
+  int S = kS;
+  bool split = false, f16 = false;
   int nc = 1;  // doubles per element: 2 for a complex system
   int No = 0, Nv = 0, P = 0, rows = 0, spp = 0, Kp = 0, Kh = 0;
   int eT = 0, eV = 0, eJ = 0;
@@ -991,7 +1037,8 @@ int make_map(CUtensorMap *m, void *base, int rank, const uint64_t *dims, const u
 }
 
 int map_a(CUtensorMap *m, void *base, const TcImpl &p, int K) {
-  const uint64_t d[4] = {(uint64_t)K, (uint64_t)p.No * p.No, (uint64_t)p.Nv, kS};
+  const uint64_t d[4] = {(uint64_t)K, (uint64_t)p.No * p.No, (uint64_t)p.Nv,
+                         (uint64_t)p.S};
   const uint32_t box[4] = {kKChunk, (uint32_t)p.rows, 1, (uint32_t)p.spp};
   return make_map(m, base, 4, d, box);
 }
@@ -1001,8 +1048,9 @@ int map_b(CUtensorMap *m, void *base, const TcImpl &p, int K) {
     const uint32_t box[5] = {kKChunk, (uint32_t)p.P / 2, 2, 1, kS};
     return make_map(m, base, 5, d, box);
   }
-  const uint64_t d[5] = {(uint64_t)K, (uint64_t)p.No, (uint64_t)p.Nv, (uint64_t)p.Nv, kS};
-  const uint32_t box[5] = {kKChunk, (uint32_t)p.P, 1, 1, kS};
+  const uint64_t d[5] = {(uint64_t)K, (uint64_t)p.No, (uint64_t)p.Nv, (uint64_t)p.Nv,
+                         (uint64_t)p.S};
+  const uint32_t box[5] = {kKChunk, (uint32_t)p.P, 1, 1, (uint32_t)p.S};
   return make_map(m, base, 5, d, box);
 }
 
@@ -1143,6 +1191,12 @@ struct ScopedDevice {  // device allocation freed on scope exit
   ~ScopedDevice() { cudaFree(p); }
 };
 
+// Rows of an item: the No^2 rows in equal shares of at most 128.
+int item_rows(int No) {
+  const int nt = (No * No + 127) / 128;
+  return ((No * No + nt - 1) / nt + 7) / 8 * 8;
+}
+
 int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cplx,
                  cudaStream_t st, int64_t *launches) {
   auto *p = new TcImpl();
@@ -1151,9 +1205,7 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cpl
   p->No = No_;
   p->Nv = Nv_;
   p->P = p->nc * ((No_ + 7) / 8 * 8);
-  // rows of an item: the No^2 rows in equal shares of at most 128
-  const int nt = (No_ * No_ + 127) / 128;
-  p->rows = ((No_ * No_ + nt - 1) / nt + 7) / 8 * 8;
+  p->rows = item_rows(No_);
   // slices per copy (a ring slot): up to 32 KB.  A role's warp needs ~200
   // cycles for a wait and a signal whatever the size, so a slot should hold
   // several MMAs' work
@@ -1312,6 +1364,48 @@ void tc_free(TcState &s) {
 // system takes the same kernel.  Cutting the slices costs ~2 ms in
 // allocations, launches and tensor maps the first time, about what the DFMA
 // kernel needs for 1e9 FLOPs at these sizes (No=4/Nv=12, 4.5e6: 0.1 ms).
+int tc_split_attach(TcState &s, int S, bool f16, int No, int Nv, int Kp, double unit,
+                    void *const *ops) {
+  tc_free(s);
+  auto *p = new TcImpl();
+  s.impl = p;
+  p->S = S;
+  p->split = true;
+  p->f16 = f16;
+  p->No = No;
+  p->Nv = Nv;
+  p->P = (No + 7) / 8 * 8;
+  p->rows = item_rows(No);
+  p->spp = S;
+  p->Kp = Kp;
+  p->Kh = kKChunk;
+  // level 0 of a cell carries S - 1 radices more
+  p->unit = std::ldexp(unit, -(f16 ? 11 : 8) * (S - 1));
+  int rc;
+  for (int i = 0; i < 4; ++i)
+    if ((rc = map_a(&p->maps.Ta[i / 2][i % 2], ops[i % 2], *p, p->Kp)) ||
+        (rc = map_a(&p->maps.Vh[i / 2][i % 2], ops[2 + i % 2], *p, p->Kh)))
+      return rc;
+  if ((rc = map_b(&p->maps.Vp, ops[4], *p, p->Kp)) || (rc = map_b(&p->maps.TpN, ops[5], *p, p->Kh)) ||
+      (rc = map_b(&p->maps.TpT, ops[6], *p, p->Kh)))
+    return rc;
+  std::memcpy(p->maps.Jh, p->maps.Vh, sizeof(p->maps.Jh));
+  p->maps.Jp = p->maps.Vp;
+  s.tried = s.usable = true;
+  return ATRIP_OK;
+}
+
+int tc_split_attach_j(TcState &s, double unit_j, void *const *ops) {
+  auto *p = static_cast<TcImpl *>(s.impl);
+  p->unit_j = std::ldexp(unit_j, -(p->f16 ? 11 : 8) * (p->S - 1));
+  int rc;
+  for (int i = 0; i < 4; ++i)
+    if ((rc = map_a(&p->maps.Jh[i / 2][i % 2], ops[i % 2], *p, p->Kh))) return rc;
+  if ((rc = map_b(&p->maps.Jp, ops[2], *p, p->Kp))) return rc;
+  s.tried_j = s.usable_j = true;
+  return ATRIP_OK;
+}
+
 bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx) {
   // complex: the columns of both components of 8 levels fill TMEM at No = 32
   const double flops = (cplx ? 4.0 : 1.0) * (double)n_tuples * 12.0 * No * No * No * (No + Nv);
@@ -1389,6 +1483,11 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   if (!b.d_queue) ATRIP_CUDA_TRY(cudaMalloc(&b.d_queue, sizeof(unsigned long long)));
   auto *h = static_cast<TcDesc *>(b.h_desc);
   int P = 0, spp = 1;
+  const auto *p0 = static_cast<const TcImpl *>(n > 0 ? sys[0].state->impl : nullptr);
+  const int S = p0 ? p0->S : kS;
+  b.S = S;
+  b.split = p0 && p0->split;
+  b.f16 = p0 && p0->f16;
   b.lay_no = 0;
   b.lay_pass = 1;
   b.aslot = 0;
@@ -1397,7 +1496,8 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   for (int k = 0; k < n; ++k) {
     const TcSystem &m = sys[k];
     auto *p = static_cast<TcImpl *>(m.state->impl);
-    if (!p || !m.state->usable || (m.use_j && !m.state->usable_j)) {
+    if (!p || !m.state->usable || (m.use_j && !m.state->usable_j) || p->S != S ||
+        p->split != b.split || p->f16 != b.f16) {
       set_error("tensor-core FP64 form: operands not prepared");
       return ATRIP_ERR_STATE;
     }
@@ -1410,6 +1510,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     d.Vhh = m.dt->Vhh;
     d.tuples = m.tuples;
     d.triples = m.triples;
+    d.tri_ef = m.tri_ef;
     d.e = m.e;
     d.ect = m.ect;
     d.unit = p->unit;
@@ -1437,11 +1538,14 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   b.grid = (int)std::min<int64_t>(b.total, sm_count);
   b.lay_cells = b.lay_no * b.lay_no * b.lay_no;
   // stack of 8 slices of P rows; an MMA's N, a multiple of 16, may read 8 rows more
-  b.bslot = kS * P * 128 + 1024;
-  // rings: a K chunk takes 8 / spp A slots and one B slot, of which there is
-  // one more than chunks (of the largest slots) can be in flight
+  b.bslot = S * P * 128 + 1024;
+  // rings: a K chunk takes S / spp A slots and one B slot, which must be free
+  // by the time its first A slot is: chunk c's first slot is waited for until
+  // the MMAs of the slot nslots before it are done, and the chunk nb before c
+  // ends at or before that one if (nb - 1) chunks have nslots - 1 slots
   const int room = kSmemLimit - 1024 - kTailBytes;
-  auto b_for = [&](int nslots) { return (nslots * spp + kS - 1) / kS + 1; };
+  const int per_chunk = S / spp;  // of the system with the fewest A slots a chunk
+  auto b_for = [&](int nslots) { return (nslots - 1 + per_chunk - 1) / per_chunk + 1; };
   b.nslots = kMaxSlots;
   while (b.nslots > 1 && b.nslots * b.aslot + b_for(b.nslots) * b.bslot > room) --b.nslots;
   b.nbslots = b_for(b.nslots);
@@ -1450,7 +1554,8 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     return ATRIP_ERR_UNSUPPORTED;
   }
   b.smem = 1024 + (size_t)b.nslots * b.aslot + (size_t)b.nbslots * b.bslot + kTailBytes;
-  const size_t per_cta = ((size_t)2 * 3 * 16 + 8) * b.nc * b.lay_pass * b.lay_cells;
+  const size_t cell = b.split ? 8 : 16;
+  const size_t per_cta = (2 * 3 * cell + 8) * b.nc * b.lay_pass * b.lay_cells;
   const size_t need = per_cta * std::max(b.grid, 1);
   if (need > b.planes_bytes) {
     cudaFree(b.planes);
@@ -1481,16 +1586,21 @@ int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st
   a.order = order;
   a.queue = b.d_queue;
   a.flags = b.d_flags;
-  a.planes = static_cast<longlong2 *>(b.planes);
+  a.planes = b.planes;
   a.wd = reinterpret_cast<double *>(static_cast<char *>(b.planes) +
-                                    (size_t)b.grid * 2 * 3 * 16 * b.nc * b.lay_pass * b.lay_cells);
+                                    (size_t)b.grid * 2 * 3 * (b.split ? 8 : 16) * b.nc * b.lay_pass * b.lay_cells);
   a.lay_cells = b.lay_cells;
   a.lay_pass = b.lay_pass;
   a.nslots = b.nslots;
   a.nbslots = b.nbslots;
   a.aslot = b.aslot;
   a.bslot = b.bslot;
-  auto kern = b.nc == 2 ? triples_fp64_tc_kernel<true> : triples_fp64_tc_kernel<false>;
+  auto kern = b.nc == 2 ? triples_tc_kernel<FmtZ> : triples_tc_kernel<FmtFp64>;
+  if (b.split)
+    kern = b.f16    ? triples_tc_kernel<Fmt<2, false, true, true>>
+           : b.S == 2 ? triples_tc_kernel<Fmt<2, false, true, false>>
+           : b.S == 3 ? triples_tc_kernel<Fmt<3, false, true, false>>
+                      : triples_tc_kernel<Fmt<4, false, true, false>>;
   ATRIP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)b.smem));
   kern<<<b.grid, kThreads, b.smem, st>>>(a);

@@ -157,8 +157,10 @@ int atrip_gpu_run(atrip_gpu_context *ctx, const atrip_run_options *opts, atrip_r
 
 /* Launch parameters chosen by the autotuner (atrip_gb300/autotune.py);
  * a zero field keeps the built-in choice.  The fp64_* fields and
- * tuples_per_claim describe the kernel of FP64 instructions: one that is set
- * selects that kernel for the FP64 form.  No counterpart in the reference,
+ * tuples_per_claim describe the kernel of FP64 instructions, the split_*
+ * fields the split forms' own kernels: one that is set selects those for its
+ * form, where otherwise all forms run on one tensor-core kernel within its
+ * limits.  No counterpart in the reference,
  * whose only tuning knob for this loop is the tuple distribution.          */
 typedef struct {
   int32_t fp64_ctas_per_sm; /* FP64 form: resident CTAs per SM (0 = occupancy max) */
@@ -178,7 +180,8 @@ typedef struct {
                             /* so the tuples in flight share their a, b, c slabs   */
                             /* in L2 (results are unchanged: per-tuple energies    */
                             /* stay indexed by list position)                      */
-  int32_t split_variant;    /* split form kernel: 0/1 = M tiles of (p,q) rows;     */
+  int32_t split_variant;    /* split form kernel: 0 = the engine's choice;         */
+                            /* 1 = M tiles of (p,q) rows;                          */
                             /* 2 = transposed (the S slices of V stacked as the    */
                             /* M rows, up to 256 (p,q) pairs as N) where S No <=   */
                             /* 128 and 2 (Nv + No) <= 1024, else variant 1;        */

@@ -134,3 +134,27 @@ def test_noalloc_tensor_cores(No, Nv, j, spoil):
     _close(got[2:2 + n], e, K)
     _close(got[2 + n:], ect, K)
     assert abs(got[0] - r.energy) <= K * 2.0 ** -52 * np.sum(np.abs(e))
+
+
+# split forms without launch parameters: the same digit products on the kernel
+# of the FP64 form.  The kernels a variant selects round the levels above 0 to
+# FP32 (2^-24 of a part 2^-8 of W or smaller, three groups, both factors of an
+# energy): 2^-28 of the largest tuple energy.
+@pytest.mark.parametrize("form,S", [("split_bf16", 2), ("split_bf16", 3), ("split_bf16", 4),
+                                    ("split_f16", 2)])
+@pytest.mark.parametrize("No,Nv,j", [(1, 9, False), (3, 17, True), (8, 40, False), (13, 64, True),
+                                     (24, 30, True), (33, 17, False), (41, 65, False),
+                                     (64, 10, True)])
+def test_split_forms_match_split_kernels(No, Nv, j, form, S):
+    d = synth.make_inputs(No, Nv, 15, with_j=j)
+    n = min(synth.n_tuples(Nv), 600)
+    with _ctx(d, j) as ctx:
+        kw = dict(form=form, slices=S, use_j=j, max_iterations=n - 1, ijkabc=True)
+        r = ctx.run(**kw)
+        e, ect = ctx.tuple_energies(0, n)
+        ctx.set_tuning(split_variant=2 if form == "split_f16" else 1)
+        v = ctx.run(**kw)
+        f, fct = ctx.tuple_energies(0, n)
+    assert np.max(np.abs(e - f)) <= 2.0 ** -28 * np.max(np.abs(f))
+    assert np.max(np.abs(ect - fct)) <= 2.0 ** -28 * np.max(np.abs(fct))
+    assert abs(r.energy - v.energy) <= 2.0 ** -28 * np.sum(np.abs(f))
