@@ -107,8 +107,10 @@ __device__ void build_w(const TriplesArgs &g, Smem &sm, double *W, const double 
             sm.Bs[kk][col] = val;
           }
           __syncthreads();
-#pragma unroll 8
-          for (int kk = 0; kk < kKC; ++kk) {
+          // nothing for K past the operands' end, nor (rows are dealt out 4 to
+          // a warp) for a warp whose rows lie past No^2: the FP64 pipe takes
+          // 16 cycles for a warp's FMA, padding or not (No=4/Nv=12: 90 % of them)
+          auto step = [&](int kk) {
             double av[RU];
 #pragma unroll
             for (int u = 0; u < RU; ++u) av[u] = sm.As[kk][ty + 32 * u];
@@ -118,6 +120,14 @@ __device__ void build_w(const TriplesArgs &g, Smem &sm, double *W, const double 
 #pragma unroll
               for (int u = 0; u < RU; ++u) acc[u][v] = fma(av[u], bv, acc[u][v]);
             }
+          };
+          const int kn = min(kKC, K - k0);
+          if (kn == kKC && m0 + MT <= No2) {
+#pragma unroll 8
+            for (int kk = 0; kk < kKC; ++kk) step(kk);
+          } else if (m0 + (tid >> 5) * 4 < No2) {
+#pragma unroll 4
+            for (int kk = 0; kk < kn; ++kk) step(kk);
           }
           __syncthreads();
         }
