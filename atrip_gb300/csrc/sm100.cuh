@@ -178,6 +178,29 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
       : "memory");
 }
 
+// The same and its commit for one lane of a converged warp (lane_on there, 0
+// elsewhere), as predicated instructions: a branch on the lane and the warp's
+// reconvergence after it cost the issuer ~20 cycles an MMA (No=8/Nv=40, whole
+// list: 1.08 -> 0.94 ms).
+__device__ __forceinline__ void mma_if(uint32_t lane_on, uint32_t d_tmem, uint64_t adesc,
+                                       uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lane_on)
+      : "memory");
+}
+__device__ __forceinline__ void commit_if(uint32_t lane_on, uint64_t *bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          smem_u32(bar)), "r"(lane_on)
+      : "memory");
+}
+
 // 32 lanes x 32 bit, 16 consecutive columns per thread.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];

@@ -348,6 +348,7 @@ __device__ __forceinline__ double energy_partial_z(const TcDesc &d, const double
   return sum;
 }
 
+
 // The MMA issuer's state, carried from tuple to tuple.
 struct MmaRole {
   int st, bs;              // A and B ring slots of the next operands
@@ -363,7 +364,7 @@ struct MmaRole {
 // columns sa P .. 8 P - 1, above N = 256 by two MMAs of about half of them.
 // NKK K steps (the run-time nkk of them where NKK is 0).
 template <class F, int P, int SA, int NKK>
-__device__ __forceinline__ void mma_slice(uint32_t d, uint64_t ad, uint64_t bd, int nkk,
+__device__ __forceinline__ void mma_slice(uint32_t on, uint32_t d, uint64_t ad, uint64_t bd, int nkk,
                                           uint32_t acc) {
   constexpr int n = ((F::S - SA) * P + 15) & ~15;
   constexpr int n1 = n <= 256 ? n : ((n >> 1) + 15) & ~15, n2 = n - n1;
@@ -371,12 +372,12 @@ __device__ __forceinline__ void mma_slice(uint32_t d, uint64_t ad, uint64_t bd, 
 #pragma unroll
   for (int kk = 0; kk < kMax; ++kk)
     if (NKK || kk < nkk)
-      mma_bf16(d + SA * P, ad + 2 * kk, bd + 2 * kk, F::idesc(n1), kk == 0 && SA == 0 ? acc : 1u);
+      mma_if(on, d + SA * P, ad + 2 * kk, bd + 2 * kk, F::idesc(n1), kk == 0 && SA == 0 ? acc : 1u);
   if constexpr (n2 > 0) {
 #pragma unroll
     for (int kk = 0; kk < kMax; ++kk)
       if (NKK || kk < nkk)
-        mma_bf16(d + SA * P + n1, ad + 2 * kk, bd + n1 * 8 + 2 * kk, F::idesc(n2),
+        mma_if(on, d + SA * P + n1, ad + 2 * kk, bd + n1 * 8 + 2 * kk, F::idesc(n2),
                  kk == 0 && SA == 0 ? acc : 1u);
   }
 }
@@ -391,16 +392,15 @@ __device__ __forceinline__ bool mma_chunk(MmaRole &m, uint32_t d, uint64_t &ad, 
       tc_fence_after();
       ad = sdesc_sw128(0) + ((m.ring_a + (uint32_t)(m.st * m.aslot)) >> 4);
     }
-    if (m.leader) mma_slice<F, P, SA, NKK>(d, ad, bd, nkk, acc);
+    mma_slice<F, P, SA, NKK>(m.leader, d, ad, bd, nkk, acc);
     ad += (uint32_t)(m.rows * 8);
     if (F::SPLIT ? SA == F::S - 1 : (SA & (m.spp - 1)) == m.spp - 1) {
-      if (m.leader) mma_commit(&m.aempty[m.st]);
+      commit_if(m.leader, &m.aempty[m.st]);
       if (++m.st == m.nslots) {
         m.st = 0;
         m.ph ^= 1u;
       }
     }
-    __syncwarp();
     return mma_chunk<F, P, SA + 1, NKK>(m, d, ad, bd, nkk, acc, status);
   }
   return true;
@@ -440,8 +440,7 @@ __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
         if (++m.bs == m.nbslots) m.bs = 0;
       }
     }
-    if (m.leader) mma_commit(&m.accf[bb]);
-    __syncwarp();
+    commit_if(m.leader, &m.accf[bb]);
   }
   return true;
 }
@@ -1209,7 +1208,7 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cpl
   // slices per copy (a ring slot): up to 32 KB.  A role's warp needs ~200
   // cycles for a wait and a signal whatever the size, so a slot should hold
   // several MMAs' work
-  p->spp = p->rows > 64 ? 2 : 4;
+  p->spp = p->rows > 104 ? 2 : 4;
   p->Kp = (Nv_ + kKChunk - 1) / kKChunk * kKChunk;
   p->Kh = kKChunk;
   const int64_t No = No_, Nv = Nv_, No2 = No * No, nc = p->nc, nblk = cplx ? kBlocksZ : 1;
