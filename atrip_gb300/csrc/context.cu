@@ -372,12 +372,22 @@ int atrip_gpu_create(const atrip_dims *dims, atrip_gpu_context **out) {
                           cudaMemcpyHostToDevice));
     c->h_tuples.swap(h);
   }
-  // (i >= j >= k) triples in the loop order of src/atrip/Equations.cxx:111-124
+  // (i >= j >= k) triples of the energy loop (src/atrip/Equations.cxx:111-124),
+  // beyond No = 20 in blocks of 4 x 4 x 2: each permuted W[..] a warp gathers
+  // then comes in runs of 4 (or 2) elements instead of one per 32-byte sector
+  // (No=37/Nv=151 with (cT) 8.0 -> 7.7 ms; No=4..20, whose W stays in L1 and
+  // L2, 2 % slower)
   {
     std::vector<uint32_t> h;
-    for (uint32_t k = 0; k < (uint32_t)c->No; ++k)
-      for (uint32_t j = k; j < (uint32_t)c->No; ++j)
-        for (uint32_t i = j; i < (uint32_t)c->No; ++i) h.push_back(i | (j << 8) | (k << 16));
+    const uint32_t no = (uint32_t)c->No;
+    const uint32_t bk = no > 20 ? 2 : 1, bj = no > 20 ? 4 : 1, bi = no > 20 ? 4 : no;
+    for (uint32_t k0 = 0; k0 < no; k0 += bk)
+      for (uint32_t j0 = k0 / bj * bj; j0 < no; j0 += bj)
+        for (uint32_t i0 = j0 / bi * bi; i0 < no; i0 += bi)
+          for (uint32_t k = k0; k < std::min(k0 + bk, no); ++k)
+            for (uint32_t j = std::max(j0, k); j < std::min(j0 + bj, no); ++j)
+              for (uint32_t i = std::max(i0, j); i < std::min(i0 + bi, no); ++i)
+                h.push_back(i | (j << 8) | (k << 16));
     c->n_triples = (int)h.size();
     CREATE_TRY(cudaMalloc(&c->d_triples, sizeof(uint32_t) * h.size()));
     CREATE_TRY(cudaMemcpy(c->d_triples, h.data(), sizeof(uint32_t) * h.size(),

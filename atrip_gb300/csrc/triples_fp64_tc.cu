@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
       if (er == 0) mbar_arrive(&tempty[ts]);
       if (!ok || s.t < 0) break;
       const TcDesc &d = g.sys[s.s];
-      const int No = d.No, No2 = No * No, No3 = No2 * No;
+      const int No = d.No, No2 = No * No;
       const int64_t Nv = d.Nv;
       const int a = s.a, b = s.b, c = s.c;
       // W, Z and the singles in units of a cell's high part (a power of two)
@@ -811,32 +811,55 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
       }
       const int wb = k & 1;
       ok = mbar_wait(&wfull[wb], (k >> 1) & 1, status, kErrAccFull);
-      const uint32_t magic = 0xffffffffu / (uint32_t)No + 1u;  // idx / No = umulhi, idx < 2^18
       const int npass = d.use_j ? 2 : 1;
+      // x / n = umulhi(x, by_n) for x < 2^18 and 2 <= n <= 64
+      const uint32_t by_no = 0xffffffffu / (uint32_t)No + 1u;
+      const uint32_t by_ti = 0xffffffffu / (uint32_t)((No + 7) >> 3) + 1u;
+      const uint32_t by_tj = 0xffffffffu / (uint32_t)((No + 3) >> 2) + 1u;
       for (int pc = 0; pc < npass * kComp; ++pc) {
         const int pass = pc / kComp, comp = pc % kComp;
         const Cell *p0 =
             planes + (size_t)((wb * g.lay_pass + pass) * 3 * kComp + comp) * cells;
         const Cell *p1 = p0 + kComp * cells, *p2 = p1 + kComp * cells;
         double *W = wd + pc * cells;
+        // a warp takes 8 x 4 elements (i,j) of one k: every plane's cells then
+        // come in whole 32-byte sectors (group 2's run along j); No=37/Nv=151
+        // with (cT) 8.4 -> 8.0 ms, No=24/Nv=240 in 3 BF16 slices 9.0 -> 8.4 ms.
+        // Few orbitals, whose cells stay in L2 and fill such tiles badly, are
+        // taken in order (No=4..20: tiles 2 % slower)
         constexpr int kU = 4;
-        for (int i0 = er; i0 < No3; i0 += kU * kEnergyThreads) {
+        const bool tiled = No > 20;
+        const int ti = tiled ? (No + 7) >> 3 : 1, tj = (No + 3) >> 2;
+        const int tiles = tiled ? ti * tj * No : (No * No2 + 31) >> 5;
+        for (int t0 = er >> 5; t0 < tiles; t0 += kU * kEnergyWarps) {
           Cell v[kU][3];
+          int at[kU];
 #pragma unroll
           for (int u = 0; u < kU; ++u) {
-            const int idx = i0 + u * kEnergyThreads;
-            if (idx < No3) {
-              const int jk = No == 1 ? idx : (int)__umulhi((uint32_t)idx, magic), i = idx - jk * No;
-              const int kx = No == 1 ? jk : (int)__umulhi((uint32_t)jk, magic), j = jk - kx * No;
-              v[u][0] = p0[idx];
+            const int t = t0 + u * kEnergyWarps;
+            int i, j, kx;
+            if (tiled) {
+              const int r = (int)__umulhi((uint32_t)t, by_ti);
+              kx = (int)__umulhi((uint32_t)r, by_tj);
+              i = (t - r * ti) * 8 + (lane & 7);
+              j = (r - kx * tj) * 4 + (lane >> 3);
+            } else {
+              const int idx = t * 32 + lane, jk = (int)__umulhi((uint32_t)idx, by_no);
+              i = idx - jk * No;
+              kx = (int)__umulhi((uint32_t)jk, by_no);
+              j = jk - kx * No;
+            }
+            at[u] = t < tiles && i < No && j < No && kx < No ? i + No * j + No2 * kx : -1;
+            if (at[u] >= 0) {
+              v[u][0] = p0[at[u]];
               v[u][1] = p1[j * No2 + i + No * kx];
               v[u][2] = p2[i * No2 + j + No * kx];
             }
           }
 #pragma unroll
           for (int u = 0; u < kU; ++u) {
-            const int idx = i0 + u * kEnergyThreads;
-            if (idx < No3) {
+            const int idx = at[u];
+            if (idx >= 0) {
               if constexpr (F::SPLIT) {  // below 2^50: exact
                 W[idx] = i64_to_f64(v[u][0] + v[u][1] + v[u][2]);
               } else {

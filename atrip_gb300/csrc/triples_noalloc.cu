@@ -410,6 +410,7 @@ struct Tail {
   int abc[3];
   double ta[64], tb[64], tc[64];
   double red[kThreads / 32];
+  int row[2][128];  // p + No q of the tile's rows, p fastest and q fastest
 };
 
 __device__ __forceinline__ double i64_to_f64(long long n) {  // |n| < 2^51
@@ -463,6 +464,13 @@ __device__ bool build_w(const Args &g, Header *h, Tail &t, unsigned char *At, un
   const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   for (int grp = 0; grp < 3; ++grp)
     for (int mt = 0; mt < nt; ++mt) {
+      const int m0 = mt * rows;
+      for (int m = threadIdx.x; m < rows; m += kThreads) {  // read again after the last drain
+        const int sl = (m0 + m) / No, f = (m0 + m) - sl * No;
+        t.row[0][m] = f + No * sl;
+        t.row[1][m] = sl + No * f;
+      }
+      __syncthreads();
       int held = 0;         // K in the accumulator
       bool first = grp == 0;  // the first piece of the first group stores W
       for (int pt = 0; pt < 4; ++pt) {
@@ -482,27 +490,27 @@ __device__ bool build_w(const Args &g, Header *h, Tail &t, unsigned char *At, un
         for (int k0 = 0; k0 < K; k0 += kChunk) {
           const int kc = min(kChunk, K - k0);
           // A: rows (p,q) of this tile, p fastest (natural) or q (transposed)
-          const int m0 = mt * rows;
-          const int64_t sf = tr ? No : 1, ss = tr ? 1 : No;  // p + No q of (f, slow)
-          const double *T = g.T, *Vh = ps.Vh, *Vp = ps.Vp;
-          if (!hole)
-            cut_rows(At, kATile, 0, min(rows, No2 - m0), h->e_t, k0, K, [&](int m, int k) {
-              const int sl = (m0 + m) / No, f = (m0 + m) - sl * No;
-              return T[x + k * Nv + (f * sf + sl * ss) * NvNv];  // T[x,E,p,q]
+          const int nrows = min(rows, No2 - m0);
+          const int *row = t.row[tr];
+          if (!hole) {
+            const double *T = g.T + x;
+            cut_rows(At, kATile, 0, nrows, h->e_t, k0, K, [&](int m, int k) {
+              return T[k * Nv + row[m] * NvNv];  // T[x,E,p,q]
             });
-          else
-            cut_rows(At, kATile, 0, min(rows, No2 - m0), ps.e, k0, K, [&](int m, int k) {
-              const int sl = (m0 + m) / No, f = (m0 + m) - sl * No;
-              return Vh[f * sf + sl * ss + (int64_t)k * No2 + (int64_t)w * No2 * No];
+          } else {
+            const double *Vh = ps.Vh + (int64_t)w * No2 * No;
+            cut_rows(At, kATile, 0, nrows, ps.e, k0, K, [&](int m, int k) {
+              return Vh[row[m] + k * No2];  // Vh[p,q,L,w]
             });
+          }
           // B: columns r
           if (!hole)
             cut_rows(Bt, P * 128, 0, No, ps.e, k0, K, [&](int r, int k) {
-              return Vp[y + z * Nv + k * NvNv + r * NvNv * Nv];  // Vp[y,z,E,r]
+              return ps.Vp[y + z * Nv + (k + r * Nv) * NvNv];  // Vp[y,z,E,r]
             });
           else
             cut_rows(Bt, P * 128, 0, No, h->e_t, k0, K, [&](int r, int k) {
-              return -T[u + v * Nv + (flip ? r + (int64_t)No * k : k + (int64_t)No * r) * NvNv];
+              return -g.T[u + v * Nv + (flip ? r + No * k : k + No * r) * NvNv];
             });
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           tc_fence_before();
