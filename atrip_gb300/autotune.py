@@ -285,17 +285,15 @@ def tune_batch(batch: capi.Batch, window: int = 256) -> dict:
 
 
 def tune_batch_tiles(contexts, window: int = 256) -> list:
-    """Per-system FP64 row tile (32 or 64), timed on a window of each."""
+    """Per system, timed on a window of each: the engine's own FP64 kernel (0:
+    the tensor-core kernel where it applies) or the row tile (32 or 64) of the
+    kernel of FP64 instructions."""
     out = []
     for ctx in contexts:
-        if ctx.No > 16:
-            ctx.set_tuning(fp64_tile_rows=64)
-            out.append(64)
-            continue
         n = capi.n_tuples(ctx.Nv)
         wins = [(0, min(n, window))]
         t = {}
-        for rows in (64, 32):
+        for rows in (0, 64, 32) if ctx.No <= 16 else (0, 64):
             t[rows] = _time(ctx, wins, "fp64", 0, {"fp64_tile_rows": rows})
         rows = min(t, key=t.get)
         ctx.set_tuning(fp64_tile_rows=rows)

@@ -302,15 +302,14 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
       return ATRIP_OK;
     };
     b->multi_used = false;
-    // one launch of the kernel of fp64_tc.cuh unless a launch parameter of the
-    // split kernels is set, for the batch or one of its systems
+    // one launch of the kernel of fp64_tc.cuh unless a split variant is set,
+    // for the batch or one of its systems
     b->tcs_used = b->tune.split_variant == 0;
     for (int s = 0; s < n && b->tcs_used; ++s) {
       const atrip_gpu_context *c = b->sys[s];
       const atrip_tuning &t = c->tune;
       b->tcs_used = split_tc_eligible(slices, form == ATRIP_FORM_SPLIT_F16, c->No, c->Nv) &&
-                    t.split_variant == 0 && t.split_stages == 0 && t.split_ctas == 0 &&
-                    t.split_w_global == 0 && t.split_prefetch == 0;
+                    t.split_variant == 0;
     }
     if (b->tcs_used) {
       int rc = prepare_all(true);

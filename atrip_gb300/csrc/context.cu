@@ -469,7 +469,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
     if (rc != ATRIP_OK) return rc;
   }
   if (tc && c->tune.tuple_block == 0) {
-    const int block = tc_tuple_block(c->No, c->Nv, c->sm_count);
+    const int block = tc_tuple_block(c->No, c->Nv, kTcFp64Slices, c->sm_count);
     if (block > 0) {
       const int rc = build_order(c, t_begin, t_end, block, st);
       if (rc != ATRIP_OK) return rc;
@@ -567,14 +567,24 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
       c->split.f16 = form == ATRIP_FORM_SPLIT_F16;
       const int ctas = c->tune.split_ctas > 0 ? std::min(c->sm_count, (int)c->tune.split_ctas)
                                               : c->sm_count;
-      // the kernel of fp64_tc.cuh unless a launch parameter of the split
-      // kernels is set
+      // the engine's choice of kernel unless a variant (or a diagnostic that
+      // only the split kernels have) is set; the other launch parameters change
+      // a kernel's schedule, not the kernel
       const atrip_tuning &tn = c->tune;
-      bool on_tc = split_tc_eligible(slices, c->split.f16, c->No, c->Nv) &&
-                   tn.split_variant == 0 && tn.split_stages == 0 && tn.split_ctas == 0 &&
-                   tn.split_w_global == 0 && tn.split_prefetch == 0 &&
-                   tn.split_wait_kcycles == 0 && tn.split_test_unpublished == 0 &&
-                   tn.split_profile == 0;
+      const bool transposed = split_prefers_transposed(slices, c->split.f16, c->No, c->Nv);
+      const bool plain = tn.split_variant == 0 && tn.split_wait_kcycles == 0 &&
+                         tn.split_test_unpublished == 0 && tn.split_profile == 0;
+      const bool on_tc =
+          plain && !transposed && split_tc_eligible(slices, c->split.f16, c->No, c->Nv);
+      if (plain && transposed) c->split.variant = 2;
+      if ((on_tc || (plain && transposed)) && tn.tuple_block == 0) {
+        const int block = tc_tuple_block(c->No, c->Nv, slices, c->sm_count);
+        if (block > 0) {
+          const int rc = build_order(c, t_begin, t_end, block, st);
+          if (rc != ATRIP_OK) return rc;
+          order = c->d_order;
+        }
+      }
       const double tai_sign = opts->ijkabc ? -1.0 : 1.0;
       auto run_split = [&]() -> int {
         if (on_tc) {
@@ -584,7 +594,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
           TcSystem ts = {&c->split.tc, &c->dt, c->No, c->Nv, c->n_triples, c->d_tuples,
                          c->d_triples, t_begin, t_end, use_j, c->d_e, c->d_ect, nullptr};
           if ((rc = split_tc_attach(c->split, use_j, &ts.tri_ef)) != ATRIP_OK) return rc;
-          if ((rc = tc_launch_prepare(&ts, 1, tai_sign, c->sm_count, c->tcs)) != ATRIP_OK)
+          if ((rc = tc_launch_prepare(&ts, 1, tai_sign, ctas, c->tcs, tn.split_stages)) != ATRIP_OK)
             return rc;
           return tc_launch_enqueue(c->tcs, order, st, &launches);
         }

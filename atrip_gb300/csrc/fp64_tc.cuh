@@ -26,7 +26,8 @@ void tc_free(TcState &s);
 bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx);
 
 // The processing order of its tuples (see build_order), 0 = list order.
-int tc_tuple_block(int No, int Nv, int sm_count);
+int tc_tuple_block(int No, int Nv, int slices, int sm_count);
+constexpr int kTcFp64Slices = 8;
 
 // Examine the operands, cut the slices and build the tensor maps, once per
 // upload.  ATRIP_OK with *usable = false where the data or the free memory
@@ -75,7 +76,9 @@ struct TcBuffers {
 void tc_buffers_free(TcBuffers &b);
 
 // Size the buffers for these systems and fill the host descriptor table.
-int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count, TcBuffers &b);
+// max_slots: operand ring depth limit, 0 = as many as fit.
+int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count, TcBuffers &b,
+                      int max_slots = 0);
 // Table copies, queue and flag reset, the launch and the flags' copy back, on
 // st (capturable).
 int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st,

@@ -38,9 +38,16 @@ int split_prepare(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
                   cudaStream_t st, int64_t *launches);
 // Whether the kernel of fp64_tc.cuh takes these slices: levels exact as the
 // kernels here keep them, BF16 with K = 2 (Nv + No) <= 1024, FP16 within
-// their own limits.  It is the one run unless a launch parameter of the
-// kernels here is set.
+// their own limits.  It is the engine's choice unless the transposed kernel is.
 bool split_tc_eligible(int slices, bool f16, int No, int Nv);
+// Whether the transposed kernel is the better one for a single system all the
+// same: two slices, whose 2 No stack rows and 240-256 columns fill its MMAs
+// better than No columns an MMA do.  Device time of FP16 slices, transposed
+// (in blocks of tuples) against the other: No=20/Nv=120 12.9 / 15.2 ms,
+// No=40/Nv=400 15.8 / 19.4, No=60/Nv=160 8.3 / 10.2; No=8/Nv=100 6.3 / 4.6,
+// No=47/Nv=160 8.5 / 8.0, No=53/Nv=201 7.4 / 6.9 (few rows to stack; singles
+// blocks that no longer fit beside three stages).
+bool split_prefers_transposed(int slices, bool f16, int No, int Nv);
 // The prepared slices' maps for it, and the triple table it reads.
 int split_tc_attach(SplitState &s, bool use_j, const double2 **tri_ef);
 

@@ -2034,6 +2034,11 @@ bool split_tc_eligible(int slices, bool f16, int No, int Nv) {
   return slices >= 2 && slices <= 4 && 2 * (Nv + No) <= 1024;
 }
 
+bool split_prefers_transposed(int slices, bool f16, int No, int Nv) {
+  return slices == 2 && ((No >= 12 && No <= 40) || No > 56) &&
+         transposed_eligible(slices, No, Nv, f16);
+}
+
 int split_tc_attach(SplitState &s, bool use_j, const double2 **tri_ef) {
   auto *p = static_cast<SplitImpl *>(s.impl);
   if (!s.valid || !p || (use_j && !p->has_j)) {

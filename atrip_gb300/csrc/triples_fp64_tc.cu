@@ -1,4 +1,5 @@
-// FP64 form of the triples kernel on the tensor cores.
+// The triples kernel on the tensor cores: the FP64 form (real and complex),
+// and the split forms' slices on the same structure.
 //
 // FP64 arithmetic on this part runs at ~1.25 TFLOP/s whichever instruction
 // does it, BF16 MMAs at ~1900.  So the contractions are done as the Ozaki
@@ -44,15 +45,18 @@
 //   warps 2, 3, 8..15 energy: W in FP64, Zijk, get_energy_{distinct,same}
 //                     (src/atrip/Equations.cxx:101-238), one tuple behind
 //
-// What bounds it: shared memory.  An MMA of N columns reads 4 KB of A and
-// 32 N bytes of B at ~118 B per cycle, so the narrow ones (the last slices,
-// few columns) cost 35 + 0.27 N cycles instead of N / 2, and the TMA's writes
-// of the next tiles take their part of the same bandwidth.  Whole runs
-// measured against the DFMA kernel: No=24/Nv=240, 8000 tuples, 316 -> 15.3 ms
-// (1.11 -> 23 TFLOP/s FP64-equivalent); No=37/Nv=151 with (cT), 900 tuples,
-// 229.6 -> 12.0 ms; No=8/Nv=40, the whole list, 6.2 -> 2.2 ms.  Error of the
-// tuple energies against quad precision, 2-norm: 1.0e-16 and 2.2e-16 for
-// (cT), DFMA kernel 1.0e-16 and 4.5e-16 (No = 8..33).
+// What bounds it: the MMA issuer where there are few columns (an MMA of N <=
+// 96 costs ~50 cycles, its issue and its share of a slot's wait and signal as
+// much), shared memory beyond (an MMA of N columns reads 4 KB of A and 32 N
+// bytes of B at ~118 B per cycle, and the TMA's writes take their part), the
+// operand stream from L2 and HBM (No=24/Nv=240: 47 B per cycle and SM) and, at
+// large No, the energy warps' gathers.  Whole runs against the DFMA kernel:
+// No=24/Nv=240, 8000 tuples, 316 -> 10.4 ms (1.11 -> 34 TFLOP/s
+// FP64-equivalent); No=37/Nv=151 with (cT), 900 tuples, 229.6 -> 7.7 ms;
+// No=8/Nv=40, the whole list, 6.2 -> 0.92 ms; complex No=13/Nv=50, 9000
+// tuples, 90.8 -> 3.7 ms.  Error of the tuple energies against quad precision,
+// 2-norm: 1.0e-16 and 2.2e-16 for (cT), DFMA kernel 1.0e-16 and 4.5e-16 (No =
+// 8..33).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -1431,7 +1435,10 @@ int tc_split_attach_j(TcState &s, double unit_j, void *const *ops) {
 bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx) {
   // complex: the columns of both components of 8 levels fill TMEM at No = 32
   const double flops = (cplx ? 4.0 : 1.0) * (double)n_tuples * 12.0 * No * No * No * (No + Nv);
-  return No >= 2 && (!cplx || No <= 32) && flops >= 1e9;
+  // sums of the low levels are random: 5500 sqrt(6 K) for level 7, which stays
+  // 8 standard deviations below the checked 2^22 up to K = 1400
+  const int K = 2 * (Nv + No) * (cplx ? 2 : 1);
+  return No >= 2 && (!cplx || No <= 32) && K <= 1400 && flops >= 1e9;
 }
 
 // Side of the (a,b,c) blocks tuples are processed in, 0 = list order.  In list
@@ -1439,8 +1446,8 @@ bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx) {
 // the L2 (129 MB, each die caching what it reads) blocks of side 6 keep them
 // resident: No=24/Nv=240 13.3 -> 11.3 ms, No=40/Nv=240 10.4 -> 9.2 ms (sides
 // 3, 4, 8: 11.5, 13.1, 11.4 and 9.2, 9.1, 9.2); below it they gain nothing.
-int tc_tuple_block(int No, int Nv, int sm_count) {
-  const double slab = 16.0 * No * No * ((Nv + kKChunk - 1) / kKChunk * kKChunk);
+int tc_tuple_block(int No, int Nv, int slices, int sm_count) {
+  const double slab = 2.0 * slices * No * No * ((Nv + kKChunk - 1) / kKChunk * kKChunk);
   return slab * std::min(sm_count, Nv) > 64e6 ? 6 : 0;
 }
 
@@ -1482,7 +1489,8 @@ void tc_buffers_free(TcBuffers &b) {
   b = TcBuffers();
 }
 
-int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count, TcBuffers &b) {
+int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count, TcBuffers &b,
+                      int max_slots) {
   if (b.cap < n) {
     cudaFreeHost(b.h_desc);
     cudaFree(b.d_desc);
@@ -1504,7 +1512,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   }
   if (!b.d_queue) ATRIP_CUDA_TRY(cudaMalloc(&b.d_queue, sizeof(unsigned long long)));
   auto *h = static_cast<TcDesc *>(b.h_desc);
-  int P = 0, spp = 1;
+  int P = 0, spp = 1, window = 0;
   const auto *p0 = static_cast<const TcImpl *>(n > 0 ? sys[0].state->impl : nullptr);
   const int S = p0 ? p0->S : kS;
   b.S = S;
@@ -1551,6 +1559,8 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     b.nc = p->nc;  // the same for all: a batch holds real systems
     b.aslot = std::max(b.aslot, p->spp * p->rows * 128);
     spp = std::max(spp, p->spp);
+    // an MMA reads 128 rows from its slice on, whatever the item's rows are
+    window = std::max(window, (p->spp - 1) * p->rows * 128 + 128 * 128);
     b.lay_no = std::max(b.lay_no, m.No);
     if (m.use_j) b.lay_pass = 2;
     b.h_prefix[k + 1] = b.h_prefix[k] + std::max<int64_t>(0, m.t_end - m.t_begin);
@@ -1568,14 +1578,17 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   const int room = kSmemLimit - 1024 - kTailBytes;
   const int per_chunk = S / spp;  // of the system with the fewest A slots a chunk
   auto b_for = [&](int nslots) { return (nslots - 1 + per_chunk - 1) / per_chunk + 1; };
-  b.nslots = kMaxSlots;
+  b.nslots = max_slots > 0 ? std::min(std::max(max_slots, 2), kMaxSlots) : kMaxSlots;
   while (b.nslots > 1 && b.nslots * b.aslot + b_for(b.nslots) * b.bslot > room) --b.nslots;
   b.nbslots = b_for(b.nslots);
   if (b.nslots * b.aslot + b.nbslots * b.bslot > room || b.nslots < 2) {
     set_error("tensor-core FP64 form: shared memory too small");
     return ATRIP_ERR_UNSUPPORTED;
   }
-  b.smem = 1024 + (size_t)b.nslots * b.aslot + (size_t)b.nbslots * b.bslot + kTailBytes;
+  // the last slot's window may reach past the B ring and the tail (few rows, a
+  // shallow ring): it must still end in this block's shared memory
+  const int end = b.nslots * b.aslot + b.nbslots * b.bslot + kTailBytes;
+  b.smem = 1024 + (size_t)std::max(end, (b.nslots - 1) * b.aslot + window);
   const size_t cell = b.split ? 8 : 16;
   const size_t per_cta = (2 * 3 * cell + 8) * b.nc * b.lay_pass * b.lay_cells;
   const size_t need = per_cta * std::max(b.grid, 1);

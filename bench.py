@@ -369,7 +369,12 @@ def _max_over_ranks(world, ms, count):
     return float(t.item()), c.item()
 
 
-def _roofline(form, slices, flops_per_launch, launch_ms, peaks, live_fp64, traffic):
+def _roofline(form, slices, flops_per_launch, launch_ms, peaks, live_fp64, traffic,
+              fp64_on_tensor_cores=False):
+    if form == "fp64" and fp64_on_tensor_cores:
+        # the FP64 form's digit products: levels 0..7 of 8 BF16 slices
+        r = _roofline("split_bf16", 8, flops_per_launch, launch_ms, peaks, None, traffic)
+        return dict(r, kernel="triples_tc_kernel")
     if form == "fp64":
         achieved = flops_per_launch / (launch_ms * 1e-3) / 1e12
         peak = live_fp64
@@ -524,7 +529,8 @@ def run_single(args, workload, world, rank, local):
     kname = "triples_fp64_kernel" if form == "fp64" else "triples_split_kernel"
     tpt = traffic_per_tuple(kname, workload, form, slices)
     roof = _roofline(form, slices, launch_tuples * fpt, kernel_ms, peaks, live_fp64,
-                     tpt * launch_tuples if tpt is not None else None)
+                     tpt * launch_tuples if tpt is not None else None,
+                     not any(tune["tuning"].values()))
     roof["tuples_per_launch"] = launch_tuples
     cpu = None if args.no_cpu_baseline else cpu_baseline(d, args.cpu_seconds)
     line = {
@@ -656,7 +662,8 @@ def run_batch96(args, world, rank, local):
     peaks = load_peaks()
     kernel_ms = statistics.median(r[0].device_ms for r in res)
     roof = _roofline(form, slices, total_flops, kernel_ms, peaks,
-                     capi.measure_peaks(local)[0] if form == "fp64" else None, None)
+                     capi.measure_peaks(local)[0] if form == "fp64" else None, None,
+                     not any(btune["tuning"].values()) and not any(tiles))
     roof["note"] = "whole batch graph (all systems' launches and the energy reduction)"
     cpu = None if args.no_cpu_baseline else cpu_baseline_batch(ds, args.cpu_seconds)
     line = {

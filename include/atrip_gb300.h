@@ -157,10 +157,8 @@ int atrip_gpu_run(atrip_gpu_context *ctx, const atrip_run_options *opts, atrip_r
 
 /* Launch parameters chosen by the autotuner (atrip_gb300/autotune.py);
  * a zero field keeps the built-in choice.  The fp64_* fields and
- * tuples_per_claim describe the kernel of FP64 instructions, the split_*
- * fields the split forms' own kernels: one that is set selects those for its
- * form, where otherwise all forms run on one tensor-core kernel within its
- * limits.  No counterpart in the reference,
+ * tuples_per_claim describe the kernel of FP64 instructions: one that is set
+ * selects that kernel for the FP64 form.  No counterpart in the reference,
  * whose only tuning knob for this loop is the tuple distribution.          */
 typedef struct {
   int32_t fp64_ctas_per_sm; /* FP64 form: resident CTAs per SM (0 = occupancy max) */
