@@ -43,9 +43,10 @@ bool split_tc_eligible(int slices, bool f16, int No, int Nv);
 // Whether the transposed kernel is the better one for a single system all the
 // same: two slices, whose 2 No stack rows and 240-256 columns fill its MMAs
 // better than No columns an MMA do.  Device time of FP16 slices, transposed
-// (in blocks of tuples) against the other: No=20/Nv=120 12.9 / 15.2 ms,
-// No=40/Nv=400 15.8 / 19.4, No=60/Nv=160 8.3 / 10.2; No=8/Nv=100 6.3 / 4.6,
-// No=47/Nv=160 8.5 / 8.0, No=53/Nv=201 7.4 / 6.9 (few rows to stack; singles
+// against the other, both in blocks of 4^3 tuples: No=20/Nv=120 12.9 / 15.2 ms,
+// No=41/Nv=300 38.0 / 40.3, No=48/Nv=300 35.8 / 41.6, No=47/Nv=160 60.7 / 59.5,
+// No=52/Nv=300 35.6 / 36.9, No=60/Nv=160 8.3 / 10.2; but No=8/Nv=100 6.3 / 4.6
+// (few rows to stack), No=53/Nv=201 157 / 151, No=56/Nv=440 228 / 191 (singles
 // blocks that no longer fit beside three stages).
 bool split_prefers_transposed(int slices, bool f16, int No, int Nv);
 // The prepared slices' maps for it, and the triple table it reads.

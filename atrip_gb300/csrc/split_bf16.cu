@@ -2035,7 +2035,7 @@ bool split_tc_eligible(int slices, bool f16, int No, int Nv) {
 }
 
 bool split_prefers_transposed(int slices, bool f16, int No, int Nv) {
-  return slices == 2 && ((No >= 12 && No <= 40) || No > 56) &&
+  return slices == 2 && ((No >= 12 && No <= 52) || No > 56) &&
          transposed_eligible(slices, No, Nv, f16);
 }
 

@@ -1443,12 +1443,16 @@ bool tc_sizes_ok(int No, int Nv, int64_t n_tuples, bool cplx) {
 
 // Side of the (a,b,c) blocks tuples are processed in, 0 = list order.  In list
 // order the ~150 tuples in flight read as many T_c slabs; where those exceed
-// the L2 (129 MB, each die caching what it reads) blocks of side 6 keep them
-// resident: No=24/Nv=240 13.3 -> 11.3 ms, No=40/Nv=240 10.4 -> 9.2 ms (sides
-// 3, 4, 8: 11.5, 13.1, 11.4 and 9.2, 9.1, 9.2); below it they gain nothing.
+// the L2 (129 MB, each die caching what it reads) blocks keep them resident;
+// below it they gain nothing.  Two to four slices: side 4, in runs of 100 ms
+// and more No=56/Nv=440 191 ms (6: 264, 8: 194), No=24/Nv=240 with 3 BF16
+// slices 125 (list order 137, 6: 131), No=53/Nv=201 151 (6: 161).  The FP64
+// form: side 6, No=24/Nv=240 11.8 ms (list order 12.5, 4: 13.0, 8: 12.3),
+// No=40/Nv=300 62 (71, 77, 73); long runs at the power limit differ either
+// way (No=24/Nv=240 6: 46 ms, 8: 42; No=37/Nv=151 list order 58, 6: 66).
 int tc_tuple_block(int No, int Nv, int slices, int sm_count) {
   const double slab = 2.0 * slices * No * No * ((Nv + kKChunk - 1) / kKChunk * kKChunk);
-  return slab * std::min(sm_count, Nv) > 64e6 ? 6 : 0;
+  return slab * std::min(sm_count, Nv) > 64e6 ? (slices == kTcFp64Slices ? 6 : 4) : 0;
 }
 
 int tc_prepare(TcState &s, const DeviceTensors &dt, int No, int Nv, bool cplx, bool use_j,
