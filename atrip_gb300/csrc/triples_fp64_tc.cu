@@ -16,9 +16,12 @@
 // element of W, where the DFMA kernel's own rounding is at 2^-51.
 //
 // When that holds is examined, not assumed (tc_prepare and the kernel's
-// overflow flag): operands must be finite; the largest element of every
-// slab a tuple reads must lie within 2^kRangeBits of its tensor's largest
-// (product of both operands' ratios); the partial sums of levels 0..2 are
+// overflow flag): operands must be finite; the largest product |T V| of every
+// T_x with every V_yz must lie within 2^kRangeBits of the grids' largest
+// (kprofile.cuh): what is lost of K products (levels 8 and up, the bits below
+// the grids), at most 9 K 2^-64 of the grids' largest, is then below a third of
+// K 2^-53 of that product, the bound of an FP64 dot product's error; the
+// partial sums of levels 0..2 are
 // bounded below 2^24 by the rows' digit norms (Cauchy-Schwarz); sums of the
 // higher levels, random in sign for any data whose low-order bits are not
 // correlated, are checked to end below 2^22, a quarter of the exact range.
@@ -72,6 +75,7 @@
 #include "digits.cuh"
 #include "engine.cuh"
 #include "fp64_tc.cuh"
+#include "kprofile.cuh"
 #include "recip.cuh"
 #include "sm100.cuh"
 
@@ -90,7 +94,7 @@ constexpr int kEnergyThreads = kEnergyWarps * 32;
 constexpr int kSmemLimit = 232448;
 constexpr int kT1 = 64;  // doubles per t1 row: No <= 64, or No <= 32 complex
 constexpr int kTailBytes = 576 + 3 * kT1 * 8 + 16 * 8;
-constexpr double kRangeBits = 8.0;
+constexpr int kRangeBits = 6;               // least product against 2^(eT+eV)
 constexpr int kBlocksZ = 3;                 // column blocks stored for a complex operand
 
 enum : int { kErrFull = 1, kErrEmpty = 2, kErrAccFull = 3, kErrAccEmpty = 4 };
@@ -923,34 +927,77 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
 
 // ------------------------------------------------------------------ prep
 
-// stats[0] = max |x| over the tensor, stats[1] = min over its nonzero slabs
-// (n elements each) of the slab's max, as FP64 bit patterns (ordered like
-// the magnitudes; infinities and NaN sort above every finite value).
-__global__ void slab_max_kernel(const double *__restrict__ x, int64_t slabs, int64_t n,
-                                unsigned long long *__restrict__ stats) {
-  __shared__ unsigned long long sh[8];
-  for (int64_t s = blockIdx.x; s < slabs; s += gridDim.x) {
-    const double *p = x + s * n;
-    unsigned long long m = 0;
-    for (int64_t i = threadIdx.x; i < n; i += 256) {
-      const unsigned long long b =
-          (unsigned long long)__double_as_longlong(p[i]) & 0x7fffffffffffffffull;
-      m = b > m ? b : m;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
-      m = v > m ? v : m;
-    }
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < 8; ++w) m = sh[w] > m ? sh[w] : m;
-      if (m > *(volatile unsigned long long *)&stats[0]) atomicMax(&stats[0], m);
-      if (m != 0 && m < *(volatile unsigned long long *)&stats[1]) atomicMin(&stats[1], m);
-    }
-    __syncthreads();
+// The largest magnitude of x[0 .. n), as an FP64 bit pattern (ordered like the
+// magnitudes; infinities and NaN sort above every finite value).
+__global__ void __launch_bounds__(256) max_kernel(const double *__restrict__ x, int64_t n,
+                                                  unsigned long long *__restrict__ out) {
+  unsigned long long m = 0;
+  for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < n; i += gridDim.x * 256ll) {
+    const unsigned long long b = magnitude(x[i]);
+    m = b > m ? b : m;
   }
+  warp_max(m, out);
+}
+
+// The profile of T: t[E][x] = log of max |Ta[x][q][p][E]|, and the largest.
+template <int NC>
+__global__ void __launch_bounds__(256) t_profile_kernel(const double *__restrict__ Ta, int No2,
+                                                        int Nv, int *__restrict__ t,
+                                                        unsigned long long *__restrict__ out) {
+  __shared__ unsigned long long sh[8][32];
+  const int x = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int E = blockIdx.y * 32 + lane;
+  unsigned long long m = 0;
+  if (E < Nv) {
+    const double *p = Ta + ((int64_t)x * No2 * Nv + E) * NC;
+#pragma unroll 4
+    for (int r = warp; r < No2; r += 8)
+#pragma unroll
+      for (int h = 0; h < NC; ++h) {
+        const unsigned long long b = magnitude(p[(int64_t)r * Nv * NC + h]);
+        m = b > m ? b : m;
+      }
+  }
+  sh[warp][lane] = m;
+  __syncthreads();
+  if (warp != 0) return;
+  for (int w = 1; w < 8; ++w) m = sh[w][lane] > m ? sh[w][lane] : m;
+  if (E < Nv) t[(size_t)E * profile_pitch(Nv) + x] = log_of(m);
+  warp_max(m, out);
+}
+
+// The least product of T's profile with those of 32 slabs Vpt[y][z][r][E] a
+// block, and the largest element.  Reads V once and takes Nv^4 steps; the slab
+// maxima it replaces read as much (No=24/Nv=240, first run of 8000 tuples with
+// examination and cut: 15.3 -> 15.6 ms).
+template <int NC>
+__global__ void __launch_bounds__(256) v_profile_kernel(const double *__restrict__ Vpt,
+                                                        const int *__restrict__ t, int No, int Nv,
+                                                        unsigned long long *__restrict__ vmax,
+                                                        unsigned int *__restrict__ least) {
+  extern __shared__ int v[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t p0 = (int64_t)blockIdx.x * kProfilePairs, np = (int64_t)Nv * Nv;
+  unsigned long long best = 0;
+  for (int k = warp; k < kProfilePairs; k += 8)
+    for (int E = lane; E < Nv; E += 32) {
+      unsigned long long m = 0;
+      if (p0 + k < np) {
+        const double *p = Vpt + ((p0 + k) * No * Nv + E) * NC;
+#pragma unroll 8
+        for (int r = 0; r < No; ++r)
+#pragma unroll
+          for (int h = 0; h < NC; ++h) {
+            const unsigned long long b = magnitude(p[(int64_t)r * Nv * NC + h]);
+            m = b > m ? b : m;
+          }
+      }
+      v[E * (kProfilePairs + 1) + k] = log_of(m);
+      best = m > best ? m : best;
+    }
+  warp_max(best, vmax);
+  __syncthreads();
+  least_product(t, v, Nv, p0, least);
 }
 
 // dst[s][R][k] (pitch Kp) = digit_s(sign src(R, k)), row R = (o n1 + r1) n2
@@ -1016,7 +1063,6 @@ struct TcImpl {
   int nc = 1;  // doubles per element: 2 for a complex system
   int No = 0, Nv = 0, P = 0, rows = 0, spp = 0, Kp = 0, Kh = 0;
   int eT = 0, eV = 0, eJ = 0;
-  double max_t = 0, min_t = 0;  // T: largest element, smallest nonzero slab maximum
   double nT[3], nU[3];          // digit norms of the T rows (over E; over L)
   double unit = 1.0, unit_j = 1.0;
   char *arena = nullptr, *arena_j = nullptr;
@@ -1094,15 +1140,42 @@ double as_double(unsigned long long b) {
 }
 
 struct DeviceStats {
-  unsigned long long m[4][2];  // slab statistics of up to four tensor views
-  unsigned int n[8][4];        // digit norms of up to eight cut jobs
+  unsigned long long t_max, vp_max, vh_max;  // largest magnitudes
+  unsigned int least;                        // least product (log_of sums)
+  unsigned int n[8][4];                      // digit norms of up to eight cut jobs
 };
 
-cudaError_t slab_max(const double *x, int64_t slabs, int64_t n, unsigned long long *out,
-                     cudaStream_t st) {
-  const int grid = (int)std::min<int64_t>(slabs, 152 * 16);
-  slab_max_kernel<<<grid, 256, 0, st>>>(x, slabs, n, out);
-  return cudaGetLastError();
+// Queue the examination of T against a pair V_hhhp, V_pphp (or J): maxima and
+// the least product.  scratch: profile_bytes() of device memory.
+template <int NC>
+int examine(const double *Ta, const double *vht, const double *vpt, int No, int Nv, void *scratch,
+            DeviceStats *ds, cudaStream_t st, int64_t *launches) {
+  int *t = static_cast<int *>(scratch);
+  t_profile_kernel<NC><<<dim3(Nv, (Nv + 31) / 32), 256, 0, st>>>(Ta, No * No, Nv, t, &ds->t_max);
+  ATRIP_CUDA_TRY(cudaGetLastError());
+  ATRIP_CUDA_TRY(cudaFuncSetAttribute(v_profile_kernel<NC>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+  v_profile_kernel<NC><<<(unsigned)(((int64_t)Nv * Nv + kProfilePairs - 1) / kProfilePairs), 256,
+                         profile_smem(Nv), st>>>(vpt, t, No, Nv, &ds->vp_max, &ds->least);
+  ATRIP_CUDA_TRY(cudaGetLastError());
+  max_kernel<<<152 * 4, 256, 0, st>>>(vht, (int64_t)NC * Nv * No * No * No, &ds->vh_max);
+  ATRIP_CUDA_TRY(cudaGetLastError());
+  *launches += 3;
+  return ATRIP_OK;
+}
+
+// Clear *ds, examine and read the result back (synchronises st).
+int examine(int nc, const double *Ta, const double *vht, const double *vpt, int No, int Nv,
+            void *scratch, DeviceStats *ds, DeviceStats *h, cudaStream_t st, int64_t *launches) {
+  std::memset(h, 0, sizeof(*h));
+  h->least = ~0u;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(ds, h, sizeof(*h), cudaMemcpyHostToDevice, st));
+  const int rc = nc == 2 ? examine<2>(Ta, vht, vpt, No, Nv, scratch, ds, st, launches)
+                         : examine<1>(Ta, vht, vpt, No, Nv, scratch, ds, st, launches);
+  if (rc != ATRIP_OK) return rc;
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(h, ds, sizeof(*h), cudaMemcpyDeviceToHost, st));
+  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+  return ATRIP_OK;
 }
 
 cudaError_t cut(CutJob j, cudaStream_t st) {
@@ -1127,6 +1200,17 @@ bool alloc_arena(char **p, size_t bytes) {
 }
 
 bool exponent_ok(int e) { return e >= -200 && e <= 200; }
+
+// The grids' exponents, if an examination's result allows the form.
+bool grids_of(const DeviceStats &h, int *e_t, int *e_v) {
+  const unsigned long long mT = h.t_max, mV = std::max(h.vp_max, h.vh_max);
+  constexpr unsigned long long kInf = 0x7ff0000000000000ull;
+  if (mT == 0 || mV == 0 || mT >= kInf || mV >= kInf) return false;
+  *e_t = exponent_of(as_double(mT));
+  *e_v = exponent_of(as_double(mV));
+  if (!exponent_ok(*e_t) || !exponent_ok(*e_v)) return false;
+  return std::ldexp((double)h.least, -kLogOne) - 2 * kLogBias >= *e_t + *e_v - kRangeBits;
+}
 
 // Bound of |partial sums| of levels 0, 1 and 2: twice (natural and transposed
 // part; four times for a complex system, whose rows meet real and imaginary
@@ -1247,26 +1331,8 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cpl
   ATRIP_CUDA_TRY(cudaMalloc(&tmp.p, sizeof(DeviceStats)));
   auto *ds = static_cast<DeviceStats *>(tmp.p);
   DeviceStats h;
-  std::memset(&h, 0, sizeof(h));
-  for (auto &m : h.m) m[1] = ~0ull;
-  ATRIP_CUDA_TRY(cudaMemcpyAsync(ds, &h, sizeof(h), cudaMemcpyHostToDevice, st));
-  ATRIP_CUDA_TRY(slab_max(dt.Ta, Nv, No2 * Nv * nc, ds->m[0], st));
-  ATRIP_CUDA_TRY(slab_max(dt.Tp, Nv * Nv, No2 * nc, ds->m[1], st));
-  ATRIP_CUDA_TRY(slab_max(dt.Vpt, Nv * Nv, No * Nv * nc, ds->m[2], st));
-  ATRIP_CUDA_TRY(slab_max(dt.Vht, Nv, No2 * No * nc, ds->m[3], st));
-  *launches += 4;
-  ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
-  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
-  const unsigned long long mT = h.m[0][0], mV = std::max(h.m[2][0], h.m[3][0]);
-  constexpr unsigned long long kInf = 0x7ff0000000000000ull;
-  if (mT == 0 || mV == 0 || mT >= kInf || mV >= kInf) return ATRIP_OK;
-  p->max_t = as_double(mT);
-  p->min_t = as_double(std::min(h.m[0][1], h.m[1][1]));
-  const double max_v = as_double(mV), min_v = as_double(std::min(h.m[2][1], h.m[3][1]));
-  p->eT = exponent_of(p->max_t);
-  p->eV = exponent_of(max_v);
-  if (!exponent_ok(p->eT) || !exponent_ok(p->eV)) return ATRIP_OK;
-  if (std::log2(p->max_t / p->min_t) + std::log2(max_v / min_v) > kRangeBits) return ATRIP_OK;
+  int rc = examine(p->nc, dt.Ta, dt.Vht, dt.Vpt, No_, Nv_, p->arena, ds, &h, st, launches);
+  if (rc != ATRIP_OK || !grids_of(h, &p->eT, &p->eV)) return rc;
   p->unit = std::ldexp(1.0, p->eT + p->eV - 14 - 24);
 
   char *q = p->arena;
@@ -1286,7 +1352,7 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cpl
   j.src = dt.Ta; j.nrows = Nv * No2; j.n1 = No; j.n2 = No;
   j.so = No2 * Nv * nc; j.s1 = No * Nv * nc; j.s2 = Nv * nc; j.sk = nc; j.K = Nv_; j.Kp = p->Kp;
   j.norms = ds->n[0];
-  int rc = cut_rows(*p, j, Ta, st, launches);
+  rc = cut_rows(*p, j, Ta, st, launches);
   if (rc != ATRIP_OK) return rc;
   // columns r of -T[u,v,L,r] and -T[u,v,r,L] over L
   const int *comp = cplx ? kCompT : kReal, *neg = cplx ? kNegT : kNeg;
@@ -1335,26 +1401,14 @@ int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *lau
   ATRIP_CUDA_TRY(cudaMalloc(&tmp.p, sizeof(DeviceStats)));
   auto *ds = static_cast<DeviceStats *>(tmp.p);
   DeviceStats h;
-  std::memset(&h, 0, sizeof(h));
-  for (auto &m : h.m) m[1] = ~0ull;
-  ATRIP_CUDA_TRY(cudaMemcpyAsync(ds, &h, sizeof(h), cudaMemcpyHostToDevice, st));
-  ATRIP_CUDA_TRY(slab_max(dt.Jpt, Nv * Nv, No * Nv * nc, ds->m[2], st));
-  ATRIP_CUDA_TRY(slab_max(dt.Jht, Nv, No2 * No * nc, ds->m[3], st));
-  *launches += 2;
-  ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
-  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
-  const unsigned long long mV = std::max(h.m[2][0], h.m[3][0]);
-  if (mV == 0 || mV >= 0x7ff0000000000000ull) return ATRIP_OK;
-  const double max_v = as_double(mV), min_v = as_double(std::min(h.m[2][1], h.m[3][1]));
-  p->eJ = exponent_of(max_v);
-  if (!exponent_ok(p->eJ) ||
-      std::log2(p->max_t / p->min_t) + std::log2(max_v / min_v) > kRangeBits)
-    return ATRIP_OK;
+  int e_t;
+  int rc = examine((int)nc, dt.Ta, dt.Jht, dt.Jpt, p->No, p->Nv, p->arena_j, ds, &h, st, launches);
+  if (rc != ATRIP_OK || !grids_of(h, &e_t, &p->eJ)) return rc;
   p->unit_j = std::ldexp(1.0, p->eT + p->eJ - 14 - 24);
   __nv_bfloat16 *vh[4];
   for (int i = 0; i < 2 * nc; ++i) vh[i] = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + i * nVh);
   auto *vp = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + 2 * nc * nVh);
-  int rc = cut_pair(*p, dt.Jht, dt.Jpt, p->eJ, vh, vp, ds, st, launches);
+  rc = cut_pair(*p, dt.Jht, dt.Jpt, p->eJ, vh, vp, ds, st, launches);
   if (rc != ATRIP_OK) return rc;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
