@@ -39,6 +39,7 @@
 #include "atrip_gb300.h"
 #include "digits.cuh"
 #include "engine.cuh"
+#include "kprofile.cuh"
 #include "sm100.cuh"
 
 namespace atrip_gb300 {
@@ -63,7 +64,10 @@ struct Header {
   int tc_overflow;               // a level sum left its exact range
   int tc_status;                 // a bounded wait gave up
   int e_t, e_v, e_j;             // exponents of the digit grids
-  unsigned long long vh_max[2], vh_min_not[2];  // V_hhhp, J_hhhp slabs: max, ~min (0: none)
+  // largest magnitudes of T, of the V and of the J pair; least products of T
+  // with V_pphp and J_pphp (kprofile.cuh)
+  unsigned long long t_max, v_max[2];
+  unsigned int least[2];
 };
 static_assert(sizeof(Header) <= kHeaderBytes, "header");
 
@@ -304,15 +308,12 @@ constexpr int kThreads = 512;
 constexpr int kS = 8;           // digit slices and levels
 constexpr int kChunk = 64;      // K elements per 128-byte row
 constexpr int kATile = 128 * 128;
+constexpr int kSmemLimit = 232448;
 // K contributions an accumulator may hold: levels 0..2 stay below 2^24
 // whatever the digits are, 3 K 2^14 <= 2^24.  Longer sums are drained into W
 // in pieces.
 constexpr int kMaxK = 341;
-constexpr double kRangeBits = 8.0;
-
-__device__ __forceinline__ unsigned long long magnitude(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
-}
+constexpr int kRangeBits = 6;  // least product against the grids' largest: triples_fp64_tc.cu
 
 // out[s] = largest magnitude of slab s of x[s + nslab c], c < count.
 __global__ void column_max(const double *__restrict__ x, int64_t nslab, int64_t count,
@@ -328,30 +329,52 @@ __global__ void column_max(const double *__restrict__ x, int64_t nslab, int64_t 
   atomicMax(&out[s], m);
 }
 
-// Largest magnitudes of contiguous slabs of n elements into the header.
-__global__ void slab_max(const double *__restrict__ x, int64_t slabs, int64_t n, Header *h,
-                         int which) {
-  __shared__ unsigned long long sh[8];
-  for (int64_t s = blockIdx.x; s < slabs; s += gridDim.x) {
+// The profile of T from its columns' maxima cols[x + Nv E], and the largest.
+__global__ void __launch_bounds__(256) t_profile(const unsigned long long *__restrict__ cols,
+                                                 int Nv, int *__restrict__ t, Header *h) {
+  const int64_t i = blockIdx.x * 256ll + threadIdx.x;
+  const unsigned long long m = i < (int64_t)Nv * Nv ? cols[i] : 0;
+  if (i == 0) h->least[0] = h->least[1] = ~0u;
+  if (i < (int64_t)Nv * Nv) t[(i / Nv) * profile_pitch(Nv) + i % Nv] = log_of(m);
+  warp_max(m, &h->t_max);
+}
+
+// The least product of T's profile with those of 32 slabs V[y,z,E,r] (y
+// fastest) a block, and the largest element.
+__global__ void __launch_bounds__(256) v_profile(const double *__restrict__ Vp,
+                                                 const int *__restrict__ t, int No, int Nv,
+                                                 Header *h, int which) {
+  extern __shared__ int v[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t p0 = (int64_t)blockIdx.x * kProfilePairs, np = (int64_t)Nv * Nv;
+  unsigned long long best = 0;
+  for (int E = warp; E < Nv; E += 8) {
     unsigned long long m = 0;
-    for (int64_t i = threadIdx.x; i < n; i += 256) {
-      const unsigned long long b = magnitude(x[s * n + i]);
-      m = b > m ? b : m;
+    if (p0 + lane < np) {
+      const double *p = Vp + p0 + lane + E * np;
+#pragma unroll 8
+      for (int r = 0; r < No; ++r) {
+        const unsigned long long b = magnitude(p[(int64_t)r * Nv * np]);
+        m = b > m ? b : m;
+      }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
-      m = v > m ? v : m;
-    }
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < 8; ++w) m = sh[w] > m ? sh[w] : m;
-      atomicMax(&h->vh_max[which], m);
-      if (m != 0) atomicMax(&h->vh_min_not[which], ~m);
-    }
-    __syncthreads();
+    v[E * (kProfilePairs + 1) + lane] = log_of(m);
+    best = m > best ? m : best;
   }
+  warp_max(best, &h->v_max[which]);
+  __syncthreads();
+  least_product(t, v, Nv, p0, &h->least[which]);
+}
+
+// The largest magnitude of x[0 .. n) into the header.
+__global__ void __launch_bounds__(256) max_kernel(const double *__restrict__ x, int64_t n,
+                                                  Header *h, int which) {
+  unsigned long long m = 0;
+  for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < n; i += gridDim.x * 256ll) {
+    const unsigned long long b = magnitude(x[i]);
+    m = b > m ? b : m;
+  }
+  warp_max(m, &h->v_max[which]);
 }
 
 // Smallest e with x <= 127/128 2^e; false if the exponent is out of hand.
@@ -364,42 +387,16 @@ __device__ bool grid_exponent(unsigned long long bits, int *e) {
   return k >= -200 && k <= 200;
 }
 
-// One block: the verdict from the slab maxima (T_uv, V_yz and J_yz pair
-// slabs at slabs[0 .. 3 nvnv)); the rules of triples_fp64_tc.cu.
-__global__ void decide(const unsigned long long *__restrict__ slabs, int64_t nvnv, int use_j,
-                       Header *h) {
-  __shared__ unsigned long long mx[3], mn_not[3];
-  if (threadIdx.x < 3) mx[threadIdx.x] = mn_not[threadIdx.x] = 0;
-  __syncthreads();
-  for (int t = 0; t < (use_j ? 3 : 2); ++t) {
-    unsigned long long a = 0, b = 0;
-    for (int64_t i = threadIdx.x; i < nvnv; i += blockDim.x) {
-      const unsigned long long m = slabs[t * nvnv + i];
-      a = m > a ? m : a;
-      if (m != 0 && ~m > b) b = ~m;
-    }
-    atomicMax(&mx[t], a);
-    atomicMax(&mn_not[t], b);
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  bool ok = true;
-  double range[3] = {0.0, 0.0, 0.0};
-  int e[3] = {0, 0, 0};
-  for (int t = 0; t < (use_j ? 3 : 2); ++t) {
-    unsigned long long m = mx[t], n = mn_not[t];
-    if (t > 0) {  // V_pphp and V_hhhp share a grid
-      m = max(m, h->vh_max[t - 1]);
-      n = max(n, h->vh_min_not[t - 1]);
-    }
-    ok = ok && grid_exponent(m, &e[t]);
-    if (ok)
-      range[t] = log2(__longlong_as_double((long long)m) / __longlong_as_double((long long)~n));
-  }
-  ok = ok && range[0] + range[1] <= kRangeBits && range[0] + range[2] <= kRangeBits;
-  h->e_t = e[0];
-  h->e_v = e[1];
-  h->e_j = e[2];
+// The verdict; the rules of triples_fp64_tc.cu.
+__global__ void decide(int use_j, Header *h) {
+  int e_t = 0, e[2] = {0, 0};
+  bool ok = grid_exponent(h->t_max, &e_t);
+  for (int w = 0; w < (use_j ? 2 : 1); ++w)
+    ok = ok && grid_exponent(h->v_max[w], &e[w]) &&
+         ldexp((double)h->least[w], -kLogOne) - 2 * kLogBias >= e_t + e[w] - kRangeBits;
+  h->e_t = e_t;
+  h->e_v = e[0];
+  h->e_j = e[1];
   h->tc_ok = ok ? 1 : 0;
 }
 
@@ -740,37 +737,42 @@ size_t smem_bytes(int no) {
   return 1024 + kS * kATile + (size_t)kS * ((no + 7) / 8 * 8) * 128 + 1024 + sizeof(Tail);
 }
 
-// By sizes: slab maxima fit the scratch, and the range's work on FP64
+// By sizes: the profile of T fits the scratch, and the range's work on FP64
 // instructions (~0.8 TFLOP/s here) takes several times what examining the
-// whole tensors does (~5 TB/s and a few launches).
+// whole tensors does (~5 TB/s, ~1.6e13 steps of a profile's product a second
+// and a few launches).
 bool sizes_ok(const Args &a) {
   const double Nv = a.Nv, No = a.No, n = (double)(a.t_end - a.t_begin);
   const double nj = a.use_j ? 2.0 : 1.0;
   const double dfma = n * nj * 12.0 * No * No * No * (No + Nv) / 0.8e12;
-  const double scan = 8.0 * (Nv * Nv * No * No + nj * Nv * No * (Nv * Nv + No * No)) / 5e12 + 4e-5;
+  const double scan = 8.0 * (Nv * Nv * No * No + nj * Nv * No * (Nv * Nv + No * No)) / 5e12 +
+                      nj * Nv * Nv * Nv * Nv / 1.6e13 + 4e-5;
   return No >= 4 && dfma > 4.0 * scan &&
-         3.0 * 8.0 * Nv * Nv <= (double)(kScratchBytes - kWorkspaceOffset);
+         8 * (size_t)a.Nv * a.Nv + profile_bytes(a.Nv) + 256 <= kScratchBytes - kWorkspaceOffset;
 }
 
 // Queue the examination and the kernel.
 int enqueue(const Args &a, int device, cudaStream_t st) {
   const int64_t Nv = a.Nv, No = a.No, nvnv = Nv * Nv;
-  auto *slabs = reinterpret_cast<unsigned long long *>(a.scratch + kWorkspaceOffset);
+  int *t = reinterpret_cast<int *>(a.scratch + kWorkspaceOffset);
+  auto *cols = reinterpret_cast<unsigned long long *>(a.scratch + kWorkspaceOffset +
+                                                      (profile_bytes((int)Nv) + 255) / 256 * 256);
   Header *h = reinterpret_cast<Header *>(a.scratch);
-  ATRIP_CUDA_TRY(cudaMemsetAsync(slabs, 0, 8 * 3 * nvnv, st));
-  const dim3 blocks((unsigned)((nvnv + 255) / 256), 1);
-  auto grid = [&](int64_t count) {
-    const int64_t y = std::max<int64_t>(1, 152 * 16 / blocks.x);
-    return dim3(blocks.x, (unsigned)std::min<int64_t>(count, y));
-  };
-  column_max<<<grid(No * No), 256, 0, st>>>(a.T, nvnv, No * No, slabs);
-  column_max<<<grid(Nv * No), 256, 0, st>>>(a.Vp, nvnv, Nv * No, slabs + nvnv);
-  slab_max<<<(int)Nv, 256, 0, st>>>(a.Vh, Nv, No * No * No, h, 0);
-  if (a.use_j) {
-    column_max<<<grid(Nv * No), 256, 0, st>>>(a.Jp, nvnv, Nv * No, slabs + 2 * nvnv);
-    slab_max<<<(int)Nv, 256, 0, st>>>(a.Jh, Nv, No * No * No, h, 1);
+  ATRIP_CUDA_TRY(cudaMemsetAsync(cols, 0, 8 * nvnv, st));
+  const unsigned blocks = (unsigned)((nvnv + 255) / 256);
+  const dim3 grid(blocks, (unsigned)std::min<int64_t>(No * No,
+                                                      std::max<int64_t>(1, 152 * 16 / blocks)));
+  column_max<<<grid, 256, 0, st>>>(a.T, nvnv, No * No, cols);
+  t_profile<<<blocks, 256, 0, st>>>(cols, (int)Nv, t, h);
+  ATRIP_CUDA_TRY(cudaGetLastError());
+  ATRIP_CUDA_TRY(cudaFuncSetAttribute(v_profile, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kSmemLimit));
+  const unsigned pairs = (unsigned)((nvnv + kProfilePairs - 1) / kProfilePairs);
+  for (int w = 0; w < (a.use_j ? 2 : 1); ++w) {
+    v_profile<<<pairs, 256, profile_smem((int)Nv), st>>>(w ? a.Jp : a.Vp, t, (int)No, (int)Nv, h, w);
+    max_kernel<<<152 * 4, 256, 0, st>>>(w ? a.Jh : a.Vh, Nv * No * No * No, h, w);
   }
-  decide<<<1, 1024, 0, st>>>(slabs, nvnv, a.use_j, h);
+  decide<<<1, 1, 0, st>>>(a.use_j, h);
   ATRIP_CUDA_TRY(cudaGetLastError());
   int sms = 0;
   ATRIP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));

@@ -73,3 +73,31 @@ def test_decoupled_operands_in_a_batch():
     assert np.max(np.abs(e[2] - f[2])) <= 2 * 49 * 2.0 ** -52 * np.max(np.abs(f[2]))
     for c in ctxs:
         c.close()
+
+
+# the no-allocation entry point: its FP64-instruction kernel adds in another
+# order, so a W cell differs by K 2^-53 of the products it adds and a tuple's
+# energy by twice that, times at most its No^3 / 6 triples where they cancel
+@pytest.mark.parametrize("bits", [20, 30])
+@pytest.mark.parametrize("j", [False, True])
+def test_decoupled_operands_noalloc(bits, j):
+    torch = pytest.importorskip("torch")
+    No, Nv, n = 8, 40, 3000
+    d = _decoupled(No, Nv, bits, j)
+    names = NAMES + (J2 if j else ())
+    dev = {k: torch.from_numpy(np.ascontiguousarray(d[k].ravel(order="F"))).cuda() for k in names}
+    out = torch.empty(2 * n + 2, dtype=torch.float64, device="cuda")
+    ptrs = capi.DeviceInputs(*[dev[k].data_ptr() if k in dev else None for k in NAMES + J2])
+    lib = capi.load()
+    torch.cuda.synchronize()
+    capi.check(lib.atrip_gpu_run_fp64_noalloc(
+        No, Nv, ctypes.byref(ptrs), 0, n - 1, 0, 1, out.data_ptr() + 16,
+        out.data_ptr() + 16 + 8 * n, out.data_ptr(), None))
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()[2:].reshape(2, n)
+    with _ctx(d, j) as ctx:
+        ctx.set_tuning(fp64_tile_rows=64)
+        want = _run(ctx, n, j)
+    tol = No ** 3 / 6 * 2 * 2 * (Nv + No) * 2.0 ** -53
+    for x, y in zip(got, want):
+        assert np.all(np.abs(x - y) <= tol * np.abs(y))
