@@ -379,7 +379,8 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
                               (uintptr_t)b->tcb.planes, (uintptr_t)b->tcb.d_desc,
                               (uintptr_t)b->tcb.smem, (uintptr_t)b->tcb.lay_cells,
                               (uintptr_t)b->tcb.lay_pass, (uintptr_t)b->tcb.bslot, (uintptr_t)b->tcb.aslot,
-                              (uintptr_t)b->tcb.nslots, (uintptr_t)b->tcb.nbslots};
+                              (uintptr_t)b->tcb.nslots, (uintptr_t)b->tcb.nbslots,
+                              (uintptr_t)b->tcb.pieces};
     key.insert(key.end(), std::begin(more), std::end(more));
   }
   if (!b->exec || key != b->key) {

@@ -67,6 +67,7 @@ struct TcBuffers {
   int cap = 0;
   // launch layout of the last tc_launch_prepare
   int n = 0, S = 8, nc = 1;
+  int pieces = 1;  // items a row tile's sums are formed in
   bool split = false, f16 = false;
   int lay_no = 0, lay_cells = 0, lay_pass = 1, nslots = 0, nbslots = 0, aslot = 0,
       bslot = 0, grid = 0;

@@ -20,12 +20,12 @@
 // T_x with every V_yz must lie within 2^kRangeBits of the grids' largest
 // (kprofile.cuh): what is lost of K products (levels 8 and up, the bits below
 // the grids), at most 9 K 2^-64 of the grids' largest, is then below a third of
-// K 2^-53 of that product, the bound of an FP64 dot product's error; the
-// partial sums of levels 0..2 are
-// bounded below 2^24 by the rows' digit norms (Cauchy-Schwarz); sums of the
-// higher levels, random in sign for any data whose low-order bits are not
-// correlated, are checked to end below 2^22, a quarter of the exact range.
-// Whatever fails this is run by the DFMA kernel instead.
+// K 2^-53 of that product, the bound of an FP64 dot product's error; the sums
+// of levels 0..6 are exact by the rows' digit norms and where they end
+// (digit_sums.cuh), in one accumulator or, for longer K, the natural and the
+// transposed half in one each; level 7's weigh 2^-70 of the grids' largest
+// product, and what roundings could do to them (8 K of at most 16) stays below
+// K 2^-62 of it.  Whatever fails this is run by the DFMA kernel instead.
 //
 // Contraction structure: the six fused particle+hole terms of
 // src/atrip/Equations.cxx:455-728 pair up by their column index into three
@@ -72,6 +72,7 @@
 #include <type_traits>
 
 #include "complex.cuh"
+#include "digit_sums.cuh"
 #include "digits.cuh"
 #include "engine.cuh"
 #include "fp64_tc.cuh"
@@ -219,20 +220,27 @@ __device__ __forceinline__ TcPart part_of(const TcMaps &m, int g, int pt, int a,
 }
 
 // What a kernel instantiation multiplies: S digit slices and levels; CPLX a
-// complex system; SPLIT the split-precision forms' slices, BF16 of radix 2^8
-// or (F16) FP16 of radix 2^11, and their energy arithmetic.
-template <int S_, bool CPLX_, bool SPLIT_, bool F16_>
+// complex system; PIECES the items a row tile's sums are formed in, 2: its
+// natural and its transposed half, where K is too long for exact sums in one
+// (a constant: the issuer pays for every instruction; a run-time choice took
+// No=8/Nv=40 from 0.91 to 0.93 .. 0.97 ms); SPLIT the split-precision forms'
+// slices, BF16 of radix 2^8 or (F16) FP16 of radix 2^11, and their energy
+// arithmetic.
+template <int S_, bool CPLX_, bool SPLIT_, bool F16_, int PIECES_ = 1>
 struct Fmt {
   static constexpr int S = S_;
   static constexpr bool CPLX = CPLX_;
+  static constexpr int PIECES = PIECES_;
   static constexpr bool SPLIT = SPLIT_;  // an A ring slot holds all slices of a chunk
   __device__ static constexpr int radix() { return F16_ ? 2048 : 256; }
   __device__ static constexpr uint32_t idesc(int n) {
     return F16_ ? idesc_f16_f32(128, n) : idesc_bf16_f32(128, n);
   }
 };
-using FmtFp64 = Fmt<kS, false, false, false>;
-using FmtZ = Fmt<kS, true, false, false>;
+template <int PIECES>
+using FmtFp64 = Fmt<kS, false, false, false, PIECES>;
+template <int PIECES>
+using FmtZ = Fmt<kS, true, false, false, PIECES>;
 
 struct TcSlot {
   int64_t t;  // list position, -1 = no more work
@@ -435,7 +443,9 @@ __device__ __forceinline__ bool mma_tuple(MmaRole &m, bool fresh, int *status) {
     tc_fence_after();
     const uint32_t d = m.tm + buf * bufcols;
     uint32_t acc = 0;
-    for (int pt = 0; pt < TcParts<F::CPLX>::kCount; ++pt) {
+    constexpr int parts = TcParts<F::CPLX>::kCount / F::PIECES;
+    const int pt0 = F::PIECES == 2 && (it & 1) ? parts : 0;
+    for (int pt = pt0; pt < pt0 + parts; ++pt) {
       const int K = TcParts<F::CPLX>::hole(pt) ? m.kh : m.kp;
       for (int k0 = 0; k0 < K; k0 += kKChunk) {
         const uint64_t bd = sdesc_sw128(0) + ((m.ring_b + (uint32_t)(m.bs * m.bslot)) >> 4);
@@ -671,7 +681,8 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
         m.kh = uniform(d.No);
         m.rows = uniform(d.rows);
         m.spp = uniform(d.spp);
-        m.nitems = 3 * (uniform(d.use_j) ? 2 : 1) * ((m.kh * m.kh + m.rows - 1) / m.rows);
+        m.nitems =
+            3 * (uniform(d.use_j) ? 2 : 1) * ((m.kh * m.kh + m.rows - 1) / m.rows) * F::PIECES;
       }
       if constexpr (CPLX) {  // P = 2 round_up(No, 8)
         switch (m.P) {
@@ -721,8 +732,10 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
       const int wb = k & 1;
       const uint32_t wuse = k >> 1;
       ok = wuse == 0 || mbar_wait(&wfree[wb], (wuse - 1) & 1, status, kErrEmpty);
-      for (int it = 0; it < 3 * npass * ntiles; ++it, ++item) {
-        const int gi = it / ntiles, mt = it - gi * ntiles, grp = gi % 3, pass = gi / 3;
+      for (int it = 0; it < 3 * npass * ntiles * F::PIECES; ++it, ++item) {
+        const int tile = it / F::PIECES;
+        const bool second = F::PIECES == 2 && (it & 1);  // added to what the first stored
+        const int gi = tile / ntiles, mt = tile - gi * ntiles, grp = gi % 3, pass = gi / 3;
         Cell *plane0 = planes + (size_t)((wb * g.lay_pass + pass) * 3 + grp) * kComp * cells;
         const int bb = item & 1, buf = nbuf == 2 ? bb : 0;
         bool okw = ok && alive && mbar_wait(&accf[bb], (item >> 1) & 1, status, kErrAccFull);
@@ -777,10 +790,15 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
               const int n23 = (int)(b[2] * 256u + b[3] - kBits * 257u);
               const int n45 = (int)(b[4] * 256u + b[5] - kBits * 257u);
               const int n67 = (int)(b[6] * 256u + b[7] - kBits * 257u);
-              const long long hi = (long long)__float2int_rn(v[0][x]) * (1 << 24) +
-                                   ((long long)n1 * 65536 + n23);
-              const long long lo = (long long)n45 * 65536 + n67;
-              plane[(size_t)r * No2 + m] = make_longlong2(hi, lo);
+              long long hi = (long long)__float2int_rn(v[0][x]) * (1 << 24) +
+                             ((long long)n1 * 65536 + n23);
+              long long lo = (long long)n45 * 65536 + n67;
+              Cell &w = plane[(size_t)r * No2 + m];
+              if (second) {  // stored by this thread
+                hi += w.x;
+                lo += w.y;
+              }
+              w = make_longlong2(hi, lo);
             }
           }
         }
@@ -1001,7 +1019,7 @@ __global__ void __launch_bounds__(256) v_profile_kernel(const double *__restrict
 }
 
 // dst[s][R][k] (pitch Kp) = digit_s(sign src(R, k)), row R = (o n1 + r1) n2
-// + r2.  norms[s], s < 3: the largest row sum of q_s^2.
+// + r2.  norms[s], s < kNormSlices: the largest row sum of q_s^2.
 struct CutJob {
   const double *src;
   __nv_bfloat16 *dst;
@@ -1015,12 +1033,12 @@ __global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
   const int64_t plane = j.nrows * j.nblk * j.Kp;
   const int lane = threadIdx.x & 31;
   const int64_t nw = (int64_t)gridDim.x * 8;
-  unsigned int best[3] = {0, 0, 0};
+  unsigned int best[kNormSlices] = {};
   for (int64_t R = blockIdx.x * 8 + (threadIdx.x >> 5); R < j.nrows; R += nw) {
     const int64_t r2 = R % j.n2, t = R / j.n2, r1 = t % j.n1, o = t / j.n1;
     const double *src = j.src + o * j.so + r1 * j.s1 + r2 * j.s2;
     __nv_bfloat16 *dst = j.dst + ((t * j.nblk + j.blk) * j.n2 + r2) * j.Kp;
-    unsigned int nrm[3] = {0, 0, 0};
+    float nrm[kNormSlices] = {};  // whole numbers below 2^24
     for (int k = 2 * lane; k < j.Kp; k += 64) {
       unsigned long long y[2];
 #pragma unroll
@@ -1035,24 +1053,24 @@ __global__ void __launch_bounds__(256) cut_kernel(CutJob j) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           q[h] = digit(y[h], s);
-          if (s < 3) nrm[s] += (unsigned int)(int)(q[h] * q[h]);
+          if (s < kNormSlices) nrm[s] = fmaf(q[h], q[h], nrm[s]);
         }
         *reinterpret_cast<__nv_bfloat162 *>(dst + s * plane + k) =
             __floats2bfloat162_rn(q[0], q[1]);
       }
     }
 #pragma unroll
-    for (int s = 0; s < 3; ++s) {
-      unsigned int v = nrm[s];
-#pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o2);
+    for (int s = 0; s < kNormSlices; ++s) {
+      const unsigned int v = __reduce_add_sync(0xffffffffu, (unsigned int)nrm[s]);
       best[s] = v > best[s] ? v : best[s];
     }
   }
-  if (lane < 3) {
-    const unsigned int v = lane == 0 ? best[0] : lane == 1 ? best[1] : best[2];
-    if (v > *(volatile unsigned int *)&j.norms[lane]) atomicMax(&j.norms[lane], v);
-  }
+  unsigned int v = 0;  // lane s takes digit s
+#pragma unroll
+  for (int s = 0; s < kNormSlices; ++s)
+    if (lane == s) v = best[s];
+  if (lane < kNormSlices && v > *(volatile unsigned int *)&j.norms[lane])
+    atomicMax(&j.norms[lane], v);
 }
 
 // ------------------------------------------------------------------ host
@@ -1063,7 +1081,8 @@ struct TcImpl {
   int nc = 1;  // doubles per element: 2 for a complex system
   int No = 0, Nv = 0, P = 0, rows = 0, spp = 0, Kp = 0, Kh = 0;
   int eT = 0, eV = 0, eJ = 0;
-  double nT[3], nU[3];          // digit norms of the T rows (over E; over L)
+  DigitNorms nT, nU;            // of the T rows (over E; over L)
+  int pieces = 1, pieces_j = 1;
   double unit = 1.0, unit_j = 1.0;
   char *arena = nullptr, *arena_j = nullptr;
   TcMaps maps;
@@ -1142,7 +1161,7 @@ double as_double(unsigned long long b) {
 struct DeviceStats {
   unsigned long long t_max, vp_max, vh_max;  // largest magnitudes
   unsigned int least;                        // least product (log_of sums)
-  unsigned int n[8][4];                      // digit norms of up to eight cut jobs
+  unsigned int n[8][8];                      // digit norms of up to eight cut jobs
 };
 
 // Queue the examination of T against a pair V_hhhp, V_pphp (or J): maxima and
@@ -1212,24 +1231,18 @@ bool grids_of(const DeviceStats &h, int *e_t, int *e_v) {
   return std::ldexp((double)h.least, -kLogOne) - 2 * kLogBias >= *e_t + *e_v - kRangeBits;
 }
 
-// Bound of |partial sums| of levels 0, 1 and 2: twice (natural and transposed
-// part; four times for a complex system, whose rows meet real and imaginary
-// columns) the Cauchy-Schwarz products.
-bool sums_exact(int nc, const double *nT, const double *nV, const double *nH, const double *nU) {
-  for (int L = 0; L < 3; ++L) {
-    double b = 0;
-    for (int s = 0; s <= L; ++s)
-      b += 2.0 * nc * (std::sqrt(nT[s] * nV[L - s]) + std::sqrt(nH[s] * nU[L - s]));
-    if (!(b < 16777216.0)) return false;
-  }
-  return true;
+DigitNorms norms_of(const unsigned int *x) {
+  DigitNorms n;
+  for (int s = 0; s < kNormSlices; ++s) n.q2[s] = (double)x[s];
+  return n;
 }
 
-void set_norms(double *out, const unsigned int *x) {
-  for (int s = 0; s < 3; ++s) out[s] = (double)x[s];
-}
-void max_norms(double *out, const unsigned int *x) {
-  for (int s = 0; s < 3; ++s) out[s] = std::max(out[s], (double)x[s]);
+// Accumulators a row tile's sums need to be exact: one for its natural and
+// transposed half, or one each; 0: not exact either.  A complex system's rows
+// meet real and imaginary columns.
+int sum_pieces(int nc, const DigitNorms &nT, const DigitNorms &nV, const DigitNorms &nH,
+               const DigitNorms &nU) {
+  return level_sums_exact(2 * nc, nT, nV, nH, nU) ? 1 : level_sums_exact(nc, nT, nV, nH, nU) ? 2 : 0;
 }
 
 // A column operand: its one block, or the three of a complex system, of
@@ -1367,13 +1380,12 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cpl
   if (rc != ATRIP_OK) return rc;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
-  set_norms(p->nT, h.n[0]);
-  set_norms(p->nU, h.n[1]);
-  max_norms(p->nU, h.n[2]);
-  double nH[3], nV[3];
-  set_norms(nH, h.n[4]);
-  set_norms(nV, h.n[5]);
-  if (!sums_exact(p->nc, p->nT, nV, nH, p->nU)) return ATRIP_OK;
+  p->nT = norms_of(h.n[0]);
+  p->nU = norms_of(h.n[1]);
+  const DigitNorms nU2 = norms_of(h.n[2]);
+  for (int s = 0; s < kNormSlices; ++s) p->nU.q2[s] = std::max(p->nU.q2[s], nU2.q2[s]);
+  p->pieces = sum_pieces(p->nc, p->nT, norms_of(h.n[5]), norms_of(h.n[4]), p->nU);
+  if (p->pieces == 0) return ATRIP_OK;
 
   for (int i = 0; i < 4; ++i) {  // [component][row order]; a real system's twice
     const int k = i % (2 * nc);
@@ -1412,10 +1424,9 @@ int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *lau
   if (rc != ATRIP_OK) return rc;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
-  double nH[3], nV[3];
-  set_norms(nH, h.n[4]);
-  set_norms(nV, h.n[5]);
-  if (!sums_exact(p->nc, p->nT, nV, nH, p->nU)) return ATRIP_OK;
+  const int pieces = sum_pieces(p->nc, p->nT, norms_of(h.n[5]), norms_of(h.n[4]), p->nU);
+  if (pieces == 0) return ATRIP_OK;
+  p->pieces_j = std::max(p->pieces, pieces);
   for (int i = 0; i < 4; ++i)
     if ((rc = map_a(&p->maps.Jh[i / 2][i % 2], vh[i % (2 * nc)], *p, p->Kh))) return rc;
   if ((rc = map_b(&p->maps.Jp, vp, *p, p->Kp))) return rc;
@@ -1580,6 +1591,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   b.lay_pass = 1;
   b.aslot = 0;
   b.nc = 1;
+  b.pieces = 1;
   b.h_prefix[0] = 0;
   for (int k = 0; k < n; ++k) {
     const TcSystem &m = sys[k];
@@ -1612,6 +1624,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     d.spp = p->spp;
     d.n_triples = m.n_triples;
     d.use_j = m.use_j ? 1 : 0;
+    b.pieces = std::max(b.pieces, m.use_j ? p->pieces_j : p->pieces);
     h[k] = d;
     P = std::max(P, p->P);
     b.nc = p->nc;  // the same for all: a batch holds real systems
@@ -1688,7 +1701,9 @@ int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st
   a.nbslots = b.nbslots;
   a.aslot = b.aslot;
   a.bslot = b.bslot;
-  auto kern = b.nc == 2 ? triples_tc_kernel<FmtZ> : triples_tc_kernel<FmtFp64>;
+  auto kern = b.nc == 2 ? (b.pieces == 2 ? triples_tc_kernel<FmtZ<2>> : triples_tc_kernel<FmtZ<1>>)
+                        : b.pieces == 2 ? triples_tc_kernel<FmtFp64<2>>
+                                        : triples_tc_kernel<FmtFp64<1>>;
   if (b.split)
     kern = b.f16    ? triples_tc_kernel<Fmt<2, false, true, true>>
            : b.S == 2 ? triples_tc_kernel<Fmt<2, false, true, false>>

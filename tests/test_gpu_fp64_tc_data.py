@@ -101,3 +101,31 @@ def test_decoupled_operands_noalloc(bits, j):
     tol = No ** 3 / 6 * 2 * 2 * (Nv + No) * 2.0 ** -53
     for x, y in zip(got, want):
         assert np.all(np.abs(x - y) <= tol * np.abs(y))
+
+
+# digits of full size and random signs: the norms of their level sums allow one
+# accumulator only up to Nv + No ~ 150 (complex 75), two here
+def _digits(rng, shape):
+    x = 126.0 * rng.choice([-1.0, 1.0], size=shape)
+    for s in range(1, 6):
+        x += 127.0 * 2.0 ** (-8 * s) * rng.choice([-1.0, 1.0], size=shape)
+    return x * 2.0 ** -7
+
+
+@pytest.mark.parametrize("No,Nv,j,field", [(4, 160, False, "real"), (5, 155, True, "real"),
+                                           (40, 115, False, "real"), (9, 70, False, "complex")])
+def test_sums_in_two_accumulators(No, Nv, j, field):
+    d = synth.make_inputs(No, Nv, 24, with_j=j, field=field)
+    rng = np.random.default_rng(No)
+    for k in ("Tabij", "Vijka", "Vabci") + (J2 if j else ()):
+        x = _digits(rng, d[k].shape)
+        d[k] = x + 1j * _digits(rng, d[k].shape) if field == "complex" else x
+    n = 300
+    with _ctx(d, j, field) as ctx:
+        e, ect = _run(ctx, n, j)
+        ctx.set_tuning(fp64_tile_rows=64)
+        f, fct = _run(ctx, n, j)
+    K = 2 * (Nv + No) * (2 if field == "complex" else 1)
+    assert not np.array_equal(e, f)  # another kernel
+    assert np.max(np.abs(e - f)) <= K * 2.0 ** -52 * np.max(np.abs(f))
+    assert np.max(np.abs(ect - fct)) <= K * 2.0 ** -52 * np.max(np.abs(fct))
