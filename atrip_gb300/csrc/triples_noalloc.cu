@@ -309,10 +309,14 @@ constexpr int kS = 8;           // digit slices and levels
 constexpr int kChunk = 64;      // K elements per 128-byte row
 constexpr int kATile = 128 * 128;
 constexpr int kSmemLimit = 232448;
-// K contributions an accumulator may hold: levels 0..2 stay below 2^24
-// whatever the digits are, 3 K 2^14 <= 2^24.  Longer sums are drained into W
-// in pieces.
-constexpr int kMaxK = 341;
+// K contributions an accumulator may hold: then the sums of levels 0..5 are
+// exact whatever the digits are, 6 K 2^14 < 2^25 - 2^22 - 2^16
+// (digit_sums.cuh).  In level 6, 7 K products of at most 2^14, at least 1792
+// must go into a sum that passes 2^24 and comes back, so at most 280 are added
+// beyond, each rounded by at most 2: below 2^-52 of the grids' largest
+// product, a quarter of what an FP64 dot product of that length may lose.
+// Longer sums are drained into W in pieces.
+constexpr int kMaxK = 296;
 constexpr int kRangeBits = 6;  // least product against the grids' largest: triples_fp64_tc.cu
 
 // out[s] = largest magnitude of slab s of x[s + nslab c], c < count.
