@@ -312,8 +312,13 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
                     t.split_variant == 0;
     }
     if (b->tcs_used) {
-      int rc = prepare_all(true);
+      const int rc = prepare_all(true);
       if (rc != ATRIP_OK) return rc;
+      for (int k = 0; k < n; ++k)
+        b->tcs_used = b->tcs_used && split_finite(b->sys[b->order[k]]->split, b->h_table[k].use_j != 0);
+    }
+    if (b->tcs_used) {
+      int rc;
       std::vector<TcSystem> ts(n);
       for (int k = 0; k < n; ++k) {
         atrip_gpu_context *c = b->sys[b->order[k]];

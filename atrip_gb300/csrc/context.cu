@@ -587,10 +587,15 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
       }
       const double tai_sign = opts->ijkabc ? -1.0 : 1.0;
       auto run_split = [&]() -> int {
+        split_on_tc = false;
         if (on_tc) {
           int rc = split_prepare(c->split, c->dt, c->No, c->Nv, 0, use_j, slices, c->d_triples,
                                  c->n_triples, st, &launches);
           if (rc != ATRIP_OK) return rc;
+          split_on_tc = split_finite(c->split, use_j);
+        }
+        if (split_on_tc) {
+          int rc;
           TcSystem ts = {&c->split.tc, &c->dt, c->No, c->Nv, c->n_triples, c->d_tuples,
                          c->d_triples, t_begin, t_end, use_j, c->d_e, c->d_ect, nullptr};
           if ((rc = split_tc_attach(c->split, use_j, &ts.tri_ef)) != ATRIP_OK) return rc;
@@ -610,7 +615,6 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
         rc = run_split();
       }
       if (rc != ATRIP_OK) return rc;
-      split_on_tc = on_tc;
     }
     ATRIP_CUDA_TRY(launch_energy_sum(c->d_e + t_begin, c->d_ect + t_begin, n, c->d_partials,
                                      c->d_sum, st));

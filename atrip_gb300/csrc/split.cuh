@@ -49,6 +49,10 @@ bool split_tc_eligible(int slices, bool f16, int No, int Nv);
 // (few rows to stack), No=53/Nv=201 157 / 151, No=56/Nv=440 228 / 191 (singles
 // blocks that no longer fit beside three stages).
 bool split_prefers_transposed(int slices, bool f16, int No, int Nv);
+// Whether the prepared operands hold finite values only.  The kernel of
+// fp64_tc.cuh joins a cell's level sums as integers, which an infinity or a NaN
+// does not survive; the split kernels keep it in the FP32 part of a cell.
+bool split_finite(const SplitState &s, bool use_j);
 // The prepared slices' maps for it, and the triple table it reads.
 int split_tc_attach(SplitState &s, bool use_j, const double2 **tri_ef);
 

@@ -122,15 +122,20 @@ struct SplitArgs {
 
 // ------------------------------------------------------------------ prep
 
+// out[0] = max |x| (NaN aside), out[1] = 1 if an element is not finite.
 __global__ void absmax_kernel(const double *__restrict__ x, int64_t n,
                               unsigned long long *__restrict__ out) {
   double m = 0.0;
+  bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
+       i += (int64_t)gridDim.x * blockDim.x) {
     m = fmax(m, fabs(x[i]));
+    bad |= !isfinite(x[i]);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
+  if (bad) out[1] = 1;
 }
 
 // Per (i,j,k) triple of the energy loop, independent of the tuple: the
@@ -1206,6 +1211,7 @@ struct SplitImpl {
                 *VpS = nullptr, *TpS = nullptr, *TpTS = nullptr;
   __nv_bfloat16 *JhS = nullptr, *JhST = nullptr, *JpS = nullptr;  // (cT), cut on demand
   bool has_j = false;
+  bool finite = true, finite_j = true;  // every element of the operands
   int eT = 0;
   double unit = 1.0, unit_j = 1.0;
   float *wglobal = nullptr;
@@ -1287,18 +1293,18 @@ int exponent_of(double maxabs) {
   return std::ilogb(maxabs) + 1;  // maxabs < 2^e
 }
 
-int absmax(const double *x, int64_t n, unsigned long long *d_tmp, cudaStream_t st, double *out) {
-  ATRIP_CUDA_TRY(cudaMemsetAsync(d_tmp, 0, sizeof(unsigned long long), st));
+int absmax(const double *x, int64_t n, unsigned long long *d_tmp, cudaStream_t st, double *out,
+           bool *finite) {
+  ATRIP_CUDA_TRY(cudaMemsetAsync(d_tmp, 0, 2 * sizeof(unsigned long long), st));
   if (n > 0) {
     absmax_kernel<<<152 * 8, 256, 0, st>>>(x, n, d_tmp);
     ATRIP_CUDA_TRY(cudaGetLastError());
   }
-  unsigned long long h = 0;
-  ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, d_tmp, sizeof(h), cudaMemcpyDeviceToHost, st));
+  unsigned long long h[2] = {0, 0};
+  ATRIP_CUDA_TRY(cudaMemcpyAsync(h, d_tmp, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
-  double v;
-  std::memcpy(&v, &h, sizeof(v));
-  *out = v;
+  std::memcpy(out, h, sizeof(*out));
+  if (h[1] != 0) *finite = false;
   return ATRIP_OK;
 }
 
@@ -1319,11 +1325,12 @@ int prepare(SplitImpl *p, const DeviceTensors &dt, int No, int Nv, int S, int bi
   p->Ep = (Nv + kKChunk - 1) / kKChunk * kKChunk;
   const int64_t No2 = (int64_t)No * No, Ep = p->Ep;
   unsigned long long *d_tmp = nullptr;
-  ATRIP_CUDA_TRY(cudaMalloc(&d_tmp, sizeof(unsigned long long)));
+  ATRIP_CUDA_TRY(cudaMalloc(&d_tmp, 2 * sizeof(unsigned long long)));
   double mT = 0, mVp = 0, mVh = 0;
-  int rc = absmax(dt.Ta, (int64_t)Nv * No2 * Nv, d_tmp, st, &mT);
-  if (rc == ATRIP_OK) rc = absmax(dt.Vpt, (int64_t)Nv * Nv * No * Nv, d_tmp, st, &mVp);
-  if (rc == ATRIP_OK) rc = absmax(dt.Vht, (int64_t)Nv * No2 * No, d_tmp, st, &mVh);
+  int rc = absmax(dt.Ta, (int64_t)Nv * No2 * Nv, d_tmp, st, &mT, &p->finite);
+  if (rc == ATRIP_OK)
+    rc = absmax(dt.Vpt, (int64_t)Nv * Nv * No * Nv, d_tmp, st, &mVp, &p->finite);
+  if (rc == ATRIP_OK) rc = absmax(dt.Vht, (int64_t)Nv * No2 * No, d_tmp, st, &mVh, &p->finite);
   cudaFree(d_tmp);
   if (rc != ATRIP_OK) return rc;
   *launches += 3;
@@ -1458,10 +1465,10 @@ int prepare_j(SplitImpl *p, const DeviceTensors &dt, cudaStream_t st, int64_t *l
   const int No = p->No, Nv = p->Nv, S = p->S;
   const int64_t No2 = (int64_t)No * No, Ep = p->Ep;
   unsigned long long *d_tmp = nullptr;
-  ATRIP_CUDA_TRY(cudaMalloc(&d_tmp, sizeof(unsigned long long)));
+  ATRIP_CUDA_TRY(cudaMalloc(&d_tmp, 2 * sizeof(unsigned long long)));
   double mJp = 0, mJh = 0;
-  int rc = absmax(dt.Jpt, (int64_t)Nv * Nv * No * Nv, d_tmp, st, &mJp);
-  if (rc == ATRIP_OK) rc = absmax(dt.Jht, (int64_t)Nv * No2 * No, d_tmp, st, &mJh);
+  int rc = absmax(dt.Jpt, (int64_t)Nv * Nv * No * Nv, d_tmp, st, &mJp, &p->finite_j);
+  if (rc == ATRIP_OK) rc = absmax(dt.Jht, (int64_t)Nv * No2 * No, d_tmp, st, &mJh, &p->finite_j);
   cudaFree(d_tmp);
   if (rc != ATRIP_OK) return rc;
   *launches += 2;
@@ -2037,6 +2044,11 @@ bool split_tc_eligible(int slices, bool f16, int No, int Nv) {
 bool split_prefers_transposed(int slices, bool f16, int No, int Nv) {
   return slices == 2 && ((No >= 12 && No <= 52) || No > 56) &&
          transposed_eligible(slices, No, Nv, f16);
+}
+
+bool split_finite(const SplitState &s, bool use_j) {
+  auto *p = static_cast<const SplitImpl *>(s.impl);
+  return p && p->finite && (!use_j || p->finite_j);
 }
 
 int split_tc_attach(SplitState &s, bool use_j, const double2 **tri_ef) {
