@@ -64,3 +64,44 @@ def test_not_finite_in_a_batch(form, S):
     assert np.isnan(out[1][1]).any() and not np.isnan(out[1][0]).any()
     for x, y in zip(*out):
         _same(x, y)
+
+
+# every digit product of level 1 of one sign: its sum passes 2^31 from
+# K = 2 (Nv + No) = 1100 or so on.  T and V depend on their indices by the first
+# digit: a W cell that is the same under all permutations has no energy.  Digits
+# are multiples of 16, so every sum is exact in FP32, in either kernel
+@pytest.mark.parametrize("No,Nv", [(2, 500), (2, 600), (3, 700)])
+def test_coherent_digits_f16(No, Nv):
+    torch = pytest.importorskip("torch")
+    top, low = 1008, 1008 / 2048  # first and second digit
+    x = (top + low) / 1024
+    v = torch.arange(Nv, dtype=torch.float64, device="cuda").clamp(max=4)
+    p = torch.arange(No, dtype=torch.float64, device="cuda")
+
+    def const(n, value):
+        return torch.full((n,), value, dtype=torch.float64, device="cuda")
+
+    def tensor(t):  # column-major data of t[first index, ...]
+        return t.permute(*reversed(range(t.dim()))).contiguous().ravel()
+
+    with capi.Context(No, Nv, 0) as ctx:
+        for k, t in (("epsi", const(No, -1.0)), ("epsa", const(Nv, 1.0)), ("Tai", const(Nv * No, 0.01)),
+                     ("Vabij", const(Nv * Nv * No * No, 0.1)), ("Vijka", const(No ** 3 * Nv, -x))):
+            torch.cuda.synchronize()
+            ctx.upload(k, t)
+        t = top + low - 16 * v[:, None, None, None] - 112 * p[:, None] - 208 * p
+        t = tensor(t.expand(Nv, Nv, No, No) / 1024)
+        torch.cuda.synchronize()
+        ctx.upload("Tabij", t)
+        t = top + low - 32 * v[None, :, None, None] - 160 * p
+        t = tensor(t.expand(Nv, Nv, Nv, No) / 1024)
+        torch.cuda.synchronize()
+        ctx.upload("Vabci", t)
+        ctx.run(form="split_f16", use_j=False, max_iterations=99)
+        e, _ = ctx.tuple_energies(0, 100)
+        ctx.set_tuning(split_variant=2)
+        ctx.run(form="split_f16", use_j=False, max_iterations=99)
+        f, _ = ctx.tuple_energies(0, 100)
+    del t
+    torch.cuda.empty_cache()
+    _same(e, f)
