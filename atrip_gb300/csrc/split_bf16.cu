@@ -51,6 +51,7 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "kprofile.cuh"
 #include "recip.cuh"
 #include "sm100.cuh"
 #include "split.cuh"
@@ -122,19 +123,21 @@ struct SplitArgs {
 
 // ------------------------------------------------------------------ prep
 
-// out[0] = max |x| (NaN aside), out[1] = 1 if an element is not finite.
+// out[0] = max |x| (NaN aside) as a bit pattern, out[1] = 1 if an element is
+// not finite.  Magnitudes compare as integers do, off the narrow FP64 pipe
+// (No=40/Nv=400, first run: 117.4 ms with fmax and isfinite, so 111.5).
 __global__ void absmax_kernel(const double *__restrict__ x, int64_t n,
                               unsigned long long *__restrict__ out) {
-  double m = 0.0;
+  constexpr unsigned long long kInf = 0x7ff0000000000000ull;
+  unsigned long long m = 0;
   bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    m = fmax(m, fabs(x[i]));
-    bad |= !isfinite(x[i]);
+    const unsigned long long b = magnitude(x[i]);
+    bad |= b >= kInf;
+    m = b > m && b <= kInf ? b : m;
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
+  warp_max(m, out);
   if (bad) out[1] = 1;
 }
 
