@@ -17,6 +17,7 @@ void clear_error();
   do {                                                                            \
     cudaError_t _e = (call);                                                      \
     if (_e != cudaSuccess) {                                                      \
+      cudaGetLastError(); /* a later launch's check is not to find it */          \
       ::atrip_gb300::set_error(std::string(#call) + ": " + cudaGetErrorString(_e) + \
                                " (" + __FILE__ + ":" + std::to_string(__LINE__) + ")"); \
       return _e == cudaErrorMemoryAllocation ? ATRIP_ERR_OUT_OF_MEMORY : ATRIP_ERR_CUDA; \

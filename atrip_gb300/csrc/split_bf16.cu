@@ -1946,6 +1946,7 @@ int split_prepare(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
     s.generation++;
     cudaFree(p->wglobal);
     p->wglobal = nullptr;
+    p->wglobal_floats = 0;  // a smaller run after a failed allocation must not find the old size
     ATRIP_CUDA_TRY(cudaMalloc(&p->wglobal, sizeof(float) * need));
     p->wglobal_floats = need;
   }
