@@ -82,6 +82,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, i
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code, limit));
 }
 
+// Wait for a phase whatever the status says, with a limit of its own: what is
+// in flight must land before its memory is given back.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
+  for (int it = 0; it < (1 << 20) && !mbar_try_wait(bar, parity); ++it) {
+  }
+}
+
 // True in one lane of a converged warp.  A role that issues tcgen05 or TMA
 // instructions keeps its whole warp in the loop and lets this lane issue:
 // their operands live in uniform registers, and in code that the compiler

@@ -156,12 +156,6 @@ __device__ __forceinline__ void tensormap_acquire(const void *map) {
                : "memory");
 }
 
-// Wait for a phase whatever the status says, with a limit of its own.
-__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
-  for (int it = 0; it < (1 << 20) && !mbar_try_wait(bar, parity); ++it) {
-  }
-}
-
 // |n| < 2^51: 1.5 2^52 + n holds n in its low mantissa bits.
 __device__ __forceinline__ double i64_to_f64(long long n) {
   return __longlong_as_double(0x4338000000000000ll + n) - 6755399441055744.0;

@@ -730,7 +730,9 @@ __global__ void __launch_bounds__(kThreads, 1) kernel(Args g) {
     }
   }
   if (over & 0xFF800000u) atomicOr(&h->tc_overflow, 1);
-  // no MMA outlives the block (after a failed wait some may be in flight)
+  // no MMA outlives the block: after a wait that gave up (its own, or another
+  // block's, reported) those of the last commit may be in flight
+  if (!alive && warp == 0) mbar_drain(&t.bar, (phase - 1) & 1);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
