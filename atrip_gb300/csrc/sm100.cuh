@@ -11,6 +11,10 @@
 namespace atrip_gb300 {
 namespace sm100 {
 
+// Shared memory a block may ask for.  Every kernel's attribute is set to this
+// and never to a launch's own size: it belongs to the function on the device,
+// and another thread's launch of it with more would fail.
+constexpr int kSmemLimit = 232448;
 constexpr long long kWaitCycles = 4000000000ll;  // ~2 s at 2 GHz
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {

@@ -63,7 +63,6 @@ using namespace sm100;
 
 constexpr int kThreads = 512;
 constexpr int kMaxStages = 6;
-constexpr int kSmemLimit = 232448;  // opt-in dynamic shared memory per block
 constexpr int kTailBytes = 384 + 3 * 64 * 8 + 16 * 8 + 64 * 8;  // + W copy, staging
 constexpr int kKChunk = 64;              // BF16 elements per 128-byte row
 constexpr int kATileBytes = 128 * 128;   // 128 rows x 128 B
@@ -1556,7 +1555,7 @@ int launch_shape(SplitImpl *p, const SplitArgs &a, int sm_count, cudaStream_t st
   const size_t smem = 1024 + (size_t)nst * K::kStageBytes + kTailBytes + vbytes;
   auto kern = triples_split_kernel<S, NP, SPLIT0, WSMEM, false>;
   ATRIP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+                                      kSmemLimit));
   const int64_t n = a.t_end - a.t_begin;
   const int grid = (int)(n < sm_count ? n : sm_count);
   kern<<<grid, kThreads, smem, st>>>(p->maps, args);
@@ -1644,7 +1643,7 @@ int launch_shape_t(SplitImpl *p, const SplitArgs &a, int sm_count, cudaStream_t 
     }
   }
   ATRIP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+                                      kSmemLimit));
   const int64_t n = a.t_end - a.t_begin;
   const int grid = (int)(n < sm_count ? n : sm_count);
   kern<<<grid, kThreads, smem, st>>>(p->maps, args);
@@ -1709,7 +1708,7 @@ template <int S, bool WSMEM, bool F16>
 int launch_multi(const SplitMultiBuffers &b, const SplitArgs &a, int grid, cudaStream_t st) {
   auto kern = triples_split_kernel<S, 16, false, WSMEM, true, false, F16, true>;
   ATRIP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)b.smem));
+                                      kSmemLimit));
   SplitMaps none;
   std::memset(&none, 0, sizeof(none));
   kern<<<grid, kThreads, b.smem, st>>>(none, a);

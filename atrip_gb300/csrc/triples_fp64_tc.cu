@@ -92,7 +92,6 @@ constexpr int kMaxSlots = 10;               // A ring
 constexpr int kTupleSlots = 4;
 constexpr int kEnergyWarps = 10;
 constexpr int kEnergyThreads = kEnergyWarps * 32;
-constexpr int kSmemLimit = 232448;
 constexpr int kT1 = 64;  // doubles per t1 row: No <= 64, or No <= 32 complex
 constexpr int kTailBytes = 576 + 3 * kT1 * 8 + 16 * 8;
 constexpr int kRangeBits = 6;               // least product against 2^(eT+eV)
@@ -1715,7 +1714,7 @@ int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st
            : b.S == 3 ? triples_tc_kernel<Fmt<3, false, true, false>>
                       : triples_tc_kernel<Fmt<4, false, true, false>>;
   ATRIP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)b.smem));
+                                      kSmemLimit));
   kern<<<b.grid, kThreads, b.smem, st>>>(a);
   ATRIP_CUDA_TRY(cudaGetLastError());
   *launches += 1;

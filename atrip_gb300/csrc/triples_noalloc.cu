@@ -308,7 +308,6 @@ constexpr int kThreads = 512;
 constexpr int kS = 8;           // digit slices and levels
 constexpr int kChunk = 64;      // K elements per 128-byte row
 constexpr int kATile = 128 * 128;
-constexpr int kSmemLimit = 232448;
 // K contributions an accumulator may hold: then the sums of levels 0..5 are
 // exact whatever the digits are, 6 K 2^14 < 2^25 - 2^22 - 2^16
 // (digit_sums.cuh).  In level 6, 7 K products of at most 2^14, at least 1792
@@ -788,7 +787,7 @@ int enqueue(const Args &a, int device, cudaStream_t st) {
   const int ctas = (int)std::min<int64_t>(std::min<int64_t>(sms, fit), n);
   const size_t smem = smem_bytes((int)No);
   ATRIP_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+                                      kSmemLimit));
   kernel<<<ctas, kThreads, smem, st>>>(a);
   ATRIP_CUDA_TRY(cudaGetLastError());
   return ATRIP_OK;
