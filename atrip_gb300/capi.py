@@ -112,6 +112,7 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
     lib.atrip_gpu_upload.argtypes = [P, ctypes.c_int32, P, ctypes.c_int64]
     lib.atrip_gpu_upload_device.argtypes = [P, ctypes.c_int32, P, ctypes.c_int64]
     lib.atrip_gpu_release.argtypes = [P, ctypes.c_int32]
+    lib.atrip_gpu_trim.argtypes = [P]
     lib.atrip_gpu_run.argtypes = [P, ctypes.POINTER(RunOptions), ctypes.POINTER(Result)]
     lib.atrip_gpu_tuple_energies.argtypes = [P, ctypes.c_int64, ctypes.c_int64, P, P]
     lib.atrip_gpu_n_tuples.argtypes = [ctypes.c_int32]
@@ -201,6 +202,10 @@ class Context:
 
     def release(self, name: str) -> None:
         check(self.lib.atrip_gpu_release(self.h, TENSOR_IDS[name]))
+
+    def trim(self) -> None:
+        """Give back the FP64 form's digit slices until the next FP64 run."""
+        check(self.lib.atrip_gpu_trim(self.h))
 
     def run(self, form: str = "fp64", slices: int = 0, ijkabc: bool = False, use_j: bool = True,
             first_iteration: int = 0, max_iterations: int = 0, start_energy: float = 0.0,

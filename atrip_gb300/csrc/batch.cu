@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -125,6 +126,22 @@ void fill_table(atrip_gpu_batch *b, int64_t first, int64_t max_it, double tai_si
   }
 }
 
+// The FP64 slices of the batch's systems and its own buffers for them make
+// room (the caller holds the systems' TcGuards); false if there were none.
+bool give_back_slices(atrip_gpu_batch *b) {
+  bool any = b->tcb.planes != nullptr;
+  for (atrip_gpu_context *c : b->sys)
+    if (c->tc.impl || c->tcb.planes) {
+      give_back(c);
+      any = true;
+    }
+  destroy_graph(b);
+  tc_buffers_free(b->tcb);
+  return any;
+}
+
+int run_batch(atrip_gpu_batch *b, const atrip_run_options *opts, atrip_result *results);
+
 }  // namespace
 
 extern "C" {
@@ -185,11 +202,11 @@ int atrip_gpu_batch_create(atrip_gpu_context *const *systems, int32_t n, atrip_g
   BATCH_TRY(cudaEventCreate(&b->ev0));
   BATCH_TRY(cudaEventCreate(&b->ev1));
   BATCH_TRY(cudaMallocHost(&b->h_table, sizeof(TriplesArgs) * n));
-  BATCH_TRY(cudaMalloc(&b->d_table, sizeof(TriplesArgs) * n));
+  BATCH_TRY(device_alloc(&b->d_table, sizeof(TriplesArgs) * n));
   BATCH_TRY(cudaMallocHost(&b->h_prefix, sizeof(int64_t) * (n + 1)));
-  BATCH_TRY(cudaMalloc(&b->d_prefix, sizeof(int64_t) * (n + 1)));
-  BATCH_TRY(cudaMalloc(&b->d_queue, sizeof(unsigned long long) * 8 * (n + 1)));
-  BATCH_TRY(cudaMalloc(&b->d_sums, sizeof(double) * 2 * n));
+  BATCH_TRY(device_alloc(&b->d_prefix, sizeof(int64_t) * (n + 1)));
+  BATCH_TRY(device_alloc(&b->d_queue, sizeof(unsigned long long) * 8 * (n + 1)));
+  BATCH_TRY(device_alloc(&b->d_sums, sizeof(double) * 2 * n));
   BATCH_TRY(cudaMallocHost(&b->h_sums, sizeof(double) * 2 * n));
   BATCH_TRY(cudaMallocHost(&b->h_status, sizeof(int) * n));
   b->max_per_sm = std::max({1, triples_fp64_batch_max_blocks_per_sm(b->max_no, 0),
@@ -197,7 +214,7 @@ int atrip_gpu_batch_create(atrip_gpu_context *const *systems, int32_t n, atrip_g
   b->grid = b->sm_count * std::max(1, triples_fp64_batch_max_blocks_per_sm(b->max_no, 0));
   const int64_t No = b->max_no;
   b->ws_stride = 2 * No * No * No;
-  BATCH_TRY(cudaMalloc(&b->d_workspace,
+  BATCH_TRY(device_alloc(&b->d_workspace,
                        sizeof(double) * b->ws_stride * b->sm_count * b->max_per_sm));
 #undef BATCH_TRY
   *out = b;
@@ -208,6 +225,24 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
                         atrip_result *results) {
   clear_error();
   if (!b || !opts || !results) return fail(ATRIP_ERR_ARGUMENT, "null argument");
+  ATRIP_CUDA_TRY(cudaSetDevice(b->device));
+  std::vector<atrip_gpu_context *> held = b->sys;  // in one order for every batch
+  std::sort(held.begin(), held.end());
+  std::vector<std::unique_ptr<TcGuard>> guards;
+  for (atrip_gpu_context *c : held) guards.emplace_back(new TcGuard(c));
+  int rc = run_batch(b, opts, results);
+  if (rc == ATRIP_ERR_OUT_OF_MEMORY && opts->form != ATRIP_FORM_FP64 && give_back_slices(b)) {
+    clear_error();
+    rc = run_batch(b, opts, results);
+  }
+  return rc;
+}
+
+}  // extern "C"
+
+namespace {
+
+int run_batch(atrip_gpu_batch *b, const atrip_run_options *opts, atrip_result *results) {
   if (opts->form != ATRIP_FORM_FP64 && opts->form != ATRIP_FORM_SPLIT_BF16 &&
       opts->form != ATRIP_FORM_AUTO && opts->form != ATRIP_FORM_SPLIT_F16)
     return fail(ATRIP_ERR_ARGUMENT, "unknown form " + std::to_string(opts->form));
@@ -473,7 +508,7 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
     const int rc = tc_launch_check(b->tcb, tc_states.data(), &rerun);
     if (rc != ATRIP_OK) return rc;
     // systems whose sums left the exact range are barred now: run again
-    if (rerun) return atrip_gpu_batch_run(b, opts, results);
+    if (rerun) return run_batch(b, opts, results);
   }
   if (form != ATRIP_FORM_FP64 && b->tcs_used) {
     std::vector<TcState *> states(n);
@@ -506,6 +541,10 @@ int atrip_gpu_batch_run(atrip_gpu_batch *b, const atrip_run_options *opts,
   }
   return ATRIP_OK;
 }
+
+}  // namespace
+
+extern "C" {
 
 int atrip_gpu_batch_set_tuning(atrip_gpu_batch *b, const atrip_tuning *t) {
   clear_error();

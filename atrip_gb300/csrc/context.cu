@@ -4,7 +4,9 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "atrip_gb300.h"
@@ -17,6 +19,48 @@ namespace atrip_gb300 {
 static thread_local std::string g_last_error;
 void set_error(const std::string &msg) { g_last_error = msg; }
 void clear_error() { g_last_error.clear(); }
+
+// Every context of the process, for device_alloc.
+static std::mutex g_contexts_mutex;
+static std::vector<atrip_gpu_context *> g_contexts;
+
+TcGuard::TcGuard(atrip_gpu_context *c) : c_(c) {
+  // held by another thread only for as long as giving memory back takes
+  while (c_->tc_held.exchange(true, std::memory_order_acquire)) std::this_thread::yield();
+}
+
+void free_tc(atrip_gpu_context *c) {
+  tc_free(c->tc);
+  tc_buffers_free(c->tcb);
+}
+
+void give_back(atrip_gpu_context *c) {
+  const bool barred = c->tc.tried && !c->tc.usable;
+  free_tc(c);
+  c->tc.tried = barred;
+}
+
+cudaError_t device_alloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  int device = 0;
+  cudaGetLastError();
+  if (cudaGetDevice(&device) != cudaSuccess) return e;
+  bool freed = false;
+  {
+    std::lock_guard<std::mutex> lock(g_contexts_mutex);  // no context goes away meanwhile
+    for (atrip_gpu_context *c : g_contexts) {
+      if (c->device != device || c->tc_held.exchange(true, std::memory_order_acquire)) continue;
+      if (c->tc.impl || c->tcb.planes) {
+        give_back(c);
+        freed = true;
+      }
+      c->tc_held.store(false, std::memory_order_release);
+    }
+  }
+  if (freed) e = cudaMalloc(p, bytes);
+  return e;
+}
 
 }  // namespace atrip_gb300
 
@@ -54,7 +98,7 @@ int build_order(atrip_gpu_context *c, int64_t t_begin, int64_t t_end, int L, cud
     cudaFree(c->d_order);
     c->d_order = nullptr;
     c->order_cap = 0;
-    ATRIP_CUDA_TRY(cudaMalloc(&c->d_order, sizeof(uint32_t) * (size_t)n));
+    ATRIP_CUDA_TRY(device_alloc(&c->d_order, sizeof(uint32_t) * (size_t)n));
     c->order_cap = n;
   }
   ATRIP_CUDA_TRY(cudaMemcpyAsync(c->d_order, out.data(), sizeof(uint32_t) * (size_t)n,
@@ -138,12 +182,6 @@ bool contraction_operand(int t) {
          t == ATRIP_JABCI;
 }
 
-// The FP64 slices are a copy the engine can do without: give them back.
-void free_tc(atrip_gpu_context *c) {
-  tc_free(c->tc);
-  tc_buffers_free(c->tcb);
-}
-
 void free_tensor(atrip_gpu_context *c, int t) {
   if (double **d = direct_slot(c, t)) {
     cudaFree(*d);
@@ -157,7 +195,10 @@ void free_tensor(atrip_gpu_context *c, int t) {
   }
   c->have[t] = false;
   split_invalidate(c->split);
-  if (contraction_operand(t)) tc_free(c->tc);
+  if (contraction_operand(t)) {
+    TcGuard guard(c);
+    tc_free(c->tc);
+  }
 }
 
 // Host uploads above this many elements are staged in chunks (default 2^28
@@ -185,12 +226,15 @@ int upload_impl(atrip_gpu_context *c, int32_t tensor, const double *src, int64_t
   if (!src && n > 0) return fail(ATRIP_ERR_ARGUMENT, "null source pointer");
   ATRIP_CUDA_TRY(cudaSetDevice(c->device));
   if (c->have[tensor]) free_tensor(c, tensor);
-  if (contraction_operand(tensor)) free_tc(c);  // a new operand, and its memory
+  if (contraction_operand(tensor)) {  // a new operand, and its memory
+    TcGuard guard(c);
+    free_tc(c);
+  }
   const cudaMemcpyKind kind = src_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   const bool cplx = c->field == ATRIP_FIELD_COMPLEX;
   const size_t elem = sizeof(double) * (cplx ? 2 : 1);
   if (double **d = direct_slot(c, tensor)) {
-    ATRIP_CUDA_TRY(cudaMalloc(d, elem * std::max<int64_t>(n, 1)));
+    ATRIP_CUDA_TRY(device_alloc(d, elem * std::max<int64_t>(n, 1)));
     ATRIP_CUDA_TRY(cudaMemcpyAsync(*d, src, elem * n, kind, c->stream));
   } else if (!src_on_device && n > staging_elems()) {
     // Large host tensor: stream it through a bounded staging buffer, a run
@@ -199,7 +243,7 @@ int upload_impl(atrip_gpu_context *c, int32_t tensor, const double *src, int64_t
     PermutePlan p = plan_for(c, tensor);
     const double *hsrc = src;
     for (int i = 0; i < p.count; ++i)
-      ATRIP_CUDA_TRY(cudaMalloc(p.dst[i], elem * std::max<int64_t>(n, 1)));
+      ATRIP_CUDA_TRY(device_alloc(p.dst[i], elem * std::max<int64_t>(n, 1)));
     int dslow[2];
     int64_t m = 0, S = 0;
     for (int i = 0; i < p.count; ++i) {
@@ -212,7 +256,7 @@ int upload_impl(atrip_gpu_context *c, int32_t tensor, const double *src, int64_t
     }
     const int64_t cv = std::max<int64_t>(1, staging_elems() / S);
     double *staging = nullptr;
-    ATRIP_CUDA_TRY(cudaMalloc(&staging, elem * std::min<int64_t>(n, cv * S)));
+    ATRIP_CUDA_TRY(device_alloc(&staging, elem * std::min<int64_t>(n, cv * S)));
     int rc = ATRIP_OK;
     for (int64_t v0 = 0; v0 < m && rc == ATRIP_OK; v0 += cv) {
       const int64_t nv = std::min<int64_t>(cv, m - v0);
@@ -243,7 +287,7 @@ int upload_impl(atrip_gpu_context *c, int32_t tensor, const double *src, int64_t
     const double *colmajor = src;
     double *staging = nullptr;
     if (!src_on_device) {
-      ATRIP_CUDA_TRY(cudaMalloc(&staging, elem * std::max<int64_t>(n, 1)));
+      ATRIP_CUDA_TRY(device_alloc(&staging, elem * std::max<int64_t>(n, 1)));
       cudaError_t e = cudaMemcpyAsync(staging, src, elem * n, kind, c->stream);
       if (e != cudaSuccess) {
         cudaFree(staging);
@@ -252,7 +296,7 @@ int upload_impl(atrip_gpu_context *c, int32_t tensor, const double *src, int64_t
       colmajor = staging;
     }
     for (int i = 0; i < p.count; ++i) {
-      cudaError_t e = cudaMalloc(p.dst[i], elem * std::max<int64_t>(n, 1));
+      cudaError_t e = device_alloc(p.dst[i], elem * std::max<int64_t>(n, 1));
       if (e == cudaSuccess)
         e = launch_permute4(*p.dst[i], colmajor, p.n[i], p.s[i], c->stream, cplx);
       if (e != cudaSuccess) {
@@ -367,7 +411,7 @@ int atrip_gpu_create(const atrip_dims *dims, atrip_gpu_context **out) {
       for (uint32_t b = a; b < (uint32_t)c->Nv; ++b)
         for (uint32_t cc = b; cc < (uint32_t)c->Nv; ++cc)
           if (!(a == b && b == cc)) h.push_back(a | (b << 10) | (cc << 20));
-    CREATE_TRY(cudaMalloc(&c->d_tuples, sizeof(uint32_t) * std::max<size_t>(h.size(), 1)));
+    CREATE_TRY(device_alloc(&c->d_tuples, sizeof(uint32_t) * std::max<size_t>(h.size(), 1)));
     CREATE_TRY(cudaMemcpy(c->d_tuples, h.data(), sizeof(uint32_t) * h.size(),
                           cudaMemcpyHostToDevice));
     c->h_tuples.swap(h);
@@ -389,16 +433,20 @@ int atrip_gpu_create(const atrip_dims *dims, atrip_gpu_context **out) {
               for (uint32_t i = std::max(i0, j); i < std::min(i0 + bi, no); ++i)
                 h.push_back(i | (j << 8) | (k << 16));
     c->n_triples = (int)h.size();
-    CREATE_TRY(cudaMalloc(&c->d_triples, sizeof(uint32_t) * h.size()));
+    CREATE_TRY(device_alloc(&c->d_triples, sizeof(uint32_t) * h.size()));
     CREATE_TRY(cudaMemcpy(c->d_triples, h.data(), sizeof(uint32_t) * h.size(),
                           cudaMemcpyHostToDevice));
   }
-  CREATE_TRY(cudaMalloc(&c->d_e, sizeof(double) * std::max<int64_t>(c->n_tuples, 1)));
-  CREATE_TRY(cudaMalloc(&c->d_ect, sizeof(double) * std::max<int64_t>(c->n_tuples, 1)));
-  CREATE_TRY(cudaMalloc(&c->d_queue, sizeof(unsigned long long) * 4));
-  CREATE_TRY(cudaMalloc(&c->d_partials, sizeof(double) * 4 * kSumBlocks));
-  CREATE_TRY(cudaMalloc(&c->d_sum, sizeof(double) * 8));
+  CREATE_TRY(device_alloc(&c->d_e, sizeof(double) * std::max<int64_t>(c->n_tuples, 1)));
+  CREATE_TRY(device_alloc(&c->d_ect, sizeof(double) * std::max<int64_t>(c->n_tuples, 1)));
+  CREATE_TRY(device_alloc(&c->d_queue, sizeof(unsigned long long) * 4));
+  CREATE_TRY(device_alloc(&c->d_partials, sizeof(double) * 4 * kSumBlocks));
+  CREATE_TRY(device_alloc(&c->d_sum, sizeof(double) * 8));
 #undef CREATE_TRY
+  {
+    std::lock_guard<std::mutex> lock(g_contexts_mutex);
+    g_contexts.push_back(c);
+  }
   *out = c;
   return ATRIP_OK;
 }
@@ -420,6 +468,15 @@ int atrip_gpu_release(atrip_gpu_context *ctx, int32_t tensor) {
   return ATRIP_OK;
 }
 
+int atrip_gpu_trim(atrip_gpu_context *c) {
+  clear_error();
+  if (!c) return fail(ATRIP_ERR_ARGUMENT, "null context");
+  ATRIP_CUDA_TRY(cudaSetDevice(c->device));
+  TcGuard guard(c);
+  give_back(c);
+  return ATRIP_OK;
+}
+
 int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_result *out) {
   clear_error();
   if (!c || !opts || !out) return fail(ATRIP_ERR_ARGUMENT, "null argument");
@@ -434,6 +491,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
   if (opts->first_iteration < 0 || opts->max_iterations < 0)
     return fail(ATRIP_ERR_ARGUMENT, "negative iteration bound");
   ATRIP_CUDA_TRY(cudaSetDevice(c->device));
+  TcGuard guard(c);
   cudaStream_t st = opts->stream ? (cudaStream_t)opts->stream : c->stream;
   const bool use_j = opts->use_j && c->have[ATRIP_JIJKA] && c->have[ATRIP_JABCI];
   // tuple range: first_iteration .. max_iterations inclusive
@@ -520,7 +578,14 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
         cudaFree(c->d_workspace);
         c->d_workspace = nullptr;
         c->workspace_doubles = 0;
-        ATRIP_CUDA_TRY(cudaMalloc(&c->d_workspace, sizeof(double) * ws));
+        cudaError_t e = device_alloc(&c->d_workspace, sizeof(double) * ws);
+        if (e == cudaErrorMemoryAllocation && (c->tc.impl || c->tcb.planes)) {
+          // this context's own slices make room
+          cudaGetLastError();
+          give_back(c);
+          e = device_alloc(&c->d_workspace, sizeof(double) * ws);
+        }
+        ATRIP_CUDA_TRY(e);
         c->workspace_doubles = ws;
       }
       TriplesArgs a;
@@ -608,10 +673,11 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
                          c->d_e, c->d_ect, st, &launches);
       };
       int rc = run_split();
-      if (rc == ATRIP_ERR_OUT_OF_MEMORY && c->tc.impl) {  // the FP64 slices make room
+      if (rc == ATRIP_ERR_OUT_OF_MEMORY && (c->tc.impl || c->tcb.planes)) {
+        // the FP64 slices make room
         cudaGetLastError();
         clear_error();
-        free_tc(c);
+        give_back(c);
         rc = run_split();
       }
       if (rc != ATRIP_OK) return rc;
@@ -727,6 +793,10 @@ int atrip_gpu_last_sums(const atrip_gpu_context *c, double *sums) {
 
 int atrip_gpu_destroy(atrip_gpu_context *c) {
   if (!c) return ATRIP_OK;
+  {
+    std::lock_guard<std::mutex> lock(g_contexts_mutex);
+    g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), c), g_contexts.end());
+  }
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (int t = 0; t < ATRIP_N_TENSORS; ++t)

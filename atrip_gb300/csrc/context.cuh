@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <vector>
 
@@ -31,8 +32,12 @@ struct atrip_gpu_context {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   atrip_gb300::SplitState split;
-  atrip_gb300::TcState tc;  // FP64 form on the tensor cores
+  // FP64 form on the tensor cores.  Held (TcGuard) by whatever uses or frees it:
+  // a call on the context or on a batch of it, or another thread that needs the
+  // memory while the context is idle
+  atrip_gb300::TcState tc;
   atrip_gb300::TcBuffers tcb;
+  std::atomic<bool> tc_held{false};
   atrip_gb300::TcBuffers tcs;  // split forms on the same kernel
   atrip_tuning tune = {};
   // processing order of the last range (tuple_block > 1), see build_order
@@ -41,3 +46,25 @@ struct atrip_gpu_context {
   int64_t order_cap = 0, order_lo = -1, order_hi = -1;
   int order_block = 0;
 };
+
+namespace atrip_gb300 {
+
+class TcGuard {
+ public:
+  explicit TcGuard(atrip_gpu_context *c);
+  ~TcGuard() { c_->tc_held.store(false, std::memory_order_release); }
+  TcGuard(const TcGuard &) = delete;
+  TcGuard &operator=(const TcGuard &) = delete;
+
+ private:
+  atrip_gpu_context *c_;
+};
+
+// The FP64 slices are a copy the engine can do without.  free_tc drops them,
+// their buffers and what is known of the operands; give_back keeps the verdict
+// where the operands were found not to allow the form.  The caller holds the
+// context's TcGuard.
+void free_tc(atrip_gpu_context *c);
+void give_back(atrip_gpu_context *c);
+
+}  // namespace atrip_gb300

@@ -24,6 +24,14 @@ void clear_error();
     }                                                                             \
   } while (0)
 
+// cudaMalloc on the current device.  Where it has no room, contexts that are not
+// in a call give back their FP64 slices (see triples_fp64_tc.cu) first.
+cudaError_t device_alloc(void **p, size_t bytes);
+template <class T>
+cudaError_t device_alloc(T **p, size_t bytes) {
+  return device_alloc(reinterpret_cast<void **>(p), bytes);
+}
+
 // Kernel-friendly HBM layouts of the inputs (element counts in comments).
 //   Ta [x][q][p][E]  = Tabij[x,E,p,q]   rows (p,q) of T_x, E contiguous  Nv*No*No*Nv
 //   Tp [x][y][n][m]  = Tabij[x,y,m,n]   No x No pair blocks              Nv*Nv*No*No

@@ -1327,7 +1327,7 @@ int prepare(SplitImpl *p, const DeviceTensors &dt, int No, int Nv, int S, int bi
   p->Ep = (Nv + kKChunk - 1) / kKChunk * kKChunk;
   const int64_t No2 = (int64_t)No * No, Ep = p->Ep;
   unsigned long long *d_tmp = nullptr;
-  ATRIP_CUDA_TRY(cudaMalloc(&d_tmp, 2 * sizeof(unsigned long long)));
+  ATRIP_CUDA_TRY(device_alloc(&d_tmp, 2 * sizeof(unsigned long long)));
   double mT = 0, mVp = 0, mVh = 0;
   int rc = absmax(dt.Ta, (int64_t)Nv * No2 * Nv, d_tmp, st, &mT, &p->finite);
   if (rc == ATRIP_OK)
@@ -1345,14 +1345,14 @@ int prepare(SplitImpl *p, const DeviceTensors &dt, int No, int Nv, int S, int bi
 
   const size_t nTa = (size_t)S * Nv * No2 * Ep, nVh = (size_t)S * Nv * No2 * kHoleK,
                nVp = (size_t)S * Nv * Nv * No * Ep, nTp = (size_t)S * Nv * Nv * No * kHoleK;
-  ATRIP_CUDA_TRY(cudaMalloc(&p->TaS, 2 * nTa));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->TaST, 2 * nTa));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->VhS, 2 * nVh));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->VhST, 2 * nVh));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->VpS, 2 * nVp));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->TpS, 2 * nTp));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->TpTS, 2 * nTp));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->d_status, sizeof(int)));
+  ATRIP_CUDA_TRY(device_alloc(&p->TaS, 2 * nTa));
+  ATRIP_CUDA_TRY(device_alloc(&p->TaST, 2 * nTa));
+  ATRIP_CUDA_TRY(device_alloc(&p->VhS, 2 * nVh));
+  ATRIP_CUDA_TRY(device_alloc(&p->VhST, 2 * nVh));
+  ATRIP_CUDA_TRY(device_alloc(&p->VpS, 2 * nVp));
+  ATRIP_CUDA_TRY(device_alloc(&p->TpS, 2 * nTp));
+  ATRIP_CUDA_TRY(device_alloc(&p->TpTS, 2 * nTp));
+  ATRIP_CUDA_TRY(device_alloc(&p->d_status, sizeof(int)));
 
   // rows (o, r1, r2) and source strides of each slice tensor
   SliceJob j;
@@ -1467,7 +1467,7 @@ int prepare_j(SplitImpl *p, const DeviceTensors &dt, cudaStream_t st, int64_t *l
   const int No = p->No, Nv = p->Nv, S = p->S;
   const int64_t No2 = (int64_t)No * No, Ep = p->Ep;
   unsigned long long *d_tmp = nullptr;
-  ATRIP_CUDA_TRY(cudaMalloc(&d_tmp, 2 * sizeof(unsigned long long)));
+  ATRIP_CUDA_TRY(device_alloc(&d_tmp, 2 * sizeof(unsigned long long)));
   double mJp = 0, mJh = 0;
   int rc = absmax(dt.Jpt, (int64_t)Nv * Nv * No * Nv, d_tmp, st, &mJp, &p->finite_j);
   if (rc == ATRIP_OK) rc = absmax(dt.Jht, (int64_t)Nv * No2 * No, d_tmp, st, &mJh, &p->finite_j);
@@ -1478,9 +1478,9 @@ int prepare_j(SplitImpl *p, const DeviceTensors &dt, cudaStream_t st, int64_t *l
   p->unit_j = std::ldexp(1.0, p->eT + eJ - 2 * (p->bits - 1));
   const double sJ = std::ldexp(1.0, p->bits - 1 - eJ);
   const size_t nVh = (size_t)S * Nv * No2 * kHoleK, nVp = (size_t)S * Nv * Nv * No * Ep;
-  ATRIP_CUDA_TRY(cudaMalloc(&p->JhS, 2 * nVh));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->JhST, 2 * nVh));
-  ATRIP_CUDA_TRY(cudaMalloc(&p->JpS, 2 * nVp));
+  ATRIP_CUDA_TRY(device_alloc(&p->JhS, 2 * nVh));
+  ATRIP_CUDA_TRY(device_alloc(&p->JhST, 2 * nVh));
+  ATRIP_CUDA_TRY(device_alloc(&p->JpS, 2 * nVp));
   SliceJob j;
   j.S = S;
   j.bits = p->bits;
@@ -1774,19 +1774,19 @@ int split_multi_prepare(const SplitMultiSystem *sys, int n, int slices, bool f16
     b.h_prefix = b.d_prefix = nullptr;
     b.cap = 0;
     ATRIP_CUDA_TRY(cudaMallocHost(&b.h_desc, sizeof(SysDesc) * n));
-    ATRIP_CUDA_TRY(cudaMalloc(&b.d_desc, sizeof(SysDesc) * n));
+    ATRIP_CUDA_TRY(device_alloc(&b.d_desc, sizeof(SysDesc) * n));
     ATRIP_CUDA_TRY(cudaMallocHost(&b.h_prefix, sizeof(int64_t) * (n + 1)));
-    ATRIP_CUDA_TRY(cudaMalloc(&b.d_prefix, sizeof(int64_t) * (n + 1)));
+    ATRIP_CUDA_TRY(device_alloc(&b.d_prefix, sizeof(int64_t) * (n + 1)));
     b.cap = n;
   }
-  if (!b.d_status) ATRIP_CUDA_TRY(cudaMalloc(&b.d_status, sizeof(int)));
-  if (!b.d_queue) ATRIP_CUDA_TRY(cudaMalloc(&b.d_queue, sizeof(unsigned long long)));
+  if (!b.d_status) ATRIP_CUDA_TRY(device_alloc(&b.d_status, sizeof(int)));
+  if (!b.d_queue) ATRIP_CUDA_TRY(device_alloc(&b.d_queue, sizeof(unsigned long long)));
   const size_t need = (size_t)sm_count * 2 * npass * 3 * 2 * L3;  // floats
   if (need > b.wglobal_floats) {
     cudaFree(b.wglobal);
     b.wglobal = nullptr;
     b.wglobal_floats = 0;
-    ATRIP_CUDA_TRY(cudaMalloc(&b.wglobal, sizeof(float) * need));
+    ATRIP_CUDA_TRY(device_alloc(&b.wglobal, sizeof(float) * need));
     b.wglobal_floats = need;
   }
   SysDesc *h = static_cast<SysDesc *>(b.h_desc);
@@ -1915,9 +1915,11 @@ int split_prepare(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
     s.impl = p;
     int rc = prepare(p, dt, No, Nv, slices, bits, st, launches);
     if (rc == ATRIP_OK && n_triples > 0) {
-      if (cudaMalloc(&p->tri_ef, sizeof(double2) * n_triples) != cudaSuccess) {
+      const cudaError_t e = device_alloc(&p->tri_ef, sizeof(double2) * n_triples);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
         set_error("split form: allocating the triple table failed");
-        rc = ATRIP_ERR_CUDA;
+        rc = e == cudaErrorMemoryAllocation ? ATRIP_ERR_OUT_OF_MEMORY : ATRIP_ERR_CUDA;
       } else {
         triple_table_kernel<<<(n_triples + 255) / 256, 256, 0, st>>>(triples, n_triples,
                                                                      dt.epsi, p->tri_ef);
@@ -1946,7 +1948,7 @@ int split_prepare(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
     cudaFree(p->wglobal);
     p->wglobal = nullptr;
     p->wglobal_floats = 0;  // a smaller run after a failed allocation must not find the old size
-    ATRIP_CUDA_TRY(cudaMalloc(&p->wglobal, sizeof(float) * need));
+    ATRIP_CUDA_TRY(device_alloc(&p->wglobal, sizeof(float) * need));
     p->wglobal_floats = need;
   }
   return ATRIP_OK;
@@ -1981,7 +1983,7 @@ int split_enqueue(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
   a.prof = nullptr;
   if (s.profile) {
     if (!p->d_prof)
-      ATRIP_CUDA_TRY(cudaMalloc(&p->d_prof, sizeof(unsigned long long) * kProfSlots));
+      ATRIP_CUDA_TRY(device_alloc(&p->d_prof, sizeof(unsigned long long) * kProfSlots));
     ATRIP_CUDA_TRY(cudaMemsetAsync(p->d_prof, 0, sizeof(unsigned long long) * kProfSlots, st));
     a.prof = p->d_prof;
   }

@@ -1210,7 +1210,9 @@ cudaError_t cut(CutJob j, cudaStream_t st) {
 size_t up(size_t x) { return (x + 1023) / 1024 * 1024; }
 
 // The slices may take at most half of the memory that is free: the rest is
-// the host program's.  false (no error) when they do not fit.
+// the host program's.  false (no error) when they do not fit.  They are given
+// back where the engine finds no memory for anything else (device_alloc), by
+// atrip_gpu_trim and when an operand is uploaded anew.
 bool alloc_arena(char **p, size_t bytes) {
   size_t fr = 0, tot = 0;
   if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || bytes > fr / 2 ||
@@ -1345,7 +1347,7 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cpl
                nTp = up((size_t)2 * kS * Nv * Nv * No * nblk * p->Kh);
   if (!alloc_arena(&p->arena, 2 * nc * (nTa + nVh) + nVp + 2 * nTp)) return ATRIP_OK;
   ScopedDevice tmp;
-  ATRIP_CUDA_TRY(cudaMalloc(&tmp.p, sizeof(DeviceStats)));
+  ATRIP_CUDA_TRY(device_alloc(&tmp.p, sizeof(DeviceStats)));
   auto *ds = static_cast<DeviceStats *>(tmp.p);
   DeviceStats h;
   int rc = examine(p->nc, dt.Ta, dt.Vht, dt.Vpt, No_, Nv_, p->arena, ds, &h, st, launches);
@@ -1414,7 +1416,7 @@ int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *lau
                nVp = up((size_t)2 * kS * Nv * Nv * No * nblk * p->Kp);
   if (!alloc_arena(&p->arena_j, 2 * nc * nVh + nVp)) return ATRIP_OK;
   ScopedDevice tmp;
-  ATRIP_CUDA_TRY(cudaMalloc(&tmp.p, sizeof(DeviceStats)));
+  ATRIP_CUDA_TRY(device_alloc(&tmp.p, sizeof(DeviceStats)));
   auto *ds = static_cast<DeviceStats *>(tmp.p);
   DeviceStats h;
   int e_t;
@@ -1576,14 +1578,14 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     b.h_flags = b.d_flags = nullptr;
     b.cap = 0;
     ATRIP_CUDA_TRY(cudaMallocHost(&b.h_desc, sizeof(TcDesc) * n));
-    ATRIP_CUDA_TRY(cudaMalloc(&b.d_desc, sizeof(TcDesc) * n));
+    ATRIP_CUDA_TRY(device_alloc(&b.d_desc, sizeof(TcDesc) * n));
     ATRIP_CUDA_TRY(cudaMallocHost(&b.h_prefix, sizeof(int64_t) * (n + 1)));
-    ATRIP_CUDA_TRY(cudaMalloc(&b.d_prefix, sizeof(int64_t) * (n + 1)));
+    ATRIP_CUDA_TRY(device_alloc(&b.d_prefix, sizeof(int64_t) * (n + 1)));
     ATRIP_CUDA_TRY(cudaMallocHost(&b.h_flags, sizeof(int) * (n + 1)));
-    ATRIP_CUDA_TRY(cudaMalloc(&b.d_flags, sizeof(int) * (n + 1)));
+    ATRIP_CUDA_TRY(device_alloc(&b.d_flags, sizeof(int) * (n + 1)));
     b.cap = n;
   }
-  if (!b.d_queue) ATRIP_CUDA_TRY(cudaMalloc(&b.d_queue, sizeof(unsigned long long)));
+  if (!b.d_queue) ATRIP_CUDA_TRY(device_alloc(&b.d_queue, sizeof(unsigned long long)));
   auto *h = static_cast<TcDesc *>(b.h_desc);
   int P = 0, spp = 1, window = 0;
   const auto *p0 = static_cast<const TcImpl *>(n > 0 ? sys[0].state->impl : nullptr);
@@ -1671,7 +1673,7 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
     cudaFree(b.planes);
     b.planes = nullptr;
     b.planes_bytes = 0;
-    ATRIP_CUDA_TRY(cudaMalloc(&b.planes, need));
+    ATRIP_CUDA_TRY(device_alloc(&b.planes, need));
     b.planes_bytes = need;
   }
   return ATRIP_OK;

@@ -148,6 +148,15 @@ int atrip_gpu_upload_device(atrip_gpu_context *ctx, int32_t tensor,
  * src/atrip/Atrip.cxx:310, frees the caller's V_pphp after slicing). */
 int atrip_gpu_release(atrip_gpu_context *ctx, int32_t tensor);
 
+/* Give back the device memory that the engine keeps to be fast and can do
+ * without: the FP64 form's digit slices, copies of the operands that may take
+ * up to half of the memory free at the first run (for V_pphp of m bytes and
+ * real orbitals about 2 m, and as much again for (cT)), and their W buffers.
+ * They are made again by the next FP64 run.  The engine does this by itself
+ * where it finds no memory on the device for any other buffer, for all
+ * contexts of the process that are not in a call.                           */
+int atrip_gpu_trim(atrip_gpu_context *ctx);
+
 /* Run the triples loop over the tuple range selected by opts and reduce the
  * energies.  Replaces the per-tuple loop and the final reduction of
  * Atrip::run (src/atrip/Atrip.cxx:686-1111): doubles_contribution,

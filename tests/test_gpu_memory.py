@@ -48,3 +48,66 @@ def test_split_run_after_a_failed_one():
             again = ctx.run(form="split_f16", use_j=False)
         assert again.energy == ref.energy
         assert ctx.run(form="split_f16", use_j=True).energy == ref.energy
+
+
+def _run64(ctx, n=200):
+    ctx.run(form="fp64", use_j=False, max_iterations=n - 1)
+    return ctx.tuple_energies(0, n)[0]
+
+
+def _close(x, y, K):
+    assert np.max(np.abs(x - y)) <= K * 2.0 ** -52 * np.max(np.abs(y))
+
+
+# the slices of No=16/Nv=160 take about 2.5 GB; a second context of No=16/Nv=120
+# needs 0.5 GB while V_pphp is uploaded
+def test_another_context_takes_the_slices_memory():
+    d, d2 = synth.make_inputs(16, 160, 32), synth.make_inputs(16, 120, 33)
+    with _ctx(d) as ctx:
+        e = _run64(ctx)
+        with full_device(300 * MB):
+            with _ctx(d2) as other:
+                f = _run64(other)
+            _close(_run64(ctx), e, 2 * 176)  # by whatever kernel there is memory for
+        with _ctx(d2) as other:
+            _close(f, _run64(other), 2 * 136)
+
+
+# the DFMA kernel's workspace (155 MB or more at No=40) beside the slices
+def test_tuned_run_takes_the_slices_memory():
+    d = synth.make_inputs(40, 60, 34)
+    with _ctx(d) as ctx:
+        e = _run64(ctx)
+        with full_device(50 * MB):
+            ctx.set_tuning(fp64_tile_rows=64)
+            _close(_run64(ctx), e, 2 * 100)
+
+
+# FP16 slices of four systems (0.7 GB) beside their FP64 slices (2.5 GB)
+def test_split_batch_takes_the_slices_memory():
+    ds = [synth.make_inputs(16, 100 + k, 35 + k) for k in range(4)]
+    opt = dict(use_j=False, max_iterations=499)
+    out = []
+    for leave in (100 * MB, 1 << 50):
+        ctxs = [_ctx(d) for d in ds]
+        with capi.Batch(ctxs) as b:
+            e = b.run(form="fp64", **opt)
+            with full_device(leave):
+                out.append([r.energy for r in b.run(form="split_f16", **opt)])
+            assert [r.energy for r in b.run(form="fp64", **opt)] == [r.energy for r in e]
+        for c in ctxs:
+            c.close()
+    assert out[0] == out[1]
+
+
+def test_trim_gives_the_slices_back():
+    d = synth.make_inputs(16, 160, 32)
+    with _ctx(d) as ctx:
+        e = _run64(ctx)
+        before = torch.cuda.mem_get_info()[0]
+        ctx.trim()
+        # V_pphp of 524 MB: slices of twice that and more
+        assert torch.cuda.mem_get_info()[0] - before > 1000 * MB
+        np.testing.assert_array_equal(_run64(ctx), e)
+        ctx.trim()
+        ctx.trim()
