@@ -1229,6 +1229,13 @@ struct SplitImpl {
   SplitMaps maps;
 };
 
+void free_j(SplitImpl *p) {
+  cudaFree(p->JhS);
+  cudaFree(p->JhST);
+  cudaFree(p->JpS);
+  p->JhS = p->JhST = p->JpS = nullptr;
+}
+
 void free_impl(SplitImpl *p) {
   if (!p) return;
   cudaFree(p->TaS);
@@ -1238,9 +1245,7 @@ void free_impl(SplitImpl *p) {
   cudaFree(p->VpS);
   cudaFree(p->TpS);
   cudaFree(p->TpTS);
-  cudaFree(p->JhS);
-  cudaFree(p->JhST);
-  cudaFree(p->JpS);
+  free_j(p);
   cudaFree(p->wglobal);
   cudaFree(p->d_status);
   cudaFree(p->tri_ef);
@@ -1939,7 +1944,10 @@ int split_prepare(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
   if (use_j && !p->has_j) {
     s.generation++;
     const int rc = prepare_j(p, dt, st, launches);
-    if (rc != ATRIP_OK) return rc;
+    if (rc != ATRIP_OK) {  // cut again by the next call
+      free_j(p);
+      return rc;
+    }
   }
   // W buffers (one double per element): two tuple parities x passes per CTA
   const size_t need = (size_t)sm_count * 2 * (use_j ? 2 : 1) * 3 * 2 * No * No * No;  // floats

@@ -111,3 +111,22 @@ def test_trim_gives_the_slices_back():
         np.testing.assert_array_equal(_run64(ctx), e)
         ctx.trim()
         ctx.trim()
+
+
+# (cT) slices that fit only in part are not kept: No=16/Nv=100, J_pphp in two
+# FP16 slices 131 MB after J_hhhp's
+def test_failed_ct_slices_leave_nothing_behind():
+    d = synth.make_inputs(16, 100, 36, with_j=True)
+    kw = dict(form="split_f16", max_iterations=99)
+    with _ctx(d, True) as ctx:
+        ctx.run(use_j=False, **kw)
+        with full_device(96 * MB):
+            free = []
+            for _ in range(4):
+                with pytest.raises(capi.AtripError) as err:
+                    ctx.run(use_j=True, **kw)
+                assert err.value.status == capi.ERR_OUT_OF_MEMORY
+                free.append(torch.cuda.mem_get_info()[0])
+        assert free[-1] == free[0]
+        ref = ctx.run(use_j=True, **kw)
+        assert np.isfinite(ref.ct_energy)
