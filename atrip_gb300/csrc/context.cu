@@ -13,6 +13,7 @@
 #include "engine.cuh"
 #include "split.cuh"
 #include "context.cuh"
+#include "tuple_order.cuh"
 
 namespace atrip_gb300 {
 
@@ -73,27 +74,16 @@ int fail(int code, const std::string &msg) {
   return code;
 }
 
-// Processing order of tuples [t_begin, t_end) for block side L >= 2: a
-// stable counting sort of the list positions by the block triple
-// (a/L, b/L, c/L), so that the tuples the persistent CTAs hold at any
-// moment read the slabs of few a, b, c values and find them in L2 (in list
-// order ~150 tuples in flight touch ~150 different c slabs).  Within a block
-// triple the list order is kept.  Writes order[q] = position - t_begin.
+// Processing order of tuples [t_begin, t_end) for block side L >= 2, so that
+// the tuples the persistent CTAs hold at any moment read the slabs of few a, b,
+// c values and find them in L2 (in list order ~150 tuples in flight touch ~150
+// different c slabs).  d_order[q] = position - t_begin.
 int build_order(atrip_gpu_context *c, int64_t t_begin, int64_t t_end, int L, cudaStream_t st) {
   if (c->order_lo == t_begin && c->order_hi == t_end && c->order_block == L && c->d_order)
     return ATRIP_OK;
   const int64_t n = t_end - t_begin;
-  while (((int64_t)c->Nv + L - 1) / L > 400) ++L;  // at most 400^3 block triples
-  const int64_t nb = (c->Nv + L - 1) / L;
-  std::vector<uint32_t> count((size_t)(nb * nb * nb) + 1, 0), out((size_t)n);
-  auto key = [&](uint32_t pk) {
-    const int64_t a = pk & 0x3ff, b = (pk >> 10) & 0x3ff, cc = (pk >> 20) & 0x3ff;
-    return (size_t)(((a / L) * nb + b / L) * nb + cc / L);
-  };
-  for (int64_t t = t_begin; t < t_end; ++t) count[key(c->h_tuples[(size_t)t]) + 1]++;
-  for (size_t k = 1; k < count.size(); ++k) count[k] += count[k - 1];
-  for (int64_t t = t_begin; t < t_end; ++t)
-    out[count[key(c->h_tuples[(size_t)t])]++] = (uint32_t)(t - t_begin);
+  std::vector<uint32_t> out((size_t)n);
+  block_order(c->h_tuples.data() + t_begin, n, c->Nv, L, out.data());
   if (n > c->order_cap) {
     cudaFree(c->d_order);
     c->d_order = nullptr;
@@ -107,6 +97,17 @@ int build_order(atrip_gpu_context *c, int64_t t_begin, int64_t t_end, int L, cud
   c->order_lo = t_begin;
   c->order_hi = t_end;
   c->order_block = L;
+  return ATRIP_OK;
+}
+
+// The engine's own choice of an order, list order where there is no memory for it.
+int choose_order(atrip_gpu_context *c, int64_t t_begin, int64_t t_end, int L, cudaStream_t st,
+                 const uint32_t **order) {
+  if (L == 0) return ATRIP_OK;
+  const int rc = build_order(c, t_begin, t_end, L, st);
+  if (rc == ATRIP_OK) *order = c->d_order;
+  if (rc != ATRIP_ERR_OUT_OF_MEMORY) return rc;
+  clear_error();
   return ATRIP_OK;
 }
 
@@ -527,12 +528,9 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
     if (rc != ATRIP_OK) return rc;
   }
   if (tc && c->tune.tuple_block == 0) {
-    const int block = tc_tuple_block(c->No, c->Nv, kTcFp64Slices, c->sm_count);
-    if (block > 0) {
-      const int rc = build_order(c, t_begin, t_end, block, st);
-      if (rc != ATRIP_OK) return rc;
-      order = c->d_order;
-    }
+    const int rc = choose_order(c, t_begin, t_end, tc_tuple_block(c->No, c->Nv, kTcFp64Slices,
+                                                                  c->sm_count), st, &order);
+    if (rc != ATRIP_OK) return rc;
   }
   if (tc) {
     const TcSystem ts = {&c->tc, &c->dt, c->No, c->Nv, c->n_triples, c->d_tuples, c->d_triples,
@@ -643,12 +641,9 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
           plain && !transposed && split_tc_eligible(slices, c->split.f16, c->No, c->Nv);
       if (plain && transposed) c->split.variant = 2;
       if ((on_tc || (plain && transposed)) && tn.tuple_block == 0) {
-        const int block = tc_tuple_block(c->No, c->Nv, slices, c->sm_count);
-        if (block > 0) {
-          const int rc = build_order(c, t_begin, t_end, block, st);
-          if (rc != ATRIP_OK) return rc;
-          order = c->d_order;
-        }
+        const int rc = choose_order(c, t_begin, t_end, tc_tuple_block(c->No, c->Nv, slices,
+                                                                      c->sm_count), st, &order);
+        if (rc != ATRIP_OK) return rc;
       }
       const double tai_sign = opts->ijkabc ? -1.0 : 1.0;
       auto run_split = [&]() -> int {
