@@ -25,7 +25,8 @@ window sums).  Scaling every input by 2^k leaves the split form's digits
 unchanged and multiplies every energy and its error by 2^(4k), so the
 twin's error is the estimate times the same factor as its energy.
 
-Choices are cached in a JSON file keyed by device name, No, Nv and form.
+Choices are cached in a JSON file keyed by device name, the generation of the
+engine's kernels, No, Nv and form.
 The reference has no tuner: its only knob for this loop is the tuple
 distribution (src/atrip/Tuples.hpp:49-52).
 """
@@ -123,8 +124,15 @@ def _save_cache(c: dict) -> None:
     os.replace(tmp, CACHE)
 
 
+# Which kernels a tuning's fields select.  A cached choice is good only for the
+# engine it was timed on: raised whenever a field comes to select another kernel
+# (2: fp64_* and tuples_per_claim select the FP64-instruction kernel, an empty
+# tuning and split_variant 0 the engine's choice).
+KERNELS = 2
+
+
 def _key(ctx: capi.Context, form: str) -> str:
-    return f"{_device_name(ctx.device)}|No={ctx.No}|Nv={ctx.Nv}|{form}"
+    return f"{_device_name(ctx.device)}|kernels={KERNELS}|No={ctx.No}|Nv={ctx.Nv}|{form}"
 
 
 def _time(ctx, wins, form, slices, tuning, reps=3):
