@@ -100,6 +100,12 @@ int build_order(atrip_gpu_context *c, int64_t t_begin, int64_t t_end, int L, cud
   return ATRIP_OK;
 }
 
+// The tensor-core kernel's test of a wait that runs out: its limit, 0 = off.
+long long test_wait(const atrip_tuning &t) {
+  if (t.split_test_unpublished == 0) return 0;
+  return t.split_wait_kcycles > 0 ? (long long)t.split_wait_kcycles * 1000 : 4000000000ll;
+}
+
 // The engine's own choice of an order, list order where there is no memory for it.
 int choose_order(atrip_gpu_context *c, int64_t t_begin, int64_t t_end, int L, cudaStream_t st,
                  const uint32_t **order) {
@@ -547,6 +553,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
     }
   }
   if (tc) {
+    c->tcb.unpublished = test_wait(c->tune);
     int rc = tc_launch_enqueue(c->tcb, order, st, &launches);
     if (rc != ATRIP_OK) return rc;
     ATRIP_CUDA_TRY(launch_energy_sum(c->d_e + t_begin, c->d_ect + t_begin, n, c->d_partials,
@@ -630,17 +637,18 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
       c->split.f16 = form == ATRIP_FORM_SPLIT_F16;
       const int ctas = c->tune.split_ctas > 0 ? std::min(c->sm_count, (int)c->tune.split_ctas)
                                               : c->sm_count;
-      // the engine's choice of kernel unless a variant (or a diagnostic that
-      // only the split kernels have) is set; the other launch parameters change
-      // a kernel's schedule, not the kernel
+      // the engine's choice of kernel unless a variant (or a wait limit, which the
+      // split kernels have, or the role profile, which the transposed one has) is
+      // set; the other launch parameters change a kernel's schedule, not the kernel
       const atrip_tuning &tn = c->tune;
-      const bool transposed = split_prefers_transposed(slices, c->split.f16, c->No, c->Nv);
-      const bool plain = tn.split_variant == 0 && tn.split_wait_kcycles == 0 &&
-                         tn.split_test_unpublished == 0 && tn.split_profile == 0;
-      const bool on_tc =
-          plain && !transposed && split_tc_eligible(slices, c->split.f16, c->No, c->Nv);
-      if (plain && transposed) c->split.variant = 2;
-      if ((on_tc || (plain && transposed)) && tn.tuple_block == 0) {
+      const bool engine = tn.split_variant == 0 &&
+                          (tn.split_wait_kcycles == 0 || tn.split_test_unpublished != 0);
+      const bool transposed =
+          engine && split_prefers_transposed(slices, c->split.f16, c->No, c->Nv);
+      const bool on_tc = engine && !transposed && tn.split_profile == 0 &&
+                         split_tc_eligible(slices, c->split.f16, c->No, c->Nv);
+      if (transposed && tn.split_profile == 0) c->split.variant = 2;
+      if ((on_tc || (transposed && tn.split_profile == 0)) && tn.tuple_block == 0) {
         const int rc = choose_order(c, t_begin, t_end, tc_tuple_block(c->No, c->Nv, slices,
                                                                       c->sm_count), st, &order);
         if (rc != ATRIP_OK) return rc;
@@ -661,6 +669,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
           if ((rc = split_tc_attach(c->split, use_j, &ts.tri_ef)) != ATRIP_OK) return rc;
           if ((rc = tc_launch_prepare(&ts, 1, tai_sign, ctas, c->tcs, tn.split_stages)) != ATRIP_OK)
             return rc;
+          c->tcs.unpublished = test_wait(tn);
           return tc_launch_enqueue(c->tcs, order, st, &launches);
         }
         return split_run(c->split, c->dt, c->No, c->Nv, ctas, c->d_tuples, c->d_triples,

@@ -73,6 +73,8 @@ struct TcBuffers {
       bslot = 0, grid = 0;
   size_t smem = 0;
   int64_t total = 0;
+  // set by the owner: test of a wait that runs out, after so many SM cycles (0: off)
+  long long unpublished = 0;
 };
 void tc_buffers_free(TcBuffers &b);
 

@@ -132,6 +132,10 @@ struct TcArgs {
   void *planes;       // [CTA][parity][pass][group][cell]
   double *wd;         // [CTA][pass][cell]
   int lay_cells, lay_pass, nslots, nbslots, aslot, bslot;
+  // test of a wait that runs out: no tuple is published, and the producer waits
+  // for one this many SM cycles (0: off).  A limit that every wait takes from
+  // here costs the issuer 1 %
+  long long unpublished;
 };
 
 __device__ __forceinline__ void bar_sync(int id, int n) {
@@ -509,6 +513,8 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
     for (int s = 0; s < kTupleSlots; ++s) {
       mbar_init(&tfull[s], 1);
       mbar_init(&tempty[s], 3);
+      tslot[s].t = -1;  // read, not used, where a wait for a tuple runs out
+      tslot[s].s = 0;
     }
     mbar_init(drain, 1);
     fence_mbar_init();
@@ -551,7 +557,9 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
     int64_t q0 = 0, pos = 0;
     int have = 0, next = 0;
     uint32_t packed = 0;
-    for (uint32_t k = 0;; ++k) {
+    // its status ends the other roles' first waits
+    if (g.unpublished != 0) mbar_wait_warp(&tfull[0], 0, status, kErrFull, g.unpublished);
+    for (uint32_t k = 0; g.unpublished == 0; ++k) {
       const int ts = k % kTupleSlots;
       const uint32_t tuse = k / kTupleSlots;
       if (tuse > 0 && !mbar_wait_warp(&tempty[ts], (tuse - 1) & 1, status, kErrEmpty))
@@ -1707,6 +1715,7 @@ int tc_launch_enqueue(const TcBuffers &b, const uint32_t *order, cudaStream_t st
   a.nbslots = b.nbslots;
   a.aslot = b.aslot;
   a.bslot = b.bslot;
+  a.unpublished = b.unpublished;
   auto kern = b.nc == 2 ? (b.pieces == 2 ? triples_tc_kernel<FmtZ<2>> : triples_tc_kernel<FmtZ<1>>)
                         : b.pieces == 2 ? triples_tc_kernel<FmtFp64<2>>
                                         : triples_tc_kernel<FmtFp64<1>>;
@@ -1729,7 +1738,7 @@ int tc_launch_check(const TcBuffers &b, TcState *const *states, bool *rerun) {
   *rerun = false;
   if (b.total == 0) return ATRIP_OK;
   if (b.h_flags[0] != 0) {
-    set_error("tensor-core FP64 kernel: a bounded wait gave up (code " +
+    set_error("tensor-core kernel: a bounded wait gave up (code " +
               std::to_string(b.h_flags[0]) + ")");
     return ATRIP_ERR_TIMEOUT;
   }
