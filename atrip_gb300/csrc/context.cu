@@ -648,7 +648,7 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
       const bool on_tc = engine && !transposed && tn.split_profile == 0 &&
                          split_tc_eligible(slices, c->split.f16, c->No, c->Nv);
       if (transposed && tn.split_profile == 0) c->split.variant = 2;
-      if ((on_tc || (transposed && tn.split_profile == 0)) && tn.tuple_block == 0) {
+      if ((on_tc || transposed) && tn.tuple_block == 0) {
         const int rc = choose_order(c, t_begin, t_end, tc_tuple_block(c->No, c->Nv, slices,
                                                                       c->sm_count), st, &order);
         if (rc != ATRIP_OK) return rc;
