@@ -29,8 +29,12 @@ EXPORTED = [
     "atrip_gpu_run_fp64_noalloc", "atrip_gpu_batch_create", "atrip_gpu_batch_run",
     "atrip_gpu_batch_destroy", "atrip_gpu_batch_plan", "atrip_gpu_set_tuning",
     "atrip_gpu_get_tuning", "atrip_gpu_batch_set_tuning", "atrip_gpu_last_sums",
-    "atrip_gpu_device_count", "atrip_gpu_split_profile",
+    "atrip_gpu_device_count", "atrip_gpu_split_profile", "atrip_gpu_trim",
+    "atrip_gpu_last_kernel",
 ]
+
+# enum atrip_kernel
+KERNELS = (None, "fp64_instructions", "tensor_core", "split")
 
 # counters of atrip_gpu_split_profile, by index
 SPLIT_PROFILE = ("producer_total", "producer_wait_stage", "producer_wait_tuple_slot",
@@ -113,6 +117,7 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
     lib.atrip_gpu_upload_device.argtypes = [P, ctypes.c_int32, P, ctypes.c_int64]
     lib.atrip_gpu_release.argtypes = [P, ctypes.c_int32]
     lib.atrip_gpu_trim.argtypes = [P]
+    lib.atrip_gpu_last_kernel.argtypes = [P, ctypes.POINTER(ctypes.c_int32)]
     lib.atrip_gpu_run.argtypes = [P, ctypes.POINTER(RunOptions), ctypes.POINTER(Result)]
     lib.atrip_gpu_tuple_energies.argtypes = [P, ctypes.c_int64, ctypes.c_int64, P, P]
     lib.atrip_gpu_n_tuples.argtypes = [ctypes.c_int32]
@@ -234,6 +239,12 @@ class Context:
         out = (ctypes.c_double * 4)()
         check(self.lib.atrip_gpu_last_sums(self.h, out))
         return tuple(out)
+
+    def last_kernel(self):
+        """Kernel of the last run, one of KERNELS (None: no run yet)."""
+        k = ctypes.c_int32()
+        check(self.lib.atrip_gpu_last_kernel(self.h, ctypes.byref(k)))
+        return KERNELS[k.value]
 
     def split_profile(self) -> dict:
         """Role profile of the last split run made with tuning

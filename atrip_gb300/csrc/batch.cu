@@ -529,6 +529,15 @@ int run_batch(atrip_gpu_batch *b, const atrip_run_options *opts, atrip_result *r
     const TriplesArgs &a = b->h_table[k];
     c->e_lo = a.t_begin;
     c->e_hi = a.t_end;
+    const bool on_tc =
+        form != ATRIP_FORM_FP64 ? b->tcs_used
+                                : std::any_of(tc.begin(), tc.end(), [&](const TcSystem &m) {
+                                    return m.state == &c->tc;
+                                  });
+    c->last_kernel = a.t_begin == a.t_end      ? ATRIP_KERNEL_NONE
+                     : on_tc                   ? ATRIP_KERNEL_TENSOR_CORE
+                     : form == ATRIP_FORM_FP64 ? ATRIP_KERNEL_FP64_INSTRUCTIONS
+                                               : ATRIP_KERNEL_SPLIT;
     atrip_result &r = results[s];
     r.energy = sign * b->h_sums[2 * k];
     r.ct_energy = sign * b->h_sums[2 * k + 1];

@@ -708,6 +708,10 @@ int atrip_gpu_run(atrip_gpu_context *c, const atrip_run_options *opts, atrip_res
   ATRIP_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   c->e_lo = t_begin;
   c->e_hi = t_end;
+  c->last_kernel = n == 0                    ? ATRIP_KERNEL_NONE
+                   : tc || split_on_tc       ? ATRIP_KERNEL_TENSOR_CORE
+                   : form == ATRIP_FORM_FP64 ? ATRIP_KERNEL_FP64_INSTRUCTIONS
+                                             : ATRIP_KERNEL_SPLIT;
   for (int k = 0; k < 4; ++k) c->last_sums[k] = sums[2 + k];
   // local energy starts at -checkpoint energy (src/atrip/Atrip.cxx:612-616);
   // final sign flip unless ijkabc (src/atrip/Atrip.cxx:1108-1111)
@@ -786,6 +790,13 @@ int atrip_gpu_split_profile(const atrip_gpu_context *c, uint64_t *counters, int3
   cudaSetDevice(c->device);
   static_assert(sizeof(uint64_t) == sizeof(unsigned long long), "counter width");
   return split_profile_read(c->split, reinterpret_cast<unsigned long long *>(counters), n);
+}
+
+int atrip_gpu_last_kernel(const atrip_gpu_context *c, int32_t *kernel) {
+  clear_error();
+  if (!c || !kernel) return fail(ATRIP_ERR_ARGUMENT, "null argument");
+  *kernel = c->last_kernel;
+  return ATRIP_OK;
 }
 
 int atrip_gpu_last_sums(const atrip_gpu_context *c, double *sums) {

@@ -24,6 +24,7 @@ struct atrip_gpu_context {
   uint32_t *d_triples = nullptr;
   double *d_e = nullptr, *d_ect = nullptr;
   int64_t e_lo = 0, e_hi = 0;  // tuple range holding energies of the last run
+  int last_kernel = ATRIP_KERNEL_NONE;
   double last_sums[4] = {};    // (sum, compensation) of e and ect over that range
   double *d_workspace = nullptr;
   size_t workspace_doubles = 0;

@@ -369,24 +369,30 @@ def _max_over_ranks(world, ms, count):
     return float(t.item()), c.item()
 
 
-def _roofline(form, slices, flops_per_launch, launch_ms, peaks, live_fp64, traffic,
-              fp64_on_tensor_cores=False):
-    if form == "fp64" and fp64_on_tensor_cores:
+def _kernel_name(form, kernels):
+    """The kernel behind runs of `form`: the one most of its systems report
+    (Context.last_kernel; a batch's smallest systems may take another)."""
+    if 2 * kernels.count("tensor_core") > len(kernels):
+        return "triples_tc_kernel"
+    return "triples_fp64_kernel" if form == "fp64" else "triples_split_kernel"
+
+
+def _roofline(form, slices, flops_per_launch, launch_ms, peaks, live_fp64, traffic, kernel=None):
+    if form == "fp64" and kernel == "triples_tc_kernel":
         # the FP64 form's digit products: levels 0..7 of 8 BF16 slices
-        r = _roofline("split_bf16", 8, flops_per_launch, launch_ms, peaks, None, traffic)
-        return dict(r, kernel="triples_tc_kernel")
+        return _roofline("split_bf16", 8, flops_per_launch, launch_ms, peaks, None, traffic, kernel)
     if form == "fp64":
         achieved = flops_per_launch / (launch_ms * 1e-3) / 1e12
         peak = live_fp64
         src = "measured FP64 DFMA/DMMA peak (live, atrip_gpu_measure_peaks)"
-        kernel = "triples_fp64_kernel"
+        kernel = kernel or "triples_fp64_kernel"
     else:
         products = slices * (slices + 1) // 2
         achieved = flops_per_launch * products / (launch_ms * 1e-3) / 1e12
         peak = peaks.get("bf16_tflops", 1900.0)  # FP16 MMAs run at the BF16 rate
         src = ("of measured BF16 dense peak (bf16_tflops, burst)" if "bf16_tflops" in peaks
                else "of fallback BF16 peak")
-        kernel = "triples_split_kernel"
+        kernel = kernel or "triples_split_kernel"
     return {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "traffic": traffic, "peak_source": src, "kernel": kernel,
             "algorithmic": ("FP64-equivalent FLOPs per launch" if form == "fp64" else
@@ -447,6 +453,7 @@ def run_single(args, workload, world, rank, local):
     ms, res, clk = _timed(args.steps, stream, step)
     tuples = sum(r.tuples_done for r in res)
     launches = sum(r.kernel_launches for r in res)
+    kname = _kernel_name(form, [ctx.last_kernel()])
     ms, tuples_all = _max_over_ranks(world, ms, tuples)
     value = tuples_all * fpt / (ms * 1e-3) / 1e12
     time_to_et = n * fpt / (value * 1e12)  # whole list at the whole job's rate
@@ -526,11 +533,9 @@ def run_single(args, workload, world, rank, local):
     peaks = load_peaks()
     # per launch: the steps' mean tuples and mean device time of the loop
     launch_tuples = tuples / len(res)
-    kname = "triples_fp64_kernel" if form == "fp64" else "triples_split_kernel"
     tpt = traffic_per_tuple(kname, workload, form, slices)
     roof = _roofline(form, slices, launch_tuples * fpt, kernel_ms, peaks, live_fp64,
-                     tpt * launch_tuples if tpt is not None else None,
-                     not any(tune["tuning"].values()))
+                     tpt * launch_tuples if tpt is not None else None, kname)
     roof["tuples_per_launch"] = launch_tuples
     cpu = None if args.no_cpu_baseline else cpu_baseline(d, args.cpu_seconds)
     line = {
@@ -617,6 +622,7 @@ def run_batch96(args, world, rank, local):
         torch.distributed.barrier()
     ms, res, clk = _timed(args.steps, stream, step)
     launches = sum(r[0].kernel_launches for r in res)
+    kernels = [c.last_kernel() for c in ctxs]
     ms, _ = _max_over_ranks(world, ms, 0)
     value = total_flops * args.steps * max(world, 1) / (ms * 1e-3) / 1e12
 
@@ -663,8 +669,9 @@ def run_batch96(args, world, rank, local):
     kernel_ms = statistics.median(r[0].device_ms for r in res)
     roof = _roofline(form, slices, total_flops, kernel_ms, peaks,
                      capi.measure_peaks(local)[0] if form == "fp64" else None, None,
-                     not any(btune["tuning"].values()) and not any(tiles))
+                     _kernel_name(form, kernels))
     roof["note"] = "whole batch graph (all systems' launches and the energy reduction)"
+    roof["systems_per_kernel"] = {k: kernels.count(k) for k in sorted(set(kernels))}
     cpu = None if args.no_cpu_baseline else cpu_baseline_batch(ds, args.cpu_seconds)
     line = {
         "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": world,

@@ -241,6 +241,17 @@ int atrip_gpu_last_sums(const atrip_gpu_context *ctx, double *sums);
 #define ATRIP_SPLIT_PROFILE_COUNTERS 20
 int atrip_gpu_split_profile(const atrip_gpu_context *ctx, uint64_t *counters, int32_t n);
 
+/* The kernel of the last run, alone or in a batch: the FP64 form takes the FP64
+ * instructions where sizes, data, free memory or a tuning rule out the tensor
+ * cores, the split forms one of two kernels.  Written to *kernel.            */
+enum atrip_kernel {
+  ATRIP_KERNEL_NONE = 0,             /* no run yet, or one of no tuples        */
+  ATRIP_KERNEL_FP64_INSTRUCTIONS = 1,
+  ATRIP_KERNEL_TENSOR_CORE = 2,      /* digit products, integer level sums     */
+  ATRIP_KERNEL_SPLIT = 3             /* split kernels (M tiles or transposed)  */
+};
+int atrip_gpu_last_kernel(const atrip_gpu_context *ctx, int32_t *kernel);
+
 /* Per-tuple energies of the last run, tuple-list positions t0 .. t0+n-1
  * (the sign atrip accumulates before its final negation). ect may be NULL. */
 int atrip_gpu_tuple_energies(atrip_gpu_context *ctx, int64_t t0, int64_t n, double *e,
