@@ -42,12 +42,15 @@ int split_prepare(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
 bool split_tc_eligible(int slices, bool f16, int No, int Nv);
 // Whether the transposed kernel is the better one for a single system all the
 // same: two slices, whose 2 No stack rows and 240-256 columns fill its MMAs
-// better than No columns an MMA do.  Device time of FP16 slices, transposed
-// against the other, both in blocks of 4^3 tuples: No=20/Nv=120 12.9 / 15.2 ms,
-// No=41/Nv=300 38.0 / 40.3, No=48/Nv=300 35.8 / 41.6, No=47/Nv=160 60.7 / 59.5,
-// No=52/Nv=300 35.6 / 36.9, No=60/Nv=160 8.3 / 10.2; but No=8/Nv=100 6.3 / 4.6
-// (few rows to stack), No=53/Nv=201 157 / 151, No=56/Nv=440 228 / 191 (singles
-// blocks that no longer fit beside three stages).
+// better than No columns an MMA do, but for few rows to stack (No < 12) and for
+// No = 53..56, whose items of 56 columns waste least, as long as the 24 slabs of
+// T that a block of 4^3 tuples reads stay in L2 (129 MB).  Device time of FP16
+// slices in blocks of 4^3 tuples, transposed / the other, runs of 5e12 .. 2e13
+// FLOP: No=8/Nv=100 6.3 / 4.6 ms, No=20/Nv=120 12.9 / 15.2, No=41/Nv=300 38.0 /
+// 40.3, No=52/Nv=200 141 / 152; No=53, 54, 55, 56 at Nv=200 155 / 149, 149 / 149,
+// 180 / 148, 150 / 147, at Nv=360 110 / 100, 101 / 97, 125 / 99, 107 / 95, but at
+// Nv=440 88 / 88, 83 / 121, 113 / 122, 101 / 120 and No=56/Nv=560 93 / 116;
+// No=57, 60, 64 at Nv=200 179 / 231, 150 / 205, 136 / 175.
 bool split_prefers_transposed(int slices, bool f16, int No, int Nv);
 // Whether the prepared operands hold finite values only.  The kernel of
 // fp64_tc.cuh joins a cell's level sums as integers, which an infinity or a NaN

@@ -2055,7 +2055,8 @@ bool split_tc_eligible(int slices, bool f16, int No, int Nv) {
 }
 
 bool split_prefers_transposed(int slices, bool f16, int No, int Nv) {
-  return slices == 2 && ((No >= 12 && No <= 52) || No > 56) &&
+  const double slab = 2.0 * slices * No * No * ((Nv + kKChunk - 1) / kKChunk * kKChunk);
+  return slices == 2 && No >= 12 && (No <= 52 || No > 56 || 24 * slab > 120e6) &&
          transposed_eligible(slices, No, Nv, f16);
 }
 
