@@ -1663,7 +1663,13 @@ int tc_launch_prepare(const TcSystem *sys, int n, double tai_sign, int sm_count,
   const int room = kSmemLimit - 1024 - kTailBytes;
   const int per_chunk = S / spp;  // of the system with the fewest A slots a chunk
   auto b_for = [&](int nslots) { return (nslots - 1 + per_chunk - 1) / per_chunk + 1; };
-  b.nslots = max_slots > 0 ? std::min(std::max(max_slots, 2), kMaxSlots) : kMaxSlots;
+  // three slices and many orbitals: two slots, whose copies still cover the
+  // MMAs of the other, leave 90 KB to L1 for the energy warps' gathers instead
+  // of 24 (3 BF16 slices, 3 slots / 2: No=37 and Nv=60 56.1 / 47.5 ms, Nv=260 60.6
+  // / 54.2, No=46/Nv=120 89 / 65, No=56/Nv=260 61 / 43; but No=36 43.8 / 43.9 and
+  // 44.9 / 57.5, No=32 29.7 / 29.7 and 43.8 / 56.6)
+  const int most = b.split && S == 3 && b.lay_no > 36 ? 2 : kMaxSlots;
+  b.nslots = max_slots > 0 ? std::min(std::max(max_slots, 2), kMaxSlots) : most;
   while (b.nslots > 1 && b.nslots * b.aslot + b_for(b.nslots) * b.bslot > room) --b.nslots;
   b.nbslots = b_for(b.nslots);
   if (b.nslots * b.aslot + b.nbslots * b.bslot > room || b.nslots < 2) {
