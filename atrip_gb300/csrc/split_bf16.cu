@@ -2051,6 +2051,10 @@ int split_enqueue(SplitState &s, const DeviceTensors &dt, int No, int Nv, int sm
 bool split_tc_eligible(int slices, bool f16, int No, int Nv) {
   if (No < 2) return false;  // one triple a tuple, whose energy is 0 but for rounding
   if (f16) return slices == 2 && No <= 64 && 2 * (Nv + No) < 2048;
+  // four slices of 64 columns: two ring slots leave next to no L1 (see
+  // tc_launch_prepare).  M-tile kernel / this one: No=57/Nv=60 99 / 148 ms, No=60/
+  // Nv=260 67 / 71, No=64/Nv=120 69 / 82; No=56/Nv=60 95 / 91, Nv=260 80 / 53
+  if (slices == 4 && No > 56) return false;
   return slices >= 2 && slices <= 4 && 2 * (Nv + No) <= 1024;
 }
 

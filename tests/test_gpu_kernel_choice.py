@@ -31,3 +31,10 @@ def test_two_fp16_slices(No, Nv, kernel):
     with _ctx(No, Nv) as ctx:
         ctx.run(form="split_f16", use_j=False, max_iterations=9)
         assert ctx.last_kernel() == kernel
+
+
+@pytest.mark.parametrize("No,kernel", [(56, "tensor_core"), (57, "split"), (64, "split")])
+def test_four_bf16_slices(No, kernel):
+    with _ctx(No, 12) as ctx:
+        ctx.run(form="split_bf16", slices=4, use_j=False, max_iterations=9)
+        assert ctx.last_kernel() == kernel
