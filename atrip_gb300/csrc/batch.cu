@@ -126,6 +126,30 @@ void fill_table(atrip_gpu_batch *b, int64_t first, int64_t max_it, double tai_si
   }
 }
 
+// Whether the transposed kernel's one launch over all systems is the better one
+// for a batch's split form, by the systems alone.  Two slices, No >= 12 (as for
+// single systems) and Nv < 200, where tuples in list order find their slabs in
+// L2; systems below No = 12, whose tuples are latency there, may do no more than
+// 1/200 of the work.  Three slices of one No in 16..28 and Nv <= 100.  Device
+// time, transposed / the other: 2 FP16 slices, three systems of No=16/Nv=150 94 /
+// 106 ms, No=20/Nv=80 59 / 67, No=28/Nv=150 79 / 84, five of No=12..20 88 / 92,
+// but three of No=10/Nv=150 127 / 99, No=20/Nv=260 79 / 63, and No=6/Nv=60 with
+// 28/120 174 / 189 (0.06 % of the work), No=4/Nv=117 with 20/90 44.5 / 42.1 (2 %);
+// 3 BF16 slices, three of No=20/Nv=80 61 / 69, 28/80 129 / 140, but 20/150 128 /
+// 104, and No=20, 24, 28, 30 together 57 / 54.
+bool batch_prefers_transposed(const atrip_gpu_batch *b, int slices) {
+  if (slices > 3) return false;
+  double all = 0.0, few = 0.0;
+  for (const atrip_gpu_context *c : b->sys) {
+    if (c->Nv >= (slices == 2 ? 200 : 101)) return false;
+    if (slices == 3 && (c->No != b->sys[0]->No || c->No < 16 || c->No > 28)) return false;
+    const double work = (double)c->n_tuples * c->No * c->No * c->No * (c->No + c->Nv);
+    all += work;
+    if (c->No < 12) few += work;
+  }
+  return few <= all / 200;
+}
+
 // The FP64 slices of the batch's systems and its own buffers for them make
 // room (the caller holds the systems' TcGuards); false if there were none.
 bool give_back_slices(atrip_gpu_batch *b) {
@@ -352,6 +376,28 @@ int run_batch(atrip_gpu_batch *b, const atrip_run_options *opts, atrip_result *r
       for (int k = 0; k < n; ++k)
         b->tcs_used = b->tcs_used && split_finite(b->sys[b->order[k]]->split, b->h_table[k].use_j != 0);
     }
+    bool better = false;
+    if (b->tcs_used && batch_prefers_transposed(b, slices)) {
+      better = true;  // of the two, if it takes all systems in one launch
+      b->tcs_used = false;
+    }
+    if (!b->tcs_used && b->tune.split_variant != 1) {
+      int rc = prepare_all(true);
+      if (rc != ATRIP_OK) return rc;
+      std::vector<SplitMultiSystem> ms(n);
+      for (int k = 0; k < n; ++k) {
+        atrip_gpu_context *c = b->sys[b->order[k]];
+        const TriplesArgs &a = b->h_table[k];
+        ms[k] = {&c->split, &c->dt, c->No, c->Nv, a.tuples, a.triples, a.n_triples,
+                 a.t_begin, a.t_end, a.use_j != 0, a.e, a.ect};
+      }
+      rc = split_multi_prepare(ms.data(), n, slices, form == ATRIP_FORM_SPLIT_F16, b->sm_count,
+                               b->multi);
+      if (rc == ATRIP_OK) b->multi_used = true;
+      else if (rc != ATRIP_ERR_UNSUPPORTED) return rc;
+      clear_error();
+    }
+    if (better && !b->multi_used) b->tcs_used = true;
     if (b->tcs_used) {
       int rc;
       std::vector<TcSystem> ts(n);
@@ -371,21 +417,6 @@ int run_batch(atrip_gpu_batch *b, const atrip_run_options *opts, atrip_result *r
                                 (uintptr_t)b->tcs.aslot, (uintptr_t)b->tcs.nslots,
                                 (uintptr_t)b->tcs.nbslots};
       key.insert(key.end(), std::begin(more), std::end(more));
-    } else if (b->tune.split_variant != 1) {
-      int rc = prepare_all(true);
-      if (rc != ATRIP_OK) return rc;
-      std::vector<SplitMultiSystem> ms(n);
-      for (int k = 0; k < n; ++k) {
-        atrip_gpu_context *c = b->sys[b->order[k]];
-        const TriplesArgs &a = b->h_table[k];
-        ms[k] = {&c->split, &c->dt, c->No, c->Nv, a.tuples, a.triples, a.n_triples,
-                 a.t_begin, a.t_end, a.use_j != 0, a.e, a.ect};
-      }
-      rc = split_multi_prepare(ms.data(), n, slices, form == ATRIP_FORM_SPLIT_F16, b->sm_count,
-                               b->multi);
-      if (rc == ATRIP_OK) b->multi_used = true;
-      else if (rc != ATRIP_ERR_UNSUPPORTED) return rc;
-      clear_error();
     }
     if (!b->multi_used && !b->tcs_used) {
       const int rc = prepare_all(false);  // one launch per system (batch split_variant 1)

@@ -38,3 +38,20 @@ def test_four_bf16_slices(No, kernel):
     with _ctx(No, 12) as ctx:
         ctx.run(form="split_bf16", slices=4, use_j=False, max_iterations=9)
         assert ctx.last_kernel() == kernel
+
+
+@pytest.mark.parametrize("form,S,sizes,kernel", [
+    ("split_f16", 2, [(12, 12), (20, 9)], "split"), ("split_f16", 2, [(11, 12), (11, 13)], "tensor_core"),
+    ("split_f16", 2, [(11, 12), (20, 12)], "tensor_core"), ("split_f16", 2, [(3, 5), (28, 20)], "split"),
+    ("split_f16", 2, [(12, 199)], "split"), ("split_f16", 2, [(12, 200)], "tensor_core"),
+    ("split_bf16", 3, [(16, 12), (16, 14)], "split"), ("split_bf16", 3, [(16, 12), (17, 14)], "tensor_core"),
+    ("split_bf16", 3, [(29, 8)], "tensor_core"), ("split_bf16", 4, [(16, 12)], "tensor_core")])
+def test_batches(form, S, sizes, kernel):
+    ctxs = [_ctx(*s) for s in sizes]
+    with capi.Batch(ctxs) as b:
+        got = b.run(form=form, slices=S, use_j=False, max_iterations=99)
+        assert {c.last_kernel() for c in ctxs} == {kernel}
+    for c, r in zip(ctxs, got):
+        one = c.run(form="fp64", use_j=False, max_iterations=99)
+        assert abs(r.energy - one.energy) <= 1e-3 * abs(one.energy)  # the split forms': 1e-5 or less
+        c.close()
