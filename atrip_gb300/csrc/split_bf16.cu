@@ -457,6 +457,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t *mempty = mfull + kMSlots;
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(mempty + kMSlots);
   TupleSlot *tslot = reinterpret_cast<TupleSlot *>(tail + 264);
+  uint64_t *drain = reinterpret_cast<uint64_t *>(tail + 376);
+  static_assert(264 + kTupleSlots * sizeof(TupleSlot) <= 376, "tail");
   double *ta = reinterpret_cast<double *>(tail + 384);
   double *tb = ta + 64;
   double *tc = tb + 64;
@@ -483,6 +485,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&tfull[s], 1);
       mbar_init(&tempty[s], 3);
     }
+    mbar_init(drain, 1);
     fence_mbar_init();
   }
   if (threadIdx.x == 0 && !MULTI) {
@@ -676,6 +679,17 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
           }
       }
+      if (leader) {  // after a wait that gave up, here or elsewhere: copies in flight land first
+        for (int i = 0; i < kStages; ++i) {
+          const uint32_t n = puse + (i < pst ? 1 : 0);
+          if (n > 0) mbar_drain(&full[i], (n - 1) & 1);
+        }
+        if constexpr (MSHARE)
+          for (uint32_t i = 0; i < kMSlots; ++i) {
+            const uint32_t n = (mcount + kMSlots - 1 - i) / kMSlots;
+            if (n > 0) mbar_drain(&mfull[i], (n - 1) & 1);
+          }
+      }
       if (PROF && leader) {
         prof_add(g.prof, kProfProdTotal, clock64() - c_start);
         prof_add(g.prof, kProfProdEmpty, c_empty);
@@ -833,6 +847,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           ++item_count;
         }
         if (!alive) break;
+      }
+      // no MMA outlives this role (after a failed wait some may be in flight)
+      if (leader) {
+        mma_commit(drain);
+        mbar_drain(drain, 0);
       }
       if (PROF && leader) {
         prof_add(g.prof, kProfMmaTotal, clock64() - c_start);
@@ -1199,7 +1218,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 
   // Leave only after every tcgen05 op of this CTA has completed: the
-  // epilogue has drained every accumulator it was handed.
+  // epilogue has drained every accumulator it was handed, the issuer its MMAs.
   __syncthreads();
   tc_fence_after();
   if (warp == 1) tmem_dealloc(tmem, K::kAllocCols);

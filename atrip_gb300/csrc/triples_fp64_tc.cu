@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
             }
           }
     }
-    if (!alive && leader) {  // wait for the copies still in flight
+    if (leader) {  // after a wait that gave up, here or elsewhere: copies in flight land first
       for (int i = 0; i < g.nslots; ++i) {
         const uint32_t n = use + (i < st ? 1 : 0);
         if (n > 0) mbar_drain(&afull[i], (n - 1) & 1);
