@@ -58,8 +58,8 @@
 // FP64-equivalent); No=37/Nv=151 with (cT), 900 tuples, 229.6 -> 7.7 ms;
 // No=8/Nv=40, the whole list, 6.2 -> 0.92 ms; complex No=13/Nv=50, 9000
 // tuples, 90.8 -> 3.7 ms.  Error of the tuple energies against quad precision,
-// 2-norm: 1.0e-16 and 2.2e-16 for (cT), DFMA kernel 1.0e-16 and 4.5e-16 (No =
-// 8..33).
+// 2-norm, No = 8..37: 0.9 to 1.1e-16 and 1.8 to 2.7e-16 for (cT), DFMA kernel
+// 0.8 to 1.1e-16 and 4.2 to 6.2e-16.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>

@@ -66,9 +66,10 @@ enum atrip_tensor {
 /* Arithmetic form of the contractions. */
 enum atrip_form {
   ATRIP_FORM_FP64 = 0,       /* FP64 results: exact digit-slice products on   */
-                             /* the tensor cores where sizes and data allow   */
-                             /* (error no larger than FP64 dot products'),    */
-                             /* else FP64 instructions throughout             */
+                             /* the tensor cores where sizes, free memory and */
+                             /* data allow (error within the bound of FP64    */
+                             /* dot products'), else FP64 instructions        */
+                             /* throughout; see atrip_gpu_last_kernel         */
   ATRIP_FORM_SPLIT_BF16 = 1, /* operands cut into BF16 slices, tensor cores,  */
                              /* FP32 accumulation, FP64 recombination         */
   ATRIP_FORM_AUTO = 2,       /* split-BF16 for real inputs (3 slices unless  */
