@@ -23,7 +23,8 @@
 // K 2^-53 of that product, the bound of an FP64 dot product's error; the sums
 // of levels 0..6 are exact by the rows' digit norms and where they end
 // (digit_sums.cuh), in one accumulator or, for longer K, the natural and the
-// transposed half in one each; level 7's weigh 2^-70 of the grids' largest
+// transposed half in one each (level 6 may be rounded a little where the least
+// product is within 2^kLooseBits); level 7's weigh 2^-70 of the grids' largest
 // product, and what roundings could do to them (8 K of at most 16) stays below
 // K 2^-62 of it.  Whatever fails this is run by the DFMA kernel instead.
 //
@@ -95,6 +96,7 @@ constexpr int kEnergyThreads = kEnergyWarps * 32;
 constexpr int kT1 = 64;  // doubles per t1 row: No <= 64, or No <= 32 complex
 constexpr int kTailBytes = 576 + 3 * kT1 * 8 + 16 * 8;
 constexpr int kRangeBits = 6;               // least product against 2^(eT+eV)
+constexpr int kLooseBits = 4;               // the same, for loose level sums
 constexpr int kBlocksZ = 3;                 // column blocks stored for a complex operand
 
 enum : int { kErrFull = 1, kErrEmpty = 2, kErrAccFull = 3, kErrAccEmpty = 4 };
@@ -864,7 +866,10 @@ __global__ void __launch_bounds__(kThreads, 1) triples_tc_kernel(const TcArgs g)
         // come in whole 32-byte sectors (group 2's run along j); No=37/Nv=151
         // with (cT) 8.4 -> 8.0 ms, No=24/Nv=240 in 3 BF16 slices 9.0 -> 8.4 ms.
         // Few orbitals, whose cells stay in L2 and fill such tiles badly, are
-        // taken in order (No=4..20: tiles 2 % slower)
+        // taken in order (No=4..20: tiles 2 % slower; together with the order of
+        // the triples, No=21..24 and Nv=60..200: No=24 in order 6 to 18 % slower,
+        // No=22 FP64 5 to 7 % slower and 3 slices 1 to 2 % faster, No=21, 23 FP64
+        // 1 to 2 % faster and 3 slices 3 to 8 % slower)
         constexpr int kU = 4;
         const bool tiled = No > 20;
         const int ti = tiled ? (No + 7) >> 3 : 1, tj = (No + 3) >> 2;
@@ -1234,15 +1239,18 @@ bool alloc_arena(char **p, size_t bytes) {
 
 bool exponent_ok(int e) { return e >= -200 && e <= 200; }
 
-// The grids' exponents, if an examination's result allows the form.
-bool grids_of(const DeviceStats &h, int *e_t, int *e_v) {
+// The grids' exponents, if an examination's result allows the form; *loose:
+// loose level sums too.
+bool grids_of(const DeviceStats &h, int *e_t, int *e_v, bool *loose) {
   const unsigned long long mT = h.t_max, mV = std::max(h.vp_max, h.vh_max);
   constexpr unsigned long long kInf = 0x7ff0000000000000ull;
   if (mT == 0 || mV == 0 || mT >= kInf || mV >= kInf) return false;
   *e_t = exponent_of(as_double(mT));
   *e_v = exponent_of(as_double(mV));
   if (!exponent_ok(*e_t) || !exponent_ok(*e_v)) return false;
-  return std::ldexp((double)h.least, -kLogOne) - 2 * kLogBias >= *e_t + *e_v - kRangeBits;
+  const double least = std::ldexp((double)h.least, -kLogOne) - 2 * kLogBias - (*e_t + *e_v);
+  *loose = least >= -kLooseBits;
+  return least >= -kRangeBits;
 }
 
 DigitNorms norms_of(const unsigned int *x) {
@@ -1255,8 +1263,10 @@ DigitNorms norms_of(const unsigned int *x) {
 // transposed half, or one each; 0: not exact either.  A complex system's rows
 // meet real and imaginary columns.
 int sum_pieces(int nc, const DigitNorms &nT, const DigitNorms &nV, const DigitNorms &nH,
-               const DigitNorms &nU) {
-  return level_sums_exact(2 * nc, nT, nV, nH, nU) ? 1 : level_sums_exact(nc, nT, nV, nH, nU) ? 2 : 0;
+               const DigitNorms &nU, bool loose) {
+  return level_sums_exact(2 * nc, nT, nV, nH, nU, loose) ? 1
+         : level_sums_exact(nc, nT, nV, nH, nU, loose)   ? 2
+                                                         : 0;
 }
 
 // A column operand: its one block, or the three of a complex system, of
@@ -1359,7 +1369,8 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cpl
   auto *ds = static_cast<DeviceStats *>(tmp.p);
   DeviceStats h;
   int rc = examine(p->nc, dt.Ta, dt.Vht, dt.Vpt, No_, Nv_, p->arena, ds, &h, st, launches);
-  if (rc != ATRIP_OK || !grids_of(h, &p->eT, &p->eV)) return rc;
+  bool loose = false;
+  if (rc != ATRIP_OK || !grids_of(h, &p->eT, &p->eV, &loose)) return rc;
   p->unit = std::ldexp(1.0, p->eT + p->eV - 14 - 24);
 
   char *q = p->arena;
@@ -1398,7 +1409,7 @@ int prepare_main(TcState &s, const DeviceTensors &dt, int No_, int Nv_, bool cpl
   p->nU = norms_of(h.n[1]);
   const DigitNorms nU2 = norms_of(h.n[2]);
   for (int s = 0; s < kNormSlices; ++s) p->nU.q2[s] = std::max(p->nU.q2[s], nU2.q2[s]);
-  p->pieces = sum_pieces(p->nc, p->nT, norms_of(h.n[5]), norms_of(h.n[4]), p->nU);
+  p->pieces = sum_pieces(p->nc, p->nT, norms_of(h.n[5]), norms_of(h.n[4]), p->nU, loose);
   if (p->pieces == 0) return ATRIP_OK;
 
   for (int i = 0; i < 4; ++i) {  // [component][row order]; a real system's twice
@@ -1429,7 +1440,8 @@ int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *lau
   DeviceStats h;
   int e_t;
   int rc = examine((int)nc, dt.Ta, dt.Jht, dt.Jpt, p->No, p->Nv, p->arena_j, ds, &h, st, launches);
-  if (rc != ATRIP_OK || !grids_of(h, &e_t, &p->eJ)) return rc;
+  bool loose = false;
+  if (rc != ATRIP_OK || !grids_of(h, &e_t, &p->eJ, &loose)) return rc;
   p->unit_j = std::ldexp(1.0, p->eT + p->eJ - 14 - 24);
   __nv_bfloat16 *vh[4];
   for (int i = 0; i < 2 * nc; ++i) vh[i] = reinterpret_cast<__nv_bfloat16 *>(p->arena_j + i * nVh);
@@ -1438,7 +1450,7 @@ int prepare_j(TcState &s, const DeviceTensors &dt, cudaStream_t st, int64_t *lau
   if (rc != ATRIP_OK) return rc;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(&h, ds, sizeof(h), cudaMemcpyDeviceToHost, st));
   ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
-  const int pieces = sum_pieces(p->nc, p->nT, norms_of(h.n[5]), norms_of(h.n[4]), p->nU);
+  const int pieces = sum_pieces(p->nc, p->nT, norms_of(h.n[5]), norms_of(h.n[4]), p->nU, loose);
   if (pieces == 0) return ATRIP_OK;
   p->pieces_j = std::max(p->pieces, pieces);
   for (int i = 0; i < 4; ++i)

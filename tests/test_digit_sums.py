@@ -16,18 +16,19 @@ def rule(tmp_path_factory):
     d = tmp_path_factory.mktemp("digit_sums")
     src = d / "rule.cpp"
     src.write_text('#include "digit_sums.cuh"\n'
-                   'extern "C" int rule(int terms, const double *n) {\n'
+                   'extern "C" int rule(int terms, const double *n, int loose) {\n'
                    '  const auto *x = reinterpret_cast<const atrip_gb300::DigitNorms *>(n);\n'
-                   '  return atrip_gb300::level_sums_exact(terms, x[0], x[1], x[2], x[3]);\n}\n')
+                   '  return atrip_gb300::level_sums_exact(terms, x[0], x[1], x[2], x[3], loose != 0);\n'
+                   '}\n')
     lib = d / "rule.so"
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I",
                            os.path.join(ROOT, "atrip_gb300", "csrc"), str(src), "-o", str(lib)])
     fn = ctypes.CDLL(str(lib)).rule
 
-    def call(terms, norms):
+    def call(terms, norms, loose=False):
         a = np.ascontiguousarray(norms, dtype=np.float64)
         assert a.shape == (4, NORMS)
-        return bool(fn(terms, a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))))
+        return bool(fn(terms, a.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), int(loose)))
     return call
 
 
@@ -61,12 +62,30 @@ def test_accepted_sums_are_exact(rule, top, nv):
     if rule(1, [n[0], n[1], zero, zero]):
         # a half alone: exact where its end lies within what is checked
         assert all(x == y for x, y in half if abs(y) < 2 ** 22)
+    if rule(2, [n[0], n[1], zero, zero], loose=True):
+        assert all(x == y for x, y in both[:6])
+        assert abs(both[6][0] - both[6][1]) <= 2 * 7 * 2 * nv  # 2 for each product
     exact = all(x == y for x, y in both)
     assert exact or not rule(2, [n[0], n[1], zero, zero])
 
 
-# normal operands: one accumulator up to Nv + No ~ 360, two (one per half) up
-# to the longest K the form serves
+# operands that only the loose rule accepts: level 6 passes 2^24 and is rounded
+def test_loose_level_six(rule):
+    nv = 560
+    rng = np.random.default_rng(1)
+    q = np.array([64, 1, 1] + [127] * 5, dtype=np.int64)[:, None] * np.ones((1, nv), np.int64)
+    r = q.copy()
+    r[1:] -= rng.integers(0, 2, (SLICES - 1, nv))
+    n = [[float((x[s] ** 2).sum()) for s in range(NORMS)] for x in (q, r)] + [[0.0] * NORMS] * 2
+    assert not rule(2, n) and rule(2, n, loose=True)
+    rows, cols = np.concatenate([q, q], 1), np.concatenate([r, -r], 1)
+    for L in range(NORMS):
+        x, y = _level_sums(rows, cols, L)
+        assert x == y if L < 6 else abs(x - y) <= 2 * 7 * 2 * nv
+
+
+# normal operands: one accumulator up to Nv + No ~ 360 (loose 450), two (one per
+# half) up to the longest K the form serves
 @pytest.mark.parametrize("no,nv,terms", [(8, 40, 2), (24, 240, 2), (42, 240, 2), (37, 151, 2),
                                          (56, 440, 1), (30, 660, 1)])
 def test_normal_operands_are_accepted(rule, no, nv, terms):
@@ -82,6 +101,22 @@ def test_normal_operands_are_accepted(rule, no, nv, terms):
             y = (y - d) >> 8
         return out[::-1] + [out[0]]  # digit 6 like digit 5
     n = [norms(nv, 4000), norms(nv, 4000), norms(no, 4000), norms(no, 4000)]
-    assert rule(terms, n)
+    assert rule(terms, n) and rule(terms, n, loose=True)
     if terms == 1:
         assert not rule(2, n)
+
+
+def test_normal_operands_loose(rule):
+    rng = np.random.default_rng(7)
+
+    def norms(k):
+        x = rng.normal(size=(4000, k))
+        y = np.rint(x * (126 / np.abs(x).max() * 0.6) * 2.0 ** 40).astype(np.int64)
+        out = []
+        for s in range(6):
+            d = (y + 128) % 256 - 128
+            out.append(float((d * d).sum(1).max()))
+            y = (y - d) >> 8
+        return out[::-1] + [out[0]]
+    n = [norms(400), norms(400), norms(40), norms(40)]
+    assert rule(2, n, loose=True) and not rule(2, n)
