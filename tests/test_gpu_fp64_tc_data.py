@@ -131,3 +131,23 @@ def test_sums_in_two_accumulators(No, Nv, j, field):
     K = 2 * (Nv + No) * (2 if field == "complex" else 1)
     assert np.max(np.abs(e - f)) <= K * 2.0 ** -52 * np.max(np.abs(f))
     assert np.max(np.abs(ect - fct)) <= K * 2.0 ** -52 * np.max(np.abs(fct))
+
+
+# T = 1, V = 1 but for one T_x, or one V_yz, of 2^-bits: the grids' largest
+# product is 4, so 4 bits are within 2^6 of it and 5 are not, wherever they are
+@pytest.mark.parametrize("bits,kernel", [(4, "tensor_core"), (5, "fp64_instructions")])
+@pytest.mark.parametrize("No,Nv", [(8, 40), (8, 41), (9, 39)])
+@pytest.mark.parametrize("at", [(0, 1), (-1, -2), (-1, -1), (17, 3), (0,), (33,), (-1,)])
+def test_least_product_is_found(bits, kernel, No, Nv, at):
+    d = synth.make_inputs(No, Nv, 25)
+    d["Tabij"][:] = 1.0
+    d["Vabci"][:] = 1.0
+    d["Vijka"][:] = 0.5
+    if len(at) == 2:
+        d["Vabci"][at] = 2.0 ** -bits
+        d["Vabci"][at][Nv // 2, No - 1] = 2.0 ** -bits
+    else:
+        d["Tabij"][at[0]] = 2.0 ** -bits
+    with _ctx(d) as ctx:
+        ctx.run(form="fp64", use_j=False, max_iterations=9)
+        assert ctx.last_kernel() == kernel

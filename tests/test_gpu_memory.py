@@ -130,3 +130,36 @@ def test_failed_ct_slices_leave_nothing_behind():
         assert free[-1] == free[0]
         ref = ctx.run(use_j=True, **kw)
         assert np.isfinite(ref.ct_energy)
+
+
+# a thread that runs FP64 ranges while another creates, uploads and closes a
+# context for which there is room only without the first one's slices
+def test_slices_are_taken_between_a_threads_runs():
+    import threading
+    d, d2 = synth.make_inputs(12, 110, 37), synth.make_inputs(16, 120, 38)
+    bad, done = [], threading.Event()
+
+    def runs(ctx, ref):
+        try:
+            for _ in range(300):
+                _close(_run64(ctx, 100), ref, 2 * 122)
+        except Exception as e:  # noqa: BLE001 - reported below
+            bad.append(repr(e))
+        done.set()
+
+    with _ctx(d) as ctx:
+        ref = _run64(ctx, 100)
+        with full_device(400 * MB):
+            t = threading.Thread(target=runs, args=(ctx, ref))
+            t.start()
+            made = 0
+            while not done.is_set():
+                try:
+                    with _ctx(d2):
+                        made += 1
+                except capi.AtripError as e:  # the other one is in a call
+                    if e.status != capi.ERR_OUT_OF_MEMORY:
+                        bad.append(repr(e))
+            t.join()
+        assert not bad
+        _close(_run64(ctx, 100), ref, 2 * 122)
