@@ -1002,10 +1002,11 @@ __global__ void __launch_bounds__(256) t_profile_kernel(const double *__restrict
 }
 
 // The least product of T's profile with those of 32 slabs Vpt[y][z][r][E] a
-// block, and the largest element.  Reads V once and takes Nv^4 steps; the slab
-// maxima it replaces read as much (No=24/Nv=240, first run of 8000 tuples with
-// examination and cut: 15.3 -> 15.6 ms).
-template <int NC>
+// block (FULL: exact, else a lower bound), and the largest element.  Reads V
+// once; the slab maxima it replaces read as much (No=24/Nv=240, first run of 8000
+// tuples with examination and cut: 15.2 ms with either, 15.6 with the exact
+// products).
+template <int NC, bool FULL>
 __global__ void __launch_bounds__(256) v_profile_kernel(const double *__restrict__ Vpt,
                                                         const int *__restrict__ t, int No, int Nv,
                                                         unsigned long long *__restrict__ vmax,
@@ -1032,7 +1033,7 @@ __global__ void __launch_bounds__(256) v_profile_kernel(const double *__restrict
     }
   warp_max(best, vmax);
   __syncthreads();
-  least_product(t, v, Nv, p0, least);
+  least_product<FULL>(t, v, Nv, p0, least);
 }
 
 // dst[s][R][k] (pitch Kp) = digit_s(sign src(R, k)), row R = (o n1 + r1) n2
@@ -1177,40 +1178,54 @@ double as_double(unsigned long long b) {
 
 struct DeviceStats {
   unsigned long long t_max, vp_max, vh_max;  // largest magnitudes
-  unsigned int least;                        // least product (log_of sums)
+  unsigned int least[2];                     // least product (log_of sums): lower bound, exact
   unsigned int n[8][8];                      // digit norms of up to eight cut jobs
 };
 
 // Queue the examination of T against a pair V_hhhp, V_pphp (or J): maxima and
-// the least product.  scratch: profile_bytes() of device memory.
-template <int NC>
+// the least product, or (FULL) only that, exact.  scratch: profile_bytes() of
+// device memory.
+template <int NC, bool FULL>
 int examine(const double *Ta, const double *vht, const double *vpt, int No, int Nv, void *scratch,
             DeviceStats *ds, cudaStream_t st, int64_t *launches) {
   int *t = static_cast<int *>(scratch);
-  t_profile_kernel<NC><<<dim3(Nv, (Nv + 31) / 32), 256, 0, st>>>(Ta, No * No, Nv, t, &ds->t_max);
+  if (!FULL) {
+    t_profile_kernel<NC><<<dim3(Nv, (Nv + 31) / 32), 256, 0, st>>>(Ta, No * No, Nv, t, &ds->t_max);
+    ATRIP_CUDA_TRY(cudaGetLastError());
+  }
+  auto kern = v_profile_kernel<NC, FULL>;
+  ATRIP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kProfileSmem));
+  kern<<<(unsigned)(((int64_t)Nv * Nv + kProfilePairs - 1) / kProfilePairs), 256, profile_smem(Nv),
+         st>>>(vpt, t, No, Nv, &ds->vp_max, &ds->least[FULL]);
   ATRIP_CUDA_TRY(cudaGetLastError());
-  ATRIP_CUDA_TRY(cudaFuncSetAttribute(v_profile_kernel<NC>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
-  v_profile_kernel<NC><<<(unsigned)(((int64_t)Nv * Nv + kProfilePairs - 1) / kProfilePairs), 256,
-                         profile_smem(Nv), st>>>(vpt, t, No, Nv, &ds->vp_max, &ds->least);
-  ATRIP_CUDA_TRY(cudaGetLastError());
+  *launches += 1;
+  if (FULL) return ATRIP_OK;
   max_kernel<<<152 * 4, 256, 0, st>>>(vht, (int64_t)NC * Nv * No * No * No, &ds->vh_max);
   ATRIP_CUDA_TRY(cudaGetLastError());
-  *launches += 3;
+  *launches += 2;
   return ATRIP_OK;
 }
 
 // Clear *ds, examine and read the result back (synchronises st).
+bool grids_of(const DeviceStats &h, int *e_t, int *e_v, bool *loose);
 int examine(int nc, const double *Ta, const double *vht, const double *vpt, int No, int Nv,
             void *scratch, DeviceStats *ds, DeviceStats *h, cudaStream_t st, int64_t *launches) {
   std::memset(h, 0, sizeof(*h));
-  h->least = ~0u;
+  h->least[0] = h->least[1] = ~0u;
   ATRIP_CUDA_TRY(cudaMemcpyAsync(ds, h, sizeof(*h), cudaMemcpyHostToDevice, st));
-  const int rc = nc == 2 ? examine<2>(Ta, vht, vpt, No, Nv, scratch, ds, st, launches)
-                         : examine<1>(Ta, vht, vpt, No, Nv, scratch, ds, st, launches);
-  if (rc != ATRIP_OK) return rc;
-  ATRIP_CUDA_TRY(cudaMemcpyAsync(h, ds, sizeof(*h), cudaMemcpyDeviceToHost, st));
-  ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+  for (int full = 0; full < 2; ++full) {
+    const auto run = nc == 2 ? (full ? examine<2, true> : examine<2, false>)
+                             : (full ? examine<1, true> : examine<1, false>);
+    const int rc = run(Ta, vht, vpt, No, Nv, scratch, ds, st, launches);
+    if (rc != ATRIP_OK) return rc;
+    ATRIP_CUDA_TRY(cudaMemcpyAsync(h, ds, sizeof(*h), cudaMemcpyDeviceToHost, st));
+    ATRIP_CUDA_TRY(cudaStreamSynchronize(st));
+    if (!full) h->least[1] = h->least[0];
+    int e_t, e_v;
+    bool loose = false;
+    if (grids_of(*h, &e_t, &e_v, &loose) && loose) break;  // as good as it gets
+  }
   return ATRIP_OK;
 }
 
@@ -1248,7 +1263,7 @@ bool grids_of(const DeviceStats &h, int *e_t, int *e_v, bool *loose) {
   *e_t = exponent_of(as_double(mT));
   *e_v = exponent_of(as_double(mV));
   if (!exponent_ok(*e_t) || !exponent_ok(*e_v)) return false;
-  const double least = std::ldexp((double)h.least, -kLogOne) - 2 * kLogBias - (*e_t + *e_v);
+  const double least = std::ldexp((double)h.least[1], -kLogOne) - 2 * kLogBias - (*e_t + *e_v);
   *loose = least >= -kLooseBits;
   return least >= -kRangeBits;
 }

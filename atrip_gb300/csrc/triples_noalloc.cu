@@ -65,9 +65,11 @@ struct Header {
   int tc_status;                 // a bounded wait gave up
   int e_t, e_v, e_j;             // exponents of the digit grids
   // largest magnitudes of T, of the V and of the J pair; least products of T
-  // with V_pphp and J_pphp (kprofile.cuh)
+  // with V_pphp and J_pphp (kprofile.cuh): lower bounds, exact; the latter are
+  // needed
   unsigned long long t_max, v_max[2];
-  unsigned int least[2];
+  unsigned int least[2][2];
+  int full;
 };
 static_assert(sizeof(Header) <= kHeaderBytes, "header");
 
@@ -337,17 +339,19 @@ __global__ void __launch_bounds__(256) t_profile(const unsigned long long *__res
                                                  int Nv, int *__restrict__ t, Header *h) {
   const int64_t i = blockIdx.x * 256ll + threadIdx.x;
   const unsigned long long m = i < (int64_t)Nv * Nv ? cols[i] : 0;
-  if (i == 0) h->least[0] = h->least[1] = ~0u;
+  if (i < 4) h->least[i >> 1][i & 1] = ~0u;
   if (i < (int64_t)Nv * Nv) t[(i / Nv) * profile_pitch(Nv) + i % Nv] = log_of(m);
   warp_max(m, &h->t_max);
 }
 
 // The least product of T's profile with those of 32 slabs V[y,z,E,r] (y
 // fastest) a block, and the largest element.
+template <bool FULL>
 __global__ void __launch_bounds__(256) v_profile(const double *__restrict__ Vp,
                                                  const int *__restrict__ t, int No, int Nv,
                                                  Header *h, int which) {
   extern __shared__ int v[];
+  if (FULL && !h->full) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t p0 = (int64_t)blockIdx.x * kProfilePairs, np = (int64_t)Nv * Nv;
   unsigned long long best = 0;
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(256) v_profile(const double *__restrict__ Vp,
   }
   warp_max(best, &h->v_max[which]);
   __syncthreads();
-  least_product(t, v, Nv, p0, &h->least[which]);
+  least_product<FULL>(t, v, Nv, p0, &h->least[FULL][which]);
 }
 
 // The largest magnitude of x[0 .. n) into the header.
@@ -390,17 +394,20 @@ __device__ bool grid_exponent(unsigned long long bits, int *e) {
   return k >= -200 && k <= 200;
 }
 
-// The verdict; the rules of triples_fp64_tc.cu.
-__global__ void decide(int use_j, Header *h) {
+// The verdict; the rules of triples_fp64_tc.cu.  From the lower bounds, then, if
+// they did not do, from the exact products.
+__global__ void decide(int use_j, Header *h, int full) {
+  if (full && !h->full) return;
   int e_t = 0, e[2] = {0, 0};
   bool ok = grid_exponent(h->t_max, &e_t);
   for (int w = 0; w < (use_j ? 2 : 1); ++w)
     ok = ok && grid_exponent(h->v_max[w], &e[w]) &&
-         ldexp((double)h->least[w], -kLogOne) - 2 * kLogBias >= e_t + e[w] - kRangeBits;
+         ldexp((double)h->least[full][w], -kLogOne) - 2 * kLogBias >= e_t + e[w] - kRangeBits;
   h->e_t = e_t;
   h->e_v = e[0];
   h->e_j = e[1];
   h->tc_ok = ok ? 1 : 0;
+  h->full = ok || full ? 0 : 1;
 }
 
 struct Tail {
@@ -744,14 +751,13 @@ size_t smem_bytes(int no) {
 
 // By sizes: the profile of T fits the scratch, and the range's work on FP64
 // instructions (~0.8 TFLOP/s here) takes several times what examining the
-// whole tensors does (~5 TB/s, ~1.6e13 steps of a profile's product a second
-// and a few launches).
+// whole tensors does (~5 TB/s, the lower bounds' Nv^3 steps and a few launches).
 bool sizes_ok(const Args &a) {
   const double Nv = a.Nv, No = a.No, n = (double)(a.t_end - a.t_begin);
   const double nj = a.use_j ? 2.0 : 1.0;
   const double dfma = n * nj * 12.0 * No * No * No * (No + Nv) / 0.8e12;
   const double scan = 8.0 * (Nv * Nv * No * No + nj * Nv * No * (Nv * Nv + No * No)) / 5e12 +
-                      nj * Nv * Nv * Nv * Nv / 1.6e13 + 4e-5;
+                      nj * Nv * Nv * Nv / 2e11 + 4e-5;
   return No >= 4 && dfma > 4.0 * scan &&
          8 * (size_t)a.Nv * a.Nv + profile_bytes(a.Nv) + 256 <= kScratchBytes - kWorkspaceOffset;
 }
@@ -770,14 +776,17 @@ int enqueue(const Args &a, int device, cudaStream_t st) {
   column_max<<<grid, 256, 0, st>>>(a.T, nvnv, No * No, cols);
   t_profile<<<blocks, 256, 0, st>>>(cols, (int)Nv, t, h);
   ATRIP_CUDA_TRY(cudaGetLastError());
-  ATRIP_CUDA_TRY(cudaFuncSetAttribute(v_profile, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      kSmemLimit));
   const unsigned pairs = (unsigned)((nvnv + kProfilePairs - 1) / kProfilePairs);
-  for (int w = 0; w < (a.use_j ? 2 : 1); ++w) {
-    v_profile<<<pairs, 256, profile_smem((int)Nv), st>>>(w ? a.Jp : a.Vp, t, (int)No, (int)Nv, h, w);
-    max_kernel<<<152 * 4, 256, 0, st>>>(w ? a.Jh : a.Vh, Nv * No * No * No, h, w);
+  for (int full = 0; full < 2; ++full) {
+    auto profile = full ? v_profile<true> : v_profile<false>;
+    ATRIP_CUDA_TRY(cudaFuncSetAttribute(profile, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        kProfileSmem));
+    for (int w = 0; w < (a.use_j ? 2 : 1); ++w) {
+      profile<<<pairs, 256, profile_smem((int)Nv), st>>>(w ? a.Jp : a.Vp, t, (int)No, (int)Nv, h, w);
+      if (!full) max_kernel<<<152 * 4, 256, 0, st>>>(w ? a.Jh : a.Vh, Nv * No * No * No, h, w);
+    }
+    decide<<<1, 1, 0, st>>>(a.use_j, h, full);
   }
-  decide<<<1, 1, 0, st>>>(a.use_j, h);
   ATRIP_CUDA_TRY(cudaGetLastError());
   int sms = 0;
   ATRIP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
