@@ -137,3 +137,27 @@ def test_as_accurate_as_fp64_instructions(No, Nv, j, field):
         print(No, Nv, field, "tensor cores %.2e, FP64 instructions %.2e of the 2-norm" %
               tuple(e / float(np.sqrt(np.sum(ref ** 2))) for e in err))
         assert err[0] <= 4 * err[1]
+
+
+# pair slabs of T that symmetry leaves at round-off: no product of a whole T_x is
+# small, so the tensor cores take them
+@pytest.mark.gpu
+@pytest.mark.parametrize("No,Nv", [(8, 40), (15, 33)])
+def test_pair_slabs_at_round_off(No, Nv):
+    d = synth.make_inputs(No, Nv, 43)
+    u = np.arange(Nv)
+    d["Tabij"][(u[:, None] + u[None, :]) % 2 == 1] *= 1e-17
+    n, t0 = 24, synth.n_tuples(Nv) // 2
+    kw = dict(form="fp64", use_j=False, first_iteration=t0, max_iterations=t0 + n - 1)
+    with capi.Context(No, Nv, 0) as ctx:
+        for k in NAMES:
+            ctx.upload(k, d[k])
+        ctx.run(**kw)
+        assert ctx.last_kernel() == "tensor_core"
+        tc = ctx.tuple_energies(t0, n)[0]
+        ctx.set_tuning(fp64_tile_rows=64)
+        ctx.run(**kw)
+        dfma = ctx.tuple_energies(t0, n)[0]
+    ref = _energies(d, _tuples(Nv, t0, n), False)[0]
+    err = [float(np.sqrt(np.sum((v.astype(np.longdouble) - ref) ** 2))) for v in (tc, dfma)]
+    assert err[0] <= 4 * err[1]
